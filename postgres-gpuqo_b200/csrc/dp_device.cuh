@@ -66,7 +66,10 @@ __device__ __forceinline__ int f2i_x86(float f) {
     return __float2int_rz(f);
 }
 
+// 0 for num = 0, as the reference's x86-64 build computes it (a row wider than
+// work_mem asks for it): 1 << -1 is 1 << 63 there, which differs from 0
 __device__ __forceinline__ int ceil_log2_l(long long num) {
+    if (num == 0) return 0;
     int res = 63 - __clzll(num);
     if ((1LL << res) == num) return res;
     return res + 1;
@@ -75,9 +78,8 @@ __device__ __forceinline__ int ceil_log2_l(long long num) {
 // order-preserving map of a float to uint32 (NaN handled by the caller);
 // -0.0 is folded to +0.0 because the reference compares with '<'
 __device__ __forceinline__ uint32_t ord_float(float f) {
-    if (f == 0.0f) f = 0.0f;
-    uint32_t b = __float_as_uint(f);
-    return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
+    const uint32_t b = __float_as_uint(f + 0.0f);   // -0 + 0 = +0
+    return b ^ ((uint32_t)((int32_t)b >> 31) | 0x80000000u);
 }
 
 // ---------------------------------------------------------------------------
@@ -119,10 +121,19 @@ __device__ __forceinline__ float clamp_row_est(float nrows) {
 }
 
 // :820-841 (MAXALIGN with MAXIMUM_ALIGNOF 8, RELATION_OVERHEAD 24, BLCKSZ 8192)
-__device__ __forceinline__ float relation_byte_size(float tuples, int width) {
+// A width >= 0 stays below 2^32 after the alignment and the overhead, so it is
+// converted from 32 bits: the same integer, the same rounding.  The 64-bit
+// conversion runs at a sixteenth of the 32-bit one's rate and was executed
+// three times per costed orientation.
+static __device__ __noinline__ float row_bytes_wide(int width) {
     unsigned long long a = ((unsigned long long)(long long)width + 7ull) & ~7ull;
-    return tuples * (float)(a + 24ull);
+    return (float)(a + 24ull);
 }
+__device__ __forceinline__ float row_bytes(int width) {
+    if (__builtin_expect(width < 0, 0)) return row_bytes_wide(width);
+    return (float)((((uint32_t)width + 7u) & ~7u) + 24u);
+}
+__device__ __forceinline__ float relation_byte_size(float tuples, int width) { return tuples * row_bytes(width); }
 __device__ __forceinline__ float page_size(float tuples, int width) {
     return ceilf(relation_byte_size(tuples, width) / 8192.0f);
 }
@@ -132,7 +143,7 @@ struct Htsz {
 };
 
 // :480-621 ExecChooseHashTableSize
-__device__ __forceinline__ Htsz exec_choose_hash_table_size(float ntuples, int tupwidth, int work_mem) {
+static __device__ __noinline__ Htsz choose_hash_table_size_wide(float ntuples, int tupwidth, int work_mem) {
     Htsz res;
     res.numbatches = 1;
     if (ntuples <= 0.0f) ntuples = 1000.0f;
@@ -173,6 +184,40 @@ __device__ __forceinline__ Htsz exec_choose_hash_table_size(float ntuples, int t
         int p2 = 1 << ceil_log2_l(minbatch);
         res.numbatches = p2 > 2 ? p2 : 2;
     }
+    return res;
+}
+
+__device__ __forceinline__ int ceil_log2_u32(uint32_t num) { return num <= 1u ? 0 : 32 - __clz(num - 1u); }
+
+// The same in 32-bit integers where every quantity fits: 4 MB <= work_mem <
+// 1 GB and 0 <= width < 2^21 keep the table's bytes, its pointers and its
+// bucket bytes below 2^30 and the quotient of bytes and bucket size above
+// zero.  Every float operation and conversion has the operands of the 64-bit
+// form, which the other settings take.  It runs once per connected set, on the
+// critical path of a level (the memo entry carries its result).
+__device__ __forceinline__ Htsz exec_choose_hash_table_size(float ntuples, int tupwidth, int work_mem) {
+    if (__builtin_expect(work_mem < 4096 || work_mem >= (1 << 20) || (uint32_t)tupwidth >= (1u << 21), 0))
+        return choose_hash_table_size_wide(ntuples, tupwidth, work_mem);
+    Htsz res;
+    res.numbatches = 1;
+    if (ntuples <= 0.0f) ntuples = 1000.0f;
+    const uint32_t tupsize = 32u + (((uint32_t)tupwidth + 7u) & ~7u);
+    const float inner_rel_bytes = ntuples * (float)tupsize;
+    uint32_t bytes = (uint32_t)work_mem * 1024u;
+    // (bytes as float) / 8, truncated, is below 0x3fffffff / 8 here
+    const uint32_t max_pointers = 1u << (31 - __clz((uint32_t)((float)bytes / 8.0f)));
+    const uint32_t skew = bytes * 2u / 100u;
+    if (skew >= tupsize + 84u) bytes -= skew;
+    uint32_t nb = (uint32_t)fminf(ceilf(ntuples), (float)max_pointers);
+    nb = 1u << ceil_log2_u32(nb < 1024u ? 1024u : nb);
+    if (inner_rel_bytes + (float)(8u * nb) > (float)bytes) {
+        nb = 1u << ceil_log2_u32(bytes / (tupsize + 8u));
+        if (nb > max_pointers) nb = max_pointers;
+        const float dbatch = fminf(ceilf(inner_rel_bytes / (float)(bytes - 8u * nb)), (float)max_pointers);
+        const int p2 = 1 << ceil_log2_u32((uint32_t)dbatch);
+        res.numbatches = p2 > 2 ? p2 : 2;
+    }
+    res.numbuckets = (int)nb;
     return res;
 }
 
@@ -268,8 +313,7 @@ __device__ __forceinline__ void cost_hashjoin(const DevHeader &h, const RelVal &
         startup_cost += h.seq_page_cost * innerpages;
         run_cost += h.seq_page_cost * (innerpages + 2.0f * outerpages);
     }
-    if (relation_byte_size(clamp_row_est(inner_path_rows * bs_mcvfreq), inner.width) >
-        (float)((long long)h.work_mem * 1024LL))
+    if (relation_byte_size(clamp_row_est(inner_path_rows * bs_mcvfreq), inner.width) > h.work_mem_bytes)
         startup_cost += h.disable_cost;
     if (extra.inner_unique) {
         float outer_matched_rows = rintf(outer_path_rows * extra.outer_match_frac);
@@ -763,6 +807,79 @@ __device__ __forceinline__ void join_eval_mirror_tree(const DevInfoView &d, uint
         out_lr = join_eval(d, L, l, R, r);
         out_rl = join_eval(d, R, r, L, l);
     }
+}
+
+// ---------------------------------------------------------------------------
+// Both orientations of a split edge of a plain tree (DevHeader::tree_plain).
+// What join_eval_mirror_w computes for it, without the parts that are constant
+// there: no unique inner side, no index, bucket size 0.1, MCV frequency 0 (one
+// row within work_mem: no skew penalty), the sums over the edge's classes in
+// TreeEdge, and the terms that both orientations share taken once (products
+// and sums of two operands do not depend on their order; a run cost may start
+// from its first term instead of 0 because only the sum with a startup cost,
+// which is never -0, is kept).  Every other operation is in the order of
+// cost_nestloop and cost_hashjoin.
+// ---------------------------------------------------------------------------
+struct PlainParams {
+    float nl_base, tuple_cost, page_cost;
+};
+
+__device__ __forceinline__ PlainParams plain_params(const DevHeader &h) {
+    PlainParams p;
+    p.nl_base = h.enable_nestloop ? 0.0f : h.disable_cost;
+    p.tuple_cost = h.cpu_tuple_cost;
+    p.page_cost = h.seq_page_cost;
+    return p;
+}
+
+struct JoinCost {
+    float rows, startup, total;
+};
+
+__device__ __forceinline__ void plain_join(const PlainParams &c, const TreeEdge &e, float sel, const float4 o,
+                                           const float4 i, float d_o, float d_i, float nl_startup, float nl_tuples,
+                                           bool batched, float pages_o, float pages_i, JoinCost &out) {
+    const float rows = sel * o.x * i.x;
+    out.rows = rows > 1.0f ? roundf(rows) : 1.0f;
+    float run = d_o;
+    const float again = o.x - 1.0f;
+    if (o.x > 1.0f) run += again * i.y;
+    run += d_i;
+    if (o.x > 1.0f) run += again * d_i;
+    run += nl_tuples;
+    const float nl_total = nl_startup + run;
+    float hs = 0.0f + o.y;
+    float hr = d_o;
+    hs += i.z;
+    hs += e.hj_row * i.x;
+    hr += e.quals_cost * o.x;
+    if (batched) {
+        hs += c.page_cost * pages_i;
+        hr += c.page_cost * (pages_i + 2.0f * pages_o);
+    }
+    hr += e.per_tuple * o.x * clamp_row_est(i.x * 0.1f) * 0.5f;
+    hr += c.tuple_cost * out.rows;
+    const float hj_total = hs + hr;
+    const bool hash = hj_total < nl_total;
+    out.startup = hash ? hs : nl_startup;
+    out.total = hash ? hj_total : nl_total;
+}
+
+// l: memo entry of the side that holds the edge's lower end, r: of the other
+__device__ __forceinline__ void plain_mirror(const PlainParams &c, const TreeEdge &e, const float4 l, const float4 r,
+                                             JoinCost &lr, JoinCost &rl) {
+    const uint32_t lw = __float_as_uint(l.w), rw = __float_as_uint(r.w);
+    const bool lb = (lw >> (kWidthBits + 6)) != 0u, rb = (rw >> (kWidthBits + 6)) != 0u;   // more than one batch
+    float lp = 0.0f, rp = 0.0f;
+    if (lb || rb) {
+        lp = page_size(l.x, (int)(lw & kWidthMask));
+        rp = page_size(r.x, (int)(rw & kWidthMask));
+    }
+    const float dl = l.z - l.y, dr = r.z - r.y;
+    const float nl_startup = c.nl_base + (r.y + l.y);
+    const float nl_tuples = e.nl_tuple * (l.x * r.x);
+    plain_join(c, e, e.sel_lo, l, r, dl, dr, nl_startup, nl_tuples, rb, lp, rp, lr);
+    plain_join(c, e, e.sel_hi, r, l, dr, dl, nl_startup, nl_tuples, lb, rp, lp, rl);
 }
 
 // (L, R) and (R, L); classes beyond 256 take two join_eval calls

@@ -287,12 +287,16 @@ __global__ void __launch_bounds__(kBlock) k_level_sets(const uint32_t *__restric
 // ---------------------------------------------------------------------------
 // candidate enumeration + evaluation shared by k_eval / k_ovf_chunks
 // ---------------------------------------------------------------------------
+// A lane's first strict minimum over the candidates it costed.  The NaN rule
+// (a NaN first candidate is kept) needs the lowest index of all candidates and
+// of those with a NaN cost; NaN costs are rare, so a candidate pays one
+// minimum and one untaken branch for it.
 struct LaneBest {
     unsigned long long key;
     RelVal val;
     uint32_t left;
-    uint32_t first_p;
-    bool first_nan;
+    uint32_t first_p;             // lowest index of a valid candidate
+    uint32_t nan_p;               // lowest index of one with a NaN cost
     RelVal nan_val;
     uint32_t nan_left;
     uint32_t n_valid;
@@ -301,33 +305,31 @@ struct LaneBest {
         key = ~0ull;
         left = 0;
         first_p = kFull;
-        first_nan = false;
+        nan_p = kFull;
         nan_left = 0;
         n_valid = 0;
     }
+    __device__ __forceinline__ bool first_nan() const { return nan_p != kFull && nan_p == first_p; }
 };
 
 // one valid candidate p = (outer L, inner side) with its cost: the lane keeps
-// its first strict minimum (key (ordered cost, p)) and its first candidate
-// in enumeration order with that candidate's NaN status
+// its first strict minimum (key (ordered cost, p))
 __device__ __forceinline__ void best_update(LaneBest &best, uint32_t p, uint32_t L, const RelVal &out) {
-    const bool nan = isnan(out.total);
     best.n_valid++;
-    if (p < best.first_p) {
-        best.first_p = p;
-        best.first_nan = nan;
-        if (nan) {
+    best.first_p = min(best.first_p, p);
+    if (__builtin_expect(isnan(out.total), 0)) {
+        if (p < best.nan_p) {
+            best.nan_p = p;
             best.nan_val = out;
             best.nan_left = L;
         }
+        return;
     }
-    if (!nan) {
-        const unsigned long long key = ((unsigned long long)ord_float(out.total) << 32) | p;
-        if (key < best.key) {
-            best.key = key;
-            best.val = out;
-            best.left = L;
-        }
+    const unsigned long long key = ((unsigned long long)ord_float(out.total) << 32) | p;
+    if (key < best.key) {
+        best.key = key;
+        best.val = out;
+        best.left = L;
     }
 }
 
@@ -519,7 +521,7 @@ __device__ __forceinline__ WarpWinner warp_winner(const LaneBest &b, unsigned lo
     uint32_t mh = __reduce_min_sync(kFull, kh);
     uint32_t ml = __reduce_min_sync(kFull, kh == mh ? kl : kFull);
     uint32_t mf = __reduce_min_sync(kFull, b.first_p);
-    bool nan_first = (b.first_p == mf) && b.first_nan;
+    bool nan_first = (b.first_p == mf) && b.first_nan();
     unsigned nm = __ballot_sync(kFull, nan_first);
     min_key = ((unsigned long long)mh << 32) | ml;
     first_key = ((unsigned long long)mf << 1) | (nm ? 1ull : 0ull);
@@ -677,7 +679,7 @@ __device__ __forceinline__ void mpdp_groups(const DevInfoView &d, const uint32_t
             }
             if (of < fp) fp = of;
         }
-        const bool nan_first = has && !ovf && best.first_p == fp && best.first_nan;
+        const bool nan_first = has && !ovf && best.first_p == fp && best.first_nan();
         const unsigned nm = __ballot_sync(kFull, nan_first) & group_mask;
         const unsigned long long gkey = ((unsigned long long)kh << 32) | kl;
         if (has && !ovf) {
@@ -734,253 +736,304 @@ __global__ void __launch_bounds__(kBlock) k_eval_mpdp(const uint32_t *__restrict
 }
 
 // ---------------------------------------------------------------------------
-// k_eval_tree: MPDP on a tree-shaped query graph (star, snowflake, chain, and
-// the contracted trees of IDP sub-problems), any relation numbering.
+// MPDP on a tree-shaped query graph (star, snowflake, chain, and the
+// contracted trees of IDP sub-problems), any relation numbering.
 // A connected set S is a subtree; the reference's block search walks it from
-// its lowest relation r, and every block is a bridge {a, b}, a < b.  With the
-// query tree rooted at r, let c be the child end of the edge: removing the
-// edge leaves S & sub_r[c] and the rest, so no DFS is needed.  Candidate
-// order: blocks are emitted in post-order of their child end, and the
-// reference's enumeration index is 2 * post_r(c) + (lb == {a} ? 0 : 1) with
-//     post_r(c) = |S & before_r[c]| - |S & anc_r[c]| + |S & sub_r[c]| - 1
-// (preorder rank minus depth plus subtree size minus one).  With ec_masked
-// only the classes on edge {a, b} can match.
+// its lowest relation r, and every block is a bridge.  With the query tree
+// rooted at r, every relation v of S but r is the child end of one split edge
+// (v, parent of v), and removing it leaves S & sub_r[v] and the rest: no DFS,
+// no search for the edge, one 8-byte table load per split.  Blocks are
+// emitted in post-order of their child end, so the reference's enumeration
+// index of a split is 2 * post_r(v) + (the lower end's side outer ? 0 : 1) with
+//     post_r(v) = |S & before_r[v]| - |S & anc_r[v]| + |S & sub_r[v]| - 1
+// (preorder rank minus depth plus subtree size minus one); it is computed only
+// where it decides something, between equal costs and for NaN costs.
 // ---------------------------------------------------------------------------
-struct EdgeIter {
-    uint32_t vs;      // vertices of S not yet started
-    uint32_t nb;      // remaining higher neighbours of v
-    int v;
-    uint32_t e;       // index of the next edge to be returned
+// what the classes of a query allow (one instantiation each, so that a kernel
+// carries only the evaluation its queries take): kTreePlain
+// DevHeader::tree_plain, kTreeMasked DevHeader::ec_masked, kTreeGeneral any
+constexpr int kTreeGeneral = 0, kTreeMasked = 1, kTreePlain = 2;
+
+__host__ __device__ __forceinline__ int tree_layout(const DevHeader &h) {
+    return h.tree_plain ? kTreePlain : (h.ec_masked ? kTreeMasked : kTreeGeneral);
+}
+
+// one set's view of the tree tables: the rows of its lowest relation
+struct TreeRows {
+    const uint32_t *tab;   // tree tables
+    const uint32_t *row;   // rows of the root
+    int n;
 };
 
-__device__ __forceinline__ void edge_next(const uint32_t *adj, uint32_t S, EdgeIter &it, int &a, int &b) {
-    while (it.nb == 0u) {
-        it.v = __ffs(it.vs) - 1;
-        it.vs &= it.vs - 1u;
-        it.nb = adj[it.v] & S & ~((2u << it.v) - 1u);
-    }
-    a = it.v;
-    b = __ffs(it.nb) - 1;
-    it.nb &= it.nb - 1u;
-    it.e++;
+__device__ __forceinline__ TreeRows tree_rows(const DevHeader &h, uint32_t S) {
+    TreeRows t;
+    t.tab = reinterpret_cast<const uint32_t *>(&h) + h.tree_tab;
+    t.n = h.n;
+    t.row = t.tab + (S ? t.tab[lowest_idx(S)] : 0u);
+    return t;
 }
 
-// Edge-wise evaluation: the candidates of S come in mirror pairs, c = 2e and
-// c = 2e + 1 being the two orientations of split edge e (side 0 puts the
-// component of a on the outer side).  A lane takes whole edges: it decodes
-// the edge once, loads the two memo entries once and costs both orientations
-// in one fused pass (join_eval_mirror_tree: shared class visit, two
-// independent cost chains), keyed by the reference's indices of both
-// candidates.  Lanes of a group take edges e = gl, gl + G, ...
-// PIPE: software-pipelined edge loop for G < 32, in the 2- and 3-blocks
-// persistent kernels (the next edge's memo entries are requested before the
-// current edge is costed); at 64 registers (the 4-blocks persistent kernel and
-// the per-level kernel) it spills, and those keep the plain loop.
-template <int G, bool MASKED, bool PIPE>
-__device__ __forceinline__ void tree_groups(const DevInfoView &d, uint32_t first_set, uint32_t stride_sets,
-                                            const uint32_t *sets, uint32_t count, int k, float4 *memo,
-                                            uint32_t *memo_left, unsigned long long &pairs) {
-    const DevHeader &h = *d.h;
-    const int lane = threadIdx.x & 31;
-    const int grp = lane / G, gl = lane % G;
-    const uint32_t group_mask = (G == 32) ? kFull : (((1u << G) - 1u) << (grp * G));
-    const uint32_t E = (uint32_t)(k - 1);                 // split edges of a k-set
-    const uint32_t per_lane = (E + G - 1u) / G;
-    // plain-DPsub index of the mirror: pext(S - L, S) - 1 = 2^k - 3 - p
-    const uint32_t mirror_base = (k >= 32 ? 0xFFFFFFFFu : ((1u << k) - 1u)) - 2u;
-    for (uint32_t base = first_set; base < count; base += stride_sets) {
-        const uint32_t i = base + (uint32_t)grp;
-        const bool has = i < count;
-        const uint32_t S = has ? __ldcg(sets + i) : 0u;
-        EdgeIter it;
-        it.vs = S;
-        it.nb = 0u;
-        it.v = 0;
-        it.e = 0u;
-        int a = 0, b = 0;
-        // G == 32 (one set per warp): the edges of S indexed cooperatively.
-        // Lane t takes the t-th relation of S and its higher-numbered
-        // neighbours in S; the inclusive prefix of their counts numbers the
-        // edges in edge_next's order (lower end, then higher end), so an
-        // edge is found by a binary search over the lanes instead of walking
-        // the edges before it.
-        int vt = 0;
-        uint32_t fwd = 0u, scan = 0u;
-        if (G == 32) {
-            const int kk = __popc(S);
-            if (lane < kk) {
-                vt = (int)__fns(S, 0u, lane + 1);
-                fwd = h.adj[vt] & S & ~((2u << vt) - 1u);
-            }
-            scan = (uint32_t)__popc(fwd);
-#pragma unroll
-            for (int off = 1; off < 32; off <<= 1) {
-                const uint32_t o = __shfl_up_sync(kFull, scan, off);
-                if (lane >= off) scan += o;
-            }
-        }
-        LaneBest best;
-        best.init();
-        const uint32_t *tab = reinterpret_cast<const uint32_t *>(d.h) + h.tree_tab;
-        const int n = h.n, nn = n * n;
-        // split edge (a, b): the side holding a (outer in orientation 0), the
-        // reference's indices of both orientations and the classes on the edge
-        auto decode = [&](uint32_t &L0, uint32_t &p0, uint32_t &p1, uint32_t &ecm) {
-            const int rt = __ffs(S) - 1;
-            const uint32_t *anc_r = tab + 2 * nn + rt * n;
-            const int ch = ((anc_r[b] >> a) & 1u) ? b : a;        // child end w.r.t. root rt
-            const uint32_t comp_c = S & tab[rt * n + ch];
-            L0 = (ch == a) ? comp_c : (S ^ comp_c);
-            const uint32_t post = (uint32_t)(__popc(S & tab[nn + rt * n + ch]) - __popc(S & anc_r[ch]) +
-                                             __popc(comp_c) - 1);
-            if (h.index_order) {
-                p0 = dpsub_index(L0, S);
-                p1 = mirror_base - p0;
-            } else {
-                p0 = 2u * post;
-                p1 = p0 + 1u;
-            }
-            ecm = 0u;
-            if (MASKED) {
-                const int ch0 = ((tab[2 * nn + b] >> a) & 1u) ? b : a;   // child end w.r.t. relation 0
-                ecm = h.edge_ec[ch0];
-            }
-        };
-        // costs both orientations of one edge from its two memo entries
-        auto cost2 = [&](uint32_t L0, uint32_t p0, uint32_t p1, uint32_t ecm, const float4 lv, const float4 rv) {
-            const uint32_t R0 = S ^ L0;
-            const RelVal l = unpack_rel(lv, h.hz_packed), r = unpack_rel(rv, h.hz_packed);
-            RelVal o0, o1;
-            join_eval_mirror_tree<MASKED>(d, L0, l, R0, r, ecm, o0, o1);
-            best_update(best, p0, L0, o0);
-            best_update(best, p1, R0, o1);
-        };
-        if (G != 32 && !PIPE) {
-            for (uint32_t j = 0; j < per_lane; j++) {
-                const uint32_t e = (uint32_t)gl + j * G;
-                if (has && e < E) {
-                    while (it.e <= e) edge_next(h.adj, S, it, a, b);
-                    uint32_t L0, p0, p1, ecm;
-                    decode(L0, p0, p1, ecm);
-                    cost2(L0, p0, p1, ecm, __ldcg(memo + L0), __ldcg(memo + (S ^ L0)));
-                }
-            }
-        } else if (G != 32) {
-            uint32_t cL = 0u, cp0 = 0u, cp1 = 0u, cecm = 0u;
-            float4 clv = make_float4(0.f, 0.f, 0.f, 0.f), crv = clv;
-            bool cact = false;
-            auto fetch = [&](uint32_t j, uint32_t &L0, uint32_t &p0, uint32_t &p1, uint32_t &ecm, float4 &lv,
-                             float4 &rv) -> bool {
-                const uint32_t e = (uint32_t)gl + j * G;
-                if (!(has && e < E)) return false;
-                while (it.e <= e) edge_next(h.adj, S, it, a, b);
-                decode(L0, p0, p1, ecm);
-                lv = __ldcg(memo + L0);
-                rv = __ldcg(memo + (S ^ L0));
-                return true;
-            };
-            if (per_lane > 0) cact = fetch(0u, cL, cp0, cp1, cecm, clv, crv);
-            for (uint32_t j = 0; j < per_lane; j++) {
-                uint32_t nL = 0u, np0 = 0u, np1 = 0u, necm = 0u;
-                float4 nlv = clv, nrv = crv;
-                const bool nact = (j + 1 < per_lane) ? fetch(j + 1, nL, np0, np1, necm, nlv, nrv) : false;
-                if (cact) cost2(cL, cp0, cp1, cecm, clv, crv);
-                cL = nL;
-                cp0 = np0;
-                cp1 = np1;
-                cecm = necm;
-                clv = nlv;
-                crv = nrv;
-                cact = nact;
-            }
+// the outer side of orientation `code` (child end | kSideHigher) of S
+__device__ __forceinline__ uint32_t tree_side(const TreeRows &t, uint32_t S, uint32_t code) {
+    const uint2 e = *reinterpret_cast<const uint2 *>(t.row + 2u * (code & 31u));
+    const uint32_t comp = S & e.x;
+    const bool comp_outer = ((e.y & kTreeLower) != 0u) == ((code & kSideHigher) == 0u);
+    return comp_outer ? comp : S ^ comp;
+}
+
+// the reference's enumeration index of orientation `code`
+__device__ __noinline__ uint32_t tree_index(const uint32_t *row, int n, uint32_t S, uint32_t code, uint32_t dpsub) {
+    const uint32_t v = code & 31u;
+    const uint2 e = *reinterpret_cast<const uint2 *>(row + 2u * v);
+    const uint32_t comp = S & e.x;
+    if (dpsub) {
+        const bool comp_outer = ((e.y & kTreeLower) != 0u) == ((code & kSideHigher) == 0u);
+        return dpsub_index(comp_outer ? comp : S ^ comp, S);
+    }
+    const uint2 w = *reinterpret_cast<const uint2 *>(row + 2u * (uint32_t)n + 2u * v);
+    const uint32_t post = (uint32_t)(__popc(S & w.x) - __popc(S & w.y) + __popc(comp) - 1);
+    return 2u * post + ((code & kSideHigher) ? 1u : 0u);
+}
+
+// A lane's best split of a set: the ordered cost (ord_float), the orientation
+// and the values the memo needs.  Ties go to the lower enumeration index.
+constexpr uint32_t kNoCode = 0xFFu;
+struct TreeBest {
+    uint32_t ord, code;
+    float rows, startup;
+    uint32_t nan_code;     // the candidate of lowest index with a NaN cost, kNoCode: none
+
+    __device__ __forceinline__ void init() {
+        ord = kFull;
+        code = kNoCode;
+        rows = startup = 0.0f;
+        nan_code = kNoCode;
+    }
+};
+
+__device__ __forceinline__ void tree_update(TreeBest &best, const DevHeader &h, const TreeRows &t, uint32_t S,
+                                            uint32_t code, float rows, float startup, float total) {
+    const uint32_t ord = ord_float(total);
+    bool take = ord < best.ord;
+    if (__builtin_expect(ord == best.ord || isnan(total), 0)) {
+        if (isnan(total)) {
+            if (best.nan_code == kNoCode ||
+                tree_index(t.row, t.n, S, code, h.index_order) < tree_index(t.row, t.n, S, best.nan_code, h.index_order))
+                best.nan_code = code;
+            take = false;
         } else {
-            for (uint32_t j = 0; j < per_lane; j++) {
-                const uint32_t e = (uint32_t)gl + j * G;
-                const bool active = has && e < E;
-                // smallest lane t with scan_t > e (every lane takes part in the shuffles)
-                int lo = 0;
-#pragma unroll
-                for (int step = 16; step >= 1; step >>= 1) {
-                    const uint32_t sv = __shfl_sync(kFull, scan, lo + step - 1);
-                    if (sv <= e) lo += step;
-                }
-                const int t = lo > 31 ? 31 : lo;
-                const uint32_t before = __shfl_sync(kFull, scan, t) - (uint32_t)__popc(__shfl_sync(kFull, fwd, t));
-                const uint32_t ft = __shfl_sync(kFull, fwd, t);
-                a = __shfl_sync(kFull, vt, t);
-                if (active) {
-                    b = (int)__fns(ft, 0u, (int)(e - before) + 1);
-                    uint32_t L0, p0, p1, ecm;
-                    decode(L0, p0, p1, ecm);
-                    cost2(L0, p0, p1, ecm, __ldcg(memo + L0), __ldcg(memo + (S ^ L0)));
-                }
-            }
+            take = tree_index(t.row, t.n, S, code, h.index_order) <
+                   tree_index(t.row, t.n, S, best.code, h.index_order);
         }
-        uint32_t kh = (uint32_t)(best.key >> 32), kl = (uint32_t)best.key, fp = best.first_p;
-#pragma unroll
-        for (int off = G / 2; off >= 1; off >>= 1) {
-            uint32_t oh = __shfl_xor_sync(kFull, kh, off);
-            uint32_t ol = __shfl_xor_sync(kFull, kl, off);
-            uint32_t of = __shfl_xor_sync(kFull, fp, off);
-            if (oh < kh || (oh == kh && ol < kl)) {
-                kh = oh;
-                kl = ol;
-            }
-            if (of < fp) fp = of;
-        }
-        const bool nan_first = has && best.first_p == fp && best.first_nan;
-        const unsigned nm = __ballot_sync(kFull, nan_first) & group_mask;
-        const unsigned long long gkey = ((unsigned long long)kh << 32) | kl;
-        if (has) {
-            if (nm) {
-                if (nan_first) memo_write(*d.h, memo, memo_left, S, best.nan_val, best.nan_left);
-            } else if (best.key == gkey && best.key != ~0ull) {
-                memo_write(*d.h, memo, memo_left, S, best.val, best.left);
-            }
-        }
-        pairs += best.n_valid;
+    }
+    if (take) {
+        best.ord = ord;
+        best.code = code;
+        best.rows = rows;
+        best.startup = startup;
     }
 }
 
-__global__ void __launch_bounds__(kBlock, 4) k_eval_tree(const uint32_t *__restrict__ blob, uint32_t blob_words, int k,
+// both orientations of the split of S at child end v from the memo entries of
+// the side that holds the edge's lower end (lv) and of the other (rv)
+template <int LAYOUT>
+__device__ __forceinline__ void tree_cost(const DevInfoView &d, const PlainParams &pp, const TreeRows &t, uint32_t S,
+                                          uint32_t L0, uint32_t v, uint32_t edge, const float4 lv, const float4 rv,
+                                          TreeBest &best, int &width) {
+    const DevHeader &h = *d.h;
+    if (LAYOUT == kTreePlain) {
+        const TreeEdge &e = reinterpret_cast<const TreeEdge *>(t.tab + tree_edge_off(t.n))[edge];
+        JoinCost lr, rl;
+        plain_mirror(pp, e, lv, rv, lr, rl);
+        width = (int)((__float_as_uint(lv.w) & kWidthMask) + (__float_as_uint(rv.w) & kWidthMask));
+        tree_update(best, h, t, S, v, lr.rows, lr.startup, lr.total);
+        tree_update(best, h, t, S, v | kSideHigher, rl.rows, rl.startup, rl.total);
+    } else {
+        const RelVal l = unpack_rel(lv, h.hz_packed), r = unpack_rel(rv, h.hz_packed);
+        RelVal o0, o1;
+        const uint32_t classes =
+            LAYOUT == kTreeMasked ? reinterpret_cast<const TreeEdge *>(t.tab + tree_edge_off(t.n))[edge].classes : 0u;
+        join_eval_mirror_tree<LAYOUT == kTreeMasked>(d, L0, l, S ^ L0, r, classes, o0, o1);
+        width = o0.width;
+        tree_update(best, h, t, S, v, o0.rows, o0.startup, o0.total);
+        tree_update(best, h, t, S, v | kSideHigher, o1.rows, o1.startup, o1.total);
+    }
+}
+
+// The first candidate of a set in enumeration order has a NaN cost: the
+// reference keeps it.  Rare (overflowed row estimates): every lane finds its
+// lowest index, and when the group's lowest is a NaN one, its lane costs it
+// again and writes the entry.  Returns whether the lane's group is settled.
+template <int LAYOUT>
+__device__ __noinline__ bool tree_nan_rule(const DevInfoView d, uint32_t S, bool has, int k, int G, uint32_t nan_code,
+                                           const float4 *memo, RelVal &out, uint32_t &left, bool &writer) {
+    const DevHeader &h = *d.h;
+    const TreeRows t = tree_rows(h, S);
+    const int gl = (int)(threadIdx.x & 31u) % G;
+    uint32_t first = kFull;
+    uint32_t x = has ? S & (S - 1u) : 0u;
+    for (int j = 0; x; x &= x - 1u, j++) {
+        if (j % G != gl) continue;
+        const uint32_t v = (uint32_t)lowest_idx(x);
+        first = min(first, tree_index(t.row, t.n, S, v, h.index_order));
+        first = min(first, tree_index(t.row, t.n, S, v | kSideHigher, h.index_order));
+    }
+    const uint32_t nan_p = nan_code != kNoCode ? tree_index(t.row, t.n, S, nan_code, h.index_order) : kFull;
+    uint32_t gfirst = first, gnan = nan_p;
+    for (int off = G >> 1; off >= 1; off >>= 1) {
+        gfirst = min(gfirst, __shfl_xor_sync(kFull, gfirst, off));
+        gnan = min(gnan, __shfl_xor_sync(kFull, gnan, off));
+    }
+    const bool settled = has && gnan != kFull && gnan == gfirst;
+    writer = settled && nan_p == gnan;
+    if (writer) {
+        left = tree_side(t, S, nan_code);
+        const RelVal l = load_rel(memo, left, h.hz_packed), r = load_rel(memo, S ^ left, h.hz_packed);
+        out = join_eval(d, left, l, S ^ left, r);
+    }
+    return settled;
+}
+
+// One set of k relations (has: the lane's group holds one) by a group of G
+// lanes, G a power of two.  Lanes take the child ends by rank in S; both memo
+// entries of the next split are requested before the current one is costed.
+// The whole warp calls it, with the same k and G.
+template <int LAYOUT>
+__device__ __forceinline__ void tree_set(const DevInfoView &d, const PlainParams &pp, uint32_t S, bool has, int k, int G,
+                                         float4 *memo, uint32_t *memo_left) {
+    const DevHeader &h = *d.h;
+    const int lane = threadIdx.x & 31, gl = lane & (G - 1);
+    const TreeRows t = tree_rows(h, has ? S : 0u);
+    uint32_t x = has ? S & (S - 1u) : 0u;
+    if (G == 32) {
+        x &= 1u << lane;   // at most 31 child ends: the lane's own relation
+    } else {
+        for (int i = 0; i < gl; i++) x &= x - 1u;
+    }
+    const int steps = G == 32 ? 1 : (k - 1 + G - 1) / G;
+    TreeBest best;
+    best.init();
+    int width = 0;
+    uint32_t v = 0u, L0 = 0u, edge = 0u;
+    float4 lv = make_float4(0.f, 0.f, 0.f, 0.f), rv = lv;
+    auto fetch = [&]() -> bool {
+        if (x == 0u) return false;
+        v = (uint32_t)lowest_idx(x);
+        const uint2 e = *reinterpret_cast<const uint2 *>(t.row + 2u * v);
+        const uint32_t comp = S & e.x;
+        L0 = (e.y & kTreeLower) ? comp : S ^ comp;
+        edge = e.y & 31u;
+        lv = __ldcg(memo + L0);
+        rv = __ldcg(memo + (S ^ L0));
+        return true;
+    };
+    bool active = fetch();
+    for (int j = 0; j < steps; j++) {
+        const uint32_t cv = v, cL = L0, ce = edge;
+        const float4 clv = lv, crv = rv;
+        const bool cact = active;
+        active = false;
+        if (j + 1 < steps) {
+            for (int i = 0; i < G; i++) x &= x - 1u;
+            active = fetch();
+        }
+        if (cact) tree_cost<LAYOUT>(d, pp, t, S, cL, cv, ce, clv, crv, best, width);
+    }
+    uint32_t m = best.ord;
+    for (int off = G >> 1; off >= 1; off >>= 1) m = min(m, __shfl_xor_sync(kFull, m, off));
+    bool win = has && best.ord == m && m != kFull;
+    const uint32_t group_mask = (G == 32) ? kFull : (((1u << G) - 1u) << (lane & ~(G - 1)));
+    const uint32_t tied = __ballot_sync(kFull, win) & group_mask;
+    if (__any_sync(kFull, __popc(tied) > 1)) {
+        const uint32_t p = win ? tree_index(t.row, t.n, S, best.code, h.index_order) : kFull;
+        uint32_t pm = p;
+        for (int off = G >> 1; off >= 1; off >>= 1) pm = min(pm, __shfl_xor_sync(kFull, pm, off));
+        win = win && p == pm;
+    }
+    if (__any_sync(kFull, best.nan_code != kNoCode)) {
+        RelVal out;
+        uint32_t left = 0u;
+        bool writer = false;
+        if (tree_nan_rule<LAYOUT>(d, S, has, k, G, best.nan_code, memo, out, left, writer)) win = false;
+        if (writer) memo_write(h, memo, memo_left, S, out, left);
+    }
+    if (win) {
+        RelVal out;
+        out.rows = best.rows;
+        out.startup = best.startup;
+        // the inverse of ord_float (a total is never -0: its startup cost starts from +0)
+        out.total = __uint_as_float((m & 0x80000000u) ? m ^ 0x80000000u : ~m);
+        out.width = width;
+        memo_write(h, memo, memo_left, S, out, tree_side(t, S, best.code));
+    }
+}
+
+// Lanes per set of a level of `count` sets of k relations with `lanes` lanes
+// resident.  A warp-step (one split, both orientations) issues about kIssue
+// instructions and takes kStep cycles; a set adds about one step of its own
+// (list entry, reduction, memo entry).  The level takes the larger of its
+// issue time and its longest lane's time; the smallest of the powers of two
+// wins, the narrower group on ties.
+__host__ __device__ __forceinline__ int tree_group(uint32_t count, int k, uint32_t lanes, uint32_t sms) {
+    const float kIssue = 240.0f, kStep = 1500.0f;
+    int best = 1;
+    float best_t = 3.0e38f;
+    for (int G = 1; G <= 32; G <<= 1) {
+        const float steps = G == 32 ? 1.0f : (float)((k - 1 + G - 1) / G);
+        const float warps = ceilf((float)count * (float)G / 32.0f);
+        const float rounds = ceilf(warps * 32.0f / (float)lanes);
+        const float issue = warps * (steps + 1.0f) * kIssue / (4.0f * (float)sms);
+        const float chain = rounds * (steps + 1.0f) * kStep;
+        const float t = issue > chain ? issue : chain;
+        if (t < best_t) {
+            best_t = t;
+            best = G;
+        }
+        if (G >= k - 1) break;
+    }
+    return best;
+}
+
+template <int LAYOUT>
+__device__ __forceinline__ void tree_level(const DevInfoView &d, const PlainParams &pp, uint32_t gwarp, uint32_t nwarps,
+                                           const uint32_t *sets, uint32_t count, int k, int G, float4 *memo,
+                                           uint32_t *memo_left) {
+    const uint32_t per_warp = 32u / (uint32_t)G, grp = (threadIdx.x & 31u) / (uint32_t)G;
+    for (uint32_t base = gwarp * per_warp; base < count; base += nwarps * per_warp) {
+        const bool has = base + grp < count;
+        tree_set<LAYOUT>(d, pp, has ? __ldcg(sets + base + grp) : 0u, has, k, G, memo, memo_left);
+    }
+}
+
+// one level per launch (gpuqo_b200_persistent = 0, no cooperative launch, or
+// after a barrier timeout)
+__global__ void __launch_bounds__(kBlock, 3) k_eval_tree(const uint32_t *__restrict__ blob, uint32_t blob_words, int k,
                                                       const uint32_t *__restrict__ sets,
                                                       LevelCounters *__restrict__ lc, float4 *__restrict__ memo,
                                                       uint32_t *__restrict__ memo_left,
-                                                      GlobalCounters *__restrict__ glob, uint32_t target_lanes,
-                                                      int max_group) {
+                                                      GlobalCounters *__restrict__ glob) {
     extern __shared__ __align__(16) uint32_t sm[];
     load_blob_to_smem(blob, blob_words, sm);
     const DevInfoView d = make_view(sm);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t count = lc->n_sets;
-    // group sizes 2, 8 or 32 (fewer instantiations keep the code in the
-    // instruction cache)
-    int G = 2;
-    while (G < max_group && (uint64_t)count * (uint64_t)G < (uint64_t)target_lanes) G <<= 1;
-    G = G <= 2 ? 2 : (G <= 8 ? 8 : 32);
-    const uint32_t gwarp = blockIdx.x * kWarpsPerBlock + warp;
+    const uint32_t gwarp = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
     const uint32_t nwarps = gridDim.x * kWarpsPerBlock;
-    const bool masked = d.h->ec_masked != 0u;
-    unsigned long long pairs = 0;
-    switch (G * 2 + (masked ? 1 : 0)) {
-#define GQB_T(g)                                                                                                 \
-    case 2 * g:                                                                                                  \
-        tree_groups<g, false, false>(d, gwarp * (32 / g), nwarps * (32 / g), sets, count, k, memo,               \
-                                     memo_left, pairs);                                                          \
-        break;                                                                                                   \
-    case 2 * g + 1:                                                                                              \
-        tree_groups<g, true, false>(d, gwarp * (32 / g), nwarps * (32 / g), sets, count, k, memo,                \
-                                     memo_left, pairs);                                                          \
+    const int G = tree_group(count, k, nwarps * 32u, gridDim.x);
+    const PlainParams pp = plain_params(*d.h);
+    switch (tree_layout(*d.h)) {
+    case kTreePlain:
+        tree_level<kTreePlain>(d, pp, gwarp, nwarps, sets, count, k, G, memo, memo_left);
         break;
-        GQB_T(2)
-        GQB_T(8)
-        GQB_T(32)
-#undef GQB_T
+    case kTreeMasked:
+        tree_level<kTreeMasked>(d, pp, gwarp, nwarps, sets, count, k, G, memo, memo_left);
+        break;
     default:
+        tree_level<kTreeGeneral>(d, pp, gwarp, nwarps, sets, count, k, G, memo, memo_left);
         break;
     }
-    pairs = __reduce_add_sync(kFull, (uint32_t)pairs);
-    if (lane == 0 && pairs) atomicAdd(&glob->evaluated_pairs, pairs);
+    // every split edge, both orientations
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+        atomicAdd(&glob->evaluated_pairs, (unsigned long long)count * 2ull * (unsigned long long)(k - 1));
 }
 
 // ---------------------------------------------------------------------------
@@ -1058,97 +1111,58 @@ __device__ __forceinline__ bool grid_barrier(unsigned *bar, unsigned &epoch, uns
     return s_ok != 0u;
 }
 
-// One enumeration phase (level k) of a tree-shaped query graph with the
-// block's shared adjacency, binomial table and per-warp staging area.
-//
-// Extension without a dedup structure: adding a neighbour v to a connected
-// set S of a tree makes v a leaf of T = S + v (v has exactly one neighbour p
-// in S), and every connected T of two or more relations has one largest
-// leaf.  T is emitted only from the S whose added v is that largest leaf: the
-// other leaves of T are the leaves of S except p (p gains the neighbour v),
-// or S itself when S is a single relation.  So each connected k-set appears
-// exactly once, with no atomics and no bitmap to clear.
-__device__ __forceinline__ void level_sets_phase(const uint32_t *adj, const uint32_t *binom, uint32_t *st, int n,
-                                                 int k, const uint32_t *prev_sets, uint32_t c_prev,
-                                                 uint32_t *out_sets, LevelCounters *lc) {
-    const int lane = threadIdx.x & 31;
-    const uint64_t total = binom[n * 33 + k];
+// One enumeration phase (level k from the connected (k-1)-sets) of a
+// tree-shaped query graph, each k-set once and without a dedup structure:
+// adding a neighbour v to a connected set S of a tree makes v a leaf of
+// T = S + v, and T is emitted only from the S whose added v is T's largest
+// leaf.  T's other leaves are the leaves of S but the relation that v hangs
+// off: with m1 > m2 the two largest leaves of S, a neighbour of m1 must exceed
+// m2 and any other neighbour must exceed m1 (a single relation: itself).  So
+// the extensions of S are one mask, counted and placed with one atomic per
+// warp; the loop over the relations of S costs about 10 instructions each.
+__device__ __forceinline__ uint32_t above(uint32_t bit) { return ~((bit << 1) - 1u); }
+
+// the relations v whose addition to S emits S + v (adj(v): neighbours of v)
+template <class Adj>
+__device__ __forceinline__ uint32_t tree_extensions(uint32_t S, Adj adj) {
+    uint32_t N = 0u, leaves = 0u;
+    for (uint32_t x = S; x; x &= x - 1u) {
+        const uint32_t a = adj(lowest_idx(x)), in = a & S;
+        N |= a;
+        if ((in & (in - 1u)) == 0u) leaves |= x & (0u - x);   // S is connected: at least one neighbour in S
+    }
+    if (S == 0u) return 0u;
+    N &= ~S;
+    const uint32_t m1 = 1u << (31 - __clz(leaves));
+    const uint32_t rest = leaves ^ m1;
+    if (rest == 0u) return N & above(m1);                      // a single relation
+    const uint32_t m2 = 1u << (31 - __clz(rest)), a1 = adj(31 - __clz(m1));
+    return N & ((above(m1) & ~a1) | (above(m2) & a1));
+}
+
+__device__ __forceinline__ void tree_enum_phase(const uint32_t *adj, int k, const uint32_t *prev_sets, uint32_t c_prev,
+                                                uint32_t *out_sets, LevelCounters *lc) {
+    const uint32_t lane = threadIdx.x & 31u;
     const uint32_t nthreads = gridDim.x * blockDim.x;
     // from the far end of the grid: the first warps evaluate the first sets
     // of the level in the same phase, so small levels split the two jobs
     const uint32_t tid = nthreads - 1u - (blockIdx.x * blockDim.x + threadIdx.x);
-    uint32_t cnt = 0;
-    auto emit = [&](bool ok, uint32_t s) {
-        uint32_t m = __ballot_sync(kFull, ok);
-        if (ok) st[cnt + __popc(m & ((1u << lane) - 1u))] = s;
-        cnt += __popc(m);
-        __syncwarp();
-        if (cnt >= 32) {
-            uint32_t base = 0;
-            if (lane == 0) base = atomicAdd(&lc->n_sets, 32u);
-            base = __shfl_sync(kFull, base, 0);
-            out_sets[base + lane] = st[lane];
-            __syncwarp();
-            if (lane < cnt - 32) st[lane] = st[32 + lane];
-            cnt -= 32;
-            __syncwarp();
+    for (uint32_t first = tid & ~31u; first < c_prev; first += nthreads) {
+        const uint32_t idx = first + (tid & 31u);
+        const uint32_t S = idx < c_prev ? ((k == 2) ? (1u << idx) : __ldcg(prev_sets + idx)) : 0u;
+        uint32_t ext = tree_extensions(S, [&](int v) { return adj[v]; });
+        const uint32_t cnt = (uint32_t)__popc(ext);
+        uint32_t incl = cnt;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const uint32_t o = __shfl_up_sync(kFull, incl, off);
+            if (lane >= (uint32_t)off) incl += o;
         }
-    };
-    const bool use_ext = (uint64_t)c_prev * (uint64_t)(k + 4 * (n - k + 1)) < total * 3ull;
-    if (use_ext) {
-        const uint32_t rounds = (c_prev + nthreads - 1u) / nthreads;
-        for (uint32_t r = 0; r < rounds; r++) {
-            const uint32_t idx = tid + r * nthreads;
-            uint32_t S = 0u, N = 0u, leaves = 0u;
-            if (idx < c_prev) {
-                S = (k == 2) ? (1u << idx) : __ldcg(prev_sets + idx);
-                uint32_t x = S;
-                while (x) {
-                    int v = __ffs(x) - 1;
-                    x &= x - 1u;
-                    const uint32_t a = adj[v];
-                    N |= a;
-                    if (__popc(a & S) == 1) leaves |= 1u << v;
-                }
-                N &= ~S;
-            }
-            const bool single = (S & (S - 1u)) == 0u;
-            const int deg = __popc(N);
-            const int maxdeg = (int)__reduce_max_sync(kFull, (uint32_t)deg);
-            for (int j = 0; j < maxdeg; j++) {
-                bool ok = false;
-                uint32_t T = 0u;
-                if (j < deg) {
-                    const uint32_t bitv = N & (0u - N);
-                    N ^= bitv;
-                    T = S | bitv;
-                    const uint32_t p = adj[__ffs(bitv) - 1] & S;            // v's only neighbour in S
-                    const uint32_t others = single ? S : (leaves & ~p);    // the other leaves of T
-                    ok = others < bitv;                                     // v is T's largest leaf
-                }
-                emit(ok, T);
-            }
-        }
-    } else {
-        const uint32_t per_thread = (uint32_t)((total + nthreads - 1) / nthreads);
-        const uint64_t r0 = (uint64_t)tid * per_thread;
-        const uint64_t r1 = r0 + per_thread < total ? r0 + per_thread : total;
-        uint32_t s = r0 < total ? unrank_ksubset(r0, n, k, binom) : 0u;
-        for (uint32_t j = 0; j < per_thread; j++) {
-            const uint64_t r = r0 + j;
-            const bool has = r < r1;
-            const bool ok = has && is_connected(s, adj);
-            emit(ok, s);
-            if (has && r + 1 < r1) s = gosper_next(s);
-        }
+        uint32_t base = 0u;
+        if (lane == 31u && incl) base = atomicAdd(&lc->n_sets, incl);
+        uint32_t at = __shfl_sync(kFull, base, 31) + incl - cnt;
+        for (; ext; ext &= ext - 1u) out_sets[at++] = S | (ext & (0u - ext));
     }
-    if (cnt > 0) {
-        uint32_t base = 0;
-        if (lane == 0) base = atomicAdd(&lc->n_sets, cnt);
-        base = __shfl_sync(kFull, base, 0);
-        if (lane < cnt) out_sets[base + lane] = st[lane];
-    }
-    __syncwarp();
 }
 
 __device__ __forceinline__ void extract_plan(const float4 *memo, const uint32_t *memo_left, uint32_t full,
@@ -1195,45 +1209,45 @@ __device__ __forceinline__ void extract_plan(const float4 *memo, const uint32_t 
     *n_out = n;
 }
 
-// MINB: blocks per SM the register budget is set for (2: up to 128
-// registers, the cost model without spills and half the barrier arrivals,
-// for small and mid-size queries whose levels are latency-bound; 3: 80
-// registers; 4: 64 registers, more warps to hide latency on large levels);
-// chosen per query from its connected sets per level, the total over the
-// relation count (Tuning::single_narrow_level_sets,
-// Tuning::single_wide_level_sets)
-// MASKED: every class of the query is a two-member class on a tree edge
-// (DevHeader::ec_masked), a separate kernel so that each carries only the
-// evaluation paths its queries take
-template <int MINB, bool MASKED>
+// Connected sets and lanes per set of every level, known on the host before
+// the launch (a tree's connected subtrees are counted by size without listing
+// them, tree_level_counts)
+struct TreePlan {
+    uint32_t count[33];
+    uint8_t group[33];
+};
+
+// Bound: a warp-step (one split, both orientations) issues about 240
+// instructions on a plain tree; wide levels are issue-bound, narrow ones wait
+// for the chain list entry -> two memo entries -> cost -> reduction -> memo
+// entry -> grid barrier.  With the child end of a split read from the root's
+// row, the sums over an edge's classes made on the host (TreeEdge), the
+// enumeration index left to ties and the extensions of a set as one mask:
+// star-22 (44.0 M pairs) 751 -> 491 us, snowflake-25 (3.2 M and 4.8 M pairs)
+// 265 / 290 -> 169 / 168 us, key chain-30 203 -> 150 us on the device.
+// MINB: blocks per SM the register budget is set for (2, 3 or 4: 128, 80 or 64
+// registers, no spill but 4 bytes with 4 blocks), chosen per query from its
+// connected sets per level, the total over the relation count
+// (Tuning::single_narrow_level_sets, Tuning::single_wide_level_sets); LAYOUT:
+// the evaluation (tree_layout)
+template <int MINB, int LAYOUT>
 __global__ void __launch_bounds__(kBlock, MINB) k_dp_tree(const uint32_t *__restrict__ blob, uint32_t blob_words,
-                                                       const uint32_t *__restrict__ binom_g, float4 *__restrict__ memo,
+                                                       float4 *__restrict__ memo,
                                                        uint32_t *__restrict__ memo_left, uint32_t *__restrict__ setsA,
                                                        uint32_t *__restrict__ setsB, LevelCounters *__restrict__ lvl,
                                                        GlobalCounters *__restrict__ glob, TreeNode *__restrict__ tree,
                                                        int *__restrict__ tree_n, unsigned *__restrict__ bar,
-                                                       uint32_t target_lanes, unsigned poll_limit) {
+                                                       const __grid_constant__ TreePlan plan, unsigned poll_limit) {
     extern __shared__ __align__(16) uint32_t sm[];
-    const uint32_t bw = (blob_words + 3u) & ~3u;
     const unsigned max_polls = barrier_polls(poll_limit);
-    uint32_t *binom = sm + bw;
-    uint32_t *stage = binom + 33 * 33 + 3;   // 16-byte aligned (bw, 1092 words)
-    for (uint32_t i = threadIdx.x; i < blob_words; i += blockDim.x) sm[i] = blob[i];
-    for (uint32_t i = threadIdx.x; i < 33 * 33; i += blockDim.x) binom[i] = binom_g[i];
-    __syncthreads();
+    load_blob_to_smem(blob, blob_words, sm);
     const DevInfoView d = make_view(sm);
     const int n = d.h->n;
     const uint32_t *adj = d.h->adj;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint32_t *st = stage + warp * 64;
-    const uint32_t gwarp = blockIdx.x * kWarpsPerBlock + warp;
+    const uint32_t gwarp = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
     const uint32_t nwarps = gridDim.x * kWarpsPerBlock;
-    unsigned long long pairs = 0;
+    const PlainParams pp = plain_params(*d.h);
     unsigned epoch = 0;   // grid barriers passed (thread 0)
-    // the pipelined candidate loop needs the registers of the 2- and 3-blocks
-    // variants; at 64 registers it spills and the 4-blocks variant keeps the
-    // plain loop
-    constexpr bool kPipe = MINB < 4;
 
     // phase 0: base relations (gpuqo_cpu_sequential.cu:80-92) and level-2 sets
     if (blockIdx.x == 0 && threadIdx.x < n) {
@@ -1241,34 +1255,23 @@ __global__ void __launch_bounds__(kBlock, MINB) k_dp_tree(const uint32_t *__rest
         memo[1u << i] = base_entry(*d.h, i);
         memo_left[1u << i] = 0u;
     }
-    if (n >= 2) level_sets_phase(adj, binom, st, n, 2, nullptr, (uint32_t)n, setsA, lvl + 2);
+    if (n >= 2) tree_enum_phase(adj, 2, nullptr, (uint32_t)n, setsA, lvl + 2);
     if (!grid_barrier<true>(bar, epoch, max_polls)) return;
     for (int k = 2; k <= n; k++) {
         uint32_t *cur = (k & 1) ? setsB : setsA;
         uint32_t *nxt = (k & 1) ? setsA : setsB;
-        const uint32_t count = __ldcg(&lvl[k].n_sets);
-        if (k < n) level_sets_phase(adj, binom, st, n, k + 1, cur, count, nxt, lvl + k + 1);
-        // lanes take whole split edges (tree_groups): k - 1 per set
-        int max_group = 1;
-        while (max_group < 32 && max_group < k - 1) max_group <<= 1;
-        int G = 2;
-        while (G < max_group && (uint64_t)count * (uint64_t)G < (uint64_t)target_lanes) G <<= 1;
-        G = G <= 2 ? 2 : (G <= 8 ? 8 : 32);
-        if (G == 2) {
-            tree_groups<2, MASKED, kPipe>(d, gwarp * 16, nwarps * 16, cur, count, k, memo, memo_left, pairs);
-        } else if (G == 8) {
-            tree_groups<8, MASKED, kPipe>(d, gwarp * 4, nwarps * 4, cur, count, k, memo, memo_left, pairs);
-        } else {
-            tree_groups<32, MASKED, kPipe>(d, gwarp, nwarps, cur, count, k, memo, memo_left, pairs);
-        }
+        const uint32_t count = plan.count[k];
+        if (k < n) tree_enum_phase(adj, k + 1, cur, count, nxt, lvl + k + 1);
+        tree_level<LAYOUT>(d, pp, gwarp, nwarps, cur, count, k, plan.group[k], memo, memo_left);
         if (!grid_barrier<true>(bar, epoch, max_polls)) return;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         const uint32_t full = (n == 32) ? 0xFFFFFFFFu : ((1u << n) - 1u);
         extract_plan(memo, memo_left, full, d.h->hz_packed ? kWidthMask : 0xFFFFFFFFu, tree, tree_n);
+        unsigned long long pairs = 0;   // every split edge, both orientations
+        for (int k = 2; k <= n; k++) pairs += (unsigned long long)plan.count[k] * 2ull * (unsigned long long)(k - 1);
+        glob->evaluated_pairs = pairs;
     }
-    pairs = __reduce_add_sync(kFull, (uint32_t)pairs);
-    if (lane == 0 && pairs) atomicAdd(&glob->evaluated_pairs, pairs);
 }
 
 // ---------------------------------------------------------------------------
@@ -1707,6 +1710,10 @@ struct GraphKey {
 struct Tuning {
     // tree queries with up to this many connected sets per level run
     // k_dp_tree<2>, those with more than single_wide_level_sets k_dp_tree<4>
+    // (device time of the 2- / 3- / 4-blocks variant: star-18, 7 k sets per
+    // level, 121 / 126 / 135 us; star-20, 26 k, 205 / 194 / 203; star-21, 50 k,
+    // 329 / 299 / 312; star-22, 95 k, 522 / 491 / 476; star-24, 350 k,
+    // 2009 / 1745 / 1632; the third crossover is left to the autotuner)
     double single_narrow_level_sets = 16384.0;
     double single_wide_level_sets = 1e30;
     double batch_single_sets = double(1u << 20);   // a batch hands larger tree queries to k_dp_tree
@@ -1716,6 +1723,51 @@ constexpr int kMaxDevices = 64;
 static Tuning g_tuning[kMaxDevices];            // per device, guarded by g_dev_mu
 
 static double tree_connected_sets(const DevHeader *h);
+
+// Connected sets of a tree-shaped query graph by size (count[k], k = 1..n; at
+// most C(30, 15) each): with g_v(x) counting the connected sets whose relation
+// nearest to relation 0 is v, g_v = x * prod over v's children c of
+// (1 + g_c), O(n^2) steps in all.  Returns their total.
+static double tree_level_counts(const DevHeader *h, uint32_t (&count)[33]) {
+    const int n = h->n;
+    int order[32], parent[32], size[32], m = 0;
+    uint32_t g[32][33];
+    uint32_t seen = 1u;
+    order[m++] = 0;
+    parent[0] = -1;
+    for (int i = 0; i < m; i++) {
+        uint32_t nb = h->adj[order[i]] & ~seen;
+        seen |= nb;
+        for (; nb; nb &= nb - 1u) {
+            const int c = __builtin_ctz(nb);
+            parent[c] = order[i];
+            order[m++] = c;
+        }
+    }
+    for (int v = 0; v < n; v++) {
+        size[v] = 1;
+        g[v][0] = 0u;
+        g[v][1] = 1u;
+    }
+    for (int k = 0; k <= 32; k++) count[k] = 0u;
+    double total = 0.0;
+    for (int i = m - 1; i >= 0; i--) {
+        const int v = order[i], p = parent[v];
+        for (int k = 1; k <= size[v]; k++) {
+            count[k] += g[v][k];
+            total += (double)g[v][k];
+        }
+        if (p < 0) continue;
+        uint32_t nx[33] = {};
+        for (int a = 1; a <= size[p]; a++) {
+            nx[a] += g[p][a];
+            for (int b = 1; b <= size[v]; b++) nx[a + b] += g[p][a] * g[v][b];
+        }
+        size[p] += size[v];
+        for (int k = 1; k <= size[p]; k++) g[p][k] = nx[k];
+    }
+    return total;
+}
 
 // cpu_dpsize's level-1 list (gpuqo_cpu_dpsize.cu:43-48 after
 // gpuqo_cpu_sequential.cu:73-84): the iteration order of its unordered_map
@@ -1968,11 +2020,8 @@ public:
                 const uint32_t target_lanes = (uint32_t)sm_count * 24u * 32u;
                 int mblocks = (int)std::min<uint64_t>((uint64_t)sm_count * 4, (total * 32 + kBlock - 1) / kBlock);
                 if (tree_mode) {
-                    // the tree kernel's lanes take split edges: k - 1 per set
-                    int max_edge_group = 1;
-                    while (max_edge_group < 32 && max_edge_group < k - 1) max_edge_group <<= 1;
                     k_eval_tree<<<mblocks, kBlock, smem, stream>>>(a.blob, blob_words, k, cur_sets, lc, a.memo,
-                                                                   a.memo_left, a.glob, target_lanes, max_edge_group);
+                                                                   a.memo_left, a.glob);
                 } else {
                     k_eval_mpdp<<<mblocks, kBlock, smem, stream>>>(a.blob, blob_words, cur_sets, lc, a.memo,
                                                                    a.memo_left, a.ovf_set, a.ovf_P, a.ovf_off,
@@ -2024,22 +2073,26 @@ public:
     // 0 and sets launched when the kernel was started.
     int launch_persistent(int n, uint32_t words, bool &launched, std::string &err) {
         launched = false;
-        const size_t smem = (size_t)(((words + 3u) & ~3u) + 33 * 33 + 3 + kWarpsPerBlock * 64) * 4u;
+        const size_t smem = (size_t)((words + 3u) & ~3u) * 4u;
         if (coop_off) return 0;
+        const DevHeader *h = reinterpret_cast<const DevHeader *>(h_blob);
+        TreePlan plan;
+        const double sets = tree_level_counts(h, plan.count);
         int minb = force_minb;
         if (minb == 0) {
-            const double per_level = tree_connected_sets(reinterpret_cast<const DevHeader *>(h_blob)) / n;
+            const double per_level = sets / n;
             const Tuning &tu = g_tuning[device];
             minb = per_level <= tu.single_narrow_level_sets ? 2 : (per_level > tu.single_wide_level_sets ? 4 : 3);
         }
-        const bool masked = reinterpret_cast<const DevHeader *>(h_blob)->ec_masked != 0u;
-        const void *fn = masked ? (minb == 4   ? (const void *)k_dp_tree<4, true>
-                                   : minb == 2 ? (const void *)k_dp_tree<2, true>
-                                               : (const void *)k_dp_tree<3, true>)
-                                : (minb == 4   ? (const void *)k_dp_tree<4, false>
-                                   : minb == 2 ? (const void *)k_dp_tree<2, false>
-                                               : (const void *)k_dp_tree<3, false>);
-        const size_t key = smem * 16u + (size_t)minb * 2u + (masked ? 1u : 0u);
+        const int layout = tree_layout(*h);
+        static const void *const variants[3][3] = {
+            {(const void *)k_dp_tree<2, 0>, (const void *)k_dp_tree<2, 1>, (const void *)k_dp_tree<2, 2>},
+            {(const void *)k_dp_tree<3, 0>, (const void *)k_dp_tree<3, 1>, (const void *)k_dp_tree<3, 2>},
+            // at 64 registers the class passes spill about 100 bytes and lose to
+            // 3 blocks at every size (star-22 with statistics 1094 against 1084 us)
+            {(const void *)k_dp_tree<3, 0>, (const void *)k_dp_tree<3, 1>, (const void *)k_dp_tree<4, 2>}};
+        const void *fn = variants[minb - 2][layout];
+        const size_t key = smem * 16u + (size_t)minb * 3u + (size_t)layout;
         auto cb = coop_blocks.find(key);
         if (cb == coop_blocks.end()) {
             int blocks = 0, dev_coop = 0, occ = 0;
@@ -2056,14 +2109,11 @@ public:
         if (grid <= 0) return 0;
         CK(cudaMemsetAsync(d_ctl, 0, kCtlClearBytes, stream));   // counters, barrier words, tree size
         uint32_t bwords = words;
-        // group width per level: count x G covers half the resident threads
-        // (measured: narrower groups, more sets in flight, shorten the levels
-        // of 20- to 25-relation trees by about 8 %; a quarter or an eighth is
-        // slower again)
-        uint32_t target_lanes = (uint32_t)grid * (uint32_t)kBlock / 2u;
+        for (int k = 2; k <= n; k++)
+            plan.group[k] = (uint8_t)tree_group(plan.count[k], k, (uint32_t)grid * kBlock, (uint32_t)sm_count);
         unsigned poll_limit = (unsigned)std::max(0, gpuqo_b200_barrier_poll_limit);
-        void *args[] = {&a.blob, &bwords, &a.binom, &a.memo, &a.memo_left, &a.sets, &a.sets2,
-                        &a.lvl, &a.glob, &a.tree, &a.tree_n, &a.bar, &target_lanes, &poll_limit};
+        void *args[] = {&a.blob, &bwords, &a.memo, &a.memo_left, &a.sets, &a.sets2,
+                        &a.lvl, &a.glob, &a.tree, &a.tree_n, &a.bar, &plan, &poll_limit};
         cudaError_t e = cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kBlock), args, smem, stream);
         if (e != cudaSuccess) {
             cudaGetLastError();
@@ -2501,6 +2551,7 @@ static int noalloc_blob(const GpuqoPlannerInfoC *c, uint32_t *blob, uint32_t &wo
     h->seq_page_cost = (float)seq_page_cost;
     h->disable_cost = (float)disable_cost;
     h->work_mem = work_mem;
+    h->work_mem_bytes = work_mem_bytes_of(work_mem);
     h->enable_nestloop = enable_nestloop ? 1 : 0;
     h->enable_hashjoin = enable_hashjoin ? 1 : 0;
     h->composite_mask = 0;
@@ -2800,7 +2851,7 @@ __device__ __forceinline__ void stage_flush64(unsigned long long *st, uint32_t &
 // connected k-sets of every query, by extension of its (k-1)-sets (c_prev
 // items in prev); thread tid of nthreads.  TREE_ONLY (every query of the wave
 // tree-shaped): each set is emitted once by the largest-leaf rule of
-// level_sets_phase, without the dedup bitmap.
+// tree_enum_phase, without the dedup bitmap.
 template <bool TREE_ONLY>
 __device__ __forceinline__ void batch_extend(const BatchQ *qs, const uint32_t *blobs, const unsigned long long *prev,
                                              uint32_t c_prev, uint32_t *seen, unsigned long long *out,
@@ -2868,27 +2919,16 @@ __global__ void __launch_bounds__(kBlock) kb_level_sets(const BatchQ *__restrict
                  blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
 }
 
-// candidate c of a tree-shaped query (see k_eval_tree): edge {a, b}, a < b
-__device__ __forceinline__ void tree_cand(const DevHeader &h, uint32_t S, int a, int b, uint32_t c, uint32_t &L,
+// candidate c of a tree-shaped query: orientation c & 1 of the split at child
+// end v
+__device__ __forceinline__ void tree_cand(const DevHeader &h, uint32_t S, uint32_t v, uint32_t c, uint32_t &L,
                                           uint32_t &R, uint32_t &p, uint32_t &ecm, bool masked) {
-    const uint32_t *tab = reinterpret_cast<const uint32_t *>(&h) + h.tree_tab;
-    const int n = h.n, nn = n * n;
-    const int rt = __ffs(S) - 1;
-    const uint32_t *anc_r = tab + 2 * nn + rt * n;
-    const int ch = ((__ldg(anc_r + b) >> a) & 1u) ? b : a;
-    const uint32_t comp_c = S & __ldg(tab + rt * n + ch);
-    const uint32_t comp_a = (ch == a) ? comp_c : (S ^ comp_c);
-    const uint32_t side = c & 1u;
-    L = side ? (S ^ comp_a) : comp_a;
+    const TreeRows t = tree_rows(h, S);
+    const uint32_t code = v | ((c & 1u) ? kSideHigher : 0u);
+    L = tree_side(t, S, code);
     R = S ^ L;
-    const uint32_t post =
-        (uint32_t)(__popc(S & __ldg(tab + nn + rt * n + ch)) - __popc(S & __ldg(anc_r + ch)) + __popc(comp_c) - 1);
-    p = h.index_order ? dpsub_index(L, S) : 2u * post + side;
-    ecm = 0u;
-    if (masked) {
-        const int ch0 = ((__ldg(tab + 2 * nn + b) >> a) & 1u) ? b : a;
-        ecm = h.edge_ec[ch0];
-    }
+    p = tree_index(t.row, t.n, S, code, h.index_order);
+    ecm = masked ? reinterpret_cast<const TreeEdge *>(t.tab + tree_edge_off(t.n))[t.row[2u * v + 1u] & 31u].classes : 0u;
 }
 
 // ALL_MASKED (with TREE_ONLY): every query of the wave has only two-member
@@ -2950,12 +2990,8 @@ __device__ __forceinline__ void batch_groups(const BatchQ *qs, const uint32_t *b
         const uint32_t iters = __reduce_max_sync(kFull, (P + G - 1u) / G);
         LaneBest best;
         best.init();
-        EdgeIter ei;
-        ei.vs = S;
-        ei.nb = 0u;
-        ei.v = 0;
-        ei.e = 0u;
-        int ea = 0, eb = 0, bcur = 0;
+        uint32_t ends = S & (S - 1u), end_rank = 0u;   // child ends not passed yet, rank of the lowest
+        int bcur = 0;
         for (uint32_t j = 0; j < iters; j++) {
             const uint32_t c = (uint32_t)gl + j * G;
             const bool active = has && c < P;
@@ -2963,8 +2999,8 @@ __device__ __forceinline__ void batch_groups(const BatchQ *qs, const uint32_t *b
             bool valid = false;
             if (active) {
                 if (tree) {
-                    while (ei.e <= (c >> 1)) edge_next(h.adj, S, ei, ea, eb);
-                    tree_cand(h, S, ea, eb, c, L, R, p, ecm, masked);
+                    for (; end_rank < (c >> 1); end_rank++) ends &= ends - 1u;
+                    tree_cand(h, S, (uint32_t)lowest_idx(ends), c, L, R, p, ecm, masked);
                     valid = true;
                 } else if (!TREE_ONLY) {
                     uint32_t key;
@@ -2991,7 +3027,7 @@ __device__ __forceinline__ void batch_groups(const BatchQ *qs, const uint32_t *b
             }
             if (of < fp) fp = of;
         }
-        const bool nan_first = has && best.first_p == fp && best.first_nan;
+        const bool nan_first = has && best.first_p == fp && best.first_nan();
         const unsigned nm = __ballot_sync(kFull, nan_first) & group_mask;
         const unsigned long long gkey = ((unsigned long long)kh << 32) | kl;
         if (has) {

@@ -108,18 +108,52 @@ struct DevHeader {
     // every class has exactly two members (DevInfoView::pair_sel then holds
     // the selectivity of every class in both orientations)
     uint32_t all_pairs;
-    uint32_t pad_[3];
+    float work_mem_bytes;                 // (float)(work_mem * 1024) (see work_mem_bytes_of)
+    // ec_masked, hz_packed, hash joins enabled, every class plain
+    // (DevInfoView::plain) and a row of the widest set within work_mem: the
+    // cost of a split is straight-line arithmetic on TreeEdge (plain_mirror)
+    uint32_t tree_plain;
+    uint32_t pad_;
 };
 
-// Tree tables (tree_mode), appended after the class arrays: for every root r
-// of the query tree and relation v, with children visited in increasing
-// index order,
-//   tab[0*n*n + r*n + v] = relations of v's subtree,
-//   tab[1*n*n + r*n + v] = relations preceding v in preorder,
-//   tab[2*n*n + r*n + v] = proper ancestors of v.
+// the work_mem of the hash join's skew check, as the reference compares it
+inline float work_mem_bytes_of(int work_mem) { return (float)((long long)work_mem * 1024LL); }
+
+// Tree tables (tree_mode), appended after the class arrays at word tree_tab.
+// Word r of the first 32 is the word offset of root r's rows from tree_tab
+// (0: r is never the lowest relation of a connected set of two or more).
+// Then n TreeEdge records, one per relation v: the edge between v and its
+// parent in the tree rooted at relation 0.  Then, per root r with rows, with
+// children visited in increasing index order,
+//   uint2 [n]: .x = relations of v's subtree in the tree rooted at r
+//              .y = the record of v's edge to its parent there | kTreeLower
+//                   when v has the lower number of the two
+//   uint2 [n]: .x = relations preceding v in preorder, .y = v's proper ancestors
 // A connected set S is a subtree; the reference's block search walks it from
-// its lowest relation r in exactly this preorder.
-GQB_HD inline uint32_t tree_tab_words(int n) { return 3u * (uint32_t)n * (uint32_t)n; }
+// its lowest relation r in exactly this preorder.  Every relation of S but r
+// is the child end of one split edge, so the first rows give every split with
+// one 8-byte load; the second rows serve the enumeration index, which only
+// equal costs and NaN costs ask for.
+struct TreeEdge {
+    // the classes on the edge, accumulated in class order (exactly the
+    // device's float operations): the selectivity product with the lower end's
+    // side outer and with the higher end's, the per-tuple cost of the quals,
+    // cpu_operator_cost * quals, and the two sums with cpu_tuple_cost that the
+    // nested loop and the hash join start from
+    float sel_lo, sel_hi, per_tuple, quals_cost, nl_tuple, hj_row;
+    uint32_t classes;                     // class mask (DevHeader::ec_masked)
+    uint32_t pad;
+};
+static_assert(sizeof(TreeEdge) == 32, "TreeEdge layout");
+constexpr uint32_t kTreeLower = 32u;
+
+// the two orientations of a split edge, numbered by its child end
+// (TreeBest::code): bit 5 set = the higher end's side is the outer one
+constexpr uint32_t kSideHigher = 32u;
+
+GQB_HD inline uint32_t tree_edge_off(int) { return 32u; }
+GQB_HD inline uint32_t tree_rows_off(int n) { return 32u + 8u * (uint32_t)n; }
+GQB_HD inline uint32_t tree_row_words(int n) { return 4u * (uint32_t)n; }
 
 struct DevInfoView {
     const DevHeader *h;

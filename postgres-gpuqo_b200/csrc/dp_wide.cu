@@ -1255,6 +1255,7 @@ int engine_run_wide(const HostInfo &info, DpMode mode, std::vector<TreeNode> &no
     hw.h.seq_page_cost = info.p.seq_page_cost;
     hw.h.disable_cost = info.p.disable_cost;
     hw.h.work_mem = info.p.work_mem;
+    hw.h.work_mem_bytes = work_mem_bytes_of(info.p.work_mem);
     hw.h.enable_nestloop = info.p.enable_nestloop ? 1 : 0;
     hw.h.enable_hashjoin = info.p.enable_hashjoin ? 1 : 0;
     long long width_sum = 0;

@@ -365,7 +365,17 @@ std::vector<uint32_t> build_blob(const HostInfo &info) {
         tree = (seen == (n == 64 ? ~0ull : (bit64(n) - 1)));
     }
     const uint32_t base_words = blob_words_for(n, n_ec, n_sels, n_fks);
-    std::vector<uint32_t> blob(base_words + (tree ? tree_tab_words(n) : 0u), 0u);
+    // The kernels read the rows of root r only for sets whose lowest relation
+    // is r (and row 0 for the edge records): a relation without a
+    // higher-numbered neighbour is never the lowest of a connected set of two
+    // or more, and has none.
+    uint32_t tree_words = 0u;
+    if (tree) {
+        tree_words = tree_rows_off(n);
+        for (int r = 0; r < n; r++)
+            if (r == 0 || ((info.edge[r] >> 1) >> r) > 1ull) tree_words += tree_row_words(n);
+    }
+    std::vector<uint32_t> blob(base_words + tree_words, 0u);
     DevHeader *h = reinterpret_cast<DevHeader *>(blob.data());
     h->n = n;
     h->n_ec = n_ec;
@@ -376,6 +386,7 @@ std::vector<uint32_t> build_blob(const HostInfo &info) {
     h->seq_page_cost = info.p.seq_page_cost;
     h->disable_cost = info.p.disable_cost;
     h->work_mem = info.p.work_mem;
+    h->work_mem_bytes = work_mem_bytes_of(info.p.work_mem);
     h->enable_nestloop = info.p.enable_nestloop ? 1 : 0;
     h->enable_hashjoin = info.p.enable_hashjoin ? 1 : 0;
     h->composite_mask = 0;
@@ -405,14 +416,11 @@ std::vector<uint32_t> build_blob(const HostInfo &info) {
     if (tree) {
         h->tree_tab = base_words;
         uint32_t *tab = blob.data() + base_words;
-        const int nn = n * n;
         uint32_t adj[32];
+        uint32_t row = tree_rows_off(n);
         for (int v = 0; v < n; v++) adj[v] = h->adj[v];
+        uint32_t anc0[32];
         for (int r = 0; r < n; r++) {
-            // The kernels read the rows of root r only for sets whose lowest
-            // relation is r (and row 0 for the classes on edges): a relation
-            // without a higher-numbered neighbour is never the lowest of a
-            // connected set of two or more, and its rows stay zero.
             if (r > 0 && (adj[r] >> r) <= 1u) continue;
             // preorder from r, children in increasing index order (pushed from
             // the highest index, so the lowest is visited first); n <= 32, so
@@ -439,11 +447,23 @@ std::vector<uint32_t> build_blob(const HostInfo &info) {
                     stack[sp++] = c;
                 }
             }
+            if (r == 0) std::memcpy(anc0, anc, sizeof(anc0));
             for (int v = 0; v < n; v++) sub[v] = 1u << v;
             for (int i = no - 1; i > 0; i--) sub[__builtin_ctz(par_bit[order[i]])] |= sub[order[i]];
-            std::memcpy(tab + r * n, sub, (size_t)n * 4u);
-            std::memcpy(tab + nn + r * n, before_of, (size_t)n * 4u);
-            std::memcpy(tab + 2 * nn + r * n, anc, (size_t)n * 4u);
+            tab[r] = row;
+            uint32_t *split = tab + row, *index = split + 2 * n;
+            for (int v = 0; v < n; v++) {
+                uint32_t meta = 0u;
+                if (v != r) {
+                    const int par = __builtin_ctz(par_bit[v]);
+                    meta = (uint32_t)(((anc0[v] >> par) & 1u) ? v : par) | (v < par ? kTreeLower : 0u);
+                }
+                split[2 * v] = sub[v];
+                split[2 * v + 1] = meta;
+                index[2 * v] = before_of[v];
+                index[2 * v + 1] = anc[v];
+            }
+            row += tree_row_words(n);
         }
         // classes on edges: every 2-member class must sit on an edge
         bool masked = n_ec <= 32;
@@ -458,7 +478,7 @@ std::vector<uint32_t> build_blob(const HostInfo &info) {
                 masked = false;   // a class between relations that are not adjacent
                 break;
             }
-            int child0 = ((tab[2 * nn + 0 * n + b] >> a) & 1u) ? b : a;
+            int child0 = ((anc0[b] >> a) & 1u) ? b : a;
             h->edge_ec[child0] |= 1u << e;
         }
         if (masked) h->ec_masked = 1u;
@@ -510,6 +530,32 @@ std::vector<uint32_t> build_blob(const HostInfo &info) {
             h->edge_sel[0][i] = fk_xy ? h->fksel[y] : (fk_yx ? h->fksel[x] : s);
             h->edge_sel[1][i] = fk_yx ? h->fksel[x] : (fk_xy ? h->fksel[y] : s);
         }
+        TreeEdge *edges = reinterpret_cast<TreeEdge *>(blob.data() + h->tree_tab + tree_edge_off(n));
+        bool plain = true;
+        for (int c = 1; c < n; c++) {
+            TreeEdge &e = edges[c];
+            e.classes = h->edge_ec[c];
+            e.sel_lo = e.sel_hi = 1.0f;
+            e.per_tuple = 0.0f;
+            int quals = 0;
+            for (uint32_t m = e.classes; m; m &= m - 1u, quals++) {
+                const int i = __builtin_ctz(m);
+                e.sel_lo *= h->edge_sel[0][i];
+                e.sel_hi *= h->edge_sel[1][i];
+                e.per_tuple += h->cpu_operator_cost;
+                plain = plain && ((v.plain[0] >> i) & 1u);
+            }
+            // an edge without a class joins without quals: bucket size and MCV
+            // frequency stay 1, which the general pass computes
+            plain = plain && quals > 0;
+            e.quals_cost = h->cpu_operator_cost * (float)quals;
+            e.nl_tuple = h->cpu_tuple_cost + e.per_tuple;
+            e.hj_row = e.quals_cost + h->cpu_tuple_cost;
+        }
+        // the skew check of a plain split compares one row of the inner side
+        // with work_mem; the widest set's row decides for all
+        const float widest = (float)((((unsigned long long)std::max(width_sum, 0ll) + 7ull) & ~7ull) + 24ull);
+        h->tree_plain = (plain && h->hz_packed && h->enable_hashjoin && widest <= h->work_mem_bytes) ? 1u : 0u;
     }
     return blob;
 }
