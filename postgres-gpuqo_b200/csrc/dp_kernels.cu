@@ -47,6 +47,7 @@
 
 #include "dp_device.cuh"
 #include "dp_engine.h"
+#include "dp_general.cuh"
 #include "gpuqo_b200.h"
 
 extern "C" int gpuqo_b200_persistent;
@@ -1165,48 +1166,47 @@ __device__ __forceinline__ void tree_enum_phase(const uint32_t *adj, int k, cons
     }
 }
 
+// The plan, walked from the full set by one warp, level by level of the join
+// tree: a lane per node reads its memo entry and outer side (about 0.35 us
+// from L2), so the walk costs the plan's depth instead of its 2n - 1 nodes.
+// Node 0 is the root; sets: 64 words of shared memory.
 __device__ __forceinline__ void extract_plan(const float4 *memo, const uint32_t *memo_left, uint32_t full,
-                                             uint32_t wmask, TreeNode *out, int *n_out) {
-    int n = 0;
-    uint32_t stack_set[64];
-    int stack_parent[64], stack_side[64];
-    int sp = 0;
-    stack_set[sp] = full;
-    stack_parent[sp] = -1;
-    stack_side[sp] = 0;
-    sp++;
-    while (sp > 0 && n < 64) {
-        sp--;
-        const uint32_t s = stack_set[sp];
-        const int parent = stack_parent[sp], side = stack_side[sp];
-        const float4 v = __ldcg(memo + s);
+                                             uint32_t wmask, uint32_t *sets, TreeNode *out, int *n_out) {
+    const uint32_t lane = threadIdx.x & 31u;
+    if (lane == 0u) sets[0] = full;
+    __syncwarp();
+    uint32_t head = 0u, tail = 1u;
+    while (head < tail) {
+        const uint32_t me = head + lane;
+        const bool has = me < tail;
+        const uint32_t s = has ? sets[me] : 0u;
         TreeNode t;
         t.set = s;
-        t.left = -1;
-        t.right = -1;
-        t.rows = v.x;
-        t.startup = v.y;
-        t.total = v.z;
-        t.width = (int)(__float_as_uint(v.w) & wmask);
-        const int me = n++;
-        out[me] = t;
-        if (parent >= 0) {
-            if (side == 0) out[parent].left = me;
-            else out[parent].right = me;
+        t.left = t.right = -1;
+        uint32_t l = 0u;
+        if (has) {
+            const float4 v = __ldcg(memo + s);
+            l = __ldcg(memo_left + s) & s;
+            t.rows = v.x;
+            t.startup = v.y;
+            t.total = v.z;
+            t.width = (int)(__float_as_uint(v.w) & wmask);
         }
-        const uint32_t l = __ldcg(memo_left + s) & s;
-        if (__popc(s) > 1 && l != 0u && l != s && sp + 2 <= 64) {
-            stack_set[sp] = s ^ l;
-            stack_parent[sp] = me;
-            stack_side[sp] = 1;
-            sp++;
-            stack_set[sp] = l;
-            stack_parent[sp] = me;
-            stack_side[sp] = 0;
-            sp++;
+        const bool join = has && popc(s) > 1 && l != 0u && l != s;
+        const uint32_t joins = __ballot_sync(kFull, join);
+        const uint32_t child = tail + 2u * (uint32_t)popc(joins & ((1u << lane) - 1u));
+        if (join && child + 1u < 64u) {
+            t.left = (int)child;
+            t.right = (int)child + 1;
+            sets[child] = l;
+            sets[child + 1u] = s ^ l;
         }
+        if (has) out[me] = t;
+        head = min(tail, head + 32u);
+        tail = min(tail + 2u * (uint32_t)popc(joins), 64u);
+        __syncwarp();
     }
-    *n_out = n;
+    if (lane == 0u) *n_out = (int)tail;
 }
 
 // Connected sets and lanes per set of every level, known on the host before
@@ -1265,12 +1265,15 @@ __global__ void __launch_bounds__(kBlock, MINB) k_dp_tree(const uint32_t *__rest
         tree_level<LAYOUT>(d, pp, gwarp, nwarps, cur, count, k, plan.group[k], memo, memo_left);
         if (!grid_barrier<true>(bar, epoch, max_polls)) return;
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
+    if (blockIdx.x == 0 && threadIdx.x < 32) {
+        __shared__ uint32_t plan_sets[64];
         const uint32_t full = (n == 32) ? 0xFFFFFFFFu : ((1u << n) - 1u);
-        extract_plan(memo, memo_left, full, d.h->hz_packed ? kWidthMask : 0xFFFFFFFFu, tree, tree_n);
-        unsigned long long pairs = 0;   // every split edge, both orientations
-        for (int k = 2; k <= n; k++) pairs += (unsigned long long)plan.count[k] * 2ull * (unsigned long long)(k - 1);
-        glob->evaluated_pairs = pairs;
+        extract_plan(memo, memo_left, full, d.h->hz_packed ? kWidthMask : 0xFFFFFFFFu, plan_sets, tree, tree_n);
+        if (threadIdx.x == 0) {
+            unsigned long long pairs = 0;   // every split edge, both orientations
+            for (int k = 2; k <= n; k++) pairs += (unsigned long long)plan.count[k] * 2ull * (unsigned long long)(k - 1);
+            glob->evaluated_pairs = pairs;
+        }
     }
 }
 
@@ -2784,16 +2787,18 @@ struct BatchQ {
     unsigned long long seen_off;       // word offset into the dedup bitmap arena
 };
 
-// Sets of a level whose candidate count exceeds kOvfLimit (large biconnected
-// blocks: the full set of a cycle, dense sub-graphs), evaluated after the
-// level by every warp in chunks of kChunk candidates (kb_dp only).
+// Sets of a level with more splits than their warp takes alone (kb_gen): all
+// their splits are dealt out evenly over the grid after the level, in units
+// of `unit` splits.  A set that finds the list full is evaluated by its warp.
 struct BatchOvf {
     unsigned long long *item;          // [cap] query << 32 | set
-    uint32_t *P;                       // [cap] candidate count
-    uint32_t *off;                     // [cap] first chunk id (increases with the index)
-    unsigned long long *key;           // [cap] min (cost bits << 32 | candidate index) over chunks
-    unsigned long long *first;         // [cap] min (first valid candidate << 1 | its cost is NaN)
-    uint32_t cap;                      // 0: no overflow list (sets are evaluated by their group)
+    uint32_t *W;                       // [cap] unordered splits
+    uint32_t *off;                     // [cap] first unit (increases with the index)
+    unsigned long long *key;           // [cap] min (cost bits << 32 | candidate index) over the units
+    uint32_t *nan_p;                   // [cap] lowest index of a NaN candidate
+    uint32_t *done;                    // [cap] units finished
+    uint32_t cap;
+    uint32_t unit;
 };
 
 __global__ void kb_init(const BatchQ *__restrict__ qs, int nq, const uint32_t *__restrict__ blobs,
@@ -2937,8 +2942,7 @@ __device__ __forceinline__ void tree_cand(const DevHeader &h, uint32_t S, uint32
 template <int G, bool TREE_ONLY, bool ALL_MASKED = false>
 __device__ __forceinline__ void batch_groups(const BatchQ *qs, const uint32_t *blobs, uint32_t first, uint32_t stride,
                                              const unsigned long long *items, uint32_t count, int k, float4 *memo_all,
-                                             uint32_t *memo_left_all, unsigned long long &pairs,
-                                             const BatchOvf &ovf, LevelCounters *lc) {
+                                             uint32_t *memo_left_all, unsigned long long &pairs) {
     const int lane = threadIdx.x & 31;
     const int grp = lane / G, gl = lane % G;
     const uint32_t group_mask = (G == 32) ? kFull : (((1u << G) - 1u) << (grp * G));
@@ -2967,23 +2971,6 @@ __device__ __forceinline__ void batch_groups(const BatchQ *qs, const uint32_t *b
             } else if (!TREE_ONLY) {
                 find_blocks(S, h.adj, B);
                 P = B.etotal;
-                if (ovf.cap != 0u && P > kOvfLimit) {
-                    // to the level's overflow list; one packed atomic assigns the
-                    // list index and the first chunk id in the same order
-                    if (gl == 0) {
-                        const uint32_t nch = (P + kChunk - 1u) / kChunk;
-                        const unsigned long long old = atomicAdd(&lc->ovf_packed, (1ull << 40) | nch);
-                        const uint32_t idx = (uint32_t)(old >> 40);
-                        if (idx < ovf.cap) {
-                            ovf.item[idx] = it;
-                            ovf.P[idx] = P;
-                            ovf.off[idx] = (uint32_t)(old & 0xFFFFFFFFFFull);
-                            ovf.key[idx] = ~0ull;
-                            ovf.first[idx] = ~0ull;
-                        }
-                    }
-                    P = 0u;   // no candidate here, no memo write
-                }
             }
         }
         __syncwarp();
@@ -3056,97 +3043,235 @@ __global__ void __launch_bounds__(kBlock) kb_eval(const BatchQ *__restrict__ qs,
     const uint32_t gwarp = blockIdx.x * kWarpsPerBlock + warp;
     const uint32_t nwarps = gridDim.x * kWarpsPerBlock;
     unsigned long long pairs = 0;
-    BatchOvf none;
-    none.cap = 0u;
-    LevelCounters *lcw = nullptr;
-    if (G == 2) batch_groups<2, false>(qs, blobs, gwarp * 16, nwarps * 16, items, count, k, memo, memo_left, pairs, none, lcw);
-    else if (G == 8) batch_groups<8, false>(qs, blobs, gwarp * 4, nwarps * 4, items, count, k, memo, memo_left, pairs, none, lcw);
-    else batch_groups<32, false>(qs, blobs, gwarp, nwarps, items, count, k, memo, memo_left, pairs, none, lcw);
+    if (G == 2) batch_groups<2, false>(qs, blobs, gwarp * 16, nwarps * 16, items, count, k, memo, memo_left, pairs);
+    else if (G == 8) batch_groups<8, false>(qs, blobs, gwarp * 4, nwarps * 4, items, count, k, memo, memo_left, pairs);
+    else batch_groups<32, false>(qs, blobs, gwarp, nwarps, items, count, k, memo, memo_left, pairs);
     pairs = __reduce_add_sync(kFull, (uint32_t)pairs);
     if (lane == 0 && pairs) atomicAdd(&glob->evaluated_pairs, pairs);
 }
 
-// Overflow chunks of level lc: every warp takes chunks of kChunk candidates
-// of a listed set (eval_range with the CCC queue) and folds its winner into
-// the set's keys with 64-bit atomicMin, as k_ovf_chunks does for one query.
-__device__ __forceinline__ void batch_ovf_chunks(const BatchQ *qs, const uint32_t *blobs, LevelCounters *lc,
-                                                 const float4 *memo_all, const BatchOvf &ovf, uint32_t *queue,
-                                                 unsigned long long &pairs) {
-    const int lane = threadIdx.x & 31;
-    const unsigned long long packed = __ldcg(&lc->ovf_packed);
-    const uint32_t n_ovf = (uint32_t)(packed >> 40);
-    const uint32_t n_chunks = (uint32_t)(packed & 0xFFFFFFFFFFull);
-    Blocks B;
-    B.nb = 0;
-    uint32_t cur_idx = kFull;
-    for (;;) {
-        uint32_t c = 0;
-        if (lane == 0) c = atomicAdd(&lc->chunk_next, 1u);
-        c = __shfl_sync(kFull, c, 0);
-        if (c >= n_chunks) break;
-        uint32_t lo_i = 0, hi_i = n_ovf - 1u;   // largest idx with off[idx] <= c
-        while (lo_i < hi_i) {
-            const uint32_t mid = (lo_i + hi_i + 1u) >> 1;
-            if (__ldcg(ovf.off + mid) <= c) lo_i = mid;
-            else hi_i = mid - 1u;
+// kb_gen: a wave of queries whose graphs have cycles, or one such query (ONE:
+// its planner info in shared memory), in ONE cooperative, persistent launch.
+// Per level k: one warp per connected k-set evaluates it (dp_general.cuh)
+// while the far end of the grid enumerates level k + 1, also one warp per set
+// and one lane per neighbour.  Sets with more splits than `limit` go to the
+// overflow list; after the barrier their splits are dealt out evenly, and the
+// warp that finishes a set's last unit writes its entry.
+// Bound: latency on the graphs planned exactly at this size (few sets per
+// level): list entry, block search (about 2 us for 30 relations), two memo
+// entries, cost, barrier.  Before, every lane searched the blocks in local
+// memory, one warp walked up to 2048 candidates of a set, and both orientations
+// were costed apart.  Device time: key cycle-30 1031 -> 402 us, random graphs
+// of 16 relations with statistics (0.59 and 0.72 M pairs) 3304 / 3360 -> 510 /
+// 552 us.
+__device__ __forceinline__ uint32_t gen_units(const BatchOvf &ovf, uint32_t W) { return (W + ovf.unit - 1u) / ovf.unit; }
+
+// connected (k+1)-sets from the c_prev k-sets in prev; `warp` of nwarps
+__device__ __forceinline__ void gen_extend(const BatchQ *qs, const uint32_t *blobs, const uint32_t *own_adj,
+                                           const unsigned long long *prev, uint32_t c_prev, uint32_t *seen,
+                                           unsigned long long *out, LevelCounters *lc, unsigned long long *st,
+                                           uint32_t warp, uint32_t nwarps) {
+    const uint32_t lane = threadIdx.x & 31u;
+    uint32_t cnt = 0;
+    for (uint32_t i = warp; i < c_prev; i += nwarps) {
+        const unsigned long long it = __ldcg(prev + i);
+        const uint32_t q = (uint32_t)(it >> 32), S = (uint32_t)it;
+        const uint32_t *adj = own_adj;
+        unsigned long long seen_off = 0;
+        uint32_t n;
+        if (own_adj) {
+            n = reinterpret_cast<const DevHeader *>(blobs)->n;
+        } else {
+            const BatchQ Q = qs[q];
+            adj = reinterpret_cast<const DevHeader *>(blobs + Q.blob_off)->adj;
+            seen_off = Q.seen_off;
+            n = Q.n;
         }
-        const uint32_t idx = lo_i;
+        const uint32_t bit = 1u << lane, T = S | bit;
+        bool ok = lane < n && !(S & bit) && (adj[lane] & S) != 0u;
+        if (ok) {
+            const uint32_t bm = 1u << (T & 31u);
+            ok = !(atomicOr(&seen[seen_off + (T >> 5)], bm) & bm);
+        }
+        stage_emit64(st, cnt, ok, ((unsigned long long)q << 32) | T, out, lc);
+    }
+    stage_flush64(st, cnt, out, lc);
+}
+
+template <bool ONE>
+__device__ __forceinline__ void gen_overflow(const BatchQ *qs, const uint32_t *blobs, const uint32_t *own,
+                                             LevelCounters *lc, float4 *memo_all, uint32_t *memo_left_all,
+                                             const uint32_t *seen_all, const BatchOvf &ovf, GenScratch &ws,
+                                             uint32_t gwarp, uint32_t nwarps, uint32_t &pairs) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const unsigned long long packed = __ldcg(&lc->ovf_packed);
+    uint32_t n = (uint32_t)(packed >> 40), total = (uint32_t)(packed & 0xFFFFFFFFFFull);
+    if (n > ovf.cap) {
+        n = ovf.cap;
+        total = __ldcg(ovf.off + n - 1u) + gen_units(ovf, __ldcg(ovf.W + n - 1u));
+    }
+    const uint32_t per = (total + nwarps - 1u) / nwarps;
+    uint32_t first = gwarp * per;
+    const uint32_t last = min(first + per, total);
+    if (first >= last) return;
+    uint32_t lo_i = 0u, hi_i = n - 1u;   // largest idx with off[idx] <= first
+    while (lo_i < hi_i) {
+        const uint32_t mid = (lo_i + hi_i + 1u) >> 1;
+        if (__ldcg(ovf.off + mid) <= first) lo_i = mid;
+        else hi_i = mid - 1u;
+    }
+    for (uint32_t idx = lo_i; first < last; idx++) {
         const unsigned long long it = __ldcg(ovf.item + idx);
         const uint32_t q = (uint32_t)(it >> 32), S = (uint32_t)it;
-        const uint32_t P = __ldcg(ovf.P + idx);
-        const BatchQ Q = qs[q];
-        const DevInfoView d = make_view(blobs + Q.blob_off);
-        if (idx != cur_idx) find_blocks(S, d.h->adj, B);
-        cur_idx = idx;
-        const uint32_t lo = (c - __ldcg(ovf.off + idx)) * kChunk;
-        const uint32_t hi = lo + kChunk < P ? lo + kChunk : P;
-        LaneBest best;
+        const uint32_t W = __ldcg(ovf.W + idx), o = __ldcg(ovf.off + idx), units = gen_units(ovf, W);
+        BatchQ Q = {};
+        if (!ONE) Q = qs[q];
+        const DevInfoView d = make_view(ONE ? own : blobs + Q.blob_off);
+        float4 *memo = memo_all + Q.memo_off;
+        const uint32_t *seen = seen_all + Q.seen_off;
+        gen_blocks(S, d.h->adj, ws);
+        GenBest best;
         best.init();
-        eval_range<kModeMpdp>(d, d.h->adj, S, B, lo, hi, memo_all + Q.memo_off, queue, true, best);
-        unsigned long long mk, fk;
-        warp_winner(best, mk, fk);
-        if (lane == 0) {
-            if (mk != ~0ull) atomicMin(ovf.key + idx, mk);
-            atomicMin(ovf.first + idx, fk);
+        int width = 0;
+        const uint32_t end = min(units, last - o);
+        gen_range(d, ws, S, (first - o) * ovf.unit, min(W, end * ovf.unit), memo, seen, best, width);
+        pairs += best.pairs;
+        uint32_t ord, p;
+        gen_winner(*d.h, ws, S, best, true, ord, p);
+        const uint32_t nan_p = __reduce_min_sync(kFull, best.nan_p);
+        uint32_t finished = 0u;
+        if (lane == 0u) {
+            if (ord != kFull) atomicMin(ovf.key + idx, ((unsigned long long)ord << 32) | p);
+            if (nan_p != kFull) atomicMin(ovf.nan_p + idx, nan_p);
+            __threadfence();
+            const uint32_t mine = end - (first - o);
+            finished = atomicAdd(ovf.done + idx, mine) + mine == units ? 1u : 0u;
+            __threadfence();
         }
-        pairs += best.n_valid;
+        finished = __shfl_sync(kFull, finished, 0);
+        __syncwarp();
+        if (finished) {
+            const uint32_t gnan = __ldcg(ovf.nan_p + idx);
+            uint32_t w = (uint32_t)__ldcg(ovf.key + idx);
+            if (gnan != kFull && gnan == gen_first(S, d.h->index_order, seen)) w = gnan;
+            gen_write_index(d, ws, S, w, memo, memo_left_all + Q.memo_off);
+        }
+        first = o + units;
     }
 }
 
-// Winner of every listed set: the candidate the keys name is evaluated again
-// and written to the memo (k_ovf_finalize for one query).
-__device__ __forceinline__ void batch_ovf_finalize(const BatchQ *qs, const uint32_t *blobs, LevelCounters *lc,
-                                                   float4 *memo_all, uint32_t *memo_left_all, const BatchOvf &ovf,
-                                                   uint32_t tid, uint32_t nthreads) {
-    const uint32_t n_ovf = (uint32_t)(__ldcg(&lc->ovf_packed) >> 40);
-    for (uint32_t idx = tid; idx < n_ovf; idx += nthreads) {
-        const unsigned long long it = __ldcg(ovf.item + idx);
-        const uint32_t q = (uint32_t)(it >> 32), S = (uint32_t)it;
-        const BatchQ Q = qs[q];
-        const DevInfoView d = make_view(blobs + Q.blob_off);
-        const uint32_t *adj = d.h->adj;
-        float4 *memo = memo_all + Q.memo_off;
-        const unsigned long long first = __ldcg(ovf.first + idx);
-        const uint32_t p = (first & 1ull) ? (uint32_t)(first >> 1) : (uint32_t)__ldcg(ovf.key + idx);
-        uint32_t L, R;
-        if (d.h->index_order) {   // plain-DPsub index
-            L = pdep32(p + 1u, S);
-            R = S ^ L;
-        } else {
-            Blocks B;
-            find_blocks(S, adj, B);
-            int b = 0;
-            while (b + 1 < B.nb && B.prefix[b + 1] <= p) b++;
-            const uint32_t blk = B.mask[b];
-            const uint32_t lb = pdep32(p - B.prefix[b] + 1u, blk);
-            const uint32_t rb = blk ^ lb;
-            L = grow(lowest(lb), S & ~rb, adj);
-            R = grow(lowest(rb), S & ~lb, adj);
-        }
-        const RelVal l = load_rel(memo, L, d.h->hz_packed), r = load_rel(memo, R, d.h->hz_packed);
-        const RelVal out = join_eval(d, L, l, R, r);
-        memo_write(*d.h, memo, memo_left_all + Q.memo_off, S, out, L);
+template <bool ONE>
+__global__ void __launch_bounds__(kBlock, 2) kb_gen(const BatchQ *__restrict__ qs, int nq, int maxn,
+                                                    const uint32_t *__restrict__ blobs, uint32_t blob_words,
+                                                    float4 *__restrict__ memo, uint32_t *__restrict__ memo_left,
+                                                    uint32_t *seen, unsigned long long *__restrict__ listA,
+                                                    unsigned long long *__restrict__ listB,
+                                                    LevelCounters *__restrict__ lvl, GlobalCounters *__restrict__ glob,
+                                                    TreeNode *__restrict__ tree, int *__restrict__ tree_n,
+                                                    unsigned *__restrict__ bar, BatchOvf ovf, unsigned poll_limit) {
+    extern __shared__ __align__(16) unsigned char gsm[];
+    __shared__ unsigned long long stage[kWarpsPerBlock][64];
+    const unsigned max_polls = barrier_polls(poll_limit);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    GenScratch &ws = reinterpret_cast<GenScratch *>(gsm)[warp];
+    uint32_t *own = nullptr;
+    if (ONE) {
+        own = reinterpret_cast<uint32_t *>(gsm + kWarpsPerBlock * sizeof(GenScratch));
+        load_blob_to_smem(blobs, blob_words, own);
     }
+    unsigned long long *st = stage[warp];
+    const uint32_t gwarp = blockIdx.x * kWarpsPerBlock + warp;
+    const uint32_t nwarps = gridDim.x * kWarpsPerBlock;
+    unsigned long long pairs = 0;
+    unsigned epoch = 0;   // grid barriers passed (thread 0)
+
+    // phase 0: base relations (gpuqo_cpu_sequential.cu:80-92) and level-2 sets
+    // (each edge once, from its lower end), entered into the bitmap
+    {
+        uint32_t cnt = 0;
+        for (uint32_t q = gwarp; q < (uint32_t)nq; q += nwarps) {
+            const BatchQ Q = qs[q];
+            const DevHeader *h = reinterpret_cast<const DevHeader *>(ONE ? own : blobs + Q.blob_off);
+            uint32_t nb = 0u;
+            if (lane < (int)Q.n) {
+                memo[Q.memo_off + (1ull << lane)] = base_entry(*h, lane);
+                memo_left[Q.memo_off + (1ull << lane)] = 0u;
+                atomicOr(seen + Q.seen_off + ((1u << lane) >> 5), 1u << ((1u << lane) & 31u));
+                nb = h->adj[lane] & ~((2u << lane) - 1u);
+            }
+            const int maxdeg = (int)__reduce_max_sync(kFull, (uint32_t)__popc(nb));
+            for (int j = 0; j < maxdeg; j++) {
+                const bool ok = nb != 0u;
+                const uint32_t T = (1u << lane) | (nb & (0u - nb));
+                nb &= nb - 1u;
+                if (ok) atomicOr(seen + Q.seen_off + (T >> 5), 1u << (T & 31u));
+                stage_emit64(st, cnt, ok, ((unsigned long long)q << 32) | T, listA, lvl + 2);
+            }
+        }
+        stage_flush64(st, cnt, listA, lvl + 2);
+    }
+    if (!grid_barrier<ONE>(bar, epoch, max_polls)) return;
+
+    for (int k = 2; k <= maxn; k++) {
+        unsigned long long *cur = (k & 1) ? listB : listA;
+        unsigned long long *nxt = (k & 1) ? listA : listB;
+        LevelCounters *lk = lvl + k;
+        const uint32_t count = __ldcg(&lk->n_sets);
+        // enumeration from the far end of the grid, evaluation from the start
+        if (k < maxn)
+            gen_extend(qs, ONE ? own : blobs, ONE ? reinterpret_cast<const DevHeader *>(own)->adj : nullptr, cur, count,
+                       seen, nxt, lk + 1, st, nwarps - 1u - gwarp, nwarps);
+        // Splits a warp takes alone: 4 rounds of its lanes per set it holds.
+        // The overflow phase costs about two barriers and another block search
+        // per share.
+        const uint32_t limit = min(2048u, 128u * ((count + nwarps - 1u) / nwarps));
+        uint32_t found = 0u;
+        for (uint32_t i = gwarp; i < count; i += nwarps) {
+            const unsigned long long it = __ldcg(cur + i);
+            const uint32_t q = (uint32_t)(it >> 32), S = (uint32_t)it;
+            BatchQ Q = {};
+            if (!ONE) Q = qs[q];
+            const DevInfoView d = make_view(ONE ? own : blobs + Q.blob_off);
+            gen_blocks(S, d.h->adj, ws);
+            const uint32_t W = ws.half[ws.nb];
+            if (W > limit && ovf.cap != 0u) {
+                // one packed atomic assigns the list index and the first unit
+                // in the same order
+                uint32_t idx = 0u;
+                if (lane == 0) {
+                    const unsigned long long old = atomicAdd(&lk->ovf_packed, (1ull << 40) | gen_units(ovf, W));
+                    idx = (uint32_t)(old >> 40);
+                    if (idx < ovf.cap) {
+                        ovf.item[idx] = it;
+                        ovf.W[idx] = W;
+                        ovf.off[idx] = (uint32_t)(old & 0xFFFFFFFFFFull);
+                        ovf.key[idx] = ~0ull;
+                        ovf.nan_p[idx] = kFull;
+                        ovf.done[idx] = 0u;
+                    }
+                }
+                if (__shfl_sync(kFull, idx, 0) < ovf.cap) continue;
+            }
+            gen_set(d, ws, S, memo + Q.memo_off, memo_left + Q.memo_off, seen + Q.seen_off, found);
+        }
+        if (!grid_barrier<ONE>(bar, epoch, max_polls)) return;
+        // the counter is final after the barrier: every block takes the same branch
+        if (ovf.cap != 0u && (uint32_t)(__ldcg(&lk->ovf_packed) >> 40) != 0u) {
+            gen_overflow<ONE>(qs, blobs, own, lk, memo, memo_left, seen, ovf, ws, gwarp, nwarps, found);
+            if (!grid_barrier<ONE>(bar, epoch, max_polls)) return;
+        }
+        pairs += found;
+    }
+
+    for (uint32_t q = gwarp; q < (uint32_t)nq; q += nwarps) {
+        const BatchQ Q = qs[q];
+        const uint32_t full = (Q.n == 32) ? 0xFFFFFFFFu : ((1u << Q.n) - 1u);
+        const uint32_t wmask =
+            reinterpret_cast<const DevHeader *>(ONE ? own : blobs + Q.blob_off)->hz_packed ? kWidthMask : 0xFFFFFFFFu;
+        extract_plan(memo + Q.memo_off, memo_left + Q.memo_off, full, wmask, ws.queue, tree + (size_t)q * 64, tree_n + q);
+    }
+    for (int off = 16; off >= 1; off >>= 1) pairs += __shfl_xor_sync(kFull, pairs, off);
+    if (lane == 0 && pairs) atomicAdd(&glob->evaluated_pairs, pairs);
 }
 
 __global__ void kb_extract(const BatchQ *__restrict__ qs, int nq, const uint32_t *__restrict__ blobs,
@@ -3203,27 +3328,26 @@ __global__ void kb_extract(const BatchQ *__restrict__ qs, int nq, const uint32_t
     n_out[q] = n;
 }
 
-// kb_dp: a whole wave of queries in ONE cooperative, persistent launch.
+// kb_dp: a wave of tree-shaped queries in ONE cooperative, persistent launch.
 // Phase 0 writes every query's base relations and emits its level-2 sets
 // (one warp per query, one lane per relation: each edge once, from its lower
 // end).  Then, per level k, the grid evaluates level k of every query while
 // it enumerates level k+1, with a grid barrier between levels; the plans are
-// extracted (one thread per query) after the last level.  The grid barrier
+// extracted (one warp per query) after the last level.  The grid barrier
 // is bounded (grid_barrier); on timeout the host reruns the wave with
 // per-level launches.
-template <bool TREE_ONLY, bool ALL_MASKED = false>
-__global__ void __launch_bounds__(kBlock, TREE_ONLY ? 3 : 2) kb_dp(const BatchQ *__restrict__ qs, int nq, int maxn,
+template <bool ALL_MASKED>
+__global__ void __launch_bounds__(kBlock, 3) kb_dp(const BatchQ *__restrict__ qs, int nq, int maxn,
                                                    const uint32_t *__restrict__ blobs, float4 *__restrict__ memo,
-                                                   uint32_t *__restrict__ memo_left, uint32_t *__restrict__ seen,
+                                                   uint32_t *__restrict__ memo_left,
                                                    unsigned long long *__restrict__ listA,
                                                    unsigned long long *__restrict__ listB,
                                                    LevelCounters *__restrict__ lvl, GlobalCounters *__restrict__ glob,
                                                    TreeNode *__restrict__ tree, int *__restrict__ tree_n,
                                                    unsigned *__restrict__ bar, uint32_t target_lanes,
-                                                   BatchOvf ovf, unsigned poll_limit) {
+                                                   unsigned poll_limit) {
     const unsigned max_polls = barrier_polls(poll_limit);
     __shared__ unsigned long long stage[kWarpsPerBlock][64];
-    __shared__ uint32_t queues[kWarpsPerBlock][kQueueWords];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     unsigned long long *st = stage[warp];
     const uint32_t gwarp = blockIdx.x * kWarpsPerBlock + warp;
@@ -3268,42 +3392,28 @@ __global__ void __launch_bounds__(kBlock, TREE_ONLY ? 3 : 2) kb_dp(const BatchQ 
         unsigned long long *nxt = (k & 1) ? listA : listB;
         const uint32_t count = __ldcg(&lvl[k].n_sets);
         // enumeration from the far end of the grid, evaluation from the start
-        if (k < maxn) batch_extend<TREE_ONLY>(qs, blobs, cur, count, seen, nxt, lvl + k + 1, st, nthreads - 1u - tid, nthreads);
+        if (k < maxn) batch_extend<true>(qs, blobs, cur, count, nullptr, nxt, lvl + k + 1, st, nthreads - 1u - tid, nthreads);
         int max_group = 1;
         while (max_group < 32 && max_group < 2 * (k - 1)) max_group <<= 1;
         int G = 2;
         while (G < max_group && (uint64_t)count * (uint64_t)G < (uint64_t)target_lanes) G <<= 1;
         G = G <= 2 ? 2 : (G <= 8 ? 8 : 32);
-        LevelCounters *lk = lvl + k;
         if (G == 2)
-            batch_groups<2, TREE_ONLY, ALL_MASKED>(qs, blobs, gwarp * 16, nwarps * 16, cur, count, k, memo, memo_left,
-                                                   pairs, ovf, lk);
+            batch_groups<2, true, ALL_MASKED>(qs, blobs, gwarp * 16, nwarps * 16, cur, count, k, memo, memo_left, pairs);
         else if (G == 8)
-            batch_groups<8, TREE_ONLY, ALL_MASKED>(qs, blobs, gwarp * 4, nwarps * 4, cur, count, k, memo, memo_left,
-                                                   pairs, ovf, lk);
+            batch_groups<8, true, ALL_MASKED>(qs, blobs, gwarp * 4, nwarps * 4, cur, count, k, memo, memo_left, pairs);
         else
-            batch_groups<32, TREE_ONLY, ALL_MASKED>(qs, blobs, gwarp, nwarps, cur, count, k, memo, memo_left, pairs,
-                                                    ovf, lk);
+            batch_groups<32, true, ALL_MASKED>(qs, blobs, gwarp, nwarps, cur, count, k, memo, memo_left, pairs);
         if (!grid_barrier<false>(bar, epoch, max_polls)) return;
-        if (TREE_ONLY) continue;   // tree sets have 2(k - 1) candidates: never an overflow
-        // overflow sets of level k: the counter is final after the barrier, so
-        // every block takes the same branch.  A list longer than its capacity
-        // is left to the host (the affected queries are rerun one by one).
-        const uint32_t n_ovf = (uint32_t)(__ldcg(&lk->ovf_packed) >> 40);
-        if (n_ovf != 0u && n_ovf <= ovf.cap) {
-            batch_ovf_chunks(qs, blobs, lk, memo, ovf, queues[warp], pairs);
-            if (!grid_barrier<false>(bar, epoch, max_polls)) return;
-            batch_ovf_finalize(qs, blobs, lk, memo, memo_left, ovf, tid, nthreads);
-            if (!grid_barrier<false>(bar, epoch, max_polls)) return;
-        }
     }
 
-    for (uint32_t q = tid; q < (uint32_t)nq; q += nthreads) {
+    for (uint32_t q = gwarp; q < (uint32_t)nq; q += nwarps) {
         const BatchQ Q = qs[q];
         const uint32_t full = (Q.n == 32) ? 0xFFFFFFFFu : ((1u << Q.n) - 1u);
         const uint32_t wmask =
             reinterpret_cast<const DevHeader *>(blobs + Q.blob_off)->hz_packed ? kWidthMask : 0xFFFFFFFFu;
-        extract_plan(memo + Q.memo_off, memo_left + Q.memo_off, full, wmask, tree + (size_t)q * 64, tree_n + q);
+        extract_plan(memo + Q.memo_off, memo_left + Q.memo_off, full, wmask, reinterpret_cast<uint32_t *>(st),
+                     tree + (size_t)q * 64, tree_n + q);
     }
     pairs = __reduce_add_sync(kFull, (uint32_t)pairs);
     if (lane == 0 && pairs) atomicAdd(&glob->evaluated_pairs, pairs);
@@ -3382,6 +3492,10 @@ uint64_t batch_query_bytes(int n) {
     return slots * (sizeof(float4) + 4) + slots / 8 + 2 * max_level_sets(n) * 8 + 64 * sizeof(TreeNode) + 4096;
 }
 
+// dynamic shared memory of kb_gen besides the planner info
+constexpr size_t kGenSmem = kWarpsPerBlock * sizeof(GenScratch);
+static_assert(kGenSmem <= 44 * 1024 && sizeof(GenScratch) % 16 == 0, "kb_gen scratch and its static shared memory");
+
 struct BatchEngine {
     int device = -1, sm_count = 148;
     cudaStream_t stream = nullptr;
@@ -3397,12 +3511,13 @@ struct BatchEngine {
     int *tree_n = nullptr;
     LevelCounters *lvl = nullptr;
     GlobalCounters *glob = nullptr;
-    unsigned *bar = nullptr, *h_bar = nullptr;   // grid barrier words of kb_dp (device, pinned copy)
-    int coop_grid = -1;                          // co-resident blocks of kb_dp<false> (0: no cooperative launch)
-    int coop_grid_tree = -1;                     // co-resident blocks of kb_dp<true>
-    int coop_grid_masked = -1;                   // co-resident blocks of kb_dp<true, true>
-    bool barrier_timed_out = false;              // a grid barrier of kb_dp gave up: per-level launches until reset
-    BatchOvf ovf{};                              // overflow list of kb_dp
+    unsigned *bar = nullptr, *h_bar = nullptr;   // grid barrier words (device, pinned copy)
+    int coop_grid = -1;                          // co-resident blocks of kb_gen<false> (0: no cooperative launch)
+    int coop_grid_tree = -1;                     // co-resident blocks of kb_dp<false>
+    int coop_grid_masked = -1;                   // co-resident blocks of kb_dp<true>
+    std::map<size_t, int> coop_one;              // dynamic shared bytes -> co-resident blocks of kb_gen<true>
+    bool barrier_timed_out = false;              // a grid barrier gave up: per-level launches until reset
+    BatchOvf ovf{};                              // overflow list of kb_gen
     uint64_t cap_ovf = 0;
     void *flush = nullptr;                       // L2 flush buffer (device-resident timing only)
     // pinned staging of a wave: planner infos and descriptors in, plans and
@@ -3434,9 +3549,10 @@ struct BatchEngine {
         int dev_coop = 0, occ = 0, occ_tree = 0, occ_masked = 0;
         cudaDeviceGetAttribute(&dev_coop, cudaDevAttrCooperativeLaunch, device);
         coop_grid = coop_grid_tree = coop_grid_masked = 0;
-        if (dev_coop && cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kb_dp<false>, kBlock, 0) == cudaSuccess &&
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_tree, kb_dp<true>, kBlock, 0) == cudaSuccess &&
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_masked, kb_dp<true, true>, kBlock, 0) == cudaSuccess) {
+        if (dev_coop &&
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kb_gen<false>, kBlock, kGenSmem) == cudaSuccess &&
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_tree, kb_dp<false>, kBlock, 0) == cudaSuccess &&
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_masked, kb_dp<true>, kBlock, 0) == cudaSuccess) {
             coop_grid = occ * sm_count;
             coop_grid_tree = occ_tree * sm_count;
             coop_grid_masked = occ_masked * sm_count;
@@ -3467,12 +3583,32 @@ struct BatchEngine {
         return kernels + 1;
     }
 
-    // the wave as one cooperative launch of kb_dp (kb_dp<true> when every query
-    // is tree-shaped, kb_dp<true, true> when every class of every query is also
-    // a two-member class on a tree edge); false when it could not start
-    bool enqueue_persistent(int nq, int maxn, uint64_t seen_words, bool tree_only, bool all_masked) {
+    // co-resident blocks of kb_gen<true> with a planner info of `words` words,
+    // 0 when two of them do not fit an SM (about 75 KB of planner info, an
+    // 18-relation clique has 13 KB) or cooperative launches are not possible
+    int one_grid(uint32_t words) {
+        const size_t smem = kGenSmem + (size_t)words * 4u;
+        if (coop_grid <= 0 || smem > 100u * 1024u) return 0;
+        auto it = coop_one.find(smem);
+        if (it == coop_one.end()) {
+            int occ = 0;
+            if (cudaFuncSetAttribute(kb_gen<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024) != cudaSuccess ||
+                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kb_gen<true>, kBlock, smem) != cudaSuccess)
+                occ = 0;
+            cudaGetLastError();
+            it = coop_one.emplace(smem, occ * sm_count).first;
+        }
+        return it->second;
+    }
+
+    // the wave as one cooperative launch: kb_dp when every query is
+    // tree-shaped (kb_dp<true> when every class of every query is also a
+    // two-member class on a tree edge), else kb_gen (kb_gen<true> for one
+    // query); false when it could not start
+    bool enqueue_persistent(int nq, int maxn, uint32_t words, uint64_t seen_words, bool tree_only, bool all_masked) {
         const bool masked = tree_only && all_masked;
-        const int grid = masked ? coop_grid_masked : (tree_only ? coop_grid_tree : coop_grid);
+        const int one = (!tree_only && nq == 1) ? one_grid(words) : 0;
+        const int grid = masked ? coop_grid_masked : (tree_only ? coop_grid_tree : (one > 0 ? one : coop_grid));
         if (grid <= 0 || gpuqo_b200_persistent == 0 || barrier_timed_out) return false;
         cudaMemsetAsync(lvl, 0, 33 * sizeof(LevelCounters), stream);
         cudaMemsetAsync(glob, 0, sizeof(GlobalCounters), stream);
@@ -3480,11 +3616,20 @@ struct BatchEngine {
         cudaMemsetAsync(bar, 0, 4 * sizeof(unsigned), stream);
         uint32_t target_lanes = (uint32_t)grid * kBlock;
         unsigned poll_limit = (unsigned)std::max(0, gpuqo_b200_barrier_poll_limit);
-        void *args[] = {&qs, &nq, &maxn, &blobs, &memo, &memo_left, &seen, &listA, &listB,
-                        &lvl, &glob, &tree, &tree_n, &bar, &target_lanes, &ovf, &poll_limit};
-        const void *fn = masked ? (const void *)kb_dp<true, true>
-                                : (tree_only ? (const void *)kb_dp<true> : (const void *)kb_dp<false>);
-        if (cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kBlock), args, 0, stream) != cudaSuccess) {
+        cudaError_t e;
+        if (tree_only) {
+            void *args[] = {&qs, &nq, &maxn, &blobs, &memo, &memo_left, &listA, &listB,
+                            &lvl, &glob, &tree, &tree_n, &bar, &target_lanes, &poll_limit};
+            e = cudaLaunchCooperativeKernel(masked ? (const void *)kb_dp<true> : (const void *)kb_dp<false>, dim3(grid),
+                                            dim3(kBlock), args, 0, stream);
+        } else {
+            void *args[] = {&qs, &nq, &maxn, &blobs, &words, &memo, &memo_left, &seen, &listA, &listB,
+                            &lvl, &glob, &tree, &tree_n, &bar, &ovf, &poll_limit};
+            e = cudaLaunchCooperativeKernel(one > 0 ? (const void *)kb_gen<true> : (const void *)kb_gen<false>,
+                                            dim3(grid), dim3(kBlock), args,
+                                            kGenSmem + (one > 0 ? (size_t)words * 4u : 0u), stream);
+        }
+        if (e != cudaSuccess) {
             cudaGetLastError();
             coop_grid = coop_grid_tree = coop_grid_masked = 0;
             return false;
@@ -3518,9 +3663,9 @@ struct BatchEngine {
     }
 
     // One wave: all queries' memos fit.  wb: per query planner-info blob.
-    // Queries that this wave could not finish (sets beyond the group limit
-    // without the overflow phase, or an overfull overflow list) are listed in
-    // redo (wave-local indices) for the single-query engine.
+    // Queries that this wave cannot finish (sets beyond the group limit, whose
+    // splits the per-level launches do not deal out) are listed in redo
+    // (wave-local indices) for the single-query engine.
     int run_wave(const std::vector<const std::vector<uint32_t> *> &wb, std::vector<std::vector<TreeNode>> &out,
                  std::vector<int> &redo, EngineStats &st, double &ms, std::string &err) {
         redo.clear();
@@ -3545,19 +3690,15 @@ struct BatchEngine {
             ms = 0.0;
             if (rest.empty()) return 0;
             std::vector<std::vector<TreeNode>> rout;
-            bool ovf_full = false;
-            if (int rc = stage_and_run(rest, rout, st, ms, ovf_full, err)) return rc;
+            if (int rc = stage_and_run(rest, rout, st, ms, err)) return rc;
             for (size_t i = 0; i < idx.size(); i++) out[idx[i]] = std::move(rout[i]);
             return 0;
         }
-        bool ovf_full = false;
-        if (int rc = stage_and_run(wb, out, st, ms, ovf_full, err)) return rc;
-        if (ovf_full) redo = need_ovf;
-        return 0;
+        return stage_and_run(wb, out, st, ms, err);
     }
 
     int stage_and_run(const std::vector<const std::vector<uint32_t> *> &wb, std::vector<std::vector<TreeNode>> &out,
-                      EngineStats &st, double &ms, bool &ovf_full, std::string &err) {
+                      EngineStats &st, double &ms, std::string &err) {
         const int nq = (int)wb.size();
         std::vector<BatchQ> hq(nq);
         uint64_t slots = 0, words = 0, seen_words = 0, items = 0, base = 0, ovf_need = 0;
@@ -3599,14 +3740,20 @@ struct BatchEngine {
         cap_items = std::min(c5, c6);
         if (ovf_need > cap_ovf) {
             uint64_t a1 = cap_ovf, a2 = cap_ovf, a3 = cap_ovf, a4 = cap_ovf, a5 = cap_ovf;
+            uint64_t a6 = cap_ovf;
             if (int rc = grow(ovf.item, a1, ovf_need, err)) return rc;
-            if (int rc = grow(ovf.P, a2, ovf_need, err)) return rc;
+            if (int rc = grow(ovf.W, a2, ovf_need, err)) return rc;
             if (int rc = grow(ovf.off, a3, ovf_need, err)) return rc;
             if (int rc = grow(ovf.key, a4, ovf_need, err)) return rc;
-            if (int rc = grow(ovf.first, a5, ovf_need, err)) return rc;
+            if (int rc = grow(ovf.nan_p, a5, ovf_need, err)) return rc;
+            if (int rc = grow(ovf.done, a6, ovf_need, err)) return rc;
             cap_ovf = ovf_need;
         }
         ovf.cap = (uint32_t)ovf_need;
+        // units of the overflow shares: small enough to spread a level evenly,
+        // large enough that a level's units number below 2^32 (at most 2^22
+        // listed sets of 2^(n - 1) splits)
+        ovf.unit = maxn <= 24 ? 32u : (maxn <= 26 ? 1024u : 8192u);
         if (nq > cap_q) {
             cudaFree(qs);
             cudaFree(tree);
@@ -3650,13 +3797,10 @@ struct BatchEngine {
         };
         uint32_t kernels = 1;
         CK(cudaEventRecord(ev0, stream));
-        bool persistent = enqueue_persistent(nq, maxn, seen_words, tree_only, all_masked);
+        bool persistent = enqueue_persistent(nq, maxn, (uint32_t)words, seen_words, tree_only, all_masked);
         CK(cudaGetLastError());
         if (persistent) CK(cudaMemcpyAsync(h_bar, bar, 4 * sizeof(unsigned), cudaMemcpyDeviceToHost, stream));
-        if (!persistent) {
-            ovf.cap = 0u;
-            kernels = enqueue_levels(nq, maxn, seen_words);
-        }
+        if (!persistent) kernels = enqueue_levels(nq, maxn, seen_words);
         CK(cudaGetLastError());
         CK(cudaEventRecord(ev1, stream));
         if (int rc = download()) return rc;
@@ -3665,7 +3809,6 @@ struct BatchEngine {
             barrier_timed_out = true;           // and use them until gpuqo_b200_reset_persistent
             st.barrier_timeouts++;
             CK(cudaEventRecord(ev0, stream));
-            ovf.cap = 0u;
             kernels = enqueue_levels(nq, maxn, seen_words);
             CK(cudaGetLastError());
             CK(cudaEventRecord(ev1, stream));
@@ -3678,19 +3821,13 @@ struct BatchEngine {
         float fms = 0.f;
         CK(cudaEventElapsedTime(&fms, ev0, ev1));
         ms = fms;
-        // kb_dp skipped the overflow phase of a level whose list outgrew its
-        // capacity; the per-level launches (ovf.cap 0) evaluate every set in
-        // its group and need no redo
-        ovf_full = false;
-        for (int k = 2; k <= maxn; k++)
-            if (persistent && (uint32_t)(hl[k].ovf_packed >> 40) > ovf.cap) ovf_full = true;
         out.resize(nq);
         for (int q = 0; q < nq; q++) {
-            if (hn[q] != 2 * (int)hq[q].n - 1 && !(ovf_full && batch_needs_ovf(*wb[q]))) {
+            if (hn[q] != 2 * (int)hq[q].n - 1) {
                 err = "batched plan extraction produced " + std::to_string(hn[q]) + " nodes";
                 return GPUQO_B200_ERR_CUDA;
             }
-            out[q].assign(htree + (size_t)q * 64, htree + (size_t)q * 64 + std::max(hn[q], 0));
+            out[q].assign(htree + (size_t)q * 64, htree + (size_t)q * 64 + hn[q]);
         }
         for (int k = 2; k <= maxn; k++) st.connected_sets += hl[k].n_sets;
         st.evaluated_pairs += hg.evaluated_pairs;
@@ -3774,10 +3911,10 @@ int engine_run_batch(const std::vector<const std::vector<uint32_t> *> &blobs, ui
 
 // One exact DP.  Tree-shaped graphs run k_dp_tree (Engine); other graphs
 // under MPDP enumeration (MPDP, and plain DPsub on valid pairs) run as a
-// one-query wave of the general persistent kernel kb_dp<false>, which has the
+// one-query wave of the general persistent kernel kb_gen<true>, which has the
 // overflow phases in the same launch; the per-level launches of Engine serve
-// the rest (plain all-subsets DPsub, no cooperative launch, an overfull
-// overflow list, gpuqo_b200_persistent = 0).
+// the rest (plain all-subsets DPsub, no cooperative launch,
+// gpuqo_b200_persistent = 0).
 int engine_run(const std::vector<uint32_t> &blob, int n, DpMode mode, bool ccc, bool profile,
                std::vector<TreeNode> &nodes, EngineStats &stats, std::string &err) {
     if (n < 1 || n > 31) {
