@@ -55,7 +55,16 @@ __device__ __forceinline__ uint32_t grow(uint32_t from, uint32_t subset, const u
 // gpuqo_filter.cuh:149-160
 __device__ __forceinline__ bool is_connected(uint32_t s, const uint32_t *adj) {
     if (!s) return false;
-    return grow(lowest(s), s, adj) == s;
+    // the closure of the lowest relation, ended as soon as it reaches all of s
+    // (in a dense graph with the first relation's neighbours)
+    uint32_t V = 0u, N = lowest(s);
+    while (N) {
+        const int i = lowest_idx(N);
+        V |= 1u << i;
+        N = (N | adj[i]) & s & ~V;
+        if ((V | N) == s) return true;
+    }
+    return false;
 }
 
 // float -> int as the reference's x86-64 host build converts it
@@ -810,11 +819,12 @@ __device__ __forceinline__ void join_eval_mirror_tree(const DevInfoView &d, uint
 }
 
 // ---------------------------------------------------------------------------
-// Both orientations of a split edge of a plain tree (DevHeader::tree_plain).
+// Both orientations of a split whose matching classes are all plain
+// (DevHeader::tree_plain, pairs_plain).
 // What join_eval_mirror_w computes for it, without the parts that are constant
 // there: no unique inner side, no index, bucket size 0.1, MCV frequency 0 (one
-// row within work_mem: no skew penalty), the sums over the edge's classes in
-// TreeEdge, and the terms that both orientations share taken once (products
+// row within work_mem: no skew penalty), the sums over the quals from
+// PlainQuals, and the terms that both orientations share taken once (products
 // and sums of two operands do not depend on their order; a run cost may start
 // from its first term instead of 0 because only the sum with a startup cost,
 // which is never -0, is kept).  Every other operation is in the order of
@@ -836,7 +846,7 @@ struct JoinCost {
     float rows, startup, total;
 };
 
-__device__ __forceinline__ void plain_join(const PlainParams &c, const TreeEdge &e, float sel, const float4 o,
+__device__ __forceinline__ void plain_join(const PlainParams &c, const PlainQuals &e, float sel, const float4 o,
                                            const float4 i, float d_o, float d_i, float nl_startup, float nl_tuples,
                                            bool batched, float pages_o, float pages_i, JoinCost &out) {
     const float rows = sel * o.x * i.x;
@@ -865,9 +875,10 @@ __device__ __forceinline__ void plain_join(const PlainParams &c, const TreeEdge 
     out.total = hash ? hj_total : nl_total;
 }
 
-// l: memo entry of the side that holds the edge's lower end, r: of the other
-__device__ __forceinline__ void plain_mirror(const PlainParams &c, const TreeEdge &e, const float4 l, const float4 r,
-                                             JoinCost &lr, JoinCost &rl) {
+// l, r: memo entries of the two sides; sel_l, sel_r: the selectivity product
+// with l's side outer and with r's
+__device__ __forceinline__ void plain_mirror(const PlainParams &c, const PlainQuals &e, float sel_l, float sel_r,
+                                             const float4 l, const float4 r, JoinCost &lr, JoinCost &rl) {
     const uint32_t lw = __float_as_uint(l.w), rw = __float_as_uint(r.w);
     const bool lb = (lw >> (kWidthBits + 6)) != 0u, rb = (rw >> (kWidthBits + 6)) != 0u;   // more than one batch
     float lp = 0.0f, rp = 0.0f;
@@ -878,8 +889,68 @@ __device__ __forceinline__ void plain_mirror(const PlainParams &c, const TreeEdg
     const float dl = l.z - l.y, dr = r.z - r.y;
     const float nl_startup = c.nl_base + (r.y + l.y);
     const float nl_tuples = e.nl_tuple * (l.x * r.x);
-    plain_join(c, e, e.sel_lo, l, r, dl, dr, nl_startup, nl_tuples, rb, lp, rp, lr);
-    plain_join(c, e, e.sel_hi, r, l, dr, dl, nl_startup, nl_tuples, lb, rp, lp, rl);
+    plain_join(c, e, sel_l, l, r, dl, dr, nl_startup, nl_tuples, rb, lp, rp, lr);
+    plain_join(c, e, sel_r, r, l, dr, dl, nl_startup, nl_tuples, lb, rp, lp, rl);
+}
+
+// Classes of two members with one member on each side of a split, 32 per word.
+// A class has exactly one member in L when it is in an odd number of the rows
+// (rel_ecs) of L's relations, so the rows' exclusive or, restricted to the
+// classes inside S, is the match of (L, S - L); it follows L from split to
+// split by the rows of the relations that change sides.
+template <int NW>
+__device__ __forceinline__ void pairs_flip(const DevInfoView &d, uint32_t rels, uint32_t (&odd)[4 * NW]) {
+    for (uint32_t x = rels; x; x &= x - 1u) {
+        const uint4 *row = reinterpret_cast<const uint4 *>(d.rel_ecs + lowest_idx(x) * (4 * NW));
+#pragma unroll
+        for (int j = 0; j < NW; j++) {
+            const uint4 a = row[j];
+            odd[4 * j] ^= a.x;
+            odd[4 * j + 1] ^= a.y;
+            odd[4 * j + 2] ^= a.z;
+            odd[4 * j + 3] ^= a.w;
+        }
+    }
+}
+
+// the classes with both members in S
+template <int NW>
+__device__ __forceinline__ void pairs_inside(const DevInfoView &d, uint32_t S, uint32_t (&inside)[4 * NW]) {
+    uint32_t odd[4 * NW];
+#pragma unroll
+    for (int w = 0; w < 4 * NW; w++) inside[w] = odd[w] = 0u;
+    for (uint32_t x = S; x; x &= x - 1u) {
+        const uint4 *row = reinterpret_cast<const uint4 *>(d.rel_ecs + lowest_idx(x) * (4 * NW));
+#pragma unroll
+        for (int j = 0; j < NW; j++) {
+            const uint4 a = row[j];
+            const uint32_t r[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                inside[4 * j + q] |= odd[4 * j + q] & r[q];
+                odd[4 * j + q] ^= r[q];
+            }
+        }
+    }
+}
+
+// both orientations of a split whose matching classes are odd & inside; the
+// one selectivity product (pairs_plain) is taken in class order
+template <int NW>
+__device__ __forceinline__ void pairs_mirror(const DevInfoView &d, const PlainParams &pp, const uint32_t (&odd)[4 * NW],
+                                             const uint32_t (&inside)[4 * NW], const float4 l, const float4 r,
+                                             JoinCost &lr, JoinCost &rl) {
+    float sel = 1.0f;
+    int quals = 0;
+#pragma unroll
+    for (int w = 0; w < 4 * NW; w++) {
+        const uint32_t m = odd[w] & inside[w];
+        const float *s = d.pair_sel + 64 * w;
+        quals += popc(m);
+        for (uint32_t x = m; x; x &= x - 1u) sel *= s[2 * lowest_idx(x)];
+    }
+    const PlainQuals q = reinterpret_cast<const PlainQuals *>(reinterpret_cast<const uint32_t *>(d.h) + d.h->pairs_plain)[quals];
+    plain_mirror(pp, q, sel, sel, l, r, lr, rl);
 }
 
 // (L, R) and (R, L); classes beyond 256 take two join_eval calls

@@ -845,7 +845,7 @@ __device__ __forceinline__ void tree_cost(const DevInfoView &d, const PlainParam
     if (LAYOUT == kTreePlain) {
         const TreeEdge &e = reinterpret_cast<const TreeEdge *>(t.tab + tree_edge_off(t.n))[edge];
         JoinCost lr, rl;
-        plain_mirror(pp, e, lv, rv, lr, rl);
+        plain_mirror(pp, e.quals, e.sel_lo, e.sel_hi, lv, rv, lr, rl);
         width = (int)((__float_as_uint(lv.w) & kWidthMask) + (__float_as_uint(rv.w) & kWidthMask));
         tree_update(best, h, t, S, v, lr.rows, lr.startup, lr.total);
         tree_update(best, h, t, S, v | kSideHigher, rl.rows, rl.startup, rl.total);
@@ -1374,6 +1374,152 @@ __global__ void __launch_bounds__(kBlock) k_ovf_finalize(const uint32_t *__restr
         RelVal l = load_rel(memo, L, d.h->hz_packed), r = load_rel(memo, R, d.h->hz_packed);
         RelVal out = join_eval(d, L, l, R, r);
         memo_write(*d.h, memo, memo_left, S, out, L);
+    }
+}
+
+// ---------------------------------------------------------------------------
+// k_dense: plain DPsub over all subsets of dense graphs with plain classes
+// (DevHeader::pairs_plain; a clique of 18 relations has 193 M unordered splits,
+// every one valid).  A lane takes a contiguous slice of a set's splits
+// L = pdep(h + 1, S), h = lo .. hi - 1, and its mirror P - 1 - h, and carries the
+// matching classes from split to split (pairs_flip: two relations change sides
+// on average) instead of gathering the class rows of all relations; nearly
+// every split is valid, so none is queued.
+// Bound: issue, most of it the selectivity product in class order (about 33
+// classes a split on the clique).  share: splits per warp; a set of at most
+// that many is one warp's and written at once, otherwise the shares fold
+// their keys (as k_ovf_chunks does) and k_dense_finalize writes the winners.
+// ---------------------------------------------------------------------------
+constexpr uint32_t kDenseWhole = 1023u;   // splits of an 11-relation set
+
+// plain DPsub keeps the all-subsets enumeration on graphs with at least half
+// of all possible edges (apply_dpsub_csg); sparse ones only come here with
+// gpuqo_dpsub_csg_enable off, and their invalid subsets are better queued
+static bool dense_pairs(const DevHeader &h) {
+    uint64_t degrees = 0;
+    for (int i = 0; i < h.n; i++) degrees += (uint64_t)__builtin_popcount(h.adj[i]);
+    return h.pairs_plain != 0u && 2 * degrees >= (uint64_t)h.n * (uint64_t)(h.n - 1);
+}
+
+template <int NW>
+__global__ void __launch_bounds__(kBlock, 3) k_dense(const uint32_t *__restrict__ blob, uint32_t blob_words, int k,
+                                                     const uint32_t *__restrict__ sets, LevelCounters *__restrict__ lc,
+                                                     float4 *__restrict__ memo, uint32_t *__restrict__ memo_left,
+                                                     unsigned long long *__restrict__ keys,
+                                                     unsigned long long *__restrict__ firsts,
+                                                     GlobalCounters *__restrict__ glob, uint32_t share) {
+    extern __shared__ __align__(16) uint32_t sm[];
+    load_blob_to_smem(blob, blob_words, sm);
+    const DevInfoView d = make_view(sm);
+    const DevHeader &h = *d.h;
+    const uint32_t *adj = h.adj;
+    const PlainParams pp = plain_params(h);
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t count = lc->n_sets, W = (1u << (k - 1)) - 1u, P = 2u * W;
+    const uint32_t per_set = (W + share - 1u) / share;
+    const unsigned long long items = (unsigned long long)count * per_set;
+    uint32_t found = 0u;
+    for (unsigned long long item = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5); item < items;
+         item += gridDim.x * kWarpsPerBlock) {
+        const uint32_t idx = (uint32_t)(item / per_set), part = (uint32_t)(item % per_set);
+        const uint32_t S = sets[idx];
+        const uint32_t lo = part * share, hi = min(W, lo + share), per = (hi - lo + 31u) / 32u;
+        uint32_t hh = min(hi, lo + per * lane);
+        const uint32_t end = min(hi, hh + per);
+        uint32_t inside[4 * NW], odd[4 * NW];
+        pairs_inside<NW>(d, S, inside);
+#pragma unroll
+        for (int w = 0; w < 4 * NW; w++) odd[w] = 0u;
+        uint32_t L = hh < end ? pdep32(hh + 1u, S) : 0u;
+        pairs_flip<NW>(d, L, odd);
+        unsigned long long key = ~0ull;
+        uint32_t first = kFull;
+        bool first_nan = false;
+        float rows = 0.0f, startup = 0.0f;
+        int width = 0;
+        for (; hh < end; hh++) {
+            if (is_connected(L, adj) && is_connected(S ^ L, adj)) {
+                const float4 l = __ldcg(memo + L), r = __ldcg(memo + (S ^ L));
+                JoinCost lr, rl;
+                pairs_mirror<NW>(d, pp, odd, inside, l, r, lr, rl);
+                width = (int)((__float_as_uint(l.w) & kWidthMask) + (__float_as_uint(r.w) & kWidthMask));
+                found += 2u;
+                // the lane's first valid candidate is its first valid split as
+                // it stands: mirrors come after every split
+                if (first == kFull) {
+                    first = hh;
+                    first_nan = isnan(lr.total);
+                }
+                const unsigned long long k0 = ((unsigned long long)ord_float(lr.total) << 32) | hh;
+                if (k0 < key && !isnan(lr.total)) {
+                    key = k0;
+                    rows = lr.rows;
+                    startup = lr.startup;
+                }
+                const unsigned long long k1 = ((unsigned long long)ord_float(rl.total) << 32) | (P - 1u - hh);
+                if (k1 < key && !isnan(rl.total)) {
+                    key = k1;
+                    rows = rl.rows;
+                    startup = rl.startup;
+                }
+            }
+            const uint32_t next = next_subset(L, S);
+            pairs_flip<NW>(d, L ^ next, odd);
+            L = next;
+        }
+        __syncwarp();
+        const uint32_t kh = (uint32_t)(key >> 32), kl = (uint32_t)key;
+        const uint32_t mh = __reduce_min_sync(kFull, kh);
+        const uint32_t ml = __reduce_min_sync(kFull, kh == mh ? kl : kFull);
+        const uint32_t mf = __reduce_min_sync(kFull, first);
+        const bool nan = __any_sync(kFull, first == mf && first_nan);
+        const unsigned long long mk = ((unsigned long long)mh << 32) | ml;
+        if (per_set > 1u) {
+            if (lane == 0u) {
+                if (mk != ~0ull) atomicMin(keys + idx, mk);
+                atomicMin(firsts + idx, ((unsigned long long)mf << 1) | (nan ? 1ull : 0ull));
+            }
+            continue;
+        }
+        if (nan) {
+            if (first == mf && first_nan) {
+                const uint32_t nl = pdep32(mf + 1u, S);
+                const RelVal l = load_rel(memo, nl, h.hz_packed), r = load_rel(memo, S ^ nl, h.hz_packed);
+                memo_write(h, memo, memo_left, S, join_eval(d, nl, l, S ^ nl, r), nl);
+            }
+        } else if (key == mk && key != ~0ull) {
+            RelVal out;
+            out.rows = rows;
+            out.startup = startup;
+            out.total = __uint_as_float((kh & 0x80000000u) ? kh ^ 0x80000000u : ~kh);   // the inverse of ord_float
+            out.width = width;
+            memo_write(h, memo, memo_left, S, out, pdep32(kl + 1u, S));
+        }
+    }
+    found = __reduce_add_sync(kFull, found);
+    if (lane == 0u && found) atomicAdd(&glob->evaluated_pairs, (unsigned long long)found);
+}
+
+// winners of the sets that k_dense took in shares; leaves the keys at all ones
+// for the next level
+__global__ void __launch_bounds__(kBlock) k_dense_finalize(const uint32_t *__restrict__ blob, uint32_t blob_words,
+                                                           const uint32_t *__restrict__ sets,
+                                                           const LevelCounters *__restrict__ lc, float4 *__restrict__ memo,
+                                                           uint32_t *__restrict__ memo_left,
+                                                           unsigned long long *__restrict__ keys,
+                                                           unsigned long long *__restrict__ firsts) {
+    const uint32_t count = lc->n_sets;
+    extern __shared__ __align__(16) uint32_t sm[];
+    load_blob_to_smem(blob, blob_words, sm);
+    const DevInfoView d = make_view(sm);
+    for (uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x; idx < count; idx += gridDim.x * blockDim.x) {
+        const uint32_t S = sets[idx];
+        const unsigned long long first = firsts[idx];
+        const uint32_t p = (first & 1ull) ? (uint32_t)(first >> 1) : (uint32_t)keys[idx];
+        const uint32_t L = pdep32(p + 1u, S);
+        const RelVal l = load_rel(memo, L, d.h->hz_packed), r = load_rel(memo, S ^ L, d.h->hz_packed);
+        memo_write(*d.h, memo, memo_left, S, join_eval(d, L, l, S ^ L, r), L);
+        keys[idx] = firsts[idx] = ~0ull;
     }
 }
 
@@ -1992,8 +2138,14 @@ public:
         const uint32_t max_block = reinterpret_cast<const DevHeader *>(h_blob)->max_block;
         const bool tree_mode = reinterpret_cast<const DevHeader *>(h_blob)->tree_mode != 0u;
         const int eval_max_blocks = sm_count * 4;
+        const bool dense = dense_pairs(*reinterpret_cast<const DevHeader *>(h_blob));
+        const int nw = ec_stride(reinterpret_cast<const DevHeader *>(h_blob)->n_ec) / 4;
         CK(cudaMemsetAsync(d_ctl, 0, kCtlClearBytes, stream));
         CK(cudaMemsetAsync(a.seen, 0, std::max<uint64_t>((1ull << n) / 8, 4), stream));
+        if (mode == kModeDpsub && dense) {   // no winner yet (k_dense_finalize leaves them so)
+            CK(cudaMemsetAsync(a.ovf_key, 0xFF, max_level_sets(n) * sizeof(unsigned long long), stream));
+            CK(cudaMemsetAsync(a.ovf_first, 0xFF, max_level_sets(n) * sizeof(unsigned long long), stream));
+        }
         n_kernels = 0;
         k_init_base<<<1, 32, 0, stream>>>(a.blob, a.memo, a.memo_left);
         n_kernels++;
@@ -2012,7 +2164,21 @@ public:
             n_kernels += 2;
             int eblocks = (int)std::min<uint64_t>((uint64_t)eval_max_blocks, (total + kWarpsPerBlock - 1) / kWarpsPerBlock);
             CK(cudaEventRecordWithFlags(kev[2 * k], stream, cudaEventRecordExternal));
-            if (mode == kModeDpsub) {
+            const uint32_t W = (uint32_t)((1ull << (k - 1)) - 1ull);   // unordered splits of a k-set
+            if (mode == kModeDpsub && dense) {
+                // whole sets per warp while a level has enough of them, shares
+                // of a set otherwise
+                const uint64_t shares = (total * W) / ((uint64_t)sm_count * 3 * kWarpsPerBlock * 4);
+                uint32_t share = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(shares, 512u), 4096u);
+                const bool whole = W <= std::max(share, kDenseWhole);
+                if (whole) share = W;
+                n_kernels += whole ? 0 : 1;
+                (nw == 1 ? k_dense<1> : k_dense<2>)<<<sm_count * 3, kBlock, (size_t)((blob_words + 3u) & ~3u) * 4u, stream>>>(
+                    a.blob, blob_words, k, cur_sets, lc, a.memo, a.memo_left, a.ovf_key, a.ovf_first, a.glob, share);
+                if (!whole)
+                    k_dense_finalize<<<sm_count, kBlock, (size_t)((blob_words + 3u) & ~3u) * 4u, stream>>>(
+                        a.blob, blob_words, cur_sets, lc, a.memo, a.memo_left, a.ovf_key, a.ovf_first);
+            } else if (mode == kModeDpsub) {
                 k_eval<kModeDpsub><<<eblocks, kBlock, smem, stream>>>(a.blob, blob_words, k, cur_sets, lc, a.memo,
                                                                       a.memo_left, a.ovf_set, a.ovf_P, a.ovf_off,
                                                                       a.ovf_key, a.ovf_first, a.glob, ccc);
@@ -2035,7 +2201,7 @@ public:
             CK(cudaEventRecordWithFlags(kev[2 * k + 1], stream, cudaEventRecordExternal));
             bool may_overflow;
             if (mode == kModeDpsub) {
-                may_overflow = ((1ull << k) - 2ull) > kOvfLimit;
+                may_overflow = !dense && ((1ull << k) - 2ull) > kOvfLimit;
             } else {
                 // sum over blocks of 2^|b| - 2 with sum(|b| - 1) = k - 1 and
                 // |b| <= the query graph's largest block
@@ -2164,6 +2330,9 @@ public:
             CK(cudaFuncSetAttribute(k_dpsize_eval, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
             CK(cudaFuncSetAttribute(k_eval<kModeDpsub>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
             CK(cudaFuncSetAttribute(k_eval<kModeMpdp>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            CK(cudaFuncSetAttribute(k_dense<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            CK(cudaFuncSetAttribute(k_dense<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            CK(cudaFuncSetAttribute(k_dense_finalize, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
             CK(cudaFuncSetAttribute(k_ovf_chunks<kModeDpsub>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
             CK(cudaFuncSetAttribute(k_ovf_chunks<kModeMpdp>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
             CK(cudaFuncSetAttribute(k_ovf_finalize<kModeDpsub>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -2173,8 +2342,11 @@ public:
         exec = nullptr;
         const uint32_t mb = reinterpret_cast<const DevHeader *>(h_blob)->max_block;
         const uint32_t tm = reinterpret_cast<const DevHeader *>(h_blob)->tree_mode;
-        GraphKey key{n, ((int)mode * 64 + (int)std::min<uint32_t>(mb, 63u)) * 2 + (int)(tm != 0u), ccc ? 1 : 0,
-                     (int)words};
+        // the dense kernels are instantiated by the words of a class row
+        const DevHeader *hb = reinterpret_cast<const DevHeader *>(h_blob);
+        const int dense = (mode == kModeDpsub && dense_pairs(*hb)) ? ec_stride(hb->n_ec) / 4 : 0;
+        GraphKey key{n, (((int)mode * 64 + (int)std::min<uint32_t>(mb, 63u)) * 2 + (int)(tm != 0u)) * 4 + dense,
+                     ccc ? 1 : 0, (int)words};
         (void)profile;
         auto it = graphs.find(key);
         if (it != graphs.end()) {

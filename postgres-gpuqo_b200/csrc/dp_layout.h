@@ -113,11 +113,23 @@ struct DevHeader {
     // (DevInfoView::plain) and a row of the widest set within work_mem: the
     // cost of a split is straight-line arithmetic on TreeEdge (plain_mirror)
     uint32_t tree_plain;
-    uint32_t pad_;
+    // not a tree: every class plain with one selectivity for both orientations
+    // and at most 256 of them, hz_packed, hash joins enabled and a row of the
+    // widest set within work_mem: the word offset of PlainQuals[n_ec + 1] by
+    // the number of matching classes (pairs_match, plain_mirror); 0: no
+    uint32_t pairs_plain;
 };
 
 // the work_mem of the hash join's skew check, as the reference compares it
 inline float work_mem_bytes_of(int work_mem) { return (float)((long long)work_mem * 1024LL); }
+
+// What the quals of a join contribute to its cost, by their number (exactly
+// the device's float operations): the per-tuple cost summed qual by qual,
+// cpu_operator_cost * quals, and the two sums with cpu_tuple_cost that the
+// nested loop and the hash join start from.
+struct alignas(16) PlainQuals {
+    float per_tuple, quals_cost, nl_tuple, hj_row;
+};
 
 // Tree tables (tree_mode), appended after the class arrays at word tree_tab.
 // Word r of the first 32 is the word offset of root r's rows from tree_tab
@@ -135,12 +147,10 @@ inline float work_mem_bytes_of(int work_mem) { return (float)((long long)work_me
 // one 8-byte load; the second rows serve the enumeration index, which only
 // equal costs and NaN costs ask for.
 struct TreeEdge {
-    // the classes on the edge, accumulated in class order (exactly the
-    // device's float operations): the selectivity product with the lower end's
-    // side outer and with the higher end's, the per-tuple cost of the quals,
-    // cpu_operator_cost * quals, and the two sums with cpu_tuple_cost that the
-    // nested loop and the hash join start from
-    float sel_lo, sel_hi, per_tuple, quals_cost, nl_tuple, hj_row;
+    PlainQuals quals;
+    // the selectivity product over the edge's classes in class order with the
+    // lower end's side outer and with the higher end's
+    float sel_lo, sel_hi;
     uint32_t classes;                     // class mask (DevHeader::ec_masked)
     uint32_t pad;
 };

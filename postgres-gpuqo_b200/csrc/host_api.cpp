@@ -343,6 +343,16 @@ static int max_block_size(const HostInfo &info) {
     return best;
 }
 
+static PlainQuals plain_quals(const DevHeader &h, int quals) {
+    PlainQuals q;
+    q.per_tuple = 0.0f;
+    for (int i = 0; i < quals; i++) q.per_tuple += h.cpu_operator_cost;
+    q.quals_cost = h.cpu_operator_cost * (float)quals;
+    q.nl_tuple = h.cpu_tuple_cost + q.per_tuple;
+    q.hj_row = q.quals_cost + h.cpu_tuple_cost;
+    return q;
+}
+
 std::vector<uint32_t> build_blob(const HostInfo &info) {
     const int n_ec = (int)info.ec_relids.size();
     const int n_sels = (int)info.ec_sels.size();
@@ -375,7 +385,8 @@ std::vector<uint32_t> build_blob(const HostInfo &info) {
         for (int r = 0; r < n; r++)
             if (r == 0 || ((info.edge[r] >> 1) >> r) > 1ull) tree_words += tree_row_words(n);
     }
-    std::vector<uint32_t> blob(base_words + tree_words, 0u);
+    const uint32_t pairs_words = (!tree && n_ec > 0 && n_ec <= 256) ? (uint32_t)(n_ec + 1) * 4u : 0u;
+    std::vector<uint32_t> blob(base_words + tree_words + pairs_words, 0u);
     DevHeader *h = reinterpret_cast<DevHeader *>(blob.data());
     h->n = n;
     h->n_ec = n_ec;
@@ -516,6 +527,11 @@ std::vector<uint32_t> build_blob(const HostInfo &info) {
     for (int i = 0; i < n_sels; i++) sels[i] = info.ec_sels[i];
     fill_rel_ecs(v, n);
     fill_pair_sel(v);
+    // the straight-line cost (plain_mirror) leaves out the skew check, which
+    // compares one row of the inner side with work_mem: the widest set's row
+    // decides for all
+    const float widest = (float)((((unsigned long long)std::max(width_sum, 0ll) + 7ull) & ~7ull) + 24ull);
+    const bool straight = h->hz_packed && h->enable_hashjoin && widest <= h->work_mem_bytes;
     if (h->ec_masked) {
         // ec_selectivity (gpuqo_row_estimation.cuh:49-88) of each two-member
         // class in both orientations: the FK selectivity of the outer member's
@@ -536,26 +552,37 @@ std::vector<uint32_t> build_blob(const HostInfo &info) {
             TreeEdge &e = edges[c];
             e.classes = h->edge_ec[c];
             e.sel_lo = e.sel_hi = 1.0f;
-            e.per_tuple = 0.0f;
             int quals = 0;
             for (uint32_t m = e.classes; m; m &= m - 1u, quals++) {
                 const int i = __builtin_ctz(m);
                 e.sel_lo *= h->edge_sel[0][i];
                 e.sel_hi *= h->edge_sel[1][i];
-                e.per_tuple += h->cpu_operator_cost;
                 plain = plain && ((v.plain[0] >> i) & 1u);
             }
             // an edge without a class joins without quals: bucket size and MCV
             // frequency stay 1, which the general pass computes
             plain = plain && quals > 0;
-            e.quals_cost = h->cpu_operator_cost * (float)quals;
-            e.nl_tuple = h->cpu_tuple_cost + e.per_tuple;
-            e.hj_row = e.quals_cost + h->cpu_tuple_cost;
+            e.quals = plain_quals(*h, quals);
         }
-        // the skew check of a plain split compares one row of the inner side
-        // with work_mem; the widest set's row decides for all
-        const float widest = (float)((((unsigned long long)std::max(width_sum, 0ll) + 7ull) & ~7ull) + 24ull);
-        h->tree_plain = (plain && h->hz_packed && h->enable_hashjoin && widest <= h->work_mem_bytes) ? 1u : 0u;
+        h->tree_plain = (plain && straight) ? 1u : 0u;
+    }
+    if (pairs_words) {
+        bool plain = straight && h->all_pairs;
+        uint32_t joined[32] = {};   // by classes
+        for (int i = 0; plain && i < n_ec; i++) {
+            plain = ((v.plain[i / 32] >> (i % 32)) & 1u) &&
+                    std::memcmp(&v.pair_sel[2 * i], &v.pair_sel[2 * i + 1], sizeof(float)) == 0;
+            joined[__builtin_ctz(relids[i])] |= relids[i];
+            joined[31 - __builtin_clz(relids[i])] |= relids[i];
+        }
+        // every split has a qual (without one the bucket size and the MCV
+        // frequency stay 1, which the general pass computes)
+        for (int i = 0; plain && i < n; i++) plain = (h->adj[i] & ~joined[i]) == 0u;
+        if (plain) {
+            h->pairs_plain = base_words;
+            PlainQuals *q = reinterpret_cast<PlainQuals *>(blob.data() + base_words);
+            for (int i = 0; i <= n_ec; i++) q[i] = plain_quals(*h, i);
+        }
     }
     return blob;
 }
