@@ -900,11 +900,10 @@ __device__ __noinline__ bool tree_nan_rule(const DevInfoView d, uint32_t S, bool
 // entries of the next split are requested before the current one is costed.
 // The whole warp calls it, with the same k and G.
 template <int LAYOUT>
-__device__ __forceinline__ void tree_set(const DevInfoView &d, const PlainParams &pp, uint32_t S, bool has, int k, int G,
-                                         float4 *memo, uint32_t *memo_left) {
+__device__ __forceinline__ void tree_set(const DevInfoView &d, const PlainParams &pp, const TreeRows &t, uint32_t S,
+                                         bool has, int k, int G, float4 *memo, uint32_t *memo_left) {
     const DevHeader &h = *d.h;
     const int lane = threadIdx.x & 31, gl = lane & (G - 1);
-    const TreeRows t = tree_rows(h, has ? S : 0u);
     uint32_t x = has ? S & (S - 1u) : 0u;
     if (G == 32) {
         x &= 1u << lane;   // at most 31 child ends: the lane's own relation
@@ -1002,7 +1001,8 @@ __device__ __forceinline__ void tree_level(const DevInfoView &d, const PlainPara
     const uint32_t per_warp = 32u / (uint32_t)G, grp = (threadIdx.x & 31u) / (uint32_t)G;
     for (uint32_t base = gwarp * per_warp; base < count; base += nwarps * per_warp) {
         const bool has = base + grp < count;
-        tree_set<LAYOUT>(d, pp, has ? __ldcg(sets + base + grp) : 0u, has, k, G, memo, memo_left);
+        const uint32_t S = has ? __ldcg(sets + base + grp) : 0u;
+        tree_set<LAYOUT>(d, pp, tree_rows(*d.h, S), S, has, k, G, memo, memo_left);
     }
 }
 
@@ -2954,7 +2954,7 @@ struct BatchQ {
     uint32_t blob_off;                 // word offset into the wave's blob buffer
     uint32_t n;
     uint32_t first_base;               // index of its first singleton in the level-1 list
-    uint32_t pad;
+    uint32_t tree_tab;                 // word offset of its tree tables in the wave's blob buffer
     unsigned long long memo_off;       // entry offset into the memo arena
     unsigned long long seen_off;       // word offset into the dedup bitmap arena
 };
@@ -3026,10 +3026,7 @@ __device__ __forceinline__ void stage_flush64(unsigned long long *st, uint32_t &
 }
 
 // connected k-sets of every query, by extension of its (k-1)-sets (c_prev
-// items in prev); thread tid of nthreads.  TREE_ONLY (every query of the wave
-// tree-shaped): each set is emitted once by the largest-leaf rule of
-// tree_enum_phase, without the dedup bitmap.
-template <bool TREE_ONLY>
+// items in prev); thread tid of nthreads (per-level launches)
 __device__ __forceinline__ void batch_extend(const BatchQ *qs, const uint32_t *blobs, const unsigned long long *prev,
                                              uint32_t c_prev, uint32_t *seen, unsigned long long *out,
                                              LevelCounters *lc, unsigned long long *st, uint32_t tid,
@@ -3038,43 +3035,26 @@ __device__ __forceinline__ void batch_extend(const BatchQ *qs, const uint32_t *b
     const uint32_t rounds = (c_prev + nthreads - 1u) / nthreads;
     for (uint32_t r = 0; r < rounds; r++) {
         const uint32_t idx = tid + r * nthreads;
-        uint32_t S = 0u, N = 0u, q = 0u, leaves = 0u;
+        uint32_t S = 0u, N = 0u, q = 0u;
         unsigned long long seen_off = 0;
-        const uint32_t *adj = nullptr;
         if (idx < c_prev) {
             const unsigned long long it = __ldcg(prev + idx);
             q = (uint32_t)(it >> 32);
             S = (uint32_t)it;
             const BatchQ Q = qs[q];
-            adj = reinterpret_cast<const DevHeader *>(blobs + Q.blob_off)->adj;
+            const uint32_t *adj = reinterpret_cast<const DevHeader *>(blobs + Q.blob_off)->adj;
             seen_off = Q.seen_off;
-            uint32_t x = S;
-            while (x) {
-                int v = __ffs(x) - 1;
-                x &= x - 1u;
-                const uint32_t a = __ldg(adj + v);
-                N |= a;
-                if (TREE_ONLY && __popc(a & S) == 1) leaves |= 1u << v;
-            }
+            for (uint32_t x = S; x; x &= x - 1u) N |= __ldg(adj + lowest_idx(x));
             N &= ~S;
         }
-        const bool single = (S & (S - 1u)) == 0u;
-        const int deg = __popc(N);
-        const int maxdeg = (int)__reduce_max_sync(kFull, (uint32_t)deg);
+        const int maxdeg = (int)__reduce_max_sync(kFull, (uint32_t)__popc(N));
         for (int j = 0; j < maxdeg; j++) {
-            bool ok = false;
+            bool ok = N != 0u;
             unsigned long long item = 0;
-            if (j < deg) {
-                const uint32_t bitv = N & (0u - N);
-                N ^= bitv;
-                const uint32_t T = S | bitv;
-                if (TREE_ONLY) {
-                    const uint32_t p = __ldg(adj + (__ffs(bitv) - 1)) & S;   // v's only neighbour in S
-                    ok = (single ? S : (leaves & ~p)) < bitv;                // v is T's largest leaf
-                } else {
-                    const uint32_t bm = 1u << (T & 31u);
-                    ok = !(atomicOr(&seen[seen_off + (T >> 5)], bm) & bm);
-                }
+            if (ok) {
+                const uint32_t T = S | (N & (0u - N)), bm = 1u << (T & 31u);
+                N &= N - 1u;
+                ok = !(atomicOr(&seen[seen_off + (T >> 5)], bm) & bm);
                 item = ((unsigned long long)q << 32) | T;
             }
             stage_emit64(st, cnt, ok, item, out, lc);
@@ -3092,7 +3072,7 @@ __global__ void __launch_bounds__(kBlock) kb_level_sets(const BatchQ *__restrict
                                                         LevelCounters *__restrict__ lc) {
     __shared__ unsigned long long stage[kWarpsPerBlock][64];
     const int warp = threadIdx.x >> 5;
-    batch_extend<false>(qs, blobs, prev, __ldcg(&prev_lc->n_sets), seen, out, lc, stage[warp],
+    batch_extend(qs, blobs, prev, __ldcg(&prev_lc->n_sets), seen, out, lc, stage[warp],
                  blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
 }
 
@@ -3108,10 +3088,8 @@ __device__ __forceinline__ void tree_cand(const DevHeader &h, uint32_t S, uint32
     ecm = masked ? reinterpret_cast<const TreeEdge *>(t.tab + tree_edge_off(t.n))[t.row[2u * v + 1u] & 31u].classes : 0u;
 }
 
-// ALL_MASKED (with TREE_ONLY): every query of the wave has only two-member
-// classes on tree edges (DevHeader::ec_masked), so the general class pass
-// is not compiled in
-template <int G, bool TREE_ONLY, bool ALL_MASKED = false>
+// the sets of one level of every query in groups of G lanes (per-level launches)
+template <int G>
 __device__ __forceinline__ void batch_groups(const BatchQ *qs, const uint32_t *blobs, uint32_t first, uint32_t stride,
                                              const unsigned long long *items, uint32_t count, int k, float4 *memo_all,
                                              uint32_t *memo_left_all, unsigned long long &pairs) {
@@ -3133,14 +3111,14 @@ __device__ __forceinline__ void batch_groups(const BatchQ *qs, const uint32_t *b
         const DevHeader &h = *d.h;
         float4 *memo = memo_all + Q.memo_off;
         uint32_t *memo_left = memo_left_all + Q.memo_off;
-        const bool tree = has && (TREE_ONLY || h.tree_mode != 0u);
-        const bool masked = ALL_MASKED || (tree && h.ec_masked != 0u);
+        const bool tree = has && h.tree_mode != 0u;
+        const bool masked = tree && h.ec_masked != 0u;
         uint32_t P = 0;
         B.nb = 0;
         if (has) {
             if (tree) {
                 P = 2u * (uint32_t)(k - 1);
-            } else if (!TREE_ONLY) {
+            } else {
                 find_blocks(S, h.adj, B);
                 P = B.etotal;
             }
@@ -3161,7 +3139,7 @@ __device__ __forceinline__ void batch_groups(const BatchQ *qs, const uint32_t *b
                     for (; end_rank < (c >> 1); end_rank++) ends &= ends - 1u;
                     tree_cand(h, S, (uint32_t)lowest_idx(ends), c, L, R, p, ecm, masked);
                     valid = true;
-                } else if (!TREE_ONLY) {
+                } else {
                     uint32_t key;
                     valid = mpdp_candidate(S, B, h.adj, c, bcur, L, R, key, cc);
                     p = valid ? key_index(h, key, L, S) : key;
@@ -3169,8 +3147,7 @@ __device__ __forceinline__ void batch_groups(const BatchQ *qs, const uint32_t *b
             }
             if (valid) {
                 RelVal l = load_rel(memo, L, d.h->hz_packed), r = load_rel(memo, R, d.h->hz_packed);
-                RelVal out = (ALL_MASKED || masked) ? join_eval_t<true>(d, L, l, R, r, ecm)
-                                                    : join_eval_t<false>(d, L, l, R, r, 0u);
+                RelVal out = masked ? join_eval_t<true>(d, L, l, R, r, ecm) : join_eval_t<false>(d, L, l, R, r, 0u);
                 best_update(best, p, L, out);
             }
         }
@@ -3215,9 +3192,9 @@ __global__ void __launch_bounds__(kBlock) kb_eval(const BatchQ *__restrict__ qs,
     const uint32_t gwarp = blockIdx.x * kWarpsPerBlock + warp;
     const uint32_t nwarps = gridDim.x * kWarpsPerBlock;
     unsigned long long pairs = 0;
-    if (G == 2) batch_groups<2, false>(qs, blobs, gwarp * 16, nwarps * 16, items, count, k, memo, memo_left, pairs);
-    else if (G == 8) batch_groups<8, false>(qs, blobs, gwarp * 4, nwarps * 4, items, count, k, memo, memo_left, pairs);
-    else batch_groups<32, false>(qs, blobs, gwarp, nwarps, items, count, k, memo, memo_left, pairs);
+    if (G == 2) batch_groups<2>(qs, blobs, gwarp * 16, nwarps * 16, items, count, k, memo, memo_left, pairs);
+    else if (G == 8) batch_groups<8>(qs, blobs, gwarp * 4, nwarps * 4, items, count, k, memo, memo_left, pairs);
+    else batch_groups<32>(qs, blobs, gwarp, nwarps, items, count, k, memo, memo_left, pairs);
     pairs = __reduce_add_sync(kFull, (uint32_t)pairs);
     if (lane == 0 && pairs) atomicAdd(&glob->evaluated_pairs, pairs);
 }
@@ -3503,12 +3480,59 @@ __global__ void kb_extract(const BatchQ *__restrict__ qs, int nq, const uint32_t
 // kb_dp: a wave of tree-shaped queries in ONE cooperative, persistent launch.
 // Phase 0 writes every query's base relations and emits its level-2 sets
 // (one warp per query, one lane per relation: each edge once, from its lower
-// end).  Then, per level k, the grid evaluates level k of every query while
-// it enumerates level k+1, with a grid barrier between levels; the plans are
-// extracted (one warp per query) after the last level.  The grid barrier
-// is bounded (grid_barrier); on timeout the host reruns the wave with
-// per-level launches.
-template <bool ALL_MASKED>
+// end).  Then, per level k, the grid evaluates level k of every query
+// (tree_set, the planner infos in global memory) while it enumerates level
+// k+1, with a grid barrier between levels; the plans are extracted (one warp
+// per query) after the last level.  The grid barrier is bounded
+// (grid_barrier); on timeout the host reruns the wave with per-level launches.
+// Bound: issue in the wide levels, the chain item -> query -> tables -> memo
+// entries in the narrow ones.  With both orientations of a split taken
+// together and no class pass (see k_dp_tree), device time of 96 queries of 10 to
+// 20 relations (77 M pairs, its wave of cycles included) 2230 -> 1220 us, of
+// 512 queries of 8 to 16 (23.7 M pairs) 1040 -> 650 us.
+__device__ __forceinline__ void batch_tree_enum(const BatchQ *qs, const uint32_t *blobs, const unsigned long long *prev,
+                                                uint32_t c_prev, unsigned long long *out, LevelCounters *lc,
+                                                uint32_t tid, uint32_t nthreads) {
+    const uint32_t lane = threadIdx.x & 31u;
+    for (uint32_t first = tid & ~31u; first < c_prev; first += nthreads) {
+        const uint32_t idx = first + (tid & 31u);
+        const unsigned long long it = idx < c_prev ? __ldcg(prev + idx) : 0ull;
+        const uint32_t *adj = reinterpret_cast<const DevHeader *>(blobs + qs[it >> 32].blob_off)->adj;
+        uint32_t ext = tree_extensions((uint32_t)it, [&](int v) { return __ldg(adj + v); });
+        const uint32_t cnt = (uint32_t)__popc(ext);
+        uint32_t incl = cnt;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const uint32_t o = __shfl_up_sync(kFull, incl, off);
+            if (lane >= (uint32_t)off) incl += o;
+        }
+        uint32_t base = 0u;
+        if (lane == 31u && incl) base = atomicAdd(&lc->n_sets, incl);
+        uint32_t at = __shfl_sync(kFull, base, 31) + incl - cnt;
+        for (; ext; ext &= ext - 1u) out[at++] = it | (ext & (0u - ext));
+    }
+}
+
+template <int LAYOUT>
+__device__ __forceinline__ void batch_tree_level(const BatchQ *qs, const uint32_t *blobs, uint32_t gwarp, uint32_t nwarps,
+                                                 const unsigned long long *items, uint32_t count, int k, int G,
+                                                 float4 *memo, uint32_t *memo_left) {
+    const uint32_t per_warp = 32u / (uint32_t)G, grp = (threadIdx.x & 31u) / (uint32_t)G;
+    for (uint32_t base = gwarp * per_warp; base < count; base += nwarps * per_warp) {
+        const bool has = base + grp < count;
+        const unsigned long long it = has ? __ldcg(items + base + grp) : 0ull;
+        const uint32_t S = (uint32_t)it;
+        const BatchQ Q = qs[it >> 32];
+        const DevInfoView d = make_view(blobs + Q.blob_off);
+        TreeRows t;
+        t.tab = blobs + Q.tree_tab;
+        t.n = (int)Q.n;
+        t.row = t.tab + (has ? t.tab[lowest_idx(S)] : 0u);
+        tree_set<LAYOUT>(d, plain_params(*d.h), t, S, has, k, G, memo + Q.memo_off, memo_left + Q.memo_off);
+    }
+}
+
+template <int LAYOUT>
 __global__ void __launch_bounds__(kBlock, 3) kb_dp(const BatchQ *__restrict__ qs, int nq, int maxn,
                                                    const uint32_t *__restrict__ blobs, float4 *__restrict__ memo,
                                                    uint32_t *__restrict__ memo_left,
@@ -3516,8 +3540,7 @@ __global__ void __launch_bounds__(kBlock, 3) kb_dp(const BatchQ *__restrict__ qs
                                                    unsigned long long *__restrict__ listB,
                                                    LevelCounters *__restrict__ lvl, GlobalCounters *__restrict__ glob,
                                                    TreeNode *__restrict__ tree, int *__restrict__ tree_n,
-                                                   unsigned *__restrict__ bar, uint32_t target_lanes,
-                                                   unsigned poll_limit) {
+                                                   unsigned *__restrict__ bar, uint32_t sms, unsigned poll_limit) {
     const unsigned max_polls = barrier_polls(poll_limit);
     __shared__ unsigned long long stage[kWarpsPerBlock][64];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -3564,18 +3587,10 @@ __global__ void __launch_bounds__(kBlock, 3) kb_dp(const BatchQ *__restrict__ qs
         unsigned long long *nxt = (k & 1) ? listA : listB;
         const uint32_t count = __ldcg(&lvl[k].n_sets);
         // enumeration from the far end of the grid, evaluation from the start
-        if (k < maxn) batch_extend<true>(qs, blobs, cur, count, nullptr, nxt, lvl + k + 1, st, nthreads - 1u - tid, nthreads);
-        int max_group = 1;
-        while (max_group < 32 && max_group < 2 * (k - 1)) max_group <<= 1;
-        int G = 2;
-        while (G < max_group && (uint64_t)count * (uint64_t)G < (uint64_t)target_lanes) G <<= 1;
-        G = G <= 2 ? 2 : (G <= 8 ? 8 : 32);
-        if (G == 2)
-            batch_groups<2, true, ALL_MASKED>(qs, blobs, gwarp * 16, nwarps * 16, cur, count, k, memo, memo_left, pairs);
-        else if (G == 8)
-            batch_groups<8, true, ALL_MASKED>(qs, blobs, gwarp * 4, nwarps * 4, cur, count, k, memo, memo_left, pairs);
-        else
-            batch_groups<32, true, ALL_MASKED>(qs, blobs, gwarp, nwarps, cur, count, k, memo, memo_left, pairs);
+        if (k < maxn) batch_tree_enum(qs, blobs, cur, count, nxt, lvl + k + 1, nthreads - 1u - tid, nthreads);
+        batch_tree_level<LAYOUT>(qs, blobs, gwarp, nwarps, cur, count, k, tree_group(count, k, nthreads, sms), memo,
+                                 memo_left);
+        pairs += (unsigned long long)count * 2ull * (unsigned long long)(k - 1);   // every split edge, both orientations
         if (!grid_barrier<false>(bar, epoch, max_polls)) return;
     }
 
@@ -3587,8 +3602,7 @@ __global__ void __launch_bounds__(kBlock, 3) kb_dp(const BatchQ *__restrict__ qs
         extract_plan(memo + Q.memo_off, memo_left + Q.memo_off, full, wmask, reinterpret_cast<uint32_t *>(st),
                      tree + (size_t)q * 64, tree_n + q);
     }
-    pairs = __reduce_add_sync(kFull, (uint32_t)pairs);
-    if (lane == 0 && pairs) atomicAdd(&glob->evaluated_pairs, pairs);
+    if (tid == 0) glob->evaluated_pairs = pairs;
 }
 
 // Candidate bound of a query for the batch (the batch has no overflow path):
@@ -3685,8 +3699,7 @@ struct BatchEngine {
     GlobalCounters *glob = nullptr;
     unsigned *bar = nullptr, *h_bar = nullptr;   // grid barrier words (device, pinned copy)
     int coop_grid = -1;                          // co-resident blocks of kb_gen<false> (0: no cooperative launch)
-    int coop_grid_tree = -1;                     // co-resident blocks of kb_dp<false>
-    int coop_grid_masked = -1;                   // co-resident blocks of kb_dp<true>
+    int coop_grid_tree[3] = {-1, -1, -1};        // co-resident blocks of kb_dp by layout (tree_layout)
     std::map<size_t, int> coop_one;              // dynamic shared bytes -> co-resident blocks of kb_gen<true>
     bool barrier_timed_out = false;              // a grid barrier gave up: per-level launches until reset
     BatchOvf ovf{};                              // overflow list of kb_gen
@@ -3718,20 +3731,22 @@ struct BatchEngine {
         CK(cudaMalloc(&glob, sizeof(GlobalCounters)));
         CK(cudaMalloc(&bar, 4 * sizeof(unsigned)));
         CK(cudaMallocHost(&h_bar, 4 * sizeof(unsigned)));
-        int dev_coop = 0, occ = 0, occ_tree = 0, occ_masked = 0;
+        int dev_coop = 0, occ = 0, occ_tree[3] = {0, 0, 0};
         cudaDeviceGetAttribute(&dev_coop, cudaDevAttrCooperativeLaunch, device);
-        coop_grid = coop_grid_tree = coop_grid_masked = 0;
+        no_cooperative();
         if (dev_coop &&
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kb_gen<false>, kBlock, kGenSmem) == cudaSuccess &&
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_tree, kb_dp<false>, kBlock, 0) == cudaSuccess &&
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_masked, kb_dp<true>, kBlock, 0) == cudaSuccess) {
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_tree[0], kb_dp<0>, kBlock, 0) == cudaSuccess &&
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_tree[1], kb_dp<1>, kBlock, 0) == cudaSuccess &&
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_tree[2], kb_dp<2>, kBlock, 0) == cudaSuccess) {
             coop_grid = occ * sm_count;
-            coop_grid_tree = occ_tree * sm_count;
-            coop_grid_masked = occ_masked * sm_count;
+            for (int i = 0; i < 3; i++) coop_grid_tree[i] = occ_tree[i] * sm_count;
         }
         cudaGetLastError();
         return 0;
     }
+
+    void no_cooperative() { coop_grid = coop_grid_tree[0] = coop_grid_tree[1] = coop_grid_tree[2] = 0; }
 
     // per-level launches of one wave (the queries, blobs and arena are staged)
     uint32_t enqueue_levels(int nq, int maxn, uint64_t seen_words) {
@@ -3773,27 +3788,26 @@ struct BatchEngine {
         return it->second;
     }
 
-    // the wave as one cooperative launch: kb_dp when every query is
-    // tree-shaped (kb_dp<true> when every class of every query is also a
-    // two-member class on a tree edge), else kb_gen (kb_gen<true> for one
-    // query); false when it could not start
-    bool enqueue_persistent(int nq, int maxn, uint32_t words, uint64_t seen_words, bool tree_only, bool all_masked) {
-        const bool masked = tree_only && all_masked;
+    // the wave as one cooperative launch: kb_dp<layout> when every query is
+    // tree-shaped (layout: the least of the queries' tree_layout), else kb_gen
+    // (layout < 0; kb_gen<true> for one query); false when it could not start
+    bool enqueue_persistent(int nq, int maxn, uint32_t words, uint64_t seen_words, int layout) {
+        const bool tree_only = layout >= 0;
         const int one = (!tree_only && nq == 1) ? one_grid(words) : 0;
-        const int grid = masked ? coop_grid_masked : (tree_only ? coop_grid_tree : (one > 0 ? one : coop_grid));
+        const int grid = tree_only ? coop_grid_tree[layout] : (one > 0 ? one : coop_grid);
         if (grid <= 0 || gpuqo_b200_persistent == 0 || barrier_timed_out) return false;
         cudaMemsetAsync(lvl, 0, 33 * sizeof(LevelCounters), stream);
         cudaMemsetAsync(glob, 0, sizeof(GlobalCounters), stream);
         if (!tree_only) cudaMemsetAsync(seen, 0, seen_words * 4, stream);
         cudaMemsetAsync(bar, 0, 4 * sizeof(unsigned), stream);
-        uint32_t target_lanes = (uint32_t)grid * kBlock;
         unsigned poll_limit = (unsigned)std::max(0, gpuqo_b200_barrier_poll_limit);
         cudaError_t e;
         if (tree_only) {
+            static const void *const variants[3] = {(const void *)kb_dp<0>, (const void *)kb_dp<1>, (const void *)kb_dp<2>};
+            uint32_t sms = (uint32_t)sm_count;
             void *args[] = {&qs, &nq, &maxn, &blobs, &memo, &memo_left, &listA, &listB,
-                            &lvl, &glob, &tree, &tree_n, &bar, &target_lanes, &poll_limit};
-            e = cudaLaunchCooperativeKernel(masked ? (const void *)kb_dp<true> : (const void *)kb_dp<false>, dim3(grid),
-                                            dim3(kBlock), args, 0, stream);
+                            &lvl, &glob, &tree, &tree_n, &bar, &sms, &poll_limit};
+            e = cudaLaunchCooperativeKernel(variants[layout], dim3(grid), dim3(kBlock), args, 0, stream);
         } else {
             void *args[] = {&qs, &nq, &maxn, &blobs, &words, &memo, &memo_left, &seen, &listA, &listB,
                             &lvl, &glob, &tree, &tree_n, &bar, &ovf, &poll_limit};
@@ -3803,7 +3817,7 @@ struct BatchEngine {
         }
         if (e != cudaSuccess) {
             cudaGetLastError();
-            coop_grid = coop_grid_tree = coop_grid_masked = 0;
+            no_cooperative();
             return false;
         }
         return true;
@@ -3831,7 +3845,7 @@ struct BatchEngine {
     }
 
     bool persistent_ready() const {
-        return coop_grid > 0 && coop_grid_tree > 0 && gpuqo_b200_persistent != 0 && !barrier_timed_out;
+        return coop_grid > 0 && coop_grid_tree[0] > 0 && gpuqo_b200_persistent != 0 && !barrier_timed_out;
     }
 
     // One wave: all queries' memos fit.  wb: per query planner-info blob.
@@ -3875,13 +3889,14 @@ struct BatchEngine {
         std::vector<BatchQ> hq(nq);
         uint64_t slots = 0, words = 0, seen_words = 0, items = 0, base = 0, ovf_need = 0;
         int maxn = 0;
-        bool tree_only = true, all_masked = true;
+        int layout = kTreePlain;   // of a wave of trees; -1: a graph with cycles among the queries
         for (int q = 0; q < nq; q++) {
             const DevHeader *h = reinterpret_cast<const DevHeader *>(wb[q]->data());
             const int n = h->n;
             hq[q].blob_off = (uint32_t)words;
             hq[q].n = (uint32_t)n;
             hq[q].first_base = (uint32_t)base;
+            hq[q].tree_tab = hq[q].blob_off + h->tree_tab;
             hq[q].memo_off = slots;
             hq[q].seen_off = seen_words;
             words += (wb[q]->size() + 3) & ~(size_t)3;
@@ -3891,8 +3906,7 @@ struct BatchEngine {
             base += (uint64_t)n;
             maxn = std::max(maxn, n);
             if (batch_needs_ovf(*wb[q])) ovf_need += max_level_sets(n);
-            tree_only = tree_only && h->tree_mode != 0u;
-            all_masked = all_masked && h->ec_masked != 0u;
+            layout = h->tree_mode != 0u ? std::min(layout, tree_layout(*h)) : -1;
         }
         items = std::max(items, base);
         ovf_need = std::min(ovf_need, kBatchOvfCap);
@@ -3969,7 +3983,7 @@ struct BatchEngine {
         };
         uint32_t kernels = 1;
         CK(cudaEventRecord(ev0, stream));
-        bool persistent = enqueue_persistent(nq, maxn, (uint32_t)words, seen_words, tree_only, all_masked);
+        bool persistent = enqueue_persistent(nq, maxn, (uint32_t)words, seen_words, layout);
         CK(cudaGetLastError());
         if (persistent) CK(cudaMemcpyAsync(h_bar, bar, 4 * sizeof(unsigned), cudaMemcpyDeviceToHost, stream));
         if (!persistent) kernels = enqueue_levels(nq, maxn, seen_words);

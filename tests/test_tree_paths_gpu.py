@@ -82,7 +82,11 @@ def test_tree_evaluation(name, setting):
             assert got.error == 0
             if alg == 5:   # two relations are a complete graph, which plain DPsub enumerates by subsets
                 assert got.stats["kernel_launches"] == 1
-            assert same_tree(got.tree, harness.run_port(q, alg)[0])
+            want = harness.run_port(q, alg)[0]
+            assert same_tree(got.tree, want)
+            # the same through a batch wave (its planner infos stay in global memory)
+            trees, rc = lib.run_batch([q, query.star(3, 1), q], capi.GPUQO_DPSUB, bicc=(alg == 5))
+            assert rc == 0 and same_tree(trees[0], want) and same_tree(trees[2], want)
     finally:
         for var, value in saved:
             var.value = value
