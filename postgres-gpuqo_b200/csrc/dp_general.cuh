@@ -19,6 +19,7 @@
 // in plain-DPsub order it is searched for.
 #pragma once
 
+#include "dp_cactus.cuh"
 #include "dp_device.cuh"
 
 namespace gqb {
@@ -40,6 +41,7 @@ struct GenScratch {
     uint16_t off[32];             // first group in tab, or first word in pre
     uint8_t st_u[32];
     uint32_t nb, cyc;
+    CactusScratch cactus;
     alignas(8) uint32_t queue[64 * 2];       // valid splits waiting for a full warp: candidate, side
 };
 
@@ -263,49 +265,41 @@ __device__ __forceinline__ void gen_cost(const DevInfoView &d, const GenScratch 
     gen_update(best, *d.h, ws, S, c, S ^ L, o1);
 }
 
-// Splits [lo, hi) of S, the whole warp.  Where sides have to be tested, the
-// valid splits wait in a queue until they fill the warp (most subsets of a
-// sparse block are not connected).
+// Splits [lo, hi) of S, the whole warp.  Valid splits wait in a queue until
+// they fill the warp (most subsets of a sparse block are not connected).
 __device__ __forceinline__ void gen_range(const DevInfoView &d, GenScratch &ws, uint32_t S, uint32_t lo, uint32_t hi,
                                           const float4 *memo, const uint32_t *seen, GenBest &best, int &width) {
     const uint32_t lane = threadIdx.x & 31u;
     uint32_t queued = 0u;
     __syncwarp();
-    for (uint32_t base = lo; base < hi; base += 32u) {
-        const uint32_t c = base + lane;
-        bool ok = c < hi, test = false;
-        uint32_t L = 0u;
-        if (ok) {
-            L = gen_side(S, ws, c, test);
-            if (test) ok = seen_bit(seen, L) && seen_bit(seen, S ^ L);
+    for (uint32_t base = lo;;) {
+        while (queued < 32u && base < hi) {
+            const uint32_t c = base + lane;
+            bool ok = c < hi, test = false;
+            uint32_t L = 0u;
+            if (ok) {
+                L = gen_side(S, ws, c, test);
+                if (test) ok = seen_bit(seen, L) && seen_bit(seen, S ^ L);
+            }
+            const uint32_t m = __ballot_sync(0xFFFFFFFFu, ok);
+            if (ok) {
+                const uint32_t at = queued + (uint32_t)popc(m & ((1u << lane) - 1u));
+                ws.queue[2u * at] = c;
+                ws.queue[2u * at + 1u] = L;
+            }
+            queued += (uint32_t)popc(m);
+            base += 32u;
         }
-        if (queued == 0u && !__any_sync(0xFFFFFFFFu, test)) {
-            if (ok) gen_cost(d, ws, S, c, L, memo, best, width);
-            continue;
-        }
-        const uint32_t m = __ballot_sync(0xFFFFFFFFu, ok);
-        if (ok) {
-            const uint32_t at = queued + (uint32_t)popc(m & ((1u << lane) - 1u));
-            ws.queue[2u * at] = c;
-            ws.queue[2u * at + 1u] = L;
-        }
-        queued += (uint32_t)popc(m);
+        if (queued == 0u) break;
         __syncwarp();
-        if (queued >= 32u) {
-            queued -= 32u;
+        const uint32_t take = min(queued, 32u);
+        queued -= take;
+        if (lane < take) {
             const uint2 e = *reinterpret_cast<const uint2 *>(ws.queue + 2u * (queued + lane));
-            __syncwarp();
             gen_cost(d, ws, S, e.x, e.y, memo, best, width);
         }
-    }
-    if (queued) {
         __syncwarp();
-        if (lane < queued) {
-            const uint2 e = *reinterpret_cast<const uint2 *>(ws.queue + 2u * lane);
-            gen_cost(d, ws, S, e.x, e.y, memo, best, width);
-        }
     }
-    __syncwarp();
 }
 
 // index of the first valid candidate of S
@@ -374,6 +368,36 @@ __device__ __forceinline__ void gen_set(const DevInfoView &d, GenScratch &ws, ui
         memo[S] = make_float4(best.rows, best.startup, total, __uint_as_float(memo_width_word(*d.h, best.rows, width)));
         memo_left[S] = best.left;
     }
+}
+
+// a set of a cactus graph (table cv), by its pieces; false: equal lowest costs
+// or a NaN
+__device__ __forceinline__ bool gen_cactus_set(const DevInfoView &d, const CactusView &cv, const PlainParams &pp,
+                                               GenScratch &ws, uint32_t S, float4 *memo, uint32_t *memo_left,
+                                               uint32_t &pairs) {
+    const DevHeader &h = *d.h;
+    return cactus_set<uint32_t>(
+        S, cv, ws.cactus, pp, [&](uint32_t L) { return __ldcg(memo + L); },
+        [&](uint32_t L, const float4 lv, const float4 rv, uint64_t match, JoinCost &lr, JoinCost &rl) {
+            const RelVal l = unpack_rel(lv, h.hz_packed), r = unpack_rel(rv, h.hz_packed);
+            RelVal o0, o1;
+            if ((cv.h.flags & kCactusEdges) && h.n_ec <= 32)
+                join_eval_mirror_w<1, true>(d, L, l, S ^ L, r, (uint32_t)match, o0, o1);
+            else
+                join_eval_mirror(d, L, l, S ^ L, r, o0, o1);
+            lr.rows = o0.rows;
+            lr.startup = o0.startup;
+            lr.total = o0.total;
+            rl.rows = o1.rows;
+            rl.startup = o1.startup;
+            rl.total = o1.total;
+            return o0.width;
+        },
+        [&](float rows, float startup, float total, int width, uint32_t left) {
+            memo[S] = make_float4(rows, startup, total, __uint_as_float(memo_width_word(h, rows, width)));
+            memo_left[S] = left;
+        },
+        pairs);
 }
 
 }  // namespace gqb

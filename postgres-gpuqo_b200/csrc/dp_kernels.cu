@@ -3381,6 +3381,10 @@ __global__ void __launch_bounds__(kBlock, 2) kb_gen(const BatchQ *__restrict__ q
             BatchQ Q = {};
             if (!ONE) Q = qs[q];
             const DevInfoView d = make_view(ONE ? own : blobs + Q.blob_off);
+            if (d.h->tree_tab != 0u &&
+                gen_cactus_set(d, cactus_view(reinterpret_cast<const uint32_t *>(d.h) + d.h->tree_tab, d.h->n_ec),
+                               plain_params(*d.h), ws, S, memo + Q.memo_off, memo_left + Q.memo_off, found))
+                continue;
             gen_blocks(S, d.h->adj, ws);
             const uint32_t W = ws.half[ws.nb];
             if (W > limit && ovf.cap != 0u) {

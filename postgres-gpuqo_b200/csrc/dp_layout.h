@@ -79,7 +79,8 @@ struct DevHeader {
     uint32_t max_block;                   // largest biconnected block of the query graph
     uint32_t tree_mode;                   // query graph is a tree (tree tables present)
     uint32_t ec_masked;                   // tree_mode and every class is a 2-member class on an edge
-    uint32_t tree_tab;                    // word offset of the tree tables (see below), 0 if none
+    uint32_t tree_tab;                    // word offset of the tree tables (see below), or of the cactus table
+                                          // (dp_cactus.cuh) of a graph that is not a tree; 0 if none
     // memo widths carry the inner hash table size (see memo_width_word): set
     // when every width is >= 0 and all of them sum to less than 2^21
     uint32_t hz_packed;

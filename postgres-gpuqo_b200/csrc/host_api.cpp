@@ -17,6 +17,7 @@
 
 #include <cuda_runtime.h>
 
+#include "dp_cactus_table.h"
 #include "dp_engine.h"
 #include "gpuqo_b200.h"
 #include "host_idp.h"
@@ -565,6 +566,29 @@ std::vector<uint32_t> build_blob(const HostInfo &info) {
             e.quals = plain_quals(*h, quals);
         }
         h->tree_plain = (plain && straight) ? 1u : 0u;
+    }
+    if (!tree && n <= 30) {
+        // 30 relations: the end of the kernels that read the table
+        std::vector<uint64_t> adj(n), rel(n_ec);
+        for (int i = 0; i < n; i++) adj[i] = h->adj[i];
+        bool plain = straight;
+        for (int i = 0; i < n_ec; i++) {
+            rel[i] = relids[i];
+            plain = plain && ((v.plain[i / 32] >> (i % 32)) & 1u);
+        }
+        const std::vector<float> sel(v.pair_sel, v.pair_sel + 2 * n_ec);
+        const std::vector<uint64_t> tab =
+            build_cactus(adj, rel, sel, plain, [&](int quals) { return plain_quals(*h, quals); });
+        if (!tab.empty()) {
+            const uint32_t at = (uint32_t)blob.size();
+            blob.resize(at + 2 * tab.size());
+            h = reinterpret_cast<DevHeader *>(blob.data());
+            v = make_view(blob.data());
+            relids = const_cast<uint32_t *>(v.ec_relids);
+            std::memcpy(blob.data() + at, tab.data(), tab.size() * 8);
+            h->tree_tab = at;
+            h->blob_words = (uint32_t)blob.size();
+        }
     }
     if (pairs_words) {
         bool plain = straight && h->all_pairs;

@@ -40,7 +40,7 @@ GRAPHS = {
 def _query(name, kind):
     n, pairs = GRAPHS[name]
     pairs = sorted(set((min(p), max(p)) for p in pairs))
-    rng = np.random.default_rng([len(name), n, ("plain", "stats", "equal", "overflow").index(kind)])
+    rng = np.random.default_rng([len(name), n, KINDS.index(kind)])
     if kind == "equal":
         rows, edges = [1000.0] * n, [(a, b, 0.01, None) for a, b in pairs]
     elif kind == "overflow":
@@ -49,10 +49,25 @@ def _query(name, kind):
         rows = np.exp(rng.uniform(5, 14, n))
         edges = [(a, b, 1.0 / query.f32(round(float(rows[b]))), "a") if rng.uniform() < 0.5 else
                  (a, b, float(np.exp(rng.uniform(-9, -2))), None) for a, b in pairs]
-    return query._assemble(name, n, rows, [int(w) for w in rng.integers(4, 65, n)], edges, rng, rich=(kind == "stats"))
+    q = query._assemble(name, n, rows, [int(w) for w in rng.integers(4, 65, n)], edges, rng,
+                        rich=kind in ("stats", "stats_two_classes"))
+    if kind in ("two_classes", "stats_two_classes"):   # beyond 32 classes on the larger graphs, keys both ways
+        for ec in list(q.eq_classes):
+            a, b = ec.members
+            q.eq_classes.append(query.EqClass([a, b], [query.f32(0.7)], [[b], [a]], [query.VarInfo(), query.VarInfo()]))
+    elif kind == "off_edge" and n > 3:
+        far = [(a, b) for a in range(n) for b in range(a + 1, n) if b not in q.edges[a]]
+        if far:
+            q.eq_classes.append(query.EqClass(list(far[0]), [query.f32(0.6)], [[], []], [query.VarInfo()] * 2))
+    elif kind == "no_class":
+        del q.eq_classes[1]
+    return q
 
 
-@pytest.mark.parametrize("kind", ["plain", "stats", "equal", "overflow"])
+KINDS = ["plain", "stats", "equal", "overflow", "two_classes", "stats_two_classes", "off_edge", "no_class"]
+
+
+@pytest.mark.parametrize("kind", KINDS)
 @pytest.mark.parametrize("name", sorted(GRAPHS))
 def test_general_evaluation(name, kind):
     q = _query(name, kind)
