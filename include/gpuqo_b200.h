@@ -253,11 +253,13 @@ extern int gpuqo_b200_device_memory_mb;
  * above 63 keeps the default. */
 extern int gpuqo_b200_sparse_from_rels;
 
-/* Connected sets the host lists for a sparse-memo DP of a graph that is not
- * a tree before it hands the listing to the device (level by level, the
- * device table deduplicating; the arrays are then sized for the sparse memo's
- * whole capacity).  0 (default): 65536.  Trees are always listed on the
- * device.  Plans do not depend on it. */
+/* Connected sets that a sparse-memo DP of a graph that is not a tree makes
+ * room for at first.  A cactus graph (bridges and simple cycles; default
+ * 131072) is listed on the device, which starts again with 16 times the room
+ * when a level outgrows it; of any other graph (default 65536) the host lists
+ * that many before it hands the listing to the device (level by level, the
+ * arrays then sized for the sparse memo's whole capacity).  0: the defaults.
+ * Trees are counted beforehand.  Plans do not depend on it. */
 extern int gpuqo_b200_sparse_host_list;
 
 /*

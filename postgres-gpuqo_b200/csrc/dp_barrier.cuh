@@ -1,0 +1,72 @@
+// dp_barrier.cuh - the bounded grid barrier of the persistent kernels.
+#pragma once
+
+#include <cuda_runtime.h>
+
+namespace gqb {
+
+constexpr unsigned long long kBarrierTimeoutNs = 4000000000ull;   // 4 s of global time
+constexpr unsigned kBarrierSpinLimit = 1u << 26;                  // hard cap on polls as well (~30 s)
+
+// poll limit of one barrier wait: the launch argument when non-zero (the
+// gpuqo_b200_barrier_poll_limit setting, which makes waits run out on purpose
+// so that the timeout path can be exercised), else kBarrierSpinLimit
+__device__ __forceinline__ unsigned barrier_polls(unsigned poll_limit) {
+    return poll_limit != 0u ? poll_limit : kBarrierSpinLimit;
+}
+
+__device__ __forceinline__ unsigned long long global_ns() {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
+
+// bar[0] = arrivals, bar[2] = error flag (both zero at launch).  The arrival
+// counter only grows: a block's e-th barrier of the launch completes when it
+// reaches e * gridDim.x, so nobody resets it and the last block to arrive has
+// nothing more to do.  Thread 0 arrives with a gpu-scope release reduction
+// (ordering every write its block made before the __syncthreads) and polls
+// with gpu-scope acquire loads (ACQUIRE_POLL), or with relaxed loads and one
+// fence once the count is reached: an acquire load also drops the SM's L1
+// contents, which a kernel that keeps its working data in shared memory does
+// not mind (k_dp_tree: the faster barrier) but which costs the batch kernel,
+// whose per-query data is read through L1 while waiting blocks poll on the
+// same SM.  The verdict is the same for every thread of the block (thread 0
+// decides); blocks may disagree only after a timeout, and then every later
+// barrier sees the error flag and returns false at once, so all blocks leave.
+// epoch: the caller's count of barriers passed (thread 0); max_polls: polls
+// before the wait gives up (barrier_polls).
+template <bool ACQUIRE_POLL>
+__device__ __forceinline__ bool grid_barrier(unsigned *bar, unsigned &epoch, unsigned max_polls) {
+    __shared__ unsigned s_ok;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        epoch++;
+        const unsigned target = epoch * gridDim.x;
+        volatile unsigned *verr = bar + 2;
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
+        const unsigned long long t0 = global_ns();
+        unsigned spins = 0;
+        for (;;) {
+            unsigned c;
+            if (ACQUIRE_POLL) {
+                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(c) : "l"(bar) : "memory");
+            } else {
+                asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(c) : "l"(bar) : "memory");
+            }
+            if (c >= target || *verr != 0u) {
+                if (!ACQUIRE_POLL) __threadfence();
+                break;
+            }
+            if (++spins >= max_polls || global_ns() - t0 > kBarrierTimeoutNs) {
+                atomicExch(bar + 2, 1u);
+                break;
+            }
+        }
+        s_ok = (*verr == 0u) ? 1u : 0u;
+    }
+    __syncthreads();
+    return s_ok != 0u;
+}
+
+}  // namespace gqb

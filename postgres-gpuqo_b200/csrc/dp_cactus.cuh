@@ -15,8 +15,9 @@
 // two edges when every class sits on an edge.
 //
 // The splits come in another order than the reference's, whose index decides
-// between equal costs and for a NaN: such sets are left to the block search
-// (cactus_set returns false).
+// between equal costs and for a NaN: such sets get their blocks searched in the
+// reference's order (cactus_order) and their splits costed once more, with
+// indices.
 #pragma once
 
 #include "dp_cactus_table.h"
@@ -24,18 +25,27 @@
 
 namespace gqb {
 
-// One warp's scratch: per block the first split, the piece's first walk
-// position and its relations
+// One warp's scratch: per block of the graph the first split, the piece's
+// first walk position and its relations; then the set's own blocks in the
+// reference's order and the search stack (cactus_order)
+template <class M>
 struct CactusScratch {
-    uint16_t off[66];
-    uint8_t start[64], size[64];
+    static constexpr int kRels = (int)sizeof(M) * 8;
+    M mask[kRels], st_desc[kRels], st_reach[kRels], st_rem[kRels], st_adj[kRels];
+    uint64_t prefix[kRels];
+    uint16_t off[kRels + 2];
+    uint8_t start[kRels], size[kRels], st_u[kRels];
+    uint32_t nb;
 };
 
 template <class M> __device__ __forceinline__ int cactus_popc(M x) { return sizeof(M) == 8 ? __popcll(x) : __popc((uint32_t)x); }
+template <class M> __device__ __forceinline__ uint32_t cactus_low(M x) {
+    return (uint32_t)((sizeof(M) == 8 ? __ffsll((long long)x) : __ffs((int)(uint32_t)x)) - 1);
+}
 
 // the splits of S per block; returns their total
 template <class M>
-__device__ __forceinline__ uint32_t cactus_pieces(M S, const CactusView &v, CactusScratch &sc) {
+__device__ __forceinline__ uint32_t cactus_pieces(M S, const CactusView &v, CactusScratch<M> &sc) {
     const uint32_t lane = threadIdx.x & 31u;
     __syncwarp();
     for (uint32_t b = 0; b < v.h.n_cycles; b++) {
@@ -79,7 +89,7 @@ __device__ __forceinline__ uint32_t cactus_pieces(M S, const CactusView &v, Cact
 
 // one side of split c of S and the classes on the cut edges
 template <class M>
-__device__ __forceinline__ M cactus_side(M S, const CactusView &v, const CactusScratch &sc, uint32_t c, uint64_t &match) {
+__device__ __forceinline__ M cactus_side(M S, const CactusView &v, const CactusScratch<M> &sc, uint32_t c, uint64_t &match) {
     // the last block whose first split is at most c (blocks without splits
     // share their successor's)
     uint32_t b = 0u;
@@ -125,13 +135,85 @@ __device__ __forceinline__ void cactus_update(CactusBest<M> &best, M L, float ro
     }
 }
 
+// The set's blocks in the reference's output order and the candidates ahead of
+// each (2^m - 2 per block): depth-first from the lowest relation, neighbours in
+// increasing order, by lane 0 with masks (as gen_blocks)
+template <class M, class Adj>
+__device__ __noinline__ void cactus_order(M S, const Adj *adj, CactusScratch<M> &sc) {
+    if ((threadIdx.x & 31u) == 0u) {
+        int sp = 0;
+        uint32_t nb = 0u, u = cactus_low<M>(S);
+        M desc = (M)1 << u, rem = desc, reach = (M)adj[u], visited = desc, anc = 0, a = reach & S;
+        uint64_t ahead = 0ull;
+        for (;;) {
+            const M c = a & ~visited;
+            if (c) {
+                sc.st_u[sp] = (uint8_t)u;
+                sc.st_desc[sp] = desc;
+                sc.st_reach[sp] = reach;
+                sc.st_rem[sp] = rem;
+                sc.st_adj[sp] = a;
+                sp++;
+                anc |= (M)1 << u;
+                u = cactus_low<M>(c);
+                desc = rem = (M)1 << u;
+                visited |= desc;
+                reach = (M)adj[u];
+                a = reach & S;
+            } else {
+                if (sp == 0) break;
+                sp--;
+                const uint32_t p = sc.st_u[sp];
+                const M bit = (M)1 << p;
+                M up = sc.st_rem[sp];
+                anc &= ~bit;
+                if ((reach & anc) == 0) {
+                    sc.mask[nb] = rem | bit;
+                    sc.prefix[nb] = ahead;
+                    ahead += (1ull << cactus_popc<M>(rem | bit)) - 2ull;
+                    nb++;
+                } else {
+                    up |= rem;
+                }
+                desc |= sc.st_desc[sp];
+                reach |= sc.st_reach[sp];
+                rem = up;
+                a = sc.st_adj[sp];
+                u = p;
+            }
+        }
+        sc.nb = nb;
+    }
+    __syncwarp();
+}
+
+// the bits of x at the positions of mask, packed (x within mask)
+template <class M>
+__device__ __forceinline__ uint64_t cactus_pext(M x, M mask) {
+    uint64_t r = 0ull;
+    for (; x; x &= x - 1) r |= 1ull << cactus_popc<M>(mask & ((x & (~x + 1)) - 1));
+    return r;
+}
+
+// the reference's index of the candidate with outer side L (after
+// cactus_order, or plain DPsub's)
+template <class M>
+__device__ __noinline__ uint64_t cactus_index(M S, const CactusScratch<M> &sc, M L, bool dpsub) {
+    if (dpsub) return cactus_pext<M>(L, S) - 1ull;
+    const M R = S ^ L;
+    uint32_t b = 0u;
+    // the one block that the split cuts
+    while (b + 1u < sc.nb && ((sc.mask[b] & L) == 0 || (sc.mask[b] & R) == 0)) b++;
+    return sc.prefix[b] + cactus_pext<M>(L & sc.mask[b], sc.mask[b]) - 1ull;
+}
+
 // A connected set by one warp: load(L) gives a side's memo entry, general(L,
 // l, r, match, lr, rl) costs both orientations where plain_mirror does not
-// apply, write(rows, startup, total, width, left) stores the winner (one
-// lane).  False, and nothing written: equal lowest costs or a NaN.
-template <class M, class Load, class General, class Write>
-__device__ __forceinline__ bool cactus_set(M S, const CactusView &v, CactusScratch &sc, const PlainParams &pp, Load load,
-                                           General general, Write write, uint32_t &pairs) {
+// apply, write(rows, startup, total, width, left) stores the winner (one lane).
+template <class M, class Adj, class Load, class General, class Write>
+__device__ __forceinline__ void cactus_set(M S, const CactusView &v, const Adj *adj, CactusScratch<M> &sc, bool dpsub,
+                                           const PlainParams &pp, Load load, General general, Write write,
+                                           uint32_t &pairs) {
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t W = cactus_pieces<M>(S, v, sc);
     CactusBest<M> best;
@@ -141,35 +223,91 @@ __device__ __forceinline__ bool cactus_set(M S, const CactusView &v, CactusScrat
     best.rows = best.startup = 0.0f;
     best.nan = false;
     int width = 0;
-    for (uint32_t c = lane; c < W; c += 32u) {
-        uint64_t match;
-        const M L = cactus_side<M>(S, v, sc, c, match), R = S ^ L;
-        const float4 l = load(L), r = load(R);
-        JoinCost lr, rl;
-        if (v.h.flags & kCactusPlain) {
-            float sel_l = 1.0f, sel_r = 1.0f;
-            for (uint64_t x = match; x; x &= x - 1ull) {
-                const CactusClass k = v.classes[__ffsll((long long)x) - 1];
-                const bool lo = (L >> k.x) & 1u;
-                sel_l *= lo ? k.lo : k.hi;
-                sel_r *= lo ? k.hi : k.lo;
+    // second pass: the candidates' indices; the lowest one with the lowest
+    // cost, the lowest one at all and whether its cost is a NaN
+    bool exact = false, nans = false, first_nan = false;
+    uint32_t ord = 0u;
+    uint64_t best_p = ~0ull, first_p = ~0ull;
+    float first_rows = 0.0f, first_startup = 0.0f, first_total = 0.0f;
+    M first_left = 0;
+    for (;;) {
+        for (uint32_t c = lane; c < W; c += 32u) {
+            uint64_t match;
+            const M L = cactus_side<M>(S, v, sc, c, match), R = S ^ L;
+            const float4 l = load(L), r = load(R);
+            JoinCost lr, rl;
+            if (v.h.flags & kCactusPlain) {
+                float sel_l = 1.0f, sel_r = 1.0f;
+                for (uint64_t x = match; x; x &= x - 1ull) {
+                    const CactusClass k = v.classes[__ffsll((long long)x) - 1];
+                    const bool lo = (L >> k.x) & 1u;
+                    sel_l *= lo ? k.lo : k.hi;
+                    sel_r *= lo ? k.hi : k.lo;
+                }
+                plain_mirror(pp, v.quals[__popcll(match)], sel_l, sel_r, l, r, lr, rl);
+                width = (int)((__float_as_uint(l.w) & kWidthMask) + (__float_as_uint(r.w) & kWidthMask));
+            } else {
+                width = general(L, l, r, match, lr, rl);
             }
-            plain_mirror(pp, v.quals[__popcll(match)], sel_l, sel_r, l, r, lr, rl);
-            width = (int)((__float_as_uint(l.w) & kWidthMask) + (__float_as_uint(r.w) & kWidthMask));
-        } else {
-            width = general(L, l, r, match, lr, rl);
+            if (!exact) {
+                cactus_update<M>(best, L, lr.rows, lr.startup, lr.total);
+                cactus_update<M>(best, R, rl.rows, rl.startup, rl.total);
+                continue;
+            }
+#pragma unroll 1
+            for (int side = 0; side < 2; side++) {
+                const JoinCost &o = side ? rl : lr;
+                const bool nan = isnan(o.total), lowest_cost = !nan && ord_float(o.total) == ord;
+                if (!lowest_cost && !nans) continue;
+                const M X = side ? R : L;
+                const uint64_t p = cactus_index<M>(S, sc, X, dpsub);
+                if (lowest_cost && p < best_p) {
+                    best_p = p;
+                    best.left = X;
+                    best.rows = o.rows;
+                    best.startup = o.startup;
+                }
+                if (p < first_p) {
+                    first_p = p;
+                    first_nan = nan;
+                    first_left = X;
+                    first_rows = o.rows;
+                    first_startup = o.startup;
+                    first_total = o.total;
+                }
+            }
         }
-        cactus_update<M>(best, L, lr.rows, lr.startup, lr.total);
-        cactus_update<M>(best, R, rl.rows, rl.startup, rl.total);
+        if (exact) break;
+        ord = __reduce_min_sync(0xFFFFFFFFu, best.ord);
+        const uint32_t win = __ballot_sync(0xFFFFFFFFu, best.ord == ord && ord != 0xFFFFFFFFu);
+        nans = __any_sync(0xFFFFFFFFu, best.nan);
+        if (!nans && __popc(win) == 1 && !__any_sync(0xFFFFFFFFu, best.ord == ord && best.tie == ord)) {
+            best_p = (win >> lane) & 1u ? 0ull : ~0ull;
+            break;
+        }
+        exact = true;
+        if (!dpsub) cactus_order<M>(S, adj, sc);
     }
-    const uint32_t ord = __reduce_min_sync(0xFFFFFFFFu, best.ord);
-    const uint32_t win = __ballot_sync(0xFFFFFFFFu, best.ord == ord && ord != 0xFFFFFFFFu);
-    if (__popc(win) != 1 || __any_sync(0xFFFFFFFFu, best.nan || (best.ord == ord && best.tie == ord))) return false;
-    if ((win >> lane) & 1u)
-        // the inverse of ord_float (a total is never -0: its startup cost starts from +0)
+    auto least = [](uint64_t p) {
+        const uint32_t hi = __reduce_min_sync(0xFFFFFFFFu, (uint32_t)(p >> 32));
+        const uint32_t lo = __reduce_min_sync(0xFFFFFFFFu, (uint32_t)(p >> 32) == hi ? (uint32_t)p : 0xFFFFFFFFu);
+        return ((uint64_t)hi << 32) | lo;
+    };
+    bool mine = best_p != ~0ull;
+    if (exact) {   // every lane takes part in the reductions
+        const uint64_t lowest_p = least(best_p);
+        mine = mine && best_p == lowest_p;
+        if (nans) {
+            const uint64_t lowest_first = least(first_p);
+            const bool kept = first_nan && first_p == lowest_first;
+            if (__any_sync(0xFFFFFFFFu, kept)) mine = false;
+            if (kept) write(first_rows, first_startup, first_total, width, first_left);
+        }
+    }
+    // the inverse of ord_float (a total is never -0: its startup cost starts from +0)
+    if (mine)
         write(best.rows, best.startup, __uint_as_float((ord & 0x80000000u) ? ord ^ 0x80000000u : ~ord), width, best.left);
     if (lane == 0u) pairs += 2u * W;
-    return true;
 }
 
 }  // namespace gqb

@@ -77,6 +77,8 @@ struct HostInfo;
 int engine_run_wide(const HostInfo &info, DpMode mode, std::vector<TreeNode> &nodes, EngineStats &st,
                     std::string &err);
 uint64_t wide_set_capacity();
+// clears a grid-barrier timeout latched by the sparse DP's persistent kernel
+bool wide_reset_persistent(int dev);
 // whether an exact DP of n relations in this mode runs on the sparse memo
 // (n > 31, or n >= gpuqo_b200_sparse_from_rels for DPsub and MPDP)
 bool use_sparse_memo(int n, DpMode mode);

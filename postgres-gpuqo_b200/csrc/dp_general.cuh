@@ -24,7 +24,7 @@
 
 namespace gqb {
 
-// One warp's scratch (shared memory, 2.9 KB)
+// One warp's scratch (shared memory, 4 KB)
 struct GenScratch {
     uint32_t mask[32];            // blocks in the reference's output order
     uint32_t sub[32];             // ... the relations below the block's child end in the search tree
@@ -41,7 +41,7 @@ struct GenScratch {
     uint16_t off[32];             // first group in tab, or first word in pre
     uint8_t st_u[32];
     uint32_t nb, cyc;
-    CactusScratch cactus;
+    alignas(8) CactusScratch<uint32_t> cactus;
     alignas(8) uint32_t queue[64 * 2];       // valid splits waiting for a full warp: candidate, side
 };
 
@@ -370,14 +370,13 @@ __device__ __forceinline__ void gen_set(const DevInfoView &d, GenScratch &ws, ui
     }
 }
 
-// a set of a cactus graph (table cv), by its pieces; false: equal lowest costs
-// or a NaN
-__device__ __forceinline__ bool gen_cactus_set(const DevInfoView &d, const CactusView &cv, const PlainParams &pp,
+// a set of a cactus graph (table cv), by its pieces
+__device__ __forceinline__ void gen_cactus_set(const DevInfoView &d, const CactusView &cv, const PlainParams &pp,
                                                GenScratch &ws, uint32_t S, float4 *memo, uint32_t *memo_left,
                                                uint32_t &pairs) {
     const DevHeader &h = *d.h;
-    return cactus_set<uint32_t>(
-        S, cv, ws.cactus, pp, [&](uint32_t L) { return __ldcg(memo + L); },
+    cactus_set<uint32_t>(
+        S, cv, h.adj, ws.cactus, h.index_order != 0u, pp, [&](uint32_t L) { return __ldcg(memo + L); },
         [&](uint32_t L, const float4 lv, const float4 rv, uint64_t match, JoinCost &lr, JoinCost &rl) {
             const RelVal l = unpack_rel(lv, h.hz_packed), r = unpack_rel(rv, h.hz_packed);
             RelVal o0, o1;

@@ -279,4 +279,22 @@ GQB_HD inline void fill_pair_sel(const DevInfoView &v) {
     h->all_pairs = (h->n_ec > 0) ? all : 0u;
 }
 
+inline PlainQuals plain_quals(const DevHeader &h, int quals) {
+    PlainQuals q;
+    q.per_tuple = 0.0f;
+    for (int i = 0; i < quals; i++) q.per_tuple += h.cpu_operator_cost;
+    q.quals_cost = h.cpu_operator_cost * (float)quals;
+    q.nl_tuple = h.cpu_tuple_cost + q.per_tuple;
+    q.hj_row = q.quals_cost + h.cpu_tuple_cost;
+    return q;
+}
+
+// Whether the straight-line cost (plain_mirror) may serve a query of this
+// width sum: it leaves out the skew check, which compares one row of the inner
+// side with work_mem, so the widest set's row decides for all.
+inline bool plain_cost_applies(const DevHeader &h, long long width_sum) {
+    const float widest = (float)((((unsigned long long)(width_sum > 0 ? width_sum : 0) + 7ull) & ~7ull) + 24ull);
+    return h.hz_packed && h.enable_hashjoin && widest <= h.work_mem_bytes;
+}
+
 }  // namespace gqb

@@ -4,6 +4,9 @@
 // and a hash-table memo (gpuqo_main_internal.cu:177-185, Bitmapset64;
 // gpuqo_hashtable.cuh:121-166).  The dense memo of the main engine stops at
 // 31 relations (2^n entries); beyond, only the connected sets are stored:
+//   * cactus graphs (bridges and simple cycles) run in one persistent launch
+//     that lists and costs level after level (k_wide_cactus), trees by one pair
+//     of launches per level (k_wide_tree_*); of the others
 //   * the host enumerates the connected sets level by level (extension by a
 //     neighbour, deduplicated) - the graphs planned exactly at this size are
 //     sparse, with thousands to millions of connected sets, and the count is
@@ -27,12 +30,16 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <cstddef>
 #include <functional>
+#include <map>
 #include <mutex>
 #include <string>
 #include <unordered_set>
 #include <vector>
 
+#include "dp_barrier.cuh"
+#include "dp_cactus.cuh"
 #include "dp_device.cuh"
 #include "dp_engine.h"
 #include "gpuqo_b200.h"
@@ -40,6 +47,8 @@
 
 extern "C" int gpuqo_b200_device_memory_mb;
 extern "C" int gpuqo_b200_sparse_host_list;
+extern "C" int gpuqo_b200_persistent;
+extern "C" int gpuqo_b200_barrier_poll_limit;
 
 namespace gqb {
 
@@ -446,12 +455,17 @@ __global__ void k_wide_insert(WideTable t, const unsigned long long *__restrict_
         wide_insert_one(t, sets[i], i, err);
 }
 
+// LIVE: the table is filled by the same launch (read from L2, where other
+// blocks' entries are).  A slot is requested together with its key, so that a
+// first hit costs one access and not two.
+template <bool LIVE = false>
 __device__ __forceinline__ uint32_t wide_lookup(const WideTable &t, uint64_t key, unsigned *err) {
     const uint32_t cap = 1u << t.cap_log2;
     uint32_t pos = wide_hash(key, t.cap_log2);
     for (uint32_t probe = 0; probe < cap; probe++, pos = (pos + 1u) & (cap - 1u)) {
-        const unsigned long long k = __ldg(t.keys + pos);
-        if (k == key) return __ldg(t.slot + pos);
+        const unsigned long long k = LIVE ? __ldcg(t.keys + pos) : __ldg(t.keys + pos);
+        const uint32_t slot = LIVE ? __ldcg(t.slot + pos) : __ldg(t.slot + pos);
+        if (k == key) return slot;
         if (k == 0ull) break;
     }
     atomicExch(err, 2u);                  // a side that is not a connected set: cannot happen
@@ -462,7 +476,108 @@ __device__ __forceinline__ RelVal wide_rel(const float4 *memo, uint32_t slot, ui
     return unpack_rel(__ldcg(memo + slot), packed);
 }
 
-// one warp per connected set of level k (sets[first .. first + count))
+// One connected set by one warp, its blocks searched by lane 0 in the
+// reference's order: every candidate keyed by its index there.  Writes the
+// memo entry `slot`; returns the lane's costed pairs.
+__device__ __forceinline__ unsigned long long wide_set(const WideInfo &w, WarpScratch &ws, const WideTable &t, uint64_t S,
+                                                    uint32_t slot, int index_order, float4 *memo,
+                                                    unsigned long long *memo_left, unsigned *err) {
+    const int lane = threadIdx.x & 31;
+    unsigned long long pairs = 0;
+    __syncwarp();   // every lane is done with the previous set's scratch
+    if (lane == 0) {
+        find_blocks64(S, w.adj, ws.B, ws.dfs);
+        uint32_t off = 0;
+        for (int b = 0; b < ws.B.nb; b++) {
+            ws.pre_off[b] = (uint8_t)off;
+            if ((ws.B.cyc >> b) & 1ull) {
+                cycle_walk64(ws.B.mask[b], w.adj, ws.pre + off);
+                off += (uint32_t)__popcll(ws.B.mask[b]) + 1u;
+            }
+        }
+    }
+    __syncwarp();
+    const BlocksW &B = ws.B;
+    const uint64_t P = B.eprefix[B.nb];
+    if (P > kWideMaxCandidates) {   // a dense block: far beyond what an exact DP at this size can afford
+        if (lane == 0) atomicExch(err, 3u);
+        return 0ull;
+    }
+    // lane best: (ordered cost, index) lexicographic; first valid
+    // candidate (index, NaN) for the reference's NaN rule
+    uint32_t best_c = kFullW;
+    uint64_t best_k = ~0ull, first_k = ~0ull;
+    bool first_nan = false;
+    RelVal best_v, nan_v;
+    uint64_t best_l = 0, nan_l = 0;
+    int b = 0;
+    for (uint64_t c = (uint64_t)lane; c < P; c += 32u) {
+        uint64_t L, R, key;
+        if (!wide_candidate(S, ws, w.adj, c, b, L, R, key)) continue;
+        if (index_order) key = dpsub_index64(L, S);
+        const RelVal l = wide_rel(memo, wide_lookup(t, L, err), w.h.hz_packed);
+        const RelVal r = wide_rel(memo, wide_lookup(t, R, err), w.h.hz_packed);
+        RelVal out;
+        if (w.rel_masked) {
+            uint64_t cl = 0ull, cr = 0ull;
+            for (uint64_t x = L; x; x &= x - 1ull) cl |= w.rel_cls[lowest_idx64(x)];
+            for (uint64_t x = R; x; x &= x - 1ull) cr |= w.rel_cls[lowest_idx64(x)];
+            out = join_eval_w<true>(w, L, l, R, r, cl & cr);
+        } else {
+            out = join_eval_w<false>(w, L, l, R, r);
+        }
+        const bool nan = isnan(out.total);
+        pairs++;
+        if (key < first_k) {
+            first_k = key;
+            first_nan = nan;
+            if (nan) {
+                nan_v = out;
+                nan_l = L;
+            }
+        }
+        if (!nan) {
+            const uint32_t oc = ord_float(out.total);
+            if (oc < best_c || (oc == best_c && key < best_k)) {
+                best_c = oc;
+                best_k = key;
+                best_v = out;
+                best_l = L;
+            }
+        }
+    }
+    // warp: minimum cost, then minimum index among it; first candidate
+    const uint32_t mc = __reduce_min_sync(kFullW, best_c);
+    const uint64_t kc = (best_c == mc) ? best_k : ~0ull;
+    const uint32_t kh = __reduce_min_sync(kFullW, (uint32_t)(kc >> 32));
+    const uint32_t kl = __reduce_min_sync(kFullW, (uint32_t)(kc >> 32) == kh ? (uint32_t)kc : kFullW);
+    const uint64_t mk = ((uint64_t)kh << 32) | kl;
+    const uint32_t fh = __reduce_min_sync(kFullW, (uint32_t)(first_k >> 32));
+    const uint32_t fl = __reduce_min_sync(kFullW, (uint32_t)(first_k >> 32) == fh ? (uint32_t)first_k : kFullW);
+    const uint64_t mf = ((uint64_t)fh << 32) | fl;
+    const bool nan_first = first_k == mf && first_nan && mf != ~0ull;
+    const unsigned nm = __ballot_sync(kFullW, nan_first);
+    const RelVal *wv = nullptr;
+    uint64_t wl = 0;
+    if (nm) {
+        if (nan_first) {
+            wv = &nan_v;
+            wl = nan_l;
+        }
+    } else if (best_c == mc && best_k == mk && mc != kFullW) {
+        wv = &best_v;
+        wl = best_l;
+    }
+    if (wv) {
+        memo[slot] = make_float4(wv->rows, wv->startup, wv->total,
+                                  __uint_as_float(memo_width_word(w.h, wv->rows, wv->width)));
+        memo_left[slot] = wl;
+    }
+    return pairs;
+}
+
+// one warp per connected set of level k (sets[first .. first + count), whose
+// slots are their indices)
 __global__ void __launch_bounds__(kWideBlock) k_wide_eval(const WideInfo *__restrict__ wi, WideTable t,
                                                           const unsigned long long *__restrict__ sets, uint32_t first,
                                                           uint32_t count, int index_order, float4 *__restrict__ memo,
@@ -479,100 +594,8 @@ __global__ void __launch_bounds__(kWideBlock) k_wide_eval(const WideInfo *__rest
     const uint32_t gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
     unsigned long long pairs = 0;
-    for (uint32_t i = gwarp; i < count; i += nwarps) {
-        const uint64_t S = sets[first + i];
-        __syncwarp();   // every lane is done with the previous set's scratch
-        if (lane == 0) {
-            find_blocks64(S, w.adj, ws.B, ws.dfs);
-            uint32_t off = 0;
-            for (int b = 0; b < ws.B.nb; b++) {
-                ws.pre_off[b] = (uint8_t)off;
-                if ((ws.B.cyc >> b) & 1ull) {
-                    cycle_walk64(ws.B.mask[b], w.adj, ws.pre + off);
-                    off += (uint32_t)__popcll(ws.B.mask[b]) + 1u;
-                }
-            }
-        }
-        __syncwarp();
-        const BlocksW &B = ws.B;
-        const uint64_t P = B.eprefix[B.nb];
-        if (P > kWideMaxCandidates) {   // a dense block: far beyond what an exact DP at this size can afford
-            if (lane == 0) atomicExch(err, 3u);
-            continue;
-        }
-        // lane best: (ordered cost, index) lexicographic; first valid
-        // candidate (index, NaN) for the reference's NaN rule
-        uint32_t best_c = kFullW;
-        uint64_t best_k = ~0ull, first_k = ~0ull;
-        bool first_nan = false;
-        RelVal best_v, nan_v;
-        uint64_t best_l = 0, nan_l = 0;
-        int b = 0;
-        for (uint64_t c = (uint64_t)lane; c < P; c += 32u) {
-            uint64_t L, R, key;
-            if (!wide_candidate(S, ws, w.adj, c, b, L, R, key)) continue;
-            if (index_order) key = dpsub_index64(L, S);
-            const RelVal l = wide_rel(memo, wide_lookup(t, L, err), w.h.hz_packed);
-            const RelVal r = wide_rel(memo, wide_lookup(t, R, err), w.h.hz_packed);
-            RelVal out;
-            if (w.rel_masked) {
-                uint64_t cl = 0ull, cr = 0ull;
-                for (uint64_t x = L; x; x &= x - 1ull) cl |= w.rel_cls[lowest_idx64(x)];
-                for (uint64_t x = R; x; x &= x - 1ull) cr |= w.rel_cls[lowest_idx64(x)];
-                out = join_eval_w<true>(w, L, l, R, r, cl & cr);
-            } else {
-                out = join_eval_w<false>(w, L, l, R, r);
-            }
-            const bool nan = isnan(out.total);
-            pairs++;
-            if (key < first_k) {
-                first_k = key;
-                first_nan = nan;
-                if (nan) {
-                    nan_v = out;
-                    nan_l = L;
-                }
-            }
-            if (!nan) {
-                const uint32_t oc = ord_float(out.total);
-                if (oc < best_c || (oc == best_c && key < best_k)) {
-                    best_c = oc;
-                    best_k = key;
-                    best_v = out;
-                    best_l = L;
-                }
-            }
-        }
-        // warp: minimum cost, then minimum index among it; first candidate
-        const uint32_t mc = __reduce_min_sync(kFullW, best_c);
-        const uint64_t kc = (best_c == mc) ? best_k : ~0ull;
-        const uint32_t kh = __reduce_min_sync(kFullW, (uint32_t)(kc >> 32));
-        const uint32_t kl = __reduce_min_sync(kFullW, (uint32_t)(kc >> 32) == kh ? (uint32_t)kc : kFullW);
-        const uint64_t mk = ((uint64_t)kh << 32) | kl;
-        const uint32_t fh = __reduce_min_sync(kFullW, (uint32_t)(first_k >> 32));
-        const uint32_t fl = __reduce_min_sync(kFullW, (uint32_t)(first_k >> 32) == fh ? (uint32_t)first_k : kFullW);
-        const uint64_t mf = ((uint64_t)fh << 32) | fl;
-        const bool nan_first = first_k == mf && first_nan && mf != ~0ull;
-        const unsigned nm = __ballot_sync(kFullW, nan_first);
-        const uint32_t slot = (lane == 0) ? wide_lookup(t, S, err) : 0u;
-        const uint32_t sslot = __shfl_sync(kFullW, slot, 0);
-        const RelVal *wv = nullptr;
-        uint64_t wl = 0;
-        if (nm) {
-            if (nan_first) {
-                wv = &nan_v;
-                wl = nan_l;
-            }
-        } else if (best_c == mc && best_k == mk && mc != kFullW) {
-            wv = &best_v;
-            wl = best_l;
-        }
-        if (wv) {
-            memo[sslot] = make_float4(wv->rows, wv->startup, wv->total,
-                                      __uint_as_float(memo_width_word(w.h, wv->rows, wv->width)));
-            memo_left[sslot] = wl;
-        }
-    }
+    for (uint32_t i = gwarp; i < count; i += nwarps)
+        pairs += wide_set(w, ws, t, sets[first + i], first + i, index_order, memo, memo_left, err);
     for (int off = 16; off >= 1; off >>= 1) pairs += __shfl_xor_sync(kFullW, pairs, off);
     if (lane == 0 && pairs) atomicAdd(pairs_out, pairs);
 }
@@ -886,52 +909,207 @@ __global__ void __launch_bounds__(256) k_wide_list_ext(const WideInfo *__restric
     }
 }
 
-// the plan, walked from the full set by one thread (at most 2n - 1 nodes)
-__global__ void k_wide_extract(WideTable t, const float4 *__restrict__ memo,
-                               const unsigned long long *__restrict__ memo_left, uint64_t full, int n,
-                               uint32_t wmask, TreeNode *__restrict__ out, int *__restrict__ n_out,
-                               unsigned *__restrict__ err) {
-    if (blockIdx.x != 0 || threadIdx.x != 0) return;
-    uint64_t st_set[128];
-    int st_parent[128], st_side[128];
-    int sp = 0, cnt = 0;
-    st_set[sp] = full;
-    st_parent[sp] = -1;
-    st_side[sp] = 0;
-    sp++;
-    while (sp > 0 && cnt < 2 * n - 1) {
-        sp--;
-        const uint64_t s = st_set[sp];
-        const int parent = st_parent[sp], side = st_side[sp];
-        const uint32_t slot = wide_lookup(t, s, err);
-        const float4 v = __ldcg(memo + slot);
+// the plan, walked from the full set by one warp, level by level of the join
+// tree (node 0 the root; sets: 128 words of shared memory)
+template <bool LIVE>
+__device__ __forceinline__ void wide_extract(const WideTable &t, const float4 *memo, const unsigned long long *memo_left,
+                                             uint64_t full, uint32_t wmask, unsigned long long *sets, TreeNode *out,
+                                             int *n_out, unsigned *err) {
+    const uint32_t lane = threadIdx.x & 31u;
+    if (lane == 0u) sets[0] = full;
+    __syncwarp();
+    uint32_t head = 0u, tail = 1u;
+    while (head < tail) {
+        const uint32_t me = head + lane;
+        const bool has = me < tail;
         TreeNode nd;
-        nd.set = s;
-        nd.left = -1;
-        nd.right = -1;
-        nd.rows = v.x;
-        nd.startup = v.y;
-        nd.total = v.z;
-        nd.width = (int32_t)(__float_as_uint(v.w) & wmask);
-        const int me = cnt++;
-        out[me] = nd;
-        if (parent >= 0) {
-            if (side == 0) out[parent].left = me;
-            else out[parent].right = me;
+        nd.set = has ? sets[me] : 0ull;
+        nd.left = nd.right = -1;
+        uint64_t l = 0ull;
+        if (has) {
+            const uint32_t slot = wide_lookup<LIVE>(t, nd.set, err);
+            const float4 v = __ldcg(memo + slot);
+            l = __ldcg(memo_left + slot) & nd.set;
+            nd.rows = v.x;
+            nd.startup = v.y;
+            nd.total = v.z;
+            nd.width = (int32_t)(__float_as_uint(v.w) & wmask);
         }
-        const uint64_t l = __ldcg(memo_left + slot) & s;
-        if (__popcll(s) > 1 && l != 0ull && l != s && sp + 2 <= 128) {
-            st_set[sp] = s ^ l;
-            st_parent[sp] = me;
-            st_side[sp] = 1;
-            sp++;
-            st_set[sp] = l;
-            st_parent[sp] = me;
-            st_side[sp] = 0;
-            sp++;
+        const bool join = has && __popcll(nd.set) > 1 && l != 0ull && l != nd.set;
+        const uint32_t joins = __ballot_sync(kFullW, join);
+        const uint32_t child = tail + 2u * (uint32_t)__popc(joins & ((1u << lane) - 1u));
+        if (join && child + 1u < 128u) {
+            nd.left = (int)child;
+            nd.right = (int)child + 1;
+            sets[child] = l;
+            sets[child + 1u] = nd.set ^ l;
         }
+        if (has) out[me] = nd;
+        head = min(tail, head + 32u);
+        tail = min(tail + 2u * (uint32_t)__popc(joins), 128u);
+        __syncwarp();
     }
-    *n_out = cnt;
+    if (lane == 0u) *n_out = (int)tail;
+}
+
+__global__ void k_wide_extract(WideTable t, const float4 *__restrict__ memo,
+                               const unsigned long long *__restrict__ memo_left, uint64_t full, uint32_t wmask,
+                               TreeNode *__restrict__ out, int *__restrict__ n_out, unsigned *__restrict__ err) {
+    __shared__ unsigned long long sets[128];
+    wide_extract<false>(t, memo, memo_left, full, wmask, sets, out, n_out, err);
+}
+
+// ---------------------------------------------------------------------------
+// k_wide_cactus: the whole sparse DP of a cactus graph (dp_cactus.cuh) in ONE
+// cooperative, persistent launch: per level one warp per set lists the next
+// level (a lane per neighbour, the table deduplicating) and one warp per set
+// costs this one, with a grid barrier between levels; the plan is walked at
+// the end.
+// Bound: latency, 7 to 17 us a level while a level has fewer sets than the
+// grid has warps (list entry, two table entries, two memo entries, cost,
+// barrier), issue beyond.  Before, one launch per level had lane 0 search
+// every set's blocks (112 us for the 42-relation set alone), the host listed
+// the sets and one thread walked the plan (136 us).  Ring path of 42 relations
+// (26 k and 15 k sets, equal costs on most levels): 2216 / 2062 -> 731 / 708 us
+// on the device, 4.6 -> 0.87 ms a call.
+// ---------------------------------------------------------------------------
+struct WideCtl {
+    unsigned bar[4];                   // grid barrier: arrivals, -, error flag
+    unsigned err;
+    unsigned level_n[66];              // sets listed per level (beyond the capacity too)
+    int n_nodes;
+    unsigned long long pairs;
+    TreeNode nodes[128];
+};
+constexpr size_t kWideCtlClear = offsetof(WideCtl, nodes);
+// probes of an entry before the level counts as outgrown (a table at most half
+// full needs a few dozen), and the mark that makes its count so
+constexpr uint32_t kWideProbes = 4096u;
+constexpr unsigned kWideCrowded = 0x80000000u;
+
+// both orientations where the straight-line cost does not apply
+__device__ __noinline__ int wide_join2(const WideInfo &w, uint64_t L, const float4 lv, uint64_t R, const float4 rv,
+                                       bool have, uint64_t match, JoinCost &lr, JoinCost &rl) {
+    const RelVal l = unpack_rel(lv, w.h.hz_packed), r = unpack_rel(rv, w.h.hz_packed);
+    if (!have && w.rel_masked) {
+        uint64_t cl = 0ull, cr = 0ull;
+        for (uint64_t x = L; x; x &= x - 1ull) cl |= w.rel_cls[lowest_idx64(x)];
+        for (uint64_t x = R; x; x &= x - 1ull) cr |= w.rel_cls[lowest_idx64(x)];
+        match = cl & cr;
+        have = true;
+    }
+    RelVal o[2];
+    for (int side = 0; side < 2; side++) {
+        const uint64_t A = side ? R : L, B = side ? L : R;
+        const RelVal a = side ? r : l, b = side ? l : r;
+        o[side] = have ? join_eval_w<true>(w, A, a, B, b, match) : join_eval_w<false>(w, A, a, B, b);
+    }
+    lr.rows = o[0].rows;
+    lr.startup = o[0].startup;
+    lr.total = o[0].total;
+    rl.rows = o[1].rows;
+    rl.startup = o[1].startup;
+    rl.total = o[1].total;
+    return o[0].width;
+}
+
+__global__ void __launch_bounds__(kWideBlock, 2) k_wide_cactus(const unsigned char *__restrict__ blob, uint32_t info_words,
+                                                               uint32_t blob_words, WideTable t, unsigned long long *sets,
+                                                               uint32_t total, int index_order, float4 *memo,
+                                                               unsigned long long *memo_left, WideCtl *ctl,
+                                                               unsigned poll_limit) {
+    // planner info and cactus table, then the warps' scratch
+    extern __shared__ __align__(16) unsigned char wsm[];
+    __shared__ unsigned long long plan_sets[128];
+    WideInfo &w = *reinterpret_cast<WideInfo *>(wsm);
+    for (uint32_t x = threadIdx.x; x < blob_words; x += blockDim.x)
+        reinterpret_cast<uint32_t *>(wsm)[x] = reinterpret_cast<const uint32_t *>(blob)[x];
+    __syncthreads();
+    const CactusView cv = cactus_view(wsm + (size_t)info_words * 4u, w.n_ec);
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    CactusScratch<uint64_t> &sc = reinterpret_cast<CactusScratch<uint64_t> *>(wsm + (size_t)blob_words * 4u)[warp];
+    const PlainParams pp = plain_params(w.h);
+    const uint32_t gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
+    const unsigned max_polls = barrier_polls(poll_limit);
+    const uint32_t cap = 1u << t.cap_log2, n = (uint32_t)w.n;
+    unsigned epoch = 0;
+    uint32_t pairs = 0u;
+
+    // level 1 (gpuqo_cpu_sequential.cu:80-92)
+    if (blockIdx.x == 0 && threadIdx.x < n) {
+        const uint32_t i = threadIdx.x;
+        sets[i] = 1ull << i;
+        wide_insert_one(t, 1ull << i, i, &ctl->err);
+        memo[i] = make_float4(w.rows[i], w.startup[i], w.total[i],
+                              __uint_as_float(memo_width_word(w.h, w.rows[i], w.width[i])));
+        memo_left[i] = 0ull;
+    }
+    if (!grid_barrier<true>(ctl->bar, epoch, max_polls)) return;
+    uint32_t first = 0u, count = n;
+    for (uint32_t k = 1; k <= n; k++) {
+        const uint32_t next = first + count;
+        if (k < n) {
+            // from the far end of the grid: the first warps cost the first sets
+            for (uint32_t i = nwarps - 1u - gwarp; i < count; i += nwarps) {
+                const uint64_t S = __ldcg(sets + first + i);
+                // the arrays are outgrown: nothing more is entered (the table
+                // has twice their room and stays searchable)
+                if ((uint64_t)next + __ldcg(&ctl->level_n[k + 1u]) > total) break;
+                for (uint32_t half = 0; half < n; half += 32u) {
+                    const uint32_t v = half + lane;
+                    bool claimed = false;
+                    const unsigned long long T = S | (1ull << (v & 63u));
+                    uint32_t pos = wide_hash(T, t.cap_log2);
+                    if (v < n && T != S && (w.adj[v] & S) != 0ull) {
+                        bool done = false;
+                        for (uint32_t probe = 0; probe < kWideProbes && !done; probe++) {
+                            const unsigned long long old = atomicCAS(t.keys + pos, 0ull, T);
+                            claimed = old == 0ull;
+                            done = claimed || old == T;
+                            if (!done) pos = (pos + 1u) & (cap - 1u);
+                        }
+                        if (!done) atomicOr(&ctl->level_n[k + 1u], kWideCrowded);
+                    }
+                    const uint32_t m = __ballot_sync(kFullW, claimed);
+                    uint32_t base = 0u;
+                    if (lane == 0u && m) base = atomicAdd(&ctl->level_n[k + 1u], (unsigned)__popc(m));
+                    const uint32_t idx = next + __shfl_sync(kFullW, base, 0) + (uint32_t)__popc(m & ((1u << lane) - 1u));
+                    if (claimed && idx < total) {
+                        sets[idx] = T;
+                        t.slot[pos] = idx;
+                    }
+                }
+            }
+        }
+        if (k >= 2u) {
+            for (uint32_t i = gwarp; i < count; i += nwarps) {
+                const uint64_t S = __ldcg(sets + first + i);
+                const uint32_t slot = first + i;
+                cactus_set<uint64_t>(
+                    S, cv, w.adj, sc, index_order != 0, pp, [&](uint64_t L) { return __ldcg(memo + wide_lookup<true>(t, L, &ctl->err)); },
+                    [&](uint64_t L, const float4 l, const float4 r, uint64_t match, JoinCost &lr, JoinCost &rl) {
+                        return wide_join2(w, L, l, S ^ L, r, (cv.h.flags & kCactusEdges) != 0u, match, lr, rl);
+                    },
+                    [&](float rows, float startup, float cost, int width, uint64_t left) {
+                        memo[slot] = make_float4(rows, startup, cost, __uint_as_float(memo_width_word(w.h, rows, width)));
+                        memo_left[slot] = left;
+                    },
+                    pairs);
+            }
+        }
+        if (!grid_barrier<true>(ctl->bar, epoch, max_polls)) return;
+        if (k == n) break;
+        // final since the barrier, so every block takes the same branch: more
+        // sets than the arrays hold (the host retries with larger ones), or a
+        // graph that is not connected
+        first = next;
+        count = __ldcg(&ctl->level_n[k + 1u]);
+        if (count == 0u || (uint64_t)first + count > total) return;
+    }
+    if (blockIdx.x == 0 && warp == 0u)
+        wide_extract<true>(t, memo, memo_left, (1ull << n) - 1ull, w.h.hz_packed ? kWidthMask : 0xFFFFFFFFu, plan_sets,
+                           ctl->nodes, &ctl->n_nodes, &ctl->err);
+    if (lane == 0u && pairs) atomicAdd(&ctl->pairs, (unsigned long long)pairs);
 }
 
 #define CKW(call)                                                                         \
@@ -999,8 +1177,20 @@ struct WideArena {
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     void *buf[24] = {};
     size_t cap[24] = {};
+    unsigned char *h_stage = nullptr;       // pinned: planner info in, control block out (k_wide_cactus)
+    size_t cap_stage = 0;
+    std::map<size_t, int> coop_blocks;      // dynamic shared bytes -> co-resident blocks of k_wide_cactus
+    bool barrier_timed_out = false;         // its grid barrier gave up: per-level launches until reset
 };
 static WideArena g_wide_arena[64];
+
+bool wide_reset_persistent(int dev) {
+    if (dev < 0 || dev >= 64) return false;
+    std::lock_guard<std::mutex> lk(g_wide_arena[dev].mu);
+    const bool was = g_wide_arena[dev].barrier_timed_out;
+    g_wide_arena[dev].barrier_timed_out = false;
+    return was;
+}
 
 static cudaError_t arena_get(WideArena &a, int idx, size_t bytes, void **out) {
     if (a.cap[idx] < bytes) {
@@ -1094,6 +1284,191 @@ static void tree_tables(const std::vector<uint64_t> &adj, std::vector<uint64_t> 
     }
 }
 
+// the host arrays of a query's planner info
+struct CactusQuery {
+    const WideInfo &info;
+    const std::vector<uint64_t> &tab, &relids;
+    const std::vector<uint32_t> &off;
+    const std::vector<float> &sels;
+    const std::vector<uint64_t> &fks;
+    const std::vector<DevVar> &vars;
+    const std::vector<float4> &pair;
+};
+
+// The sparse DP of a cactus graph as one launch of k_wide_cactus.  The number
+// of connected sets is not known beforehand: the arrays start with room for
+// gpuqo_b200_sparse_host_list sets (131072 by default, 10 MB) and the launch
+// ends at the level that outgrows them, to be repeated with 16 times the room up
+// to the sparse memo's cap.  ran: false when no cooperative launch is possible
+// or its barrier gave up (per-level launches then).
+template <class TooMany>
+static int run_cactus(const CactusQuery &q, int n, DpMode mode, uint64_t cap_sets, TooMany too_many, bool &ran,
+                      std::vector<TreeNode> &nodes, EngineStats &st, std::string &err) {
+    ran = false;
+    int dev = 0, sm_count = 148, rc = 0;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= 64) return 0;
+    cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
+    WideArena &A = g_wide_arena[dev];
+    std::lock_guard<std::mutex> arena_lock(A.mu);
+    if (A.barrier_timed_out) return 0;
+    const uint32_t info_words = (uint32_t)(kWideInfoBytes / 4), blob_words = info_words + 2u * (uint32_t)q.tab.size();
+    const size_t smem = (size_t)blob_words * 4u + (kWideBlock / 32) * sizeof(CactusScratch<uint64_t>);
+    auto cb = A.coop_blocks.find(smem);
+    if (cb == A.coop_blocks.end()) {
+        int occ = 0, coop = 0;
+        cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
+        if (!coop || cudaFuncSetAttribute(k_wide_cactus, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024) != cudaSuccess ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_wide_cactus, kWideBlock, smem) != cudaSuccess)
+            occ = 0;
+        cudaGetLastError();
+        cb = A.coop_blocks.emplace(smem, occ * sm_count).first;
+    }
+    const int grid = cb->second;
+    if (grid <= 0) return 0;
+    ran = true;
+    // table slots and bytes for a number of sets: those of the per-level path
+    auto log2_slots = [](uint64_t sets) {
+        uint32_t l = 1;
+        while ((1ull << l) < 2ull * sets) l++;
+        return l;
+    };
+    const size_t n_ec = q.relids.size();
+    auto bytes_for = [&](uint64_t sets) {
+        return (1ull << log2_slots(sets)) * 12ull + sets * (8 + 16 + 8) + n_ec * 12 + q.sels.size() * 4 + q.fks.size() * 40 +
+               sizeof(WideInfo) + 64 * sizeof(TreeNode) + 4 * 66 + 64;
+    };
+    uint64_t limit = cap_sets;
+    if (gpuqo_b200_device_memory_mb > 0) {
+        const uint64_t budget = (uint64_t)gpuqo_b200_device_memory_mb << 20;
+        uint64_t lo = 0, hi = cap_sets;   // the most sets whose arrays fit
+        while (lo < hi) {
+            const uint64_t mid = (lo + hi + 1) / 2;
+            if (bytes_for(mid) <= budget) lo = mid;
+            else hi = mid - 1;
+        }
+        limit = lo;
+    }
+    const uint64_t room = gpuqo_b200_sparse_host_list > 0 ? (uint64_t)gpuqo_b200_sparse_host_list : (1ull << 17);
+    uint64_t total = std::min(std::max<uint64_t>(room, 2 * (uint64_t)n), limit);
+    if (total < (uint64_t)n) return too_many();
+    // one staging block: planner info and cactus table, then the class arrays
+    size_t at = (size_t)blob_words * 4u;
+    auto place = [&](size_t bytes) {
+        const size_t here = at;
+        at += (bytes + 15) & ~size_t(15);
+        return here;
+    };
+    const size_t o_relids = place(n_ec * 8), o_off = place(n_ec * 4), o_sels = place(q.sels.size() * 4),
+                 o_fks = place(q.fks.size() * 8), o_vars = place(q.vars.size() * sizeof(DevVar)),
+                 o_pair = place(q.pair.size() * sizeof(float4));
+    const size_t in_bytes = at, o_ctl = place(sizeof(WideCtl));
+    unsigned char *d_blob = nullptr;
+    WideCtl *d_ctl = nullptr;
+    unsigned long long *d_keys = nullptr, *d_sets = nullptr, *d_left = nullptr;
+    uint32_t *d_slot = nullptr;
+    float4 *d_memo = nullptr;
+    const WideCtl *ctl = nullptr;
+    float ms = 0.f;
+    if (!A.stream) CKW(cudaStreamCreateWithFlags(&A.stream, cudaStreamNonBlocking));
+    if (!A.ev0) CKW(cudaEventCreate(&A.ev0));
+    if (!A.ev1) CKW(cudaEventCreate(&A.ev1));
+    if (at > A.cap_stage) {
+        if (A.h_stage) cudaFreeHost(A.h_stage);
+        A.h_stage = nullptr;
+        A.cap_stage = 0;
+        CKW(cudaMallocHost(&A.h_stage, at));
+        A.cap_stage = at;
+    }
+    ctl = reinterpret_cast<const WideCtl *>(A.h_stage + o_ctl);
+    CKW(arena_get(A, 20, in_bytes, reinterpret_cast<void **>(&d_blob)));
+    CKW(arena_get(A, 21, sizeof(WideCtl), reinterpret_cast<void **>(&d_ctl)));
+    {
+        WideInfo w = q.info;
+        w.ec_relids = reinterpret_cast<const uint64_t *>(d_blob + o_relids);
+        w.ec_off = reinterpret_cast<const uint32_t *>(d_blob + o_off);
+        w.sels = reinterpret_cast<const float *>(d_blob + o_sels);
+        w.fks = reinterpret_cast<const uint64_t *>(d_blob + o_fks);
+        w.vars = reinterpret_cast<const DevVar *>(d_blob + o_vars);
+        w.pair = reinterpret_cast<const float4 *>(d_blob + o_pair);
+        auto put = [&](size_t o, const void *src, size_t bytes) {
+            if (bytes) std::memcpy(A.h_stage + o, src, bytes);
+        };
+        put(0, &w, sizeof(w));
+        put((size_t)info_words * 4u, q.tab.data(), q.tab.size() * 8);
+        put(o_relids, q.relids.data(), n_ec * 8);
+        put(o_off, q.off.data(), n_ec * 4);
+        put(o_sels, q.sels.data(), q.sels.size() * 4);
+        put(o_fks, q.fks.data(), q.fks.size() * 8);
+        put(o_vars, q.vars.data(), q.vars.size() * sizeof(DevVar));
+        put(o_pair, q.pair.data(), q.pair.size() * sizeof(float4));
+    }
+    CKW(cudaMemcpyAsync(d_blob, A.h_stage, in_bytes, cudaMemcpyHostToDevice, A.stream));
+    for (;;) {
+        const uint32_t cap_log2 = log2_slots(total);
+        CKW(arena_get(A, 7, (size_t)8 << cap_log2, reinterpret_cast<void **>(&d_keys)));
+        CKW(arena_get(A, 8, (size_t)4 << cap_log2, reinterpret_cast<void **>(&d_slot)));
+        CKW(arena_get(A, 9, (size_t)total * 8, reinterpret_cast<void **>(&d_sets)));
+        CKW(arena_get(A, 10, (size_t)total * sizeof(float4), reinterpret_cast<void **>(&d_memo)));
+        CKW(arena_get(A, 11, (size_t)total * 8, reinterpret_cast<void **>(&d_left)));
+        CKW(cudaMemsetAsync(d_keys, 0, (size_t)8 << cap_log2, A.stream));
+        CKW(cudaMemsetAsync(d_ctl, 0, kWideCtlClear, A.stream));
+        CKW(cudaEventRecord(A.ev0, A.stream));
+        {
+            WideTable t{d_keys, d_slot, cap_log2};
+            uint32_t iw = info_words, bw = blob_words, tot = (uint32_t)total;
+            int index_order = mode == kModeDpsub ? 1 : 0;
+            unsigned poll_limit = (unsigned)std::max(0, gpuqo_b200_barrier_poll_limit);
+            void *args[] = {&d_blob, &iw, &bw, &t, &d_sets, &tot, &index_order, &d_memo, &d_left, &d_ctl, &poll_limit};
+            if (cudaLaunchCooperativeKernel((const void *)k_wide_cactus, dim3(grid), dim3(kWideBlock), args, smem, A.stream) !=
+                cudaSuccess) {
+                cudaGetLastError();
+                cb->second = 0;
+                CKW(cudaStreamSynchronize(A.stream));
+                ran = false;
+                return 0;
+            }
+        }
+        CKW(cudaEventRecord(A.ev1, A.stream));
+        CKW(cudaMemcpyAsync(A.h_stage + o_ctl, d_ctl, sizeof(WideCtl), cudaMemcpyDeviceToHost, A.stream));
+        CKW(cudaStreamSynchronize(A.stream));
+        CKW(cudaEventElapsedTime(&ms, A.ev0, A.ev1));
+        st.device_ms += ms;
+        st.kernel_launches++;
+        if (ctl->bar[2] != 0u) {
+            A.barrier_timed_out = true;
+            st.barrier_timeouts++;
+            ran = false;
+            return 0;
+        }
+        uint64_t listed = (uint64_t)n;
+        for (int k = 2; k <= n; k++) listed += ctl->level_n[k];
+        if (listed > total) {
+            if (total >= limit) return too_many();
+            total = std::min(limit, total * 16);
+            continue;
+        }
+        if (ctl->err) {
+            err = "sparse memo table inconsistent";
+            rc = GPUQO_B200_ERR_CUDA;
+            goto done;
+        }
+        if (ctl->n_nodes != 2 * n - 1) {
+            err = "plan extraction produced " + std::to_string(ctl->n_nodes) + " nodes";
+            rc = GPUQO_B200_ERR_CUDA;
+            goto done;
+        }
+        nodes.assign(ctl->nodes, ctl->nodes + ctl->n_nodes);
+        st.connected_sets += listed - (uint64_t)n;
+        st.evaluated_pairs += ctl->pairs;
+        st.memo_bytes = std::max<uint64_t>(st.memo_bytes, bytes_for(total));
+        break;
+    }
+done:
+    if (rc) nodes.clear();
+    return rc;
+}
+
 int engine_run_wide(const HostInfo &info, DpMode mode, std::vector<TreeNode> &nodes, EngineStats &st,
                     std::string &err) {
     const int n = info.n;
@@ -1139,10 +1514,114 @@ int engine_run_wide(const HostInfo &info, DpMode mode, std::vector<TreeNode> &no
               "(use IDP)";
         return GPUQO_B200_ERR_TOO_LARGE;
     };
+    const bool tree = degree_sum == 2 * (n - 1);
+    const size_t n_ec = info.ec_relids.size(), n_sels = info.ec_sels.size(), n_fks = info.ec_fks.size();
+    // planner info (host)
+    WideInfo hw;
+    std::memset(&hw, 0, sizeof(hw));
+    hw.n = n;
+    hw.n_ec = (int)n_ec;
+    hw.h.n = n;
+    hw.h.cpu_operator_cost = info.p.cpu_operator_cost;
+    hw.h.cpu_tuple_cost = info.p.cpu_tuple_cost;
+    hw.h.seq_page_cost = info.p.seq_page_cost;
+    hw.h.disable_cost = info.p.disable_cost;
+    hw.h.work_mem = info.p.work_mem;
+    hw.h.work_mem_bytes = work_mem_bytes_of(info.p.work_mem);
+    hw.h.enable_nestloop = info.p.enable_nestloop ? 1 : 0;
+    hw.h.enable_hashjoin = info.p.enable_hashjoin ? 1 : 0;
+    long long width_sum = 0;
+    bool width_ok = true;
+    for (int i = 0; i < n; i++) {
+        width_sum += info.base[i].width;
+        width_ok = width_ok && info.base[i].width >= 0;
+        hw.adj[i] = adj[i];
+        hw.rows[i] = info.base[i].rows;
+        hw.tuples[i] = info.base[i].tuples;
+        hw.startup[i] = info.base[i].cost.startup;
+        hw.total[i] = info.base[i].cost.total;
+        hw.width[i] = info.base[i].width;
+        hw.fksel[i] = (float)(1.0 / (double)std::fmax(1.0f, info.base[i].tuples));
+        if (info.base[i].composite) hw.composite |= 1ull << i;
+    }
+    hw.h.hz_packed = (width_ok && width_sum < (1ll << kWidthBits)) ? 1u : 0u;
+    std::vector<uint64_t> h_relids(n_ec), h_fks(n_fks);
+    std::vector<uint32_t> h_off(n_ec);
+    std::vector<DevVar> h_vars(n_fks);
+    {
+        int off_sels = 0, off_fks = 0;
+        for (size_t e = 0; e < n_ec; e++) {
+            h_relids[e] = info.ec_relids[e] >> 1;
+            h_off[e] = ((uint32_t)off_sels << 16) | (uint32_t)off_fks;
+            int j = 0;
+            for (uint64_t m = h_relids[e]; m; m &= m - 1ull, j++) {
+                const int rel = __builtin_ctzll(m);
+                const int f = off_fks + j;
+                h_fks[f] = info.ec_fks[f] >> 1;
+                const VarInfo &vi = info.ec_vars[f];
+                DevVar &dv = h_vars[f];
+                std::memset(&dv, 0, sizeof(dv));
+                dv.idx_rows = vi.index.rows;
+                dv.idx_startup = vi.index.cost.startup;
+                dv.idx_total = vi.index.cost.total;
+                dv.flags = (vi.index.available ? 1u : 0u) | (vi.index.unique ? 2u : 0u);
+                devvar_bucket_terms(dv, vi.stats.stadistinct, vi.stats.stanullfrac, vi.stats.mcvfreq, hw.rows[rel],
+                                    hw.tuples[rel]);
+            }
+            off_sels += j * (j - 1) / 2;
+            off_fks += j;
+        }
+    }
+    // the plain-class table (the pair selectivities of gpuqo_row_estimation.cuh
+    // :26-88 for a two-member class, both orientations)
+    std::vector<float4> h_pair(std::max<size_t>(n_ec, 1), make_float4(0.f, 0.f, 0.f, 0.f));
+    for (size_t e = 0; e < n_ec; e++) {
+        if (__builtin_popcountll(h_relids[e]) != 2) continue;
+        const int off_s = (int)(h_off[e] >> 16), off_f = (int)(h_off[e] & 0xFFFFu);
+        const int x = __builtin_ctzll(h_relids[e]), y = 63 - __builtin_clzll(h_relids[e]);
+        const bool fk_xy = (h_fks[off_f] >> y) & 1ull;       // member x's key matches y
+        const bool fk_yx = (h_fks[off_f + 1] >> x) & 1ull;   // member y's key matches x
+        const float sel = info.ec_sels[off_s];
+        bool plain = true;
+        for (int j = 0; j < 2; j++) {
+            const DevVar &dv = h_vars[off_f + j];
+            plain = plain && (dv.flags & (1u | kVarMcvRatio)) == 0u && (dv.flags & kVarNoDistinct) != 0u &&
+                    dv.mcvfreq == 0.0f;
+        }
+        float4 &pe = h_pair[e];
+        pe.x = fk_xy ? hw.fksel[y] : (fk_yx ? hw.fksel[x] : sel);
+        pe.y = fk_yx ? hw.fksel[x] : (fk_xy ? hw.fksel[y] : sel);
+        uint32_t flag = plain ? 1u : 0u;
+        std::memcpy(&pe.z, &flag, 4);
+    }
+    if (n_ec <= 64) {
+        hw.rel_masked = 1;
+        for (size_t e = 0; e < n_ec; e++)
+            for (uint64_t m = h_relids[e]; m; m &= m - 1ull) hw.rel_cls[__builtin_ctzll(m)] |= 1ull << e;
+    }
+    // a cactus graph: one persistent launch (k_wide_cactus)
+    if (!tree && n >= 2 && gpuqo_b200_persistent != 0) {
+        std::vector<float> sel(2 * n_ec, 0.0f);
+        bool plain = plain_cost_applies(hw.h, width_sum);
+        for (size_t e = 0; e < n_ec; e++) {
+            sel[2 * e] = h_pair[e].x;
+            sel[2 * e + 1] = h_pair[e].y;
+            uint32_t flag;
+            std::memcpy(&flag, &h_pair[e].z, 4);
+            plain = plain && flag != 0u;
+        }
+        const std::vector<uint64_t> tab =
+            build_cactus(adj, h_relids, sel, plain, [&](int quals) { return plain_quals(hw.h, quals); });
+        if (!tab.empty()) {
+            bool ran = false;
+            const int rc = run_cactus({hw, tab, h_relids, h_off, info.ec_sels, h_fks, h_vars, h_pair}, n, mode, cap_sets,
+                                      too_many, ran, nodes, st, err);
+            if (ran) return rc;
+        }
+    }
     // Connected sets by level.  A tree's are counted on the host and listed
     // on the device level by level (k_wide_tree_enum); other graphs' are
     // listed on the host by extension with one neighbour, deduplicated.
-    const bool tree = degree_sum == 2 * (n - 1);
     const uint64_t kHostListMax = gpuqo_b200_sparse_host_list > 0 ? (uint64_t)gpuqo_b200_sparse_host_list : (1ull << 16);
     bool dev_list = false;   // a general graph whose levels the device lists
     std::vector<uint64_t> all;
@@ -1235,7 +1714,6 @@ int engine_run_wide(const HostInfo &info, DpMode mode, std::vector<TreeNode> &no
     uint32_t cap_log2 = 1;
     while ((1ull << cap_log2) < 2ull * total) cap_log2++;
     const uint64_t cap = 1ull << cap_log2;
-    const size_t n_ec = info.ec_relids.size(), n_sels = info.ec_sels.size(), n_fks = info.ec_fks.size();
     const uint64_t tree_bytes = tree ? (uint64_t)n * n * 25 : 0ull;
     const uint64_t bytes = cap * 12ull + (uint64_t)total * (8 + 16 + 8) + n_ec * 12 + n_sels * 4 + n_fks * 40 +
                            sizeof(WideInfo) + tree_bytes + 64 * sizeof(TreeNode) + 4 * 66 + 64;
@@ -1243,89 +1721,6 @@ int engine_run_wide(const HostInfo &info, DpMode mode, std::vector<TreeNode> &no
         err = "the sparse exact DP needs " + std::to_string(bytes >> 20) + " MB of device memory; "
               "gpuqo_b200_device_memory_mb allows " + std::to_string(gpuqo_b200_device_memory_mb);
         return GPUQO_B200_ERR_NOMEM;
-    }
-    // planner info (host)
-    WideInfo hw;
-    std::memset(&hw, 0, sizeof(hw));
-    hw.n = n;
-    hw.n_ec = (int)n_ec;
-    hw.h.n = n;
-    hw.h.cpu_operator_cost = info.p.cpu_operator_cost;
-    hw.h.cpu_tuple_cost = info.p.cpu_tuple_cost;
-    hw.h.seq_page_cost = info.p.seq_page_cost;
-    hw.h.disable_cost = info.p.disable_cost;
-    hw.h.work_mem = info.p.work_mem;
-    hw.h.work_mem_bytes = work_mem_bytes_of(info.p.work_mem);
-    hw.h.enable_nestloop = info.p.enable_nestloop ? 1 : 0;
-    hw.h.enable_hashjoin = info.p.enable_hashjoin ? 1 : 0;
-    long long width_sum = 0;
-    bool width_ok = true;
-    for (int i = 0; i < n; i++) {
-        width_sum += info.base[i].width;
-        width_ok = width_ok && info.base[i].width >= 0;
-        hw.adj[i] = adj[i];
-        hw.rows[i] = info.base[i].rows;
-        hw.tuples[i] = info.base[i].tuples;
-        hw.startup[i] = info.base[i].cost.startup;
-        hw.total[i] = info.base[i].cost.total;
-        hw.width[i] = info.base[i].width;
-        hw.fksel[i] = (float)(1.0 / (double)std::fmax(1.0f, info.base[i].tuples));
-        if (info.base[i].composite) hw.composite |= 1ull << i;
-    }
-    hw.h.hz_packed = (width_ok && width_sum < (1ll << kWidthBits)) ? 1u : 0u;
-    std::vector<uint64_t> h_relids(n_ec), h_fks(n_fks);
-    std::vector<uint32_t> h_off(n_ec);
-    std::vector<DevVar> h_vars(n_fks);
-    {
-        int off_sels = 0, off_fks = 0;
-        for (size_t e = 0; e < n_ec; e++) {
-            h_relids[e] = info.ec_relids[e] >> 1;
-            h_off[e] = ((uint32_t)off_sels << 16) | (uint32_t)off_fks;
-            int j = 0;
-            for (uint64_t m = h_relids[e]; m; m &= m - 1ull, j++) {
-                const int rel = __builtin_ctzll(m);
-                const int f = off_fks + j;
-                h_fks[f] = info.ec_fks[f] >> 1;
-                const VarInfo &vi = info.ec_vars[f];
-                DevVar &dv = h_vars[f];
-                std::memset(&dv, 0, sizeof(dv));
-                dv.idx_rows = vi.index.rows;
-                dv.idx_startup = vi.index.cost.startup;
-                dv.idx_total = vi.index.cost.total;
-                dv.flags = (vi.index.available ? 1u : 0u) | (vi.index.unique ? 2u : 0u);
-                devvar_bucket_terms(dv, vi.stats.stadistinct, vi.stats.stanullfrac, vi.stats.mcvfreq, hw.rows[rel],
-                                    hw.tuples[rel]);
-            }
-            off_sels += j * (j - 1) / 2;
-            off_fks += j;
-        }
-    }
-    // the plain-class table (the pair selectivities of gpuqo_row_estimation.cuh
-    // :26-88 for a two-member class, both orientations)
-    std::vector<float4> h_pair(std::max<size_t>(n_ec, 1), make_float4(0.f, 0.f, 0.f, 0.f));
-    for (size_t e = 0; e < n_ec; e++) {
-        if (__builtin_popcountll(h_relids[e]) != 2) continue;
-        const int off_s = (int)(h_off[e] >> 16), off_f = (int)(h_off[e] & 0xFFFFu);
-        const int x = __builtin_ctzll(h_relids[e]), y = 63 - __builtin_clzll(h_relids[e]);
-        const bool fk_xy = (h_fks[off_f] >> y) & 1ull;       // member x's key matches y
-        const bool fk_yx = (h_fks[off_f + 1] >> x) & 1ull;   // member y's key matches x
-        const float sel = info.ec_sels[off_s];
-        bool plain = true;
-        for (int j = 0; j < 2; j++) {
-            const DevVar &dv = h_vars[off_f + j];
-            plain = plain && (dv.flags & (1u | kVarMcvRatio)) == 0u && (dv.flags & kVarNoDistinct) != 0u &&
-                    dv.mcvfreq == 0.0f;
-        }
-        float4 &pe = h_pair[e];
-        pe.x = fk_xy ? hw.fksel[y] : (fk_yx ? hw.fksel[x] : sel);
-        pe.y = fk_yx ? hw.fksel[x] : (fk_xy ? hw.fksel[y] : sel);
-        uint32_t flag = plain ? 1u : 0u;
-        std::memcpy(&pe.z, &flag, 4);
-    }
-    if (n_ec <= 64) {
-        hw.rel_masked = 1;
-        for (size_t e = 0; e < n_ec; e++)
-            for (uint64_t m = h_relids[e]; m; m &= m - 1ull) hw.rel_cls[__builtin_ctzll(m)] |= 1ull << e;
     }
     std::vector<uint64_t> t_sub, t_before, t_anc;
     std::vector<uint8_t> t_par;
@@ -1553,7 +1948,7 @@ int engine_run_wide(const HostInfo &info, DpMode mode, std::vector<TreeNode> &no
                 CKW(cudaGetLastError());
             }
         }
-        k_wide_extract<<<1, 32, 0, stream>>>(t, d_memo, d_left, full, n, hw.h.hz_packed ? kWidthMask : 0xFFFFFFFFu,
+        k_wide_extract<<<1, 32, 0, stream>>>(t, d_memo, d_left, full, hw.h.hz_packed ? kWidthMask : 0xFFFFFFFFu,
                                              d_nodes, d_nn, d_err);
         launches++;
         CKW(cudaGetLastError());

@@ -344,16 +344,6 @@ static int max_block_size(const HostInfo &info) {
     return best;
 }
 
-static PlainQuals plain_quals(const DevHeader &h, int quals) {
-    PlainQuals q;
-    q.per_tuple = 0.0f;
-    for (int i = 0; i < quals; i++) q.per_tuple += h.cpu_operator_cost;
-    q.quals_cost = h.cpu_operator_cost * (float)quals;
-    q.nl_tuple = h.cpu_tuple_cost + q.per_tuple;
-    q.hj_row = q.quals_cost + h.cpu_tuple_cost;
-    return q;
-}
-
 std::vector<uint32_t> build_blob(const HostInfo &info) {
     const int n_ec = (int)info.ec_relids.size();
     const int n_sels = (int)info.ec_sels.size();
@@ -528,11 +518,7 @@ std::vector<uint32_t> build_blob(const HostInfo &info) {
     for (int i = 0; i < n_sels; i++) sels[i] = info.ec_sels[i];
     fill_rel_ecs(v, n);
     fill_pair_sel(v);
-    // the straight-line cost (plain_mirror) leaves out the skew check, which
-    // compares one row of the inner side with work_mem: the widest set's row
-    // decides for all
-    const float widest = (float)((((unsigned long long)std::max(width_sum, 0ll) + 7ull) & ~7ull) + 24ull);
-    const bool straight = h->hz_packed && h->enable_hashjoin && widest <= h->work_mem_bytes;
+    const bool straight = plain_cost_applies(*h, width_sum);
     if (h->ec_masked) {
         // ec_selectivity (gpuqo_row_estimation.cuh:49-88) of each two-member
         // class in both orientations: the FK selectivity of the outer member's
