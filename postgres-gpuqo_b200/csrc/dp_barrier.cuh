@@ -1,6 +1,7 @@
 // dp_barrier.cuh - the bounded grid barrier of the persistent kernels.
 #pragma once
 
+#include <cstdint>
 #include <cuda_runtime.h>
 
 namespace gqb {
@@ -67,6 +68,19 @@ __device__ __forceinline__ bool grid_barrier(unsigned *bar, unsigned &epoch, uns
     }
     __syncthreads();
     return s_ok != 0u;
+}
+
+// The barrier of a grid that is one thread-block cluster, in hardware (no
+// polling, nothing to time out): every thread of the cluster.
+__device__ __forceinline__ uint32_t cluster_blocks() {
+    uint32_t n;
+    asm volatile("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(n));
+    return n;
+}
+
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
 }  // namespace gqb

@@ -387,6 +387,23 @@ __device__ __forceinline__ uint32_t memo_width_word(const DevHeader &h, float ro
     return (uint32_t)width | (1u << kWidthBits) | (lb << (kWidthBits + 1)) | (lt << (kWidthBits + 6));
 }
 
+// The width word where only plain_mirror reads it: it asks whether the hash
+// table takes more than one batch, which exec_choose_hash_table_size decides
+// by its first comparison; the batch count's field is 1 then and 0 otherwise.
+__device__ __forceinline__ uint32_t plain_width_word(const DevHeader &h, float rows, int width) {
+    if (__builtin_expect(h.work_mem < 4096 || h.work_mem >= (1 << 20), 0)) return memo_width_word(h, rows, width);
+    const float ntuples = rows <= 0.0f ? 1000.0f : rows;
+    const uint32_t tupsize = 32u + (((uint32_t)width + 7u) & ~7u);
+    uint32_t bytes = (uint32_t)h.work_mem * 1024u;
+    const uint32_t max_pointers = 1u << (31 - __clz((uint32_t)(h.work_mem_bytes / 8.0f)));
+    const uint32_t skew = bytes * 2u / 100u;
+    if (skew >= tupsize + 84u) bytes -= skew;
+    uint32_t nb = (uint32_t)fminf(ceilf(ntuples), (float)max_pointers);
+    nb = 1u << ceil_log2_u32(nb < 1024u ? 1024u : nb);
+    const bool batched = ntuples * (float)tupsize + (float)(8u * nb) > (float)bytes;
+    return (uint32_t)width | (batched ? 1u << (kWidthBits + 6) : 0u);
+}
+
 // memo entry of base relation i (gpuqo_cpu_sequential.cu:80-92)
 __device__ __forceinline__ float4 base_entry(const DevHeader &h, int i) {
     return make_float4(h.rows[i], h.startup[i], h.total[i], __uint_as_float(memo_width_word(h, h.rows[i], h.width[i])));

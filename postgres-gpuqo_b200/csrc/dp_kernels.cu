@@ -748,8 +748,7 @@ __global__ void __launch_bounds__(kBlock) k_eval_mpdp(const uint32_t *__restrict
 // emitted in post-order of their child end, so the reference's enumeration
 // index of a split is 2 * post_r(v) + (the lower end's side outer ? 0 : 1) with
 //     post_r(v) = |S & before_r[v]| - |S & anc_r[v]| + |S & sub_r[v]| - 1
-// (preorder rank minus depth plus subtree size minus one); it is computed only
-// where it decides something, between equal costs and for NaN costs.
+// (preorder rank minus depth plus subtree size minus one).
 // ---------------------------------------------------------------------------
 // what the classes of a query allow (one instantiation each, so that a kernel
 // carries only the evaluation its queries take): kTreePlain
@@ -775,81 +774,68 @@ __device__ __forceinline__ TreeRows tree_rows(const DevHeader &h, uint32_t S) {
     return t;
 }
 
-// the outer side of orientation `code` (child end | kSideHigher) of S
-__device__ __forceinline__ uint32_t tree_side(const TreeRows &t, uint32_t S, uint32_t code) {
-    const uint2 e = *reinterpret_cast<const uint2 *>(t.row + 2u * (code & 31u));
-    const uint32_t comp = S & e.x;
-    const bool comp_outer = ((e.y & kTreeLower) != 0u) == ((code & kSideHigher) == 0u);
-    return comp_outer ? comp : S ^ comp;
-}
-
-// the reference's enumeration index of orientation `code`
-__device__ __noinline__ uint32_t tree_index(const uint32_t *row, int n, uint32_t S, uint32_t code, uint32_t dpsub) {
-    const uint32_t v = code & 31u;
-    const uint2 e = *reinterpret_cast<const uint2 *>(row + 2u * v);
-    const uint32_t comp = S & e.x;
+// The reference's order of a split's two orientations: outer side L0 (the
+// lower end's) and S - L0.  Block order: 2 * post_r(v) and the next; plain
+// DPsub's: the subsets of S in increasing order, so the outer side itself.
+__device__ __forceinline__ void tree_order(const TreeRows &t, uint32_t S, uint32_t v, uint32_t sub, uint32_t L0,
+                                           uint32_t dpsub, uint32_t &p0, uint32_t &p1) {
     if (dpsub) {
-        const bool comp_outer = ((e.y & kTreeLower) != 0u) == ((code & kSideHigher) == 0u);
-        return dpsub_index(comp_outer ? comp : S ^ comp, S);
+        p0 = L0;
+        p1 = S ^ L0;
+    } else {
+        const uint2 w = *reinterpret_cast<const uint2 *>(t.row + 2u * (uint32_t)t.n + 2u * v);
+        p0 = 2u * (uint32_t)(__popc(S & w.x) - __popc(S & w.y) + __popc(S & sub) - 1);
+        p1 = p0 + 1u;
     }
-    const uint2 w = *reinterpret_cast<const uint2 *>(row + 2u * (uint32_t)n + 2u * v);
-    const uint32_t post = (uint32_t)(__popc(S & w.x) - __popc(S & w.y) + __popc(comp) - 1);
-    return 2u * post + ((code & kSideHigher) ? 1u : 0u);
 }
 
-// A lane's best split of a set: the ordered cost (ord_float), the orientation
-// and the values the memo needs.  Ties go to the lower enumeration index.
-constexpr uint32_t kNoCode = 0xFFu;
+// A lane's best split of a set: (ordered cost, place in the reference's order)
+// and the values the memo needs.  Equal costs are common (key joins leave the
+// row counts of the larger side alone, so the order of several joins does not
+// matter), hence the place is at hand and not computed on demand.
 struct TreeBest {
-    uint32_t ord, code;
+    unsigned long long key;
+    uint32_t left;
     float rows, startup;
-    uint32_t nan_code;     // the candidate of lowest index with a NaN cost, kNoCode: none
+    uint32_t nan_p;        // lowest place of a candidate with a NaN cost, kFull: none
 
     __device__ __forceinline__ void init() {
-        ord = kFull;
-        code = kNoCode;
+        key = ~0ull;
+        left = 0u;
         rows = startup = 0.0f;
-        nan_code = kNoCode;
+        nan_p = kFull;
     }
 };
 
-__device__ __forceinline__ void tree_update(TreeBest &best, const DevHeader &h, const TreeRows &t, uint32_t S,
-                                            uint32_t code, float rows, float startup, float total) {
-    const uint32_t ord = ord_float(total);
-    bool take = ord < best.ord;
-    if (__builtin_expect(ord == best.ord || isnan(total), 0)) {
-        if (isnan(total)) {
-            if (best.nan_code == kNoCode ||
-                tree_index(t.row, t.n, S, code, h.index_order) < tree_index(t.row, t.n, S, best.nan_code, h.index_order))
-                best.nan_code = code;
-            take = false;
-        } else {
-            take = tree_index(t.row, t.n, S, code, h.index_order) <
-                   tree_index(t.row, t.n, S, best.code, h.index_order);
-        }
+__device__ __forceinline__ void tree_update(TreeBest &best, uint32_t p, uint32_t L, float rows, float startup,
+                                            float total) {
+    if (__builtin_expect(isnan(total), 0)) {
+        best.nan_p = min(best.nan_p, p);
+        return;
     }
-    if (take) {
-        best.ord = ord;
-        best.code = code;
+    const unsigned long long key = ((unsigned long long)ord_float(total) << 32) | p;
+    if (key < best.key) {
+        best.key = key;
+        best.left = L;
         best.rows = rows;
         best.startup = startup;
     }
 }
 
-// both orientations of the split of S at child end v from the memo entries of
-// the side that holds the edge's lower end (lv) and of the other (rv)
+// both orientations of the split of S with the lower end's side L0 from the
+// memo entries of that side (lv) and of the other (rv)
 template <int LAYOUT>
 __device__ __forceinline__ void tree_cost(const DevInfoView &d, const PlainParams &pp, const TreeRows &t, uint32_t S,
-                                          uint32_t L0, uint32_t v, uint32_t edge, const float4 lv, const float4 rv,
-                                          TreeBest &best, int &width) {
+                                          uint32_t L0, uint32_t p0, uint32_t p1, uint32_t edge, const float4 lv,
+                                          const float4 rv, TreeBest &best, int &width) {
     const DevHeader &h = *d.h;
     if (LAYOUT == kTreePlain) {
         const TreeEdge &e = reinterpret_cast<const TreeEdge *>(t.tab + tree_edge_off(t.n))[edge];
         JoinCost lr, rl;
         plain_mirror(pp, e.quals, e.sel_lo, e.sel_hi, lv, rv, lr, rl);
         width = (int)((__float_as_uint(lv.w) & kWidthMask) + (__float_as_uint(rv.w) & kWidthMask));
-        tree_update(best, h, t, S, v, lr.rows, lr.startup, lr.total);
-        tree_update(best, h, t, S, v | kSideHigher, rl.rows, rl.startup, rl.total);
+        tree_update(best, p0, L0, lr.rows, lr.startup, lr.total);
+        tree_update(best, p1, S ^ L0, rl.rows, rl.startup, rl.total);
     } else {
         const RelVal l = unpack_rel(lv, h.hz_packed), r = unpack_rel(rv, h.hz_packed);
         RelVal o0, o1;
@@ -857,30 +843,33 @@ __device__ __forceinline__ void tree_cost(const DevInfoView &d, const PlainParam
             LAYOUT == kTreeMasked ? reinterpret_cast<const TreeEdge *>(t.tab + tree_edge_off(t.n))[edge].classes : 0u;
         join_eval_mirror_tree<LAYOUT == kTreeMasked>(d, L0, l, S ^ L0, r, classes, o0, o1);
         width = o0.width;
-        tree_update(best, h, t, S, v, o0.rows, o0.startup, o0.total);
-        tree_update(best, h, t, S, v | kSideHigher, o1.rows, o1.startup, o1.total);
+        tree_update(best, p0, L0, o0.rows, o0.startup, o0.total);
+        tree_update(best, p1, S ^ L0, o1.rows, o1.startup, o1.total);
     }
 }
 
 // The first candidate of a set in enumeration order has a NaN cost: the
 // reference keeps it.  Rare (overflowed row estimates): every lane finds its
-// lowest index, and when the group's lowest is a NaN one, its lane costs it
+// lowest place, and when the group's lowest is a NaN one, its lane costs it
 // again and writes the entry.  Returns whether the lane's group is settled.
-template <int LAYOUT>
-__device__ __noinline__ bool tree_nan_rule(const DevInfoView d, uint32_t S, bool has, int k, int G, uint32_t nan_code,
+__device__ __noinline__ bool tree_nan_rule(const DevInfoView d, uint32_t S, bool has, int G, uint32_t nan_p,
                                            const float4 *memo, RelVal &out, uint32_t &left, bool &writer) {
     const DevHeader &h = *d.h;
     const TreeRows t = tree_rows(h, S);
     const int gl = (int)(threadIdx.x & 31u) % G;
-    uint32_t first = kFull;
+    uint32_t first = kFull, nan_left = 0u;
     uint32_t x = has ? S & (S - 1u) : 0u;
     for (int j = 0; x; x &= x - 1u, j++) {
-        if (j % G != gl) continue;
         const uint32_t v = (uint32_t)lowest_idx(x);
-        first = min(first, tree_index(t.row, t.n, S, v, h.index_order));
-        first = min(first, tree_index(t.row, t.n, S, v | kSideHigher, h.index_order));
+        if (G == 32 ? (int)v != gl : j % G != gl) continue;
+        const uint2 e = *reinterpret_cast<const uint2 *>(t.row + 2u * v);
+        const uint32_t L0 = (e.y & kTreeLower) ? S & e.x : S ^ (S & e.x);
+        uint32_t p0, p1;
+        tree_order(t, S, v, e.x, L0, h.index_order, p0, p1);
+        first = min(first, min(p0, p1));
+        if (p0 == nan_p) nan_left = L0;
+        if (p1 == nan_p) nan_left = S ^ L0;
     }
-    const uint32_t nan_p = nan_code != kNoCode ? tree_index(t.row, t.n, S, nan_code, h.index_order) : kFull;
     uint32_t gfirst = first, gnan = nan_p;
     for (int off = G >> 1; off >= 1; off >>= 1) {
         gfirst = min(gfirst, __shfl_xor_sync(kFull, gfirst, off));
@@ -889,7 +878,7 @@ __device__ __noinline__ bool tree_nan_rule(const DevInfoView d, uint32_t S, bool
     const bool settled = has && gnan != kFull && gnan == gfirst;
     writer = settled && nan_p == gnan;
     if (writer) {
-        left = tree_side(t, S, nan_code);
+        left = nan_left;
         const RelVal l = load_rel(memo, left, h.hz_packed), r = load_rel(memo, S ^ left, h.hz_packed);
         out = join_eval(d, left, l, S ^ left, r);
     }
@@ -897,9 +886,9 @@ __device__ __noinline__ bool tree_nan_rule(const DevInfoView d, uint32_t S, bool
 }
 
 // One set of k relations (has: the lane's group holds one) by a group of G
-// lanes, G a power of two.  Lanes take the child ends by rank in S; both memo
-// entries of the next split are requested before the current one is costed.
-// The whole warp calls it, with the same k and G.
+// lanes, G a power of two.  Lanes take the child ends by rank in S (a whole
+// warp: by number); both memo entries of the next split are requested before
+// the current one is costed.  The whole warp calls it, with the same k and G.
 template <int LAYOUT>
 __device__ __forceinline__ void tree_set(const DevInfoView &d, const PlainParams &pp, const TreeRows &t, uint32_t S,
                                          bool has, int k, int G, float4 *memo, uint32_t *memo_left) {
@@ -915,22 +904,23 @@ __device__ __forceinline__ void tree_set(const DevInfoView &d, const PlainParams
     TreeBest best;
     best.init();
     int width = 0;
-    uint32_t v = 0u, L0 = 0u, edge = 0u;
+    uint32_t p0 = 0u, p1 = 0u, L0 = 0u, edge = 0u;
     float4 lv = make_float4(0.f, 0.f, 0.f, 0.f), rv = lv;
     auto fetch = [&]() -> bool {
         if (x == 0u) return false;
-        v = (uint32_t)lowest_idx(x);
+        const uint32_t v = (uint32_t)lowest_idx(x);
         const uint2 e = *reinterpret_cast<const uint2 *>(t.row + 2u * v);
         const uint32_t comp = S & e.x;
         L0 = (e.y & kTreeLower) ? comp : S ^ comp;
-        edge = e.y & 31u;
         lv = __ldcg(memo + L0);
         rv = __ldcg(memo + (S ^ L0));
+        edge = e.y & 31u;
+        tree_order(t, S, v, e.x, L0, h.index_order, p0, p1);
         return true;
     };
     bool active = fetch();
     for (int j = 0; j < steps; j++) {
-        const uint32_t cv = v, cL = L0, ce = edge;
+        const uint32_t c0 = p0, c1 = p1, cL = L0, ce = edge;
         const float4 clv = lv, crv = rv;
         const bool cact = active;
         active = false;
@@ -938,34 +928,37 @@ __device__ __forceinline__ void tree_set(const DevInfoView &d, const PlainParams
             for (int i = 0; i < G; i++) x &= x - 1u;
             active = fetch();
         }
-        if (cact) tree_cost<LAYOUT>(d, pp, t, S, cL, cv, ce, clv, crv, best, width);
+        if (cact) tree_cost<LAYOUT>(d, pp, t, S, cL, c0, c1, ce, clv, crv, best, width);
     }
-    uint32_t m = best.ord;
-    for (int off = G >> 1; off >= 1; off >>= 1) m = min(m, __shfl_xor_sync(kFull, m, off));
-    bool win = has && best.ord == m && m != kFull;
-    const uint32_t group_mask = (G == 32) ? kFull : (((1u << G) - 1u) << (lane & ~(G - 1)));
-    const uint32_t tied = __ballot_sync(kFull, win) & group_mask;
-    if (__any_sync(kFull, __popc(tied) > 1)) {
-        const uint32_t p = win ? tree_index(t.row, t.n, S, best.code, h.index_order) : kFull;
-        uint32_t pm = p;
-        for (int off = G >> 1; off >= 1; off >>= 1) pm = min(pm, __shfl_xor_sync(kFull, pm, off));
-        win = win && p == pm;
+    uint32_t mh = (uint32_t)(best.key >> 32), ml = (uint32_t)best.key;
+    if (G == 32) {
+        const uint32_t w = __reduce_min_sync(kFull, mh);
+        ml = __reduce_min_sync(kFull, mh == w ? ml : kFull);
+        mh = w;
+    } else {
+        for (int off = G >> 1; off >= 1; off >>= 1) {
+            const uint32_t oh = __shfl_xor_sync(kFull, mh, off), ol = __shfl_xor_sync(kFull, ml, off);
+            if (oh < mh || (oh == mh && ol < ml)) {
+                mh = oh;
+                ml = ol;
+            }
+        }
     }
-    if (__any_sync(kFull, best.nan_code != kNoCode)) {
+    bool win = has && best.key == (((unsigned long long)mh << 32) | ml) && best.key != ~0ull;
+    if (__any_sync(kFull, best.nan_p != kFull)) {
         RelVal out;
         uint32_t left = 0u;
         bool writer = false;
-        if (tree_nan_rule<LAYOUT>(d, S, has, k, G, best.nan_code, memo, out, left, writer)) win = false;
+        if (tree_nan_rule(d, S, has, G, best.nan_p, memo, out, left, writer)) win = false;
         if (writer) memo_write(h, memo, memo_left, S, out, left);
     }
     if (win) {
-        RelVal out;
-        out.rows = best.rows;
-        out.startup = best.startup;
         // the inverse of ord_float (a total is never -0: its startup cost starts from +0)
-        out.total = __uint_as_float((m & 0x80000000u) ? m ^ 0x80000000u : ~m);
-        out.width = width;
-        memo_write(h, memo, memo_left, S, out, tree_side(t, S, best.code));
+        const float total = __uint_as_float((mh & 0x80000000u) ? mh ^ 0x80000000u : ~mh);
+        const uint32_t word = LAYOUT == kTreePlain ? plain_width_word(h, best.rows, width)
+                                                   : memo_width_word(h, best.rows, width);
+        memo[S] = make_float4(best.rows, best.startup, total, __uint_as_float(word));
+        memo_left[S] = best.left;
     }
 }
 
@@ -1060,7 +1053,17 @@ __global__ void __launch_bounds__(kBlock, 3) k_eval_tree(const uint32_t *__restr
 // warp; the loop over the relations of S costs about 10 instructions each.
 __device__ __forceinline__ uint32_t above(uint32_t bit) { return ~((bit << 1) - 1u); }
 
-// the relations v whose addition to S emits S + v (adj(v): neighbours of v)
+// the relations v of the neighbours N of S whose addition emits S + v
+template <class Adj>
+__device__ __forceinline__ uint32_t tree_extension_mask(uint32_t S, uint32_t N, uint32_t leaves, Adj adj) {
+    const uint32_t m1 = 1u << (31 - __clz(leaves));
+    const uint32_t rest = leaves ^ m1;
+    if (rest == 0u) return N & above(m1);                      // a single relation
+    const uint32_t m2 = 1u << (31 - __clz(rest)), a1 = adj(31 - __clz(m1));
+    return N & ((above(m1) & ~a1) | (above(m2) & a1));
+}
+
+// the same from S alone (adj(v): neighbours of v)
 template <class Adj>
 __device__ __forceinline__ uint32_t tree_extensions(uint32_t S, Adj adj) {
     uint32_t N = 0u, leaves = 0u;
@@ -1069,13 +1072,7 @@ __device__ __forceinline__ uint32_t tree_extensions(uint32_t S, Adj adj) {
         N |= a;
         if ((in & (in - 1u)) == 0u) leaves |= x & (0u - x);   // S is connected: at least one neighbour in S
     }
-    if (S == 0u) return 0u;
-    N &= ~S;
-    const uint32_t m1 = 1u << (31 - __clz(leaves));
-    const uint32_t rest = leaves ^ m1;
-    if (rest == 0u) return N & above(m1);                      // a single relation
-    const uint32_t m2 = 1u << (31 - __clz(rest)), a1 = adj(31 - __clz(m1));
-    return N & ((above(m1) & ~a1) | (above(m2) & a1));
+    return S ? tree_extension_mask(S, N & ~S, leaves, adj) : 0u;
 }
 
 __device__ __forceinline__ void tree_enum_phase(const uint32_t *adj, int k, const uint32_t *prev_sets, uint32_t c_prev,
@@ -1085,6 +1082,21 @@ __device__ __forceinline__ void tree_enum_phase(const uint32_t *adj, int k, cons
     // from the far end of the grid: the first warps evaluate the first sets
     // of the level in the same phase, so small levels split the two jobs
     const uint32_t tid = nthreads - 1u - (blockIdx.x * blockDim.x + threadIdx.x);
+    if (c_prev * 32u <= nthreads) {
+        // a level that leaves warps idle: one warp per set and one lane per
+        // relation, about 40 instructions instead of 10 per relation of the set
+        const uint32_t i = tid >> 5;
+        if (i >= c_prev) return;
+        const uint32_t S = (k == 2) ? (1u << i) : __ldcg(prev_sets + i);
+        const uint32_t a = ((S >> lane) & 1u) ? adj[lane] : 0u, in = a & S;
+        const uint32_t leaves = __ballot_sync(kFull, a != 0u && (in & (in - 1u)) == 0u);
+        const uint32_t ext = tree_extension_mask(S, __reduce_or_sync(kFull, a) & ~S, leaves, [&](int v) { return adj[v]; });
+        uint32_t base = 0u;
+        if (lane == 0u && ext) base = atomicAdd(&lc->n_sets, (uint32_t)__popc(ext));
+        base = __shfl_sync(kFull, base, 0);
+        if ((ext >> lane) & 1u) out_sets[base + (uint32_t)__popc(ext & ((1u << lane) - 1u))] = S | (1u << lane);
+        return;
+    }
     for (uint32_t first = tid & ~31u; first < c_prev; first += nthreads) {
         const uint32_t idx = first + (tid & 31u);
         const uint32_t S = idx < c_prev ? ((k == 2) ? (1u << idx) : __ldcg(prev_sets + idx)) : 0u;
@@ -1156,12 +1168,15 @@ struct TreePlan {
 
 // Bound: a warp-step (one split, both orientations) issues about 240
 // instructions on a plain tree; wide levels are issue-bound, narrow ones wait
-// for the chain list entry -> two memo entries -> cost -> reduction -> memo
-// entry -> grid barrier.  With the child end of a split read from the root's
-// row, the sums over an edge's classes made on the host (TreeEdge), the
-// enumeration index left to ties and the extensions of a set as one mask:
-// star-22 (44.0 M pairs) 751 -> 491 us, snowflake-25 (3.2 M and 4.8 M pairs)
-// 265 / 290 -> 169 / 168 us, key chain-30 203 -> 150 us on the device.
+// for the chain list entry (about 700 cycles from L2) -> two memo entries (700)
+// -> cost (500) -> reduction (300) -> memo entry (450) -> barrier (100 cycles in
+// one block, 900 in a cluster of 8, 2000 over 296 blocks).  With the child end
+// of a split read from the root's row, the sums over an edge's classes made on
+// the host (TreeEdge), the extensions of a set as one mask, the order of a
+// split at hand for equal costs, and grids no larger than the widest level
+// needs, one cluster where that does: device time of star-22 (44.0 M pairs)
+// 751 -> 387 us, snowflake-25 (3.2 M and 4.8 M pairs) 265 / 290 -> 139 us, key
+// chain-30 203 -> 90 us, star-12 77 -> 47 us, star-6 38 -> 20 us.
 // MINB: blocks per SM the register budget is set for (2, 3 or 4: 128, 80 or 64
 // registers, no spill but 4 bytes with 4 blocks), chosen per query from its
 // connected sets per level, the total over the relation count
@@ -1185,6 +1200,17 @@ __global__ void __launch_bounds__(kBlock, MINB) k_dp_tree(const uint32_t *__rest
     const uint32_t nwarps = gridDim.x * kWarpsPerBlock;
     const PlainParams pp = plain_params(*d.h);
     unsigned epoch = 0;   // grid barriers passed (thread 0)
+    // one block, or a grid that is one cluster, synchronises in hardware; the
+    // other variants never run as one
+    const bool cluster = MINB == 2 && cluster_blocks() == gridDim.x;
+    auto barrier = [&]() -> bool {
+        if (MINB == 2 && cluster) {
+            if (gridDim.x == 1u) __syncthreads();
+            else cluster_barrier();
+            return true;
+        }
+        return grid_barrier<true>(bar, epoch, max_polls);
+    };
 
     // phase 0: base relations (gpuqo_cpu_sequential.cu:80-92) and level-2 sets
     if (blockIdx.x == 0 && threadIdx.x < n) {
@@ -1193,14 +1219,14 @@ __global__ void __launch_bounds__(kBlock, MINB) k_dp_tree(const uint32_t *__rest
         memo_left[1u << i] = 0u;
     }
     if (n >= 2) tree_enum_phase(adj, 2, nullptr, (uint32_t)n, setsA, lvl + 2);
-    if (!grid_barrier<true>(bar, epoch, max_polls)) return;
+    if (!barrier()) return;
     for (int k = 2; k <= n; k++) {
         uint32_t *cur = (k & 1) ? setsB : setsA;
         uint32_t *nxt = (k & 1) ? setsA : setsB;
         const uint32_t count = plan.count[k];
         if (k < n) tree_enum_phase(adj, k + 1, cur, count, nxt, lvl + k + 1);
         tree_level<LAYOUT>(d, pp, gwarp, nwarps, cur, count, k, plan.group[k], memo, memo_left);
-        if (!grid_barrier<true>(bar, epoch, max_polls)) return;
+        if (!barrier()) return;
     }
     if (blockIdx.x == 0 && threadIdx.x < 32) {
         __shared__ uint32_t plan_sets[64];
@@ -1797,9 +1823,9 @@ struct Tuning {
     // tree queries with up to this many connected sets per level run
     // k_dp_tree<2>, those with more than single_wide_level_sets k_dp_tree<4>
     // (device time of the 2- / 3- / 4-blocks variant: star-18, 7 k sets per
-    // level, 121 / 126 / 135 us; star-20, 26 k, 205 / 194 / 203; star-21, 50 k,
-    // 329 / 299 / 312; star-22, 95 k, 522 / 491 / 476; star-24, 350 k,
-    // 2009 / 1745 / 1632; the third crossover is left to the autotuner)
+    // level, 98 / 104 / 111 us; star-20, 26 k, 163 / 156 / 165; star-21, 50 k,
+    // 253 / 237 / 252; star-22, 95 k, 392 / 387 / 385; star-24, 350 k,
+    // 1557 / 1441 / 1407; the third crossover is left to the autotuner)
     double single_narrow_level_sets = 16384.0;
     double single_wide_level_sets = 1e30;
     double batch_single_sets = double(1u << 20);   // a batch hands larger tree queries to k_dp_tree
@@ -1880,6 +1906,11 @@ struct EngineCtl {
     TreeNode tree[64];
 };
 constexpr size_t kCtlClearBytes = offsetof(EngineCtl, pad);   // lvl .. tree_n
+
+// largest cluster of k_dp_tree (the portable size), and the blocks' worth of
+// splits of the widest level up to which a cluster runs the query
+constexpr int kTreeCluster = 8;
+constexpr int kTreeClusterLevel = 16;
 
 class Engine {
 public:
@@ -2175,6 +2206,22 @@ public:
         return 0;
     }
 
+    // Blocks of a tree query: enough lanes for every split of its widest level,
+    // so that no level takes a second round, and no more, since a barrier
+    // costs with its arrivals.  Up to kTreeClusterLevel blocks' worth run as
+    // one cluster (a power of two of blocks), which the hardware synchronises:
+    // star-12 (widest level 2772 splits, 11 blocks' worth) 66 us on 296 blocks,
+    // 54 us in a cluster of 8.
+    static int tree_grid(const TreePlan &plan, int n, int full) {
+        uint64_t lanes = 1;
+        for (int k = 2; k <= n; k++) lanes = std::max(lanes, (uint64_t)plan.count[k] * (uint64_t)(k - 1));
+        const uint64_t blocks = (lanes + kBlock - 1) / kBlock;
+        if (blocks > (uint64_t)kTreeClusterLevel) return (int)std::min<uint64_t>(blocks, (uint64_t)full);
+        int grid = 1;
+        while (grid < kTreeCluster && (uint64_t)grid < blocks) grid <<= 1;
+        return std::min(grid, full);
+    }
+
     // The whole tree-mode MPDP as one cooperative launch (k_dp_tree).  Returns
     // 0 and sets launched when the kernel was started.
     int launch_persistent(int n, uint32_t words, bool &launched, std::string &err) {
@@ -2195,7 +2242,7 @@ public:
             {(const void *)k_dp_tree<2, 0>, (const void *)k_dp_tree<2, 1>, (const void *)k_dp_tree<2, 2>},
             {(const void *)k_dp_tree<3, 0>, (const void *)k_dp_tree<3, 1>, (const void *)k_dp_tree<3, 2>},
             // at 64 registers the class passes spill about 100 bytes and lose to
-            // 3 blocks at every size (star-22 with statistics 1094 against 1084 us)
+            // 3 blocks (star-20 with statistics 406 against 356 us)
             {(const void *)k_dp_tree<3, 0>, (const void *)k_dp_tree<3, 1>, (const void *)k_dp_tree<4, 2>}};
         const void *fn = variants[minb - 2][layout];
         const size_t key = smem * 16u + (size_t)minb * 3u + (size_t)layout;
@@ -2211,16 +2258,34 @@ public:
             cudaGetLastError();
             cb = coop_blocks.emplace(key, blocks).first;
         }
-        const int grid = cb->second;
-        if (grid <= 0) return 0;
+        const int full = cb->second;
+        if (full <= 0) return 0;
+        const bool bounded = gpuqo_b200_barrier_poll_limit > 0;   // the polled barrier on purpose
+        const int grid = bounded || minb != 2 ? full : tree_grid(plan, n, full);
         CK(cudaMemsetAsync(d_ctl, 0, kCtlClearBytes, stream));   // counters, barrier words, tree size
         uint32_t bwords = words;
         for (int k = 2; k <= n; k++)
-            plan.group[k] = (uint8_t)tree_group(plan.count[k], k, (uint32_t)grid * kBlock, (uint32_t)sm_count);
+            plan.group[k] = (uint8_t)tree_group(plan.count[k], k, (uint32_t)grid * kBlock, (uint32_t)std::min(grid, sm_count));
         unsigned poll_limit = (unsigned)std::max(0, gpuqo_b200_barrier_poll_limit);
         void *args[] = {&a.blob, &bwords, &a.memo, &a.memo_left, &a.sets, &a.sets2,
                         &a.lvl, &a.glob, &a.tree, &a.tree_n, &a.bar, &plan, &poll_limit};
-        cudaError_t e = cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kBlock), args, smem, stream);
+        cudaError_t e;
+        if (grid <= kTreeCluster && !bounded && minb == 2) {
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3(grid);
+            cfg.blockDim = dim3(kBlock);
+            cfg.dynamicSmemBytes = smem;
+            cfg.stream = stream;
+            cudaLaunchAttribute attr;
+            attr.id = cudaLaunchAttributeClusterDimension;
+            attr.val.clusterDim.x = (unsigned)grid;
+            attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+            cfg.attrs = &attr;
+            cfg.numAttrs = 1;
+            e = cudaLaunchKernelExC(&cfg, fn, args);
+        } else {
+            e = cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kBlock), args, smem, stream);
+        }
         if (e != cudaSuccess) {
             cudaGetLastError();
             coop_off = true;   // do not retry on this engine
@@ -3018,11 +3083,14 @@ __global__ void __launch_bounds__(kBlock) kb_level_sets(const BatchQ *__restrict
 __device__ __forceinline__ void tree_cand(const DevHeader &h, uint32_t S, uint32_t v, uint32_t c, uint32_t &L,
                                           uint32_t &R, uint32_t &p, uint32_t &ecm, bool masked) {
     const TreeRows t = tree_rows(h, S);
-    const uint32_t code = v | ((c & 1u) ? kSideHigher : 0u);
-    L = tree_side(t, S, code);
+    const uint2 e = *reinterpret_cast<const uint2 *>(t.row + 2u * v);
+    const uint32_t comp = S & e.x, L0 = (e.y & kTreeLower) ? comp : S ^ comp;
+    uint32_t p0, p1;
+    tree_order(t, S, v, e.x, L0, h.index_order, p0, p1);
+    L = (c & 1u) ? S ^ L0 : L0;
     R = S ^ L;
-    p = tree_index(t.row, t.n, S, code, h.index_order);
-    ecm = masked ? reinterpret_cast<const TreeEdge *>(t.tab + tree_edge_off(t.n))[t.row[2u * v + 1u] & 31u].classes : 0u;
+    p = (c & 1u) ? p1 : p0;
+    ecm = masked ? reinterpret_cast<const TreeEdge *>(t.tab + tree_edge_off(t.n))[e.y & 31u].classes : 0u;
 }
 
 // the sets of one level of every query in groups of G lanes (per-level launches)
@@ -3430,8 +3498,8 @@ __global__ void kb_extract(const BatchQ *__restrict__ qs, int nq, const uint32_t
 // Bound: issue in the wide levels, the chain item -> query -> tables -> memo
 // entries in the narrow ones.  With both orientations of a split taken
 // together and no class pass (see k_dp_tree), device time of 96 queries of 10 to
-// 20 relations (77 M pairs, its wave of cycles included) 2230 -> 1220 us, of
-// 512 queries of 8 to 16 (23.7 M pairs) 1040 -> 650 us.
+// 20 relations (77 M pairs, its wave of cycles included) 2230 -> 1000 us, of
+// 512 queries of 8 to 16 (23.7 M pairs) 1040 -> 600 us.
 __device__ __forceinline__ void batch_tree_enum(const BatchQ *qs, const uint32_t *blobs, const unsigned long long *prev,
                                                 uint32_t c_prev, unsigned long long *out, LevelCounters *lc,
                                                 uint32_t tid, uint32_t nthreads) {

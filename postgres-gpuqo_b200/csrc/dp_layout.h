@@ -158,10 +158,6 @@ struct TreeEdge {
 static_assert(sizeof(TreeEdge) == 32, "TreeEdge layout");
 constexpr uint32_t kTreeLower = 32u;
 
-// the two orientations of a split edge, numbered by its child end
-// (TreeBest::code): bit 5 set = the higher end's side is the outer one
-constexpr uint32_t kSideHigher = 32u;
-
 GQB_HD inline uint32_t tree_edge_off(int) { return 32u; }
 GQB_HD inline uint32_t tree_rows_off(int n) { return 32u + 8u * (uint32_t)n; }
 GQB_HD inline uint32_t tree_row_words(int n) { return 4u * (uint32_t)n; }
