@@ -14,10 +14,11 @@
 // exclusive or of two.  The classes that a cut matches are those on its one or
 // two edges when every class sits on an edge.
 //
-// The splits come in another order than the reference's, whose index decides
-// between equal costs and for a NaN: such sets get their blocks searched in the
-// reference's order (cactus_order) and their splits costed once more, with
-// indices.
+// Between equal costs the reference's order decides.  Plain DPsub's is that of
+// the subsets of S, so of the outer sides as integers.  The block enumeration's
+// is not at hand here: sets with equal lowest costs, and with a NaN cost, get
+// their blocks searched in the reference's order (cactus_order) and their
+// splits costed once more, with indices.
 #pragma once
 
 #include "dp_cactus_table.h"
@@ -120,14 +121,15 @@ struct CactusBest {
 };
 
 template <class M>
-__device__ __forceinline__ void cactus_update(CactusBest<M> &best, M L, float rows, float startup, float total) {
+__device__ __forceinline__ void cactus_update(CactusBest<M> &best, M L, bool dpsub, float rows, float startup,
+                                              float total) {
     if (__builtin_expect(isnan(total), 0)) {
         best.nan = true;
         return;
     }
     const uint32_t ord = ord_float(total);
-    if (ord == best.ord) best.tie = ord;
-    if (ord < best.ord) {
+    if (ord == best.ord && !dpsub) best.tie = ord;
+    if (ord < best.ord || (dpsub && ord == best.ord && L < best.left)) {
         best.ord = ord;
         best.left = L;
         best.rows = rows;
@@ -196,10 +198,10 @@ __device__ __forceinline__ uint64_t cactus_pext(M x, M mask) {
 }
 
 // the reference's index of the candidate with outer side L (after
-// cactus_order, or plain DPsub's)
+// cactus_order), or its place in plain DPsub's order
 template <class M>
 __device__ __noinline__ uint64_t cactus_index(M S, const CactusScratch<M> &sc, M L, bool dpsub) {
-    if (dpsub) return cactus_pext<M>(L, S) - 1ull;
+    if (dpsub) return (uint64_t)L;
     const M R = S ^ L;
     uint32_t b = 0u;
     // the one block that the split cuts
@@ -209,10 +211,11 @@ __device__ __noinline__ uint64_t cactus_index(M S, const CactusScratch<M> &sc, M
 
 // A connected set by one warp: load(L) gives a side's memo entry, general(L,
 // l, r, match, lr, rl) costs both orientations where plain_mirror does not
-// apply, write(rows, startup, total, width, left) stores the winner (one lane).
+// apply, write(rows, startup, total, width word, left) stores the winner (one
+// lane).
 template <class M, class Adj, class Load, class General, class Write>
-__device__ __forceinline__ void cactus_set(M S, const CactusView &v, const Adj *adj, CactusScratch<M> &sc, bool dpsub,
-                                           const PlainParams &pp, Load load, General general, Write write,
+__device__ __forceinline__ void cactus_set(M S, const CactusView &v, const DevHeader &h, const Adj *adj,
+                                           CactusScratch<M> &sc, bool dpsub, const PlainParams &pp, Load load, General general, Write write,
                                            uint32_t &pairs) {
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t W = cactus_pieces<M>(S, v, sc);
@@ -250,8 +253,8 @@ __device__ __forceinline__ void cactus_set(M S, const CactusView &v, const Adj *
                 width = general(L, l, r, match, lr, rl);
             }
             if (!exact) {
-                cactus_update<M>(best, L, lr.rows, lr.startup, lr.total);
-                cactus_update<M>(best, R, rl.rows, rl.startup, rl.total);
+                cactus_update<M>(best, L, dpsub, lr.rows, lr.startup, lr.total);
+                cactus_update<M>(best, R, dpsub, rl.rows, rl.startup, rl.total);
                 continue;
             }
 #pragma unroll 1
@@ -281,6 +284,10 @@ __device__ __forceinline__ void cactus_set(M S, const CactusView &v, const Adj *
         ord = __reduce_min_sync(0xFFFFFFFFu, best.ord);
         const uint32_t win = __ballot_sync(0xFFFFFFFFu, best.ord == ord && ord != 0xFFFFFFFFu);
         nans = __any_sync(0xFFFFFFFFu, best.nan);
+        if (!nans && dpsub) {
+            best_p = (win >> lane) & 1u ? (uint64_t)best.left : ~0ull;
+            break;
+        }
         if (!nans && __popc(win) == 1 && !__any_sync(0xFFFFFFFFu, best.ord == ord && best.tie == ord)) {
             best_p = (win >> lane) & 1u ? 0ull : ~0ull;
             break;
@@ -293,20 +300,24 @@ __device__ __forceinline__ void cactus_set(M S, const CactusView &v, const Adj *
         const uint32_t lo = __reduce_min_sync(0xFFFFFFFFu, (uint32_t)(p >> 32) == hi ? (uint32_t)p : 0xFFFFFFFFu);
         return ((uint64_t)hi << 32) | lo;
     };
-    bool mine = best_p != ~0ull;
-    if (exact) {   // every lane takes part in the reductions
+    bool mine = best_p != ~0ull, kept = false;
+    if (exact || dpsub) {   // every lane takes part in the reductions
         const uint64_t lowest_p = least(best_p);
         mine = mine && best_p == lowest_p;
         if (nans) {
             const uint64_t lowest_first = least(first_p);
-            const bool kept = first_nan && first_p == lowest_first;
+            kept = first_nan && first_p == lowest_first;
             if (__any_sync(0xFFFFFFFFu, kept)) mine = false;
-            if (kept) write(first_rows, first_startup, first_total, width, first_left);
         }
     }
+    auto word = [&](float rows) {
+        return (v.h.flags & kCactusPlain) ? plain_width_word(h, rows, width) : memo_width_word(h, rows, width);
+    };
+    if (kept) write(first_rows, first_startup, first_total, word(first_rows), first_left);
     // the inverse of ord_float (a total is never -0: its startup cost starts from +0)
     if (mine)
-        write(best.rows, best.startup, __uint_as_float((ord & 0x80000000u) ? ord ^ 0x80000000u : ~ord), width, best.left);
+        write(best.rows, best.startup, __uint_as_float((ord & 0x80000000u) ? ord ^ 0x80000000u : ~ord), word(best.rows),
+              best.left);
     if (lane == 0u) pairs += 2u * W;
 }
 

@@ -16,7 +16,10 @@ struct CactusHead {
     uint32_t n_cycles;
     uint32_t n_walk;              // walk entries, m + 1 per block
     uint32_t flags;               // kCactusEdges, kCactusPlain
+    uint32_t n_sets;              // connected sets of the graph (all ones: 2^32 - 1 or more)
+    uint32_t pad[3];
 };
+static_assert(sizeof(CactusHead) == 32, "CactusHead layout");
 constexpr uint32_t kCactusEdges = 1u;   // two-member classes on edges only, at most 64
 constexpr uint32_t kCactusPlain = 2u;   // ... all plain, a class on every edge (plain_mirror applies)
 
@@ -42,7 +45,7 @@ struct CactusView {
 GQB_HD inline CactusView cactus_view(const void *tab, int n_ec) {
     CactusView v;
     v.h = *reinterpret_cast<const CactusHead *>(tab);
-    const uint64_t *p = reinterpret_cast<const uint64_t *>(tab) + 2;
+    const uint64_t *p = reinterpret_cast<const uint64_t *>(tab) + 4;
     const uint32_t ec = (v.h.flags & kCactusEdges) ? (uint32_t)n_ec : 0u;
     v.quals = reinterpret_cast<const PlainQuals *>(p);
     p += 2u * (ec + 1u);
@@ -73,6 +76,12 @@ inline std::vector<uint64_t> build_cactus(const std::vector<uint64_t> &adj, cons
         uint64_t mask;
     };
     std::vector<Block> cycles, bridges;
+    // Connected sets: f[v] of them lie in v's part of the block tree (rooted at
+    // relation 0) and contain v; a block's children are complete when it is
+    // emitted.  A set's topmost piece is one relation (f) or a run of two or
+    // more children of a cycle.
+    double f[64], sets = 0.0;
+    for (int i = 0; i < n; i++) f[i] = 1.0;
     {
         // blocks of the graph (depth-first, a relation stack); recursion
         // unrolled: at most 63 relations
@@ -124,9 +133,32 @@ inline std::vector<uint64_t> build_cactus(const std::vector<uint64_t> &adj, cons
                 if (m == 2) v = 63 - __builtin_clzll(b.mask);
                 else v = __builtin_ctzll(rest);
             }
+            int top = 0;
+            while (b.walk[(size_t)top] != p) top++;
+            std::vector<double> child;
+            for (int i = 1; i < m; i++) child.push_back(f[b.walk[(size_t)((top + i) % m)]]);
+            // runs from either side of the top relation, then the whole block
+            double with = 0.0, left = 1.0, all = 1.0;
+            for (double x : child) all *= x;
+            for (int i = 0; i <= m - 2; i++) {
+                double right = 1.0;
+                for (int j = 0; i + j <= m - 2; j++) {
+                    with += left * right;
+                    right *= child[(size_t)(m - 2 - j)];
+                }
+                left *= child[(size_t)i];
+            }
+            with += all;
+            for (int i = 0; i < m - 1; i++) {
+                double run = child[(size_t)i];
+                sets += run;
+                for (int j = i + 1; j < m - 1; j++) sets += run *= child[(size_t)j];
+            }
+            f[p] *= with;
             (m > 2 ? cycles : bridges).push_back(std::move(b));
         }
         if (t != n) return {};
+        sets += f[0];
     }
     std::vector<Block> blocks = std::move(cycles);
     CactusHead head{};
@@ -140,7 +172,8 @@ inline std::vector<uint64_t> build_cactus(const std::vector<uint64_t> &adj, cons
         else if (!((adj[__builtin_ctzll(rel[i])] & rel[i]))) edges = false;
     }
     head.flags = edges ? kCactusEdges : 0u;
-    std::vector<uint64_t> tab(2u + (edges ? 4u * (uint32_t)n_ec + 2u : 2u) + head.n_blocks + 2u * head.n_walk +
+    head.n_sets = sets < 4294967295.0 ? (uint32_t)sets : 0xFFFFFFFFu;
+    std::vector<uint64_t> tab(4u + (edges ? 4u * (uint32_t)n_ec + 2u : 2u) + head.n_blocks + 2u * head.n_walk +
                                   (head.n_blocks + 1u) / 2u + (head.n_walk + 32u + 7u) / 8u + 1u,
                               0ull);
     tab.resize((tab.size() + 1u) & ~(size_t)1);

@@ -12,11 +12,13 @@
 // parts of its relations, and it is valid when both sides are connected sets,
 // which the enumeration's bitmap answers for every smaller set.
 //
-// A candidate's enumeration index in the reference is needed only where it
+// A candidate's place in the reference's order is needed only where it
 // decides: between equal costs and for NaN costs (the first candidate of a
-// set, if its cost is NaN, is kept).  In block order the first candidate is
-// always valid (a biconnected block without its lowest relation is connected),
-// in plain-DPsub order it is searched for.
+// set, if its cost is NaN, is kept).  In block order it is the enumeration
+// index, and the first candidate is always valid (a biconnected block without
+// its lowest relation is connected); plain DPsub visits the subsets of S in
+// increasing order, so there it is the outer side itself, and the first valid
+// one is searched for.
 #pragma once
 
 #include "dp_cactus.cuh"
@@ -194,16 +196,16 @@ __device__ __forceinline__ uint32_t gen_side(uint32_t S, const GenScratch &ws, u
     return L;
 }
 
-// the reference's index of split c with L the outer side
-__device__ __noinline__ uint32_t gen_index(uint32_t S, const GenScratch &ws, uint32_t c, uint32_t L, uint32_t dpsub) {
-    if (dpsub) return dpsub_index(L, S);
+// the place of split c with L the outer side
+__device__ __forceinline__ uint32_t gen_index(uint32_t S, const GenScratch &ws, uint32_t c, uint32_t L, uint32_t dpsub) {
+    if (dpsub) return L;
     const uint32_t b = gen_block_of(ws, ws.half, c), blk = ws.mask[b];
     return ws.prefix[b] + pext32(L & blk, blk) - 1u;
 }
 
-// the outer side of the candidate with the reference's index p
+// the outer side of the candidate at place p
 __device__ __forceinline__ uint32_t gen_from_index(uint32_t S, const GenScratch &ws, uint32_t p, uint32_t dpsub) {
-    if (dpsub) return pdep32(p + 1u, S);
+    if (dpsub) return p;
     const uint32_t b = gen_block_of(ws, ws.prefix, p), blk = ws.mask[b], bs = ws.sub[b];
     uint32_t L = 0u;
     for (uint32_t x = pdep32(p - ws.prefix[b] + 1u, blk); x; x &= x - 1u) {
@@ -219,7 +221,7 @@ __device__ __forceinline__ bool seen_bit(const uint32_t *seen, uint32_t T) { ret
 struct GenBest {
     uint32_t ord, c, left;
     float rows, startup;
-    uint32_t nan_p;               // lowest index of a NaN candidate
+    uint32_t nan_p;               // lowest place of a NaN candidate
     uint32_t pairs;
 
     __device__ __forceinline__ void init() {
@@ -302,7 +304,7 @@ __device__ __forceinline__ void gen_range(const DevInfoView &d, GenScratch &ws, 
     }
 }
 
-// index of the first valid candidate of S
+// place of the first valid candidate of S
 __device__ __noinline__ uint32_t gen_first(uint32_t S, uint32_t dpsub, const uint32_t *seen) {
     if (!dpsub) return 0u;
     const uint32_t lane = threadIdx.x & 31u, total = (1u << popc(S)) - 2u;
@@ -310,12 +312,12 @@ __device__ __noinline__ uint32_t gen_first(uint32_t S, uint32_t dpsub, const uin
         const uint32_t p = base + lane;
         const uint32_t L = p < total ? pdep32(p + 1u, S) : 0u;
         const uint32_t m = __ballot_sync(0xFFFFFFFFu, p < total && seen_bit(seen, L) && seen_bit(seen, S ^ L));
-        if (m) return base + (uint32_t)lowest_idx(m);
+        if (m) return __shfl_sync(0xFFFFFFFFu, L, lowest_idx(m));
     }
     return 0xFFFFFFFFu;
 }
 
-// the memo entry of S from the candidate of index p (one lane writes)
+// the memo entry of S from the candidate at place p (one lane writes)
 __device__ __noinline__ void gen_write_index(const DevInfoView d, const GenScratch &ws, uint32_t S, uint32_t p,
                                              float4 *memo, uint32_t *memo_left) {
     if ((threadIdx.x & 31u) == 0u) {
@@ -330,7 +332,7 @@ __device__ __noinline__ void gen_write_index(const DevInfoView d, const GenScrat
 }
 
 // lanes with the warp's lowest cost, the tie broken: the winner's lane (its
-// index in p when ties were compared or want_p is set)
+// place in p when ties were compared or want_p is set)
 __device__ __forceinline__ bool gen_winner(const DevHeader &h, const GenScratch &ws, uint32_t S, const GenBest &best,
                                            bool want_p, uint32_t &ord, uint32_t &p) {
     ord = __reduce_min_sync(0xFFFFFFFFu, best.ord);
@@ -376,7 +378,7 @@ __device__ __forceinline__ void gen_cactus_set(const DevInfoView &d, const Cactu
                                                uint32_t &pairs) {
     const DevHeader &h = *d.h;
     cactus_set<uint32_t>(
-        S, cv, h.adj, ws.cactus, h.index_order != 0u, pp, [&](uint32_t L) { return __ldcg(memo + L); },
+        S, cv, h, h.adj, ws.cactus, h.index_order != 0u, pp, [&](uint32_t L) { return __ldcg(memo + L); },
         [&](uint32_t L, const float4 lv, const float4 rv, uint64_t match, JoinCost &lr, JoinCost &rl) {
             const RelVal l = unpack_rel(lv, h.hz_packed), r = unpack_rel(rv, h.hz_packed);
             RelVal o0, o1;
@@ -392,8 +394,8 @@ __device__ __forceinline__ void gen_cactus_set(const DevInfoView &d, const Cactu
             rl.total = o1.total;
             return o0.width;
         },
-        [&](float rows, float startup, float total, int width, uint32_t left) {
-            memo[S] = make_float4(rows, startup, total, __uint_as_float(memo_width_word(h, rows, width)));
+        [&](float rows, float startup, float total, uint32_t word, uint32_t left) {
+            memo[S] = make_float4(rows, startup, total, __uint_as_float(word));
             memo_left[S] = left;
         },
         pairs);

@@ -1912,6 +1912,22 @@ constexpr size_t kCtlClearBytes = offsetof(EngineCtl, pad);   // lvl .. tree_n
 constexpr int kTreeCluster = 8;
 constexpr int kTreeClusterLevel = 16;
 
+// one cluster of `blocks` blocks
+static cudaError_t launch_cluster(const void *fn, int blocks, size_t smem, void **args, cudaStream_t stream) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(kBlock);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = (unsigned)blocks;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelExC(&cfg, fn, args);
+}
+
 class Engine {
 public:
     int device = -1;
@@ -2270,22 +2286,8 @@ public:
         void *args[] = {&a.blob, &bwords, &a.memo, &a.memo_left, &a.sets, &a.sets2,
                         &a.lvl, &a.glob, &a.tree, &a.tree_n, &a.bar, &plan, &poll_limit};
         cudaError_t e;
-        if (grid <= kTreeCluster && !bounded && minb == 2) {
-            cudaLaunchConfig_t cfg = {};
-            cfg.gridDim = dim3(grid);
-            cfg.blockDim = dim3(kBlock);
-            cfg.dynamicSmemBytes = smem;
-            cfg.stream = stream;
-            cudaLaunchAttribute attr;
-            attr.id = cudaLaunchAttributeClusterDimension;
-            attr.val.clusterDim.x = (unsigned)grid;
-            attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-            cfg.attrs = &attr;
-            cfg.numAttrs = 1;
-            e = cudaLaunchKernelExC(&cfg, fn, args);
-        } else {
-            e = cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kBlock), args, smem, stream);
-        }
+        if (grid <= kTreeCluster && !bounded && minb == 2) e = launch_cluster(fn, grid, smem, args, stream);
+        else e = cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kBlock), args, smem, stream);
         if (e != cudaSuccess) {
             cudaGetLastError();
             coop_off = true;   // do not retry on this engine
@@ -3208,7 +3210,10 @@ __global__ void __launch_bounds__(kBlock) kb_eval(const BatchQ *__restrict__ qs,
 // its planner info in shared memory), in ONE cooperative, persistent launch.
 // Per level k: one warp per connected k-set evaluates it (dp_general.cuh)
 // while the far end of the grid enumerates level k + 1, also one warp per set
-// and one lane per neighbour.  Sets with more splits than `limit` go to the
+// and one lane per neighbour, deduplicated in a bitmap of all subsets, or for
+// a cactus graph, whose connected sets are counted beforehand and whose sides
+// need no test, in a table of 2^table_log2 words when that is smaller (a
+// 30-relation bitmap takes 30 us to clear).  Sets with more splits than `limit` go to the
 // overflow list; after the barrier their splits are dealt out evenly, and the
 // warp that finishes a set's last unit writes its entry.
 // Bound: latency on the graphs planned exactly at this size (few sets per
@@ -3223,8 +3228,8 @@ __device__ __forceinline__ uint32_t gen_units(const BatchOvf &ovf, uint32_t W) {
 // connected (k+1)-sets from the c_prev k-sets in prev; `warp` of nwarps
 __device__ __forceinline__ void gen_extend(const BatchQ *qs, const uint32_t *blobs, const uint32_t *own_adj,
                                            const unsigned long long *prev, uint32_t c_prev, uint32_t *seen,
-                                           unsigned long long *out, LevelCounters *lc, unsigned long long *st,
-                                           uint32_t warp, uint32_t nwarps) {
+                                           uint32_t table_log2, unsigned long long *out, LevelCounters *lc,
+                                           unsigned long long *st, uint32_t warp, uint32_t nwarps) {
     const uint32_t lane = threadIdx.x & 31u;
     uint32_t cnt = 0;
     for (uint32_t i = warp; i < c_prev; i += nwarps) {
@@ -3243,7 +3248,15 @@ __device__ __forceinline__ void gen_extend(const BatchQ *qs, const uint32_t *blo
         }
         const uint32_t bit = 1u << lane, T = S | bit;
         bool ok = lane < n && !(S & bit) && (adj[lane] & S) != 0u;
-        if (ok) {
+        if (ok && table_log2) {
+            // at most half full: an empty or the set's own slot is found
+            uint32_t at = (T * 0x9E3779B1u) >> (32u - table_log2);
+            for (uint32_t probe = 0; probe < (1u << table_log2); probe++, at = (at + 1u) & ((1u << table_log2) - 1u)) {
+                const uint32_t old = atomicCAS(seen + at, 0u, T);
+                ok = old == 0u;
+                if (ok || old == T) break;
+            }
+        } else if (ok) {
             const uint32_t bm = 1u << (T & 31u);
             ok = !(atomicOr(&seen[seen_off + (T >> 5)], bm) & bm);
         }
@@ -3322,7 +3335,8 @@ __global__ void __launch_bounds__(kBlock, 2) kb_gen(const BatchQ *__restrict__ q
                                                     unsigned long long *__restrict__ listB,
                                                     LevelCounters *__restrict__ lvl, GlobalCounters *__restrict__ glob,
                                                     TreeNode *__restrict__ tree, int *__restrict__ tree_n,
-                                                    unsigned *__restrict__ bar, BatchOvf ovf, unsigned poll_limit) {
+                                                    unsigned *__restrict__ bar, BatchOvf ovf, uint32_t table_log2,
+                                                    unsigned poll_limit) {
     extern __shared__ __align__(16) unsigned char gsm[];
     __shared__ unsigned long long stage[kWarpsPerBlock][64];
     const unsigned max_polls = barrier_polls(poll_limit);
@@ -3338,6 +3352,15 @@ __global__ void __launch_bounds__(kBlock, 2) kb_gen(const BatchQ *__restrict__ q
     const uint32_t nwarps = gridDim.x * kWarpsPerBlock;
     unsigned long long pairs = 0;
     unsigned epoch = 0;   // grid barriers passed (thread 0)
+    // small queries run as one cluster, synchronised in hardware
+    const bool cluster = ONE && cluster_blocks() == gridDim.x;
+    auto barrier = [&]() -> bool {
+        if (ONE && cluster) {
+            cluster_barrier();
+            return true;
+        }
+        return grid_barrier<ONE>(bar, epoch, max_polls);
+    };
 
     // phase 0: base relations (gpuqo_cpu_sequential.cu:80-92) and level-2 sets
     // (each edge once, from its lower end), entered into the bitmap
@@ -3350,7 +3373,7 @@ __global__ void __launch_bounds__(kBlock, 2) kb_gen(const BatchQ *__restrict__ q
             if (lane < (int)Q.n) {
                 memo[Q.memo_off + (1ull << lane)] = base_entry(*h, lane);
                 memo_left[Q.memo_off + (1ull << lane)] = 0u;
-                atomicOr(seen + Q.seen_off + ((1u << lane) >> 5), 1u << ((1u << lane) & 31u));
+                if (!table_log2) atomicOr(seen + Q.seen_off + ((1u << lane) >> 5), 1u << ((1u << lane) & 31u));
                 nb = h->adj[lane] & ~((2u << lane) - 1u);
             }
             const int maxdeg = (int)__reduce_max_sync(kFull, (uint32_t)__popc(nb));
@@ -3358,13 +3381,13 @@ __global__ void __launch_bounds__(kBlock, 2) kb_gen(const BatchQ *__restrict__ q
                 const bool ok = nb != 0u;
                 const uint32_t T = (1u << lane) | (nb & (0u - nb));
                 nb &= nb - 1u;
-                if (ok) atomicOr(seen + Q.seen_off + (T >> 5), 1u << (T & 31u));
+                if (ok && !table_log2) atomicOr(seen + Q.seen_off + (T >> 5), 1u << (T & 31u));
                 stage_emit64(st, cnt, ok, ((unsigned long long)q << 32) | T, listA, lvl + 2);
             }
         }
         stage_flush64(st, cnt, listA, lvl + 2);
     }
-    if (!grid_barrier<ONE>(bar, epoch, max_polls)) return;
+    if (!barrier()) return;
 
     for (int k = 2; k <= maxn; k++) {
         unsigned long long *cur = (k & 1) ? listB : listA;
@@ -3374,7 +3397,7 @@ __global__ void __launch_bounds__(kBlock, 2) kb_gen(const BatchQ *__restrict__ q
         // enumeration from the far end of the grid, evaluation from the start
         if (k < maxn)
             gen_extend(qs, ONE ? own : blobs, ONE ? reinterpret_cast<const DevHeader *>(own)->adj : nullptr, cur, count,
-                       seen, nxt, lk + 1, st, nwarps - 1u - gwarp, nwarps);
+                       seen, table_log2, nxt, lk + 1, st, nwarps - 1u - gwarp, nwarps);
         // Splits a warp takes alone: 4 rounds of its lanes per set it holds.
         // The overflow phase costs about two barriers and another block search
         // per share.
@@ -3413,11 +3436,11 @@ __global__ void __launch_bounds__(kBlock, 2) kb_gen(const BatchQ *__restrict__ q
             }
             gen_set(d, ws, S, memo + Q.memo_off, memo_left + Q.memo_off, seen + Q.seen_off, found);
         }
-        if (!grid_barrier<ONE>(bar, epoch, max_polls)) return;
+        if (!barrier()) return;
         // the counter is final after the barrier: every block takes the same branch
         if (ovf.cap != 0u && (uint32_t)(__ldcg(&lk->ovf_packed) >> 40) != 0u) {
             gen_overflow<ONE>(qs, blobs, own, lk, memo, memo_left, seen, ovf, ws, gwarp, nwarps, found);
-            if (!grid_barrier<ONE>(bar, epoch, max_polls)) return;
+            if (!barrier()) return;
         }
         pairs += found;
     }
@@ -3801,14 +3824,27 @@ struct BatchEngine {
     // the wave as one cooperative launch: kb_dp<layout> when every query is
     // tree-shaped (layout: the least of the queries' tree_layout), else kb_gen
     // (layout < 0; kb_gen<true> for one query); false when it could not start
-    bool enqueue_persistent(int nq, int maxn, uint32_t words, uint64_t seen_words, int layout) {
+    bool enqueue_persistent(int nq, int maxn, uint32_t words, uint64_t seen_words, int layout, uint32_t cactus_sets) {
         const bool tree_only = layout >= 0;
         const int one = (!tree_only && nq == 1) ? one_grid(words) : 0;
-        const int grid = tree_only ? coop_grid_tree[layout] : (one > 0 ? one : coop_grid);
+        int grid = tree_only ? coop_grid_tree[layout] : (one > 0 ? one : coop_grid);
+        // one cactus query: a table of twice its connected sets, and a cluster
+        // when the widest levels (taken as twice the average) leave its warps
+        // idle, half for the sets and half for their extensions
+        uint32_t table_log2 = 0;
+        bool cluster = false;
+        if (one > 0 && cactus_sets != 0u && cactus_sets < (1u << 30)) {
+            uint32_t l = 6;
+            while ((1ull << l) < 2ull * cactus_sets) l++;
+            if ((1ull << l) <= seen_words / 4) table_log2 = l;
+            const double warps = 4.0 * (double)cactus_sets / (double)maxn;
+            cluster = gpuqo_b200_barrier_poll_limit <= 0 && warps <= 2.0 * kTreeCluster * kWarpsPerBlock;
+            if (cluster) grid = std::min(grid, kTreeCluster);
+        }
         if (grid <= 0 || gpuqo_b200_persistent == 0 || barrier_timed_out) return false;
         cudaMemsetAsync(lvl, 0, 33 * sizeof(LevelCounters), stream);
         cudaMemsetAsync(glob, 0, sizeof(GlobalCounters), stream);
-        if (!tree_only) cudaMemsetAsync(seen, 0, seen_words * 4, stream);
+        if (!tree_only) cudaMemsetAsync(seen, 0, table_log2 ? (size_t)4 << table_log2 : seen_words * 4, stream);
         cudaMemsetAsync(bar, 0, 4 * sizeof(unsigned), stream);
         unsigned poll_limit = (unsigned)std::max(0, gpuqo_b200_barrier_poll_limit);
         cudaError_t e;
@@ -3820,10 +3856,11 @@ struct BatchEngine {
             e = cudaLaunchCooperativeKernel(variants[layout], dim3(grid), dim3(kBlock), args, 0, stream);
         } else {
             void *args[] = {&qs, &nq, &maxn, &blobs, &words, &memo, &memo_left, &seen, &listA, &listB,
-                            &lvl, &glob, &tree, &tree_n, &bar, &ovf, &poll_limit};
-            e = cudaLaunchCooperativeKernel(one > 0 ? (const void *)kb_gen<true> : (const void *)kb_gen<false>,
-                                            dim3(grid), dim3(kBlock), args,
-                                            kGenSmem + (one > 0 ? (size_t)words * 4u : 0u), stream);
+                            &lvl, &glob, &tree, &tree_n, &bar, &ovf, &table_log2, &poll_limit};
+            const void *fn = one > 0 ? (const void *)kb_gen<true> : (const void *)kb_gen<false>;
+            const size_t smem = kGenSmem + (one > 0 ? (size_t)words * 4u : 0u);
+            e = cluster ? launch_cluster(fn, grid, smem, args, stream)
+                        : cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kBlock), args, smem, stream);
         }
         if (e != cudaSuccess) {
             cudaGetLastError();
@@ -3900,6 +3937,7 @@ struct BatchEngine {
         uint64_t slots = 0, words = 0, seen_words = 0, items = 0, base = 0, ovf_need = 0;
         int maxn = 0;
         int layout = kTreePlain;   // of a wave of trees; -1: a graph with cycles among the queries
+        uint32_t cactus_sets = 0;  // connected sets of the last query if it is a cactus graph with cycles
         for (int q = 0; q < nq; q++) {
             const DevHeader *h = reinterpret_cast<const DevHeader *>(wb[q]->data());
             const int n = h->n;
@@ -3917,6 +3955,8 @@ struct BatchEngine {
             maxn = std::max(maxn, n);
             if (batch_needs_ovf(*wb[q])) ovf_need += max_level_sets(n);
             layout = h->tree_mode != 0u ? std::min(layout, tree_layout(*h)) : -1;
+            if (h->tree_mode == 0u && h->tree_tab != 0u)
+                cactus_sets = reinterpret_cast<const CactusHead *>(wb[q]->data() + h->tree_tab)->n_sets;
         }
         items = std::max(items, base);
         ovf_need = std::min(ovf_need, kBatchOvfCap);
@@ -3993,7 +4033,7 @@ struct BatchEngine {
         };
         uint32_t kernels = 1;
         CK(cudaEventRecord(ev0, stream));
-        bool persistent = enqueue_persistent(nq, maxn, (uint32_t)words, seen_words, layout);
+        bool persistent = enqueue_persistent(nq, maxn, (uint32_t)words, seen_words, layout, cactus_sets);
         CK(cudaGetLastError());
         if (persistent) CK(cudaMemcpyAsync(h_bar, bar, 4 * sizeof(unsigned), cudaMemcpyDeviceToHost, stream));
         if (!persistent) kernels = enqueue_levels(nq, maxn, seen_words);

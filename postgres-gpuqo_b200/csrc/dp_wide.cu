@@ -1086,12 +1086,12 @@ __global__ void __launch_bounds__(kWideBlock, 2) k_wide_cactus(const unsigned ch
                 const uint64_t S = __ldcg(sets + first + i);
                 const uint32_t slot = first + i;
                 cactus_set<uint64_t>(
-                    S, cv, w.adj, sc, index_order != 0, pp, [&](uint64_t L) { return __ldcg(memo + wide_lookup<true>(t, L, &ctl->err)); },
+                    S, cv, w.h, w.adj, sc, index_order != 0, pp, [&](uint64_t L) { return __ldcg(memo + wide_lookup<true>(t, L, &ctl->err)); },
                     [&](uint64_t L, const float4 l, const float4 r, uint64_t match, JoinCost &lr, JoinCost &rl) {
                         return wide_join2(w, L, l, S ^ L, r, (cv.h.flags & kCactusEdges) != 0u, match, lr, rl);
                     },
-                    [&](float rows, float startup, float cost, int width, uint64_t left) {
-                        memo[slot] = make_float4(rows, startup, cost, __uint_as_float(memo_width_word(w.h, rows, width)));
+                    [&](float rows, float startup, float cost, uint32_t word, uint64_t left) {
+                        memo[slot] = make_float4(rows, startup, cost, __uint_as_float(word));
                         memo_left[slot] = left;
                     },
                     pairs);
