@@ -22,10 +22,11 @@ __device__ __forceinline__ unsigned long long global_ns() {
     return t;
 }
 
-// bar[0] = arrivals, bar[2] = error flag (both zero at launch).  The arrival
-// counter only grows: a block's e-th barrier of the launch completes when it
-// reaches e * gridDim.x, so nobody resets it and the last block to arrive has
-// nothing more to do.  Thread 0 arrives with a gpu-scope release reduction
+// bar[0] = arrivals (base at launch), bar[2] = error flag (zero at launch).
+// The arrival counter only grows: a block's e-th barrier of the launch
+// completes when it reaches base + e * gridDim.x, so nobody resets it, the last
+// block to arrive has nothing more to do, and the next launch may go on from
+// where it stands.  Thread 0 arrives with a gpu-scope release reduction
 // (ordering every write its block made before the __syncthreads) and polls
 // with gpu-scope acquire loads (ACQUIRE_POLL), or with relaxed loads and one
 // fence once the count is reached: an acquire load also drops the SM's L1
@@ -38,12 +39,12 @@ __device__ __forceinline__ unsigned long long global_ns() {
 // epoch: the caller's count of barriers passed (thread 0); max_polls: polls
 // before the wait gives up (barrier_polls).
 template <bool ACQUIRE_POLL>
-__device__ __forceinline__ bool grid_barrier(unsigned *bar, unsigned &epoch, unsigned max_polls) {
+__device__ __forceinline__ bool grid_barrier(unsigned *bar, unsigned &epoch, unsigned max_polls, unsigned base = 0u) {
     __shared__ unsigned s_ok;
     __syncthreads();
     if (threadIdx.x == 0) {
         epoch++;
-        const unsigned target = epoch * gridDim.x;
+        const unsigned target = base + epoch * gridDim.x;
         volatile unsigned *verr = bar + 2;
         asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
         const unsigned long long t0 = global_ns();

@@ -1177,6 +1177,9 @@ struct TreePlan {
 // needs, one cluster where that does: device time of star-22 (44.0 M pairs)
 // 751 -> 387 us, snowflake-25 (3.2 M and 4.8 M pairs) 265 / 290 -> 139 us, key
 // chain-30 203 -> 90 us, star-12 77 -> 47 us, star-6 38 -> 20 us.
+// tree and tree_n are the host's (pinned): tree_n stays 0 when a barrier gives
+// up.  blob may be the host's too: a few blocks read it faster than a copy
+// ahead of the launch takes.
 // MINB: blocks per SM the register budget is set for (2, 3 or 4: 128, 80 or 64
 // registers, no spill but 4 bytes with 4 blocks), chosen per query from its
 // connected sets per level, the total over the relation count
@@ -1187,12 +1190,14 @@ __global__ void __launch_bounds__(kBlock, MINB) k_dp_tree(const uint32_t *__rest
                                                        float4 *__restrict__ memo,
                                                        uint32_t *__restrict__ memo_left, uint32_t *__restrict__ setsA,
                                                        uint32_t *__restrict__ setsB, LevelCounters *__restrict__ lvl,
-                                                       GlobalCounters *__restrict__ glob, TreeNode *__restrict__ tree,
-                                                       int *__restrict__ tree_n, unsigned *__restrict__ bar,
+                                                       TreeNode *__restrict__ tree, int *__restrict__ tree_n,
+                                                       unsigned *__restrict__ bar, unsigned bar_base,
                                                        const __grid_constant__ TreePlan plan, unsigned poll_limit) {
     extern __shared__ __align__(16) uint32_t sm[];
     const unsigned max_polls = barrier_polls(poll_limit);
-    load_blob_to_smem(blob, blob_words, sm);
+    for (uint32_t i = threadIdx.x; i < blob_words / 4u; i += blockDim.x)
+        reinterpret_cast<uint4 *>(sm)[i] = reinterpret_cast<const uint4 *>(blob)[i];
+    __syncthreads();
     const DevInfoView d = make_view(sm);
     const int n = d.h->n;
     const uint32_t *adj = d.h->adj;
@@ -1209,7 +1214,7 @@ __global__ void __launch_bounds__(kBlock, MINB) k_dp_tree(const uint32_t *__rest
             else cluster_barrier();
             return true;
         }
-        return grid_barrier<true>(bar, epoch, max_polls);
+        return grid_barrier<true>(bar, epoch, max_polls, bar_base);
     };
 
     // phase 0: base relations (gpuqo_cpu_sequential.cu:80-92) and level-2 sets
@@ -1232,11 +1237,8 @@ __global__ void __launch_bounds__(kBlock, MINB) k_dp_tree(const uint32_t *__rest
         __shared__ uint32_t plan_sets[64];
         const uint32_t full = (n == 32) ? 0xFFFFFFFFu : ((1u << n) - 1u);
         extract_plan(memo, memo_left, full, d.h->hz_packed ? kWidthMask : 0xFFFFFFFFu, plan_sets, tree, tree_n);
-        if (threadIdx.x == 0) {
-            unsigned long long pairs = 0;   // every split edge, both orientations
-            for (int k = 2; k <= n; k++) pairs += (unsigned long long)plan.count[k] * 2ull * (unsigned long long)(k - 1);
-            glob->evaluated_pairs = pairs;
-        }
+        // the counters as the next launch expects them (nobody adds any more)
+        for (int k = 2 + (int)threadIdx.x; k <= n; k += 32) lvl[k].n_sets = 0u;
     }
 }
 
@@ -1949,7 +1951,12 @@ public:
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     std::vector<cudaEvent_t> kev;      // per-level eval events (profile mode)
     int n_kernels = 0;                 // kernels per DP run
-    unsigned *h_bar = nullptr;         // pinned copy of the barrier words
+    // k_dp_tree leaves its counters at zero and the barrier's arrivals where
+    // the next launch goes on: whether they are so, and the arrivals
+    bool ctl_clean = false;
+    unsigned bar_base = 0, bar_after = 0;
+    double plan_sets = 0.0;            // connected sets and pairs of the last persistent run
+    uint64_t plan_pairs = 0;
     std::map<size_t, int> coop_blocks; // (dynamic shared bytes, variant) -> co-resident blocks of k_dp_tree (0: none)
     int force_minb = 0;                // autotuner: run this k_dp_tree variant (2, 3 or 4); 0 = by the tuning record
     bool coop_off = false;             // cooperative launch refused on this device
@@ -1975,7 +1982,6 @@ public:
         a.tree = d_ctl->tree;
         h_lvl = h_ctl->lvl;
         h_glob = &h_ctl->glob;
-        h_bar = h_ctl->bar;
         h_tree_n = &h_ctl->tree_n;
         h_tree = h_ctl->tree;
         CK(cudaMalloc(&a.binom, 33 * 33 * sizeof(uint32_t)));
@@ -2240,9 +2246,9 @@ public:
 
     // The whole tree-mode MPDP as one cooperative launch (k_dp_tree).  Returns
     // 0 and sets launched when the kernel was started.
-    int launch_persistent(int n, uint32_t words, bool &launched, std::string &err) {
+    int launch_persistent(int n, uint32_t words, bool on_device, bool &launched, std::string &err) {
         launched = false;
-        const size_t smem = (size_t)((words + 3u) & ~3u) * 4u;
+        const size_t smem = (size_t)((words + 511u) & ~511u) * 4u;   // few sizes: the occupancy is looked up per size
         if (coop_off) return 0;
         const DevHeader *h = reinterpret_cast<const DevHeader *>(h_blob);
         TreePlan plan;
@@ -2278,15 +2284,29 @@ public:
         if (full <= 0) return 0;
         const bool bounded = gpuqo_b200_barrier_poll_limit > 0;   // the polled barrier on purpose
         const int grid = bounded || minb != 2 ? full : tree_grid(plan, n, full);
-        CK(cudaMemsetAsync(d_ctl, 0, kCtlClearBytes, stream));   // counters, barrier words, tree size
+        const bool one_cluster = grid <= kTreeCluster && !bounded && minb == 2;
+        if (!ctl_clean || bar_base > (1u << 30)) {
+            CK(cudaMemsetAsync(d_ctl, 0, kCtlClearBytes, stream));   // counters, barrier words
+            bar_base = 0u;
+        }
+        ctl_clean = false;   // until this launch is known to have finished
+        if (!one_cluster && !on_device)
+            CK(cudaMemcpyAsync(a.blob, h_blob, (size_t)words * 4u, cudaMemcpyHostToDevice, stream));
+        CK(cudaEventRecord(ev0, stream));
+        const uint32_t *blob_src = one_cluster && !on_device ? h_blob : a.blob;
         uint32_t bwords = words;
+        plan_sets = sets;
+        plan_pairs = 0;
+        for (int k = 2; k <= n; k++) plan_pairs += (uint64_t)plan.count[k] * 2u * (uint64_t)(k - 1);
+        bar_after = one_cluster ? bar_base : bar_base + (unsigned)n * (unsigned)grid;   // a barrier per level and the first
+        *h_tree_n = 0;
         for (int k = 2; k <= n; k++)
             plan.group[k] = (uint8_t)tree_group(plan.count[k], k, (uint32_t)grid * kBlock, (uint32_t)std::min(grid, sm_count));
         unsigned poll_limit = (unsigned)std::max(0, gpuqo_b200_barrier_poll_limit);
-        void *args[] = {&a.blob, &bwords, &a.memo, &a.memo_left, &a.sets, &a.sets2,
-                        &a.lvl, &a.glob, &a.tree, &a.tree_n, &a.bar, &plan, &poll_limit};
+        void *args[] = {&blob_src, &bwords, &a.memo, &a.memo_left, &a.sets, &a.sets2, &a.lvl,
+                        &h_tree, &h_tree_n, &a.bar, &bar_base, &plan, &poll_limit};
         cudaError_t e;
-        if (grid <= kTreeCluster && !bounded && minb == 2) e = launch_cluster(fn, grid, smem, args, stream);
+        if (one_cluster) e = launch_cluster(fn, grid, smem, args, stream);
         else e = cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kBlock), args, smem, stream);
         if (e != cudaSuccess) {
             cudaGetLastError();
@@ -2298,17 +2318,20 @@ public:
         return 0;
     }
 
-    // brings the control words back (one copy) and reports whether the last
-    // persistent run's grid barrier timed out; a timeout latches the engine
-    // onto the per-level launches (gpuqo_b200_reset_persistent clears it), so
-    // later calls do not wait for another timeout first
+    // waits for the last persistent run and reports whether its grid barrier
+    // timed out (no plan arrived); a timeout latches the engine onto the
+    // per-level launches (gpuqo_b200_reset_persistent clears it), so later calls
+    // do not wait for another timeout first
     int barrier_failed(bool &failed, EngineStats &st, std::string &err) {
-        if (int rc = download(err)) return rc;
         CK(cudaStreamSynchronize(stream));
-        failed = h_bar[2] != 0u;
+        CK(cudaGetLastError());
+        failed = *const_cast<volatile int *>(h_tree_n) == 0;
         if (failed) {
             barrier_timed_out = true;
             st.barrier_timeouts++;
+        } else {
+            ctl_clean = true;
+            bar_base = bar_after;
         }
         return 0;
     }
@@ -2378,6 +2401,7 @@ public:
     }
 
     int launch(cudaGraphExec_t exec, std::string &err) {
+        ctl_clean = false;
         CK(cudaGraphLaunch(exec, stream));
         return 0;
     }
@@ -2396,11 +2420,12 @@ public:
 
     // Copies the plan and counters back and fills nodes / stats.
     int finish(int n, bool profile, std::vector<TreeNode> &nodes, EngineStats &st, std::string &err,
-               bool downloaded = false) {
-        if (!downloaded)
+               bool persistent = false) {
+        if (!persistent) {
             if (int rc = download(err)) return rc;
-        CK(cudaStreamSynchronize(stream));
-        CK(cudaGetLastError());
+            CK(cudaStreamSynchronize(stream));
+            CK(cudaGetLastError());
+        }
         if (profile)
             if (int rc = read_eval_events(n, st, err)) return rc;
         int nn = *h_tree_n;
@@ -2411,13 +2436,13 @@ public:
         nodes.assign(h_tree, h_tree + nn);
         uint64_t csgs = 0, filt = 0;
         for (int k = 2; k <= n; k++) {
-            csgs += h_lvl[k].n_sets;
+            if (!persistent) csgs += h_lvl[k].n_sets;
             filt += binom64(n, k);
-            st.fallback_sets += h_lvl[k].n_fb;
+            if (!persistent) st.fallback_sets += h_lvl[k].n_fb;
         }
-        st.connected_sets += csgs;
+        st.connected_sets += persistent ? (uint64_t)plan_sets - (uint64_t)n : csgs;
         st.filtered_subsets += filt;
-        st.evaluated_pairs += h_glob->evaluated_pairs;
+        st.evaluated_pairs += persistent ? plan_pairs : h_glob->evaluated_pairs;
         st.memo_bytes = (1ull << n) * (sizeof(float4) + 4);
         st.kernel_launches += (uint32_t)n_kernels;
         return 0;
@@ -2429,14 +2454,15 @@ public:
                h->tree_mode != 0u;
     }
 
-    // stage the blob without building a graph (persistent path)
-    int stage(const std::vector<uint32_t> &blob, int n, uint32_t &words, std::string &err) {
+    // stage the blob without building a graph (persistent path); upload: on
+    // the device too (launch_persistent copies it otherwise, where it has to)
+    int stage(const std::vector<uint32_t> &blob, int n, bool upload, uint32_t &words, std::string &err) {
         if (int rc = init(err)) return rc;
-        words = ((uint32_t)blob.size() + 511u) & ~511u;
-        if (int rc = ensure(n, words, err)) return rc;
-        std::memset(h_blob, 0, words * 4);
+        words = ((uint32_t)blob.size() + 3u) & ~3u;
+        if (int rc = ensure(n, (words + 511u) & ~511u, err)) return rc;
         std::memcpy(h_blob, blob.data(), blob.size() * 4);
-        CK(cudaMemcpyAsync(a.blob, h_blob, words * 4, cudaMemcpyHostToDevice, stream));
+        for (uint32_t i = (uint32_t)blob.size(); i < words; i++) h_blob[i] = 0u;
+        if (upload) CK(cudaMemcpyAsync(a.blob, h_blob, words * 4, cudaMemcpyHostToDevice, stream));
         return 0;
     }
 
@@ -2444,10 +2470,9 @@ public:
             std::vector<TreeNode> &nodes, EngineStats &st, std::string &err) {
         if (persistent_ok(blob, mode)) {
             uint32_t pw;
-            if (int rc = stage(blob, n, pw, err)) return rc;
-            CK(cudaEventRecord(ev0, stream));
+            if (int rc = stage(blob, n, false, pw, err)) return rc;
             bool launched = false;
-            if (int rc = launch_persistent(n, pw, launched, err)) return rc;
+            if (int rc = launch_persistent(n, pw, false, launched, err)) return rc;
             CK(cudaEventRecord(ev1, stream));
             bool failed = true;
             if (launched) {
@@ -2487,12 +2512,12 @@ public:
         const size_t flush_floats = (256u << 20) / sizeof(float);
         if (persistent_ok(blob, mode)) {
             uint32_t pw;
-            if (int rc = stage(blob, n, pw, err)) return rc;
+            if (int rc = stage(blob, n, true, pw, err)) return rc;
             if (flush_l2 && !flush) CK(cudaMalloc(&flush, flush_floats * sizeof(float)));
             bool usable = true;   // every launch so far started and passed its barriers
             for (int i = 0; i < warmup && usable; i++) {
                 bool launched = false, failed = false;
-                if (int rc = launch_persistent(n, pw, launched, err)) return rc;
+                if (int rc = launch_persistent(n, pw, true, launched, err)) return rc;
                 if (launched)
                     if (int rc = barrier_failed(failed, st, err)) return rc;
                 usable = launched && !failed;
@@ -2501,8 +2526,7 @@ public:
             for (int i = 0; usable && i < iters; i++) {
                 if (flush_l2) CK(cudaMemsetAsync(flush, i & 0xFF, flush_floats * sizeof(float), stream));
                 bool launched = false, failed = false;
-                CK(cudaEventRecord(ev0, stream));
-                if (int rc = launch_persistent(n, pw, launched, err)) return rc;
+                if (int rc = launch_persistent(n, pw, true, launched, err)) return rc;
                 CK(cudaEventRecord(ev1, stream));
                 CK(cudaEventSynchronize(ev1));
                 float ms = 0.f;
@@ -2526,6 +2550,7 @@ public:
         cudaGraphExec_t exec;
         if (int rc = prepare(blob, n, mode, ccc, false, words, exec, err)) return rc;
         if (flush_l2 && !flush) CK(cudaMalloc(&flush, flush_floats * sizeof(float)));
+        ctl_clean = false;
         for (int i = 0; i < warmup; i++) CK(cudaGraphLaunch(exec, stream));
         double total = 0.0;
         for (int i = 0; i < iters; i++) {
@@ -2957,7 +2982,8 @@ namespace gqb {
 struct BatchQ {
     uint32_t blob_off;                 // word offset into the wave's blob buffer
     uint32_t n;
-    uint32_t first_base;               // index of its first singleton in the level-1 list
+    uint32_t first_base;               // relations of the queries ahead: its first singleton in the level-1
+                                       // list, and half the index of its first plan node
     uint32_t tree_tab;                 // word offset of its tree tables in the wave's blob buffer
     unsigned long long memo_off;       // entry offset into the memo arena
     unsigned long long seen_off;       // word offset into the dedup bitmap arena
@@ -3450,7 +3476,7 @@ __global__ void __launch_bounds__(kBlock, 2) kb_gen(const BatchQ *__restrict__ q
         const uint32_t full = (Q.n == 32) ? 0xFFFFFFFFu : ((1u << Q.n) - 1u);
         const uint32_t wmask =
             reinterpret_cast<const DevHeader *>(ONE ? own : blobs + Q.blob_off)->hz_packed ? kWidthMask : 0xFFFFFFFFu;
-        extract_plan(memo + Q.memo_off, memo_left + Q.memo_off, full, wmask, ws.queue, tree + (size_t)q * 64, tree_n + q);
+        extract_plan(memo + Q.memo_off, memo_left + Q.memo_off, full, wmask, ws.queue, tree + 2u * Q.first_base, tree_n + q);
     }
     for (int off = 16; off >= 1; off >>= 1) pairs += __shfl_xor_sync(kFull, pairs, off);
     if (lane == 0 && pairs) atomicAdd(&glob->evaluated_pairs, pairs);
@@ -3465,7 +3491,7 @@ __global__ void kb_extract(const BatchQ *__restrict__ qs, int nq, const uint32_t
     const uint32_t wmask =
         reinterpret_cast<const DevHeader *>(blobs + Q.blob_off)->hz_packed ? kWidthMask : 0xFFFFFFFFu;
     const uint32_t full = (Q.n == 32) ? 0xFFFFFFFFu : ((1u << Q.n) - 1u);
-    TreeNode *o = out + (size_t)q * 64;
+    TreeNode *o = out + 2u * Q.first_base;
     const float4 *m = memo + Q.memo_off;
     const uint32_t *ml = memo_left + Q.memo_off;
     int n = 0;
@@ -3633,7 +3659,7 @@ __global__ void __launch_bounds__(kBlock, 3) kb_dp(const BatchQ *__restrict__ qs
         const uint32_t wmask =
             reinterpret_cast<const DevHeader *>(blobs + Q.blob_off)->hz_packed ? kWidthMask : 0xFFFFFFFFu;
         extract_plan(memo + Q.memo_off, memo_left + Q.memo_off, full, wmask, reinterpret_cast<uint32_t *>(st),
-                     tree + (size_t)q * 64, tree_n + q);
+                     tree + 2u * Q.first_base, tree_n + q);
     }
     if (tid == 0) glob->evaluated_pairs = pairs;
 }
@@ -3711,6 +3737,13 @@ uint64_t batch_query_bytes(int n) {
     return slots * (sizeof(float4) + 4) + slots / 8 + 2 * max_level_sets(n) * 8 + 64 * sizeof(TreeNode) + 4096;
 }
 
+// control words of a wave: cleared with one memset, brought back with its plans
+struct alignas(16) BatchCtl {
+    LevelCounters lvl[33];
+    GlobalCounters glob;
+    unsigned bar[4];                   // grid barrier: arrivals, -, error flag
+};
+
 // dynamic shared memory of kb_gen besides the planner info
 constexpr size_t kGenSmem = kWarpsPerBlock * sizeof(GenScratch);
 static_assert(kGenSmem <= 44 * 1024 && sizeof(GenScratch) % 16 == 0, "kb_gen scratch and its static shared memory");
@@ -3720,17 +3753,20 @@ struct BatchEngine {
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     // arena (grown on demand)
-    uint64_t cap_slots = 0, cap_items = 0, cap_words = 0, cap_seen = 0;
-    int cap_q = 0;
+    uint64_t cap_slots = 0, cap_items = 0, cap_seen = 0;
     float4 *memo = nullptr;
     uint32_t *memo_left = nullptr, *blobs = nullptr, *seen = nullptr;
     unsigned long long *listA = nullptr, *listB = nullptr;
     BatchQ *qs = nullptr;
     TreeNode *tree = nullptr;
     int *tree_n = nullptr;
-    LevelCounters *lvl = nullptr;
+    LevelCounters *lvl = nullptr;                // views into d_out
     GlobalCounters *glob = nullptr;
-    unsigned *bar = nullptr, *h_bar = nullptr;   // grid barrier words (device, pinned copy)
+    unsigned *bar = nullptr;
+    // device side of a wave's two copies: descriptors and planner infos in
+    // (qs, blobs), control words, node counts and plans out (BatchCtl, tree_n, tree)
+    unsigned char *d_in = nullptr, *d_out = nullptr;
+    uint64_t cap_in = 0, cap_out = 0;
     int coop_grid = -1;                          // co-resident blocks of kb_gen<false> (0: no cooperative launch)
     int coop_grid_tree[3] = {-1, -1, -1};        // co-resident blocks of kb_dp by layout (tree_layout)
     std::map<size_t, int> coop_one;              // dynamic shared bytes -> co-resident blocks of kb_gen<true>
@@ -3760,10 +3796,6 @@ struct BatchEngine {
         CK(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
         CK(cudaEventCreate(&ev0));
         CK(cudaEventCreate(&ev1));
-        CK(cudaMalloc(&lvl, 33 * sizeof(LevelCounters)));
-        CK(cudaMalloc(&glob, sizeof(GlobalCounters)));
-        CK(cudaMalloc(&bar, 4 * sizeof(unsigned)));
-        CK(cudaMallocHost(&h_bar, 4 * sizeof(unsigned)));
         int dev_coop = 0, occ = 0, occ_tree[3] = {0, 0, 0};
         cudaDeviceGetAttribute(&dev_coop, cudaDevAttrCooperativeLaunch, device);
         no_cooperative();
@@ -3783,8 +3815,7 @@ struct BatchEngine {
 
     // per-level launches of one wave (the queries, blobs and arena are staged)
     uint32_t enqueue_levels(int nq, int maxn, uint64_t seen_words) {
-        cudaMemsetAsync(lvl, 0, 33 * sizeof(LevelCounters), stream);
-        cudaMemsetAsync(glob, 0, sizeof(GlobalCounters), stream);
+        cudaMemsetAsync(d_out, 0, sizeof(BatchCtl), stream);
         cudaMemsetAsync(seen, 0, seen_words * 4, stream);
         kb_init<<<nq, 32, 0, stream>>>(qs, nq, blobs, memo, memo_left, listA, lvl + 1);
         uint32_t kernels = 1;
@@ -3842,10 +3873,8 @@ struct BatchEngine {
             if (cluster) grid = std::min(grid, kTreeCluster);
         }
         if (grid <= 0 || gpuqo_b200_persistent == 0 || barrier_timed_out) return false;
-        cudaMemsetAsync(lvl, 0, 33 * sizeof(LevelCounters), stream);
-        cudaMemsetAsync(glob, 0, sizeof(GlobalCounters), stream);
+        cudaMemsetAsync(d_out, 0, sizeof(BatchCtl), stream);
         if (!tree_only) cudaMemsetAsync(seen, 0, table_log2 ? (size_t)4 << table_log2 : seen_words * 4, stream);
-        cudaMemsetAsync(bar, 0, 4 * sizeof(unsigned), stream);
         unsigned poll_limit = (unsigned)std::max(0, gpuqo_b200_barrier_poll_limit);
         cudaError_t e;
         if (tree_only) {
@@ -3963,12 +3992,10 @@ struct BatchEngine {
         if (int rc = over_budget(slots * (sizeof(float4) + 4) + words * 4 + seen_words * 4 + items * 16 + ovf_need * 32,
                                  "the batch wave's arena", err))
             return rc;
-        uint64_t c1 = cap_slots, c2 = cap_slots, c3 = cap_words, c4 = cap_seen, c5 = cap_items, c6 = cap_items;
+        uint64_t c1 = cap_slots, c2 = cap_slots, c4 = cap_seen, c5 = cap_items, c6 = cap_items;
         if (int rc = grow(memo, c1, slots, err)) return rc;
         if (int rc = grow(memo_left, c2, slots, err)) return rc;
         cap_slots = std::min(c1, c2);
-        if (int rc = grow(blobs, c3, words, err)) return rc;
-        cap_words = c3;
         if (int rc = grow(seen, c4, seen_words, err)) return rc;
         cap_seen = c4;
         if (int rc = grow(listA, c5, items, err)) return rc;
@@ -3990,43 +4017,34 @@ struct BatchEngine {
         // large enough that a level's units number below 2^32 (at most 2^22
         // listed sets of 2^(n - 1) splits)
         ovf.unit = maxn <= 24 ? 32u : (maxn <= 26 ? 1024u : 8192u);
-        if (nq > cap_q) {
-            cudaFree(qs);
-            cudaFree(tree);
-            cudaFree(tree_n);
-            qs = nullptr;
-            tree = nullptr;
-            tree_n = nullptr;
-            cap_q = 0;
-            CK(cudaMalloc(&qs, nq * sizeof(BatchQ)));
-            CK(cudaMalloc(&tree, (size_t)nq * 64 * sizeof(TreeNode)));
-            CK(cudaMalloc(&tree_n, nq * sizeof(int)));
-            cap_q = nq;
-        }
-        // stage the planner infos and the descriptors in pinned memory (the
+        const size_t in_q = (size_t)nq * sizeof(BatchQ), in_bytes = in_q + (size_t)words * 4;
+        const size_t o_n = sizeof(BatchCtl), o_tree = (o_n + (size_t)nq * sizeof(int) + 15) & ~(size_t)15,
+                     o_end = o_tree + 2 * (size_t)base * sizeof(TreeNode);
+        if (int rc = grow(d_in, cap_in, in_bytes, err)) return rc;
+        if (int rc = grow(d_out, cap_out, o_end, err)) return rc;
+        qs = reinterpret_cast<BatchQ *>(d_in);
+        blobs = reinterpret_cast<uint32_t *>(d_in + in_q);
+        lvl = reinterpret_cast<BatchCtl *>(d_out)->lvl;
+        glob = &reinterpret_cast<BatchCtl *>(d_out)->glob;
+        bar = reinterpret_cast<BatchCtl *>(d_out)->bar;
+        tree_n = reinterpret_cast<int *>(d_out + o_n);
+        tree = reinterpret_cast<TreeNode *>(d_out + o_tree);
+        // stage the descriptors and the planner infos in pinned memory (the
         // previous wave's copies ended with its synchronisation)
-        const size_t in_blob = (size_t)words * 4, in_q = (size_t)nq * sizeof(BatchQ);
-        if (int rc = grow_pinned(h_in, cap_h_in, in_blob + in_q, err)) return rc;
-        uint32_t *hblob = reinterpret_cast<uint32_t *>(h_in);
+        if (int rc = grow_pinned(h_in, cap_h_in, in_bytes, err)) return rc;
+        if (int rc = grow_pinned(h_out, cap_h_out, o_end, err)) return rc;
+        std::memcpy(h_in, hq.data(), in_q);
+        uint32_t *hblob = reinterpret_cast<uint32_t *>(h_in + in_q);
         for (int q = 0; q < nq; q++) {
             const size_t len = wb[q]->size(), padded = (len + 3) & ~(size_t)3;
             std::memcpy(hblob + hq[q].blob_off, wb[q]->data(), len * 4);
             std::memset(hblob + hq[q].blob_off + len, 0, (padded - len) * 4);
         }
-        std::memcpy(h_in + in_blob, hq.data(), in_q);
-        CK(cudaMemcpyAsync(blobs, hblob, in_blob, cudaMemcpyHostToDevice, stream));
-        CK(cudaMemcpyAsync(qs, h_in + in_blob, in_q, cudaMemcpyHostToDevice, stream));
-        // plans and counters come back into pinned memory, with the barrier
-        // words, in one synchronisation
-        const size_t o_tree = 0, o_n = o_tree + (size_t)nq * 64 * sizeof(TreeNode),
-                     o_lvl = (o_n + (size_t)nq * sizeof(int) + 15) & ~(size_t)15,
-                     o_glob = o_lvl + 33 * sizeof(LevelCounters), o_end = o_glob + sizeof(GlobalCounters);
-        if (int rc = grow_pinned(h_out, cap_h_out, o_end, err)) return rc;
+        CK(cudaMemcpyAsync(d_in, h_in, in_bytes, cudaMemcpyHostToDevice, stream));
+        // control words and plans come back in one copy
+        const BatchCtl &ctl = *reinterpret_cast<const BatchCtl *>(h_out);
         auto download = [&]() -> int {
-            CK(cudaMemcpyAsync(h_out + o_tree, tree, (size_t)nq * 64 * sizeof(TreeNode), cudaMemcpyDeviceToHost, stream));
-            CK(cudaMemcpyAsync(h_out + o_n, tree_n, nq * sizeof(int), cudaMemcpyDeviceToHost, stream));
-            CK(cudaMemcpyAsync(h_out + o_lvl, lvl, 33 * sizeof(LevelCounters), cudaMemcpyDeviceToHost, stream));
-            CK(cudaMemcpyAsync(h_out + o_glob, glob, sizeof(GlobalCounters), cudaMemcpyDeviceToHost, stream));
+            CK(cudaMemcpyAsync(h_out, d_out, o_end, cudaMemcpyDeviceToHost, stream));
             CK(cudaStreamSynchronize(stream));
             CK(cudaGetLastError());
             return 0;
@@ -4035,12 +4053,11 @@ struct BatchEngine {
         CK(cudaEventRecord(ev0, stream));
         bool persistent = enqueue_persistent(nq, maxn, (uint32_t)words, seen_words, layout, cactus_sets);
         CK(cudaGetLastError());
-        if (persistent) CK(cudaMemcpyAsync(h_bar, bar, 4 * sizeof(unsigned), cudaMemcpyDeviceToHost, stream));
         if (!persistent) kernels = enqueue_levels(nq, maxn, seen_words);
         CK(cudaGetLastError());
         CK(cudaEventRecord(ev1, stream));
         if (int rc = download()) return rc;
-        if (persistent && h_bar[2] != 0u) {   // barrier timed out: rerun with per-level launches
+        if (persistent && ctl.bar[2] != 0u) {   // barrier timed out: rerun with per-level launches
             persistent = false;
             barrier_timed_out = true;           // and use them until gpuqo_b200_reset_persistent
             st.barrier_timeouts++;
@@ -4052,8 +4069,6 @@ struct BatchEngine {
         }
         const TreeNode *htree = reinterpret_cast<const TreeNode *>(h_out + o_tree);
         const int *hn = reinterpret_cast<const int *>(h_out + o_n);
-        const LevelCounters *hl = reinterpret_cast<const LevelCounters *>(h_out + o_lvl);
-        const GlobalCounters &hg = *reinterpret_cast<const GlobalCounters *>(h_out + o_glob);
         float fms = 0.f;
         CK(cudaEventElapsedTime(&fms, ev0, ev1));
         ms = fms;
@@ -4063,10 +4078,10 @@ struct BatchEngine {
                 err = "batched plan extraction produced " + std::to_string(hn[q]) + " nodes";
                 return GPUQO_B200_ERR_CUDA;
             }
-            out[q].assign(htree + (size_t)q * 64, htree + (size_t)q * 64 + hn[q]);
+            out[q].assign(htree + 2 * (size_t)hq[q].first_base, htree + 2 * (size_t)hq[q].first_base + hn[q]);
         }
-        for (int k = 2; k <= maxn; k++) st.connected_sets += hl[k].n_sets;
-        st.evaluated_pairs += hg.evaluated_pairs;
+        for (int k = 2; k <= maxn; k++) st.connected_sets += ctl.lvl[k].n_sets;
+        st.evaluated_pairs += ctl.glob.evaluated_pairs;
         st.memo_bytes = std::max<uint64_t>(st.memo_bytes, slots * (sizeof(float4) + 4));
         st.device_ms += fms;
         st.kernel_launches += kernels;
