@@ -5,6 +5,8 @@
 // convert -> BFS relabel -> exact DP (or IDP driver) -> map the plan back ->
 // palloc'd QueryTreeC.  The exact DP runs on the GPU (dp_kernels.cu).
 #include <algorithm>
+#include <array>
+#include <atomic>
 #include <cmath>
 #include <csignal>
 #include <cstdio>
@@ -678,7 +680,11 @@ bool algorithm_supported(int algorithm) {
 }
 
 static Bitmapset *make_bms(mask64 m) {
-    Bitmapset *b = (Bitmapset *)palloc0(offsetof(Bitmapset, words) + sizeof(bitmapword));
+    // palloc and memset: glibc's calloc (palloc0) passes its per-thread cache by,
+    // so each node's set cost a trip to the heap's lists
+    const size_t size = offsetof(Bitmapset, words) + sizeof(bitmapword);
+    Bitmapset *b = (Bitmapset *)palloc(size);
+    std::memset(b, 0, size);
     b->nwords = 1;
     b->words[0] = m;
     return b;
@@ -687,7 +693,7 @@ static Bitmapset *make_bms(mask64 m) {
 // node array (compact masks over relabelled relations) -> QueryTreeC with the
 // caller's relids (remapQueryTree gpuqo_remapper.cu:279-300, convertQueryTree
 // gpuqo_planner_info.cu:256-270)
-static QueryTreeC *nodes_to_c(const std::vector<TreeNode> &nodes, int idx, const std::vector<int> &from_of_to) {
+static QueryTreeC *nodes_to_c(const std::vector<TreeNode> &nodes, int idx, const int *from_of_to) {
     if (idx < 0) return NULL;
     const TreeNode &t = nodes[idx];
     QueryTreeC *q = (QueryTreeC *)palloc(sizeof(QueryTreeC));
@@ -745,7 +751,7 @@ QueryTreeC *run_one(int algorithm, GpuqoPlannerInfoC *info_c) {
         set_error(rc, err);
         return NULL;
     }
-    return nodes_to_c(nodes, 0, order);
+    return nodes_to_c(nodes, 0, order.data());
 }
 
 }  // namespace gqb
@@ -809,7 +815,7 @@ extern "C" int gpuqo_b200_time_resident(int gpuqo_algorithm_arg, GpuqoPlannerInf
         return rc;
     }
     stats_add(st);
-    if (tree) *tree = nodes_to_c(nodes, 0, order);
+    if (tree) *tree = nodes_to_c(nodes, 0, order.data());
     return GPUQO_B200_OK;
 }
 
@@ -948,7 +954,7 @@ extern "C" int gpuqo_b200_run_batch(int gpuqo_algorithm_arg, GpuqoPlannerInfoC *
     // queries without IDP whose candidate count fits the batched kernel go to
     // the level-synchronous batch, the rest run one by one.
     struct Prep {
-        std::vector<int> order;
+        std::array<int, 30> order;   // the caller's relations in BFS order
         std::vector<uint32_t> blob;
     };
     std::vector<Prep> prep(n_queries);
@@ -964,24 +970,32 @@ extern "C" int gpuqo_b200_run_batch(int gpuqo_algorithm_arg, GpuqoPlannerInfoC *
         HostInfo info;
         std::string err;
         if (!convert_info(c, info, err)) return;
-        prep[i].order = bfs_order(info);
-        if ((int)prep[i].order.size() != info.n) return;
-        HostInfo remapped = relabel(info, prep[i].order);
+        const std::vector<int> order = bfs_order(info);
+        if ((int)order.size() != info.n) return;
+        std::copy(order.begin(), order.end(), prep[i].order.begin());
+        HostInfo remapped = relabel(info, order);
         prep[i].blob = build_blob(remapped);
         apply_dpsub_csg(prep[i].blob, m);
         to_batch[i] = (m == kModeMpdp && batch_eligible(prep[i].blob)) ? 1 : 0;
     };
+    // This thread works too, and takes the first queries while the others
+    // start: a query takes 1.5 to 6 us, a thread some 20 us to start, and
+    // threads that fault in new pages at the same time hold each other up.
+    // 512 queries of 8 to 16 relations take 0.44 to 0.58 ms with 8 threads;
+    // 16 with fixed shares and this thread waiting took 0.58 to 0.85 ms.
     const int hw = (int)std::max(1u, std::thread::hardware_concurrency());
-    const int n_threads = n_queries >= 64 ? std::min({hw, 16, n_queries / 32}) : 1;
-    if (n_threads > 1) {
+    const int n_threads = std::max(1, std::min({hw, 8, n_queries / 32}));
+    std::atomic<int> next{0};
+    auto work_off = [&] {
+        constexpr int kTake = 8;
+        for (int at = next.fetch_add(kTake); at < n_queries; at = next.fetch_add(kTake))
+            for (int i = at; i < std::min(at + kTake, n_queries); i++) prepare(i);
+    };
+    {
         std::vector<std::thread> pool;
-        for (int t = 0; t < n_threads; t++)
-            pool.emplace_back([&, t] {
-                for (int i = t; i < n_queries; i += n_threads) prepare(i);
-            });
+        for (int t = 1; t < n_threads; t++) pool.emplace_back(work_off);
+        work_off();
         for (auto &th : pool) th.join();
-    } else {
-        for (int i = 0; i < n_queries; i++) prepare(i);
     }
     std::vector<int> batched, single;
     for (int i = 0; i < n_queries; i++) (to_batch[i] ? batched : single).push_back(i);
@@ -1058,7 +1072,7 @@ extern "C" int gpuqo_b200_run_batch(int gpuqo_algorithm_arg, GpuqoPlannerInfoC *
         stats_add(st);
         t_stats.n_subproblems = (uint32_t)batched.size();
         for (size_t j = 0; j < batched.size(); j++)
-            out[batched[j]] = nodes_to_c(nodes[j], 0, prep[batched[j]].order);
+            out[batched[j]] = nodes_to_c(nodes[j], 0, prep[batched[j]].order.data());
     }
     for (int i : single) {
         out[i] = run_one(gpuqo_algorithm_arg, infos[i]);

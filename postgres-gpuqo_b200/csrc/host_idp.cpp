@@ -26,7 +26,7 @@
 #include <cstdio>
 #include <cstring>
 #include <functional>
-#include <map>
+#include <iterator>
 #include <memory>
 #include <queue>
 #include <string>
@@ -42,7 +42,6 @@ extern "C" int gpuqo_idp_type;
 extern "C" bool gpuqo_spanning_tree_enable;
 extern "C" volatile sig_atomic_t InterruptPending;
 extern "C" void *palloc(size_t size);
-extern "C" void *palloc0(size_t size);
 
 namespace gqb {
 
@@ -227,12 +226,28 @@ struct QT {
 };
 
 // node arena of one gpuqo_run call (the reference's trees are freed piecemeal;
-// here they live until the call returns)
-struct Arena {
-    std::vector<std::unique_ptr<QT>> nodes;
+// here they live until the call returns).  Nodes come in linked blocks: a
+// 200-relation IDP2 call makes some 5000, and one allocation each was a quarter
+// of its host time.
+class Arena {
+    struct Block {
+        std::unique_ptr<Block> before;
+        QT nodes[64];
+    };
+    std::unique_ptr<Block> last;
+    int used = 0;   // of the last block
+public:
     QT *make() {
-        nodes.emplace_back(new QT());
-        return nodes.back().get();
+        if (!last || used == (int)std::size(last->nodes)) {
+            std::unique_ptr<Block> b(new Block);
+            b->before = std::move(last);
+            last = std::move(b);
+            used = 0;
+        }
+        return &last->nodes[used++];
+    }
+    ~Arena() {
+        while (last) last = std::move(last->before);   // one by one: the chain may be long
     }
 };
 
@@ -810,31 +825,22 @@ static QT *solve_sub(const GInfo &info, const std::vector<Entry> &list, Ctx &C) 
 struct GooNode {
     QT *qt;
     BB edges;      // union of the relations' edges (are_connected_ids operand)
+    int top;       // highest relation: the order of disjoint sets as integers
+    bool live;     // not yet part of a larger entry
+};
+
+// A join on the heap: the tree node is made only if the join is taken.
+struct GooJoin {
+    float rows;
+    int l, r;      // nodes
 };
 
 static QT *goo(const GInfo &g, Arena &A) {
-    auto compare = [](QT *l, QT *r) {
-        if (l != nullptr && r != nullptr) return l->rows > r->rows;
-        return r != nullptr;
-    };
-    std::vector<QT *> heap;
-    std::map<BB, GooNode> rels;
-    auto edges_of = [&](const BB &id) {
-        BB e;
-        id.for_each([&](int b) { e |= g.edge[b - 1]; });
-        return e;
-    };
-    auto join = [&](QT &l, QT &r) {
-        QT *q = A.make();
-        q->id = l.id | r.id;
-        q->rows = estimate_join_rows(g, l, r);
-        q->cost.startup = 0;
-        q->cost.total = q->rows + l.cost.total + r.cost.total;
-        q->left = &l;
-        q->right = &r;
-        q->width = l.width + r.width;
-        return q;
-    };
+    auto compare = [](const GooJoin &l, const GooJoin &r) { return l.rows > r.rows; };
+    std::vector<GooJoin> heap;
+    std::vector<GooNode> nodes;              // every entry there ever was, at most 2 n - 1
+    nodes.reserve(2 * (size_t)g.n);
+    std::vector<int> owner(g.n + 1, -1);     // relation (bit) -> its live entry
     for (int i = 0; i < g.n; i++) {
         QT *q = A.make();
         q->id = g.base[i].id;
@@ -842,63 +848,62 @@ static QT *goo(const GInfo &g, Arena &A) {
         q->cost.startup = 0;
         q->cost.total = g.base[i].rows;
         q->width = g.base[i].width;
-        rels.emplace(q->id, GooNode{q, edges_of(q->id)});
+        nodes.push_back(GooNode{q, g.edge[i], i + 1, true});
+        owner[i + 1] = i;
     }
     // are_valid_pair (gpuqo_filter.cuh:84-90): connected and disjoint.  The
     // reference tests every pair of entries in map order; the entries valid
     // with `a` are those holding a relation of a's edges outside a, so they
-    // are found through owner[] (relation -> its entry) and visited in the
-    // same map order, which keeps the heap's push sequence and so its ties.
-    using It = std::map<BB, GooNode>::iterator;
-    std::vector<It> owner(g.n + 1, rels.end());
-    for (It it = rels.begin(); it != rels.end(); ++it)
-        it->first.for_each([&](int b) {
-            if (b <= g.n) owner[b] = it;
-        });
-    std::vector<It> cand;
+    // are found through owner[] and visited in the same map order, which
+    // keeps the heap's push sequence and so its ties.  The entries are
+    // disjoint, so their order as sets is the order of their highest relations.
+    std::vector<int> cand;
     auto valid_entries = [&](const GooNode &a) {
         cand.clear();
         (a.edges - a.qt->id).for_each([&](int b) {
-            if (b <= g.n && owner[b] != rels.end()) cand.push_back(owner[b]);
+            if (b <= g.n && owner[b] >= 0) cand.push_back(owner[b]);
         });
-        std::sort(cand.begin(), cand.end(), [](const It &x, const It &y) { return x->first < y->first; });
+        std::sort(cand.begin(), cand.end(), [&](int x, int y) { return nodes[x].top < nodes[y].top; });
         cand.erase(std::unique(cand.begin(), cand.end()), cand.end());
     };
-    for (It i = rels.begin(); i != rels.end(); ++i) {
-        valid_entries(i->second);
-        for (const It &j : cand)
-            if (i->first < j->first) {
-                heap.push_back(join(*i->second.qt, *j->second.qt));
-                std::push_heap(heap.begin(), heap.end(), compare);
-            }
+    auto push_join = [&](int l, int r) {
+        heap.push_back(GooJoin{estimate_join_rows(g, *nodes[l].qt, *nodes[r].qt), l, r});
+        std::push_heap(heap.begin(), heap.end(), compare);
+    };
+    for (int i = 0; i < g.n; i++) {
+        valid_entries(nodes[i]);
+        for (int j : cand)
+            if (nodes[i].top < nodes[j].top) push_join(i, j);
     }
-    QT *smallest = nullptr;
-    do {
-        if (heap.empty()) return nullptr;   // disconnected query graph
-        std::pop_heap(heap.begin(), heap.end(), compare);
-        smallest = heap.back();
-        heap.pop_back();
-        auto lp = rels.find(smallest->left->id);
-        auto rp = rels.find(smallest->right->id);
-        if (lp == rels.end() || rp == rels.end()) {
-            smallest = nullptr;
-            continue;
-        }
-        // edges_of distributes over the union of the two entries
-        GooNode sn{smallest, lp->second.edges | rp->second.edges};
-        rels.erase(lp);
-        rels.erase(rp);
-        valid_entries(sn);
-        for (const It &j : cand) {
-            heap.push_back(join(*smallest, *j->second.qt));
-            std::push_heap(heap.begin(), heap.end(), compare);
-        }
-        const It ins = rels.emplace(smallest->id, sn).first;
-        smallest->id.for_each([&](int b) {
-            if (b <= g.n) owner[b] = ins;
+    int last = 0;
+    while (nodes[last].qt->id.size() < g.n) {
+        GooJoin best;
+        do {
+            if (heap.empty()) return nullptr;   // disconnected query graph
+            std::pop_heap(heap.begin(), heap.end(), compare);
+            best = heap.back();
+            heap.pop_back();
+        } while (!nodes[best.l].live || !nodes[best.r].live);
+        GooNode &l = nodes[best.l], &r = nodes[best.r];
+        l.live = r.live = false;
+        QT *q = A.make();
+        q->id = l.qt->id | r.qt->id;
+        q->rows = best.rows;
+        q->cost.startup = 0;
+        q->cost.total = q->rows + l.qt->cost.total + r.qt->cost.total;
+        q->left = l.qt;
+        q->right = r.qt;
+        q->width = l.qt->width + r.qt->width;
+        last = (int)nodes.size();
+        // edges of a union are the union of the edges
+        nodes.push_back(GooNode{q, l.edges | r.edges, std::max(l.top, r.top), true});
+        q->id.for_each([&](int b) {
+            if (b <= g.n) owner[b] = last;
         });
-    } while (smallest == nullptr || smallest->id.size() < g.n);
-    return smallest;
+        valid_entries(nodes[last]);
+        for (int j : cand) push_join(last, j);
+    }
+    return nodes[last].qt;
 }
 
 // ---------------------------------------------------------------------------
@@ -1076,7 +1081,9 @@ static QueryTreeC *qt_to_c(const QT *q) {
     for (int i = 0; i < kBigWords; i++)
         if (q->id.w[i]) top = i;
     int nwords = top + 1;
-    Bitmapset *b = (Bitmapset *)palloc0(offsetof(Bitmapset, words) + nwords * sizeof(bitmapword));
+    const size_t size = offsetof(Bitmapset, words) + nwords * sizeof(bitmapword);
+    Bitmapset *b = (Bitmapset *)palloc(size);
+    std::memset(b, 0, size);
     b->nwords = nwords;
     for (int i = 0; i < nwords; i++) b->words[i] = q->id.w[i];
     o->id = b;
