@@ -910,30 +910,29 @@ __device__ __forceinline__ void plain_mirror(const PlainParams &c, const PlainQu
     plain_join(c, e, sel_r, r, l, dr, dl, nl_startup, nl_tuples, lb, rp, lp, rl);
 }
 
-// Classes of two members with one member on each side of a split, 32 per word.
-// A class has exactly one member in L when it is in an odd number of the rows
-// (rel_ecs) of L's relations, so the rows' exclusive or, restricted to the
-// classes inside S, is the match of (L, S - L); it follows L from split to
-// split by the rows of the relations that change sides.
-template <int NW>
-__device__ __forceinline__ void pairs_flip(const DevInfoView &d, uint32_t rels, uint32_t (&odd)[4 * NW]) {
-    for (uint32_t x = rels; x; x &= x - 1u) {
-        const uint4 *row = reinterpret_cast<const uint4 *>(d.rel_ecs + lowest_idx(x) * (4 * NW));
-#pragma unroll
-        for (int j = 0; j < NW; j++) {
-            const uint4 a = row[j];
-            odd[4 * j] ^= a.x;
-            odd[4 * j + 1] ^= a.y;
-            odd[4 * j + 2] ^= a.z;
-            odd[4 * j + 3] ^= a.w;
-        }
-    }
+// pext: the bits of x at the positions of mask, packed (x within mask)
+__device__ __forceinline__ uint32_t pext32(uint32_t x, uint32_t mask) {
+    uint32_t r = 0u;
+    for (; x; x &= x - 1u) r |= 1u << __popc(mask & ((x & (0u - x)) - 1u));
+    return r;
 }
 
-// the classes with both members in S
+// One set's classes with both members in it (two members each), numbered in
+// class order without gaps: their selectivities and, per relation of the set,
+// the classes it is in.  A class has exactly one member in L when it is in an
+// odd number of the rows of L's relations, so the rows' exclusive or is the
+// match of (L, S - L); it follows L from split to split by the rows of the
+// relations that change sides.
 template <int NW>
-__device__ __forceinline__ void pairs_inside(const DevInfoView &d, uint32_t S, uint32_t (&inside)[4 * NW]) {
-    uint32_t odd[4 * NW];
+struct PairTable {
+    float4 sel[32 * NW];
+    uint4 row[kMaxRels][NW];
+};
+
+// by one warp; the number of classes inside S
+template <int NW>
+__device__ __forceinline__ int pairs_table(const DevInfoView &d, uint32_t S, uint32_t lane, PairTable<NW> &t) {
+    uint32_t odd[4 * NW], inside[4 * NW];
 #pragma unroll
     for (int w = 0; w < 4 * NW; w++) inside[w] = odd[w] = 0u;
     for (uint32_t x = S; x; x &= x - 1u) {
@@ -949,22 +948,76 @@ __device__ __forceinline__ void pairs_inside(const DevInfoView &d, uint32_t S, u
             }
         }
     }
+    __syncwarp();   // readers of the previous set's table
+    const bool member = (S >> lane) & 1u;
+    uint32_t *row = reinterpret_cast<uint32_t *>(t.row[lane]);
+    if (member)
+#pragma unroll
+        for (int w = 0; w < 4 * NW; w++) row[w] = 0u;
+    float *sel = reinterpret_cast<float *>(t.sel);
+    int base = 0;
+#pragma unroll
+    for (int w = 0; w < 4 * NW; w++) {
+        if ((inside[w] >> lane) & 1u) sel[base + popc(inside[w] & ((1u << lane) - 1u))] = d.pair_sel[64 * w + 2 * lane];
+        if (member) {
+            const uint32_t x = pext32(d.rel_ecs[lane * (4 * NW) + w] & inside[w], inside[w]);
+            const int at = base >> 5, sh = base & 31;
+            if (x) row[at] |= x << sh;
+            const uint32_t rest = sh ? x >> (32 - sh) : 0u;
+            if (rest) row[at + 1] |= rest;
+        }
+        base += popc(inside[w]);
+    }
+    __syncwarp();
+    return base;
 }
 
-// both orientations of a split whose matching classes are odd & inside; the
-// one selectivity product (pairs_plain) is taken in class order
 template <int NW>
-__device__ __forceinline__ void pairs_mirror(const DevInfoView &d, const PlainParams &pp, const uint32_t (&odd)[4 * NW],
-                                             const uint32_t (&inside)[4 * NW], const float4 l, const float4 r,
-                                             JoinCost &lr, JoinCost &rl) {
+__device__ __forceinline__ void pairs_flip(const PairTable<NW> &t, uint32_t rels, uint32_t (&odd)[4 * NW]) {
+    for (uint32_t x = rels; x; x &= x - 1u) {
+        const uint4 *row = t.row[lowest_idx(x)];
+#pragma unroll
+        for (int j = 0; j < NW; j++) {
+            const uint4 a = row[j];
+            odd[4 * j] ^= a.x;
+            odd[4 * j + 1] ^= a.y;
+            odd[4 * j + 2] ^= a.z;
+            odd[4 * j + 3] ^= a.w;
+        }
+    }
+}
+
+// Both orientations of a split whose matching classes are odd; the one
+// selectivity product (pairs_plain) is taken in class order.  Every lane passes
+// over all classes of the set and multiplies where its split matches: that is
+// twice the multiplications, but the class is the same for all lanes, so that
+// it costs a test and a multiplication with a selectivity loaded for four
+// classes at a time, where a search for each lane's next matching class costs
+// some seven instructions and runs as often as the fullest lane of a word asks.
+template <int NW>
+__device__ __forceinline__ void pairs_mirror(const DevInfoView &d, const PlainParams &pp, const PairTable<NW> &t,
+                                             int classes, const uint32_t (&odd)[4 * NW], const float4 l,
+                                             const float4 r, JoinCost &lr, JoinCost &rl) {
     float sel = 1.0f;
     int quals = 0;
 #pragma unroll
     for (int w = 0; w < 4 * NW; w++) {
-        const uint32_t m = odd[w] & inside[w];
-        const float *s = d.pair_sel + 64 * w;
+        if (32 * w >= classes) break;
+        const uint32_t m = odd[w];
         quals += popc(m);
-        for (uint32_t x = m; x; x &= x - 1u) sel *= s[2 * lowest_idx(x)];
+#pragma unroll
+        for (int g = 0; g < 4; g++) {
+            if (32 * w + 8 * g >= classes) break;
+#pragma unroll
+            for (int j = 0; j < 2; j++) {
+                const float4 s = t.sel[8 * w + 2 * g + j];
+                const uint32_t bit = 1u << (8 * g + 4 * j);
+                if (m & bit) sel *= s.x;
+                if (m & (bit << 1)) sel *= s.y;
+                if (m & (bit << 2)) sel *= s.z;
+                if (m & (bit << 3)) sel *= s.w;
+            }
+        }
     }
     const PlainQuals q = reinterpret_cast<const PlainQuals *>(reinterpret_cast<const uint32_t *>(d.h) + d.h->pairs_plain)[quals];
     plain_mirror(pp, q, sel, sel, l, r, lr, rl);
@@ -1011,13 +1064,6 @@ struct Blocks {
     uint32_t prefix[kMaxRels + 1];
     uint32_t eprefix[kMaxRels + 1];
 };
-
-// pext: the bits of x at the positions of mask, packed (x within mask)
-__device__ __forceinline__ uint32_t pext32(uint32_t x, uint32_t mask) {
-    uint32_t r = 0u;
-    for (; x; x &= x - 1u) r |= 1u << __popc(mask & ((x & (0u - x)) - 1u));
-    return r;
-}
 
 __device__ __forceinline__ void find_blocks(uint32_t S, const uint32_t *adj, Blocks &B) {
     uint8_t disc[kMaxRels], low[kMaxRels], parent[kMaxRels];

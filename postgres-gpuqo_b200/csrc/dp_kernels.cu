@@ -1374,12 +1374,14 @@ __global__ void __launch_bounds__(kBlock, 3) k_dense(const uint32_t *__restrict_
                                                      unsigned long long *__restrict__ firsts,
                                                      GlobalCounters *__restrict__ glob, uint32_t share) {
     extern __shared__ __align__(16) uint32_t sm[];
+    __shared__ PairTable<NW> tabs[kWarpsPerBlock];
     load_blob_to_smem(blob, blob_words, sm);
     const DevInfoView d = make_view(sm);
     const DevHeader &h = *d.h;
     const uint32_t *adj = h.adj;
     const PlainParams pp = plain_params(h);
     const uint32_t lane = threadIdx.x & 31u;
+    PairTable<NW> &tab = tabs[threadIdx.x >> 5];
     const uint32_t count = lc->n_sets, W = (1u << (k - 1)) - 1u, P = 2u * W;
     const uint32_t per_set = (W + share - 1u) / share;
     const unsigned long long items = (unsigned long long)count * per_set;
@@ -1391,12 +1393,12 @@ __global__ void __launch_bounds__(kBlock, 3) k_dense(const uint32_t *__restrict_
         const uint32_t lo = part * share, hi = min(W, lo + share), per = (hi - lo + 31u) / 32u;
         uint32_t hh = min(hi, lo + per * lane);
         const uint32_t end = min(hi, hh + per);
-        uint32_t inside[4 * NW], odd[4 * NW];
-        pairs_inside<NW>(d, S, inside);
+        const int classes = pairs_table<NW>(d, S, lane, tab);
+        uint32_t odd[4 * NW];
 #pragma unroll
         for (int w = 0; w < 4 * NW; w++) odd[w] = 0u;
         uint32_t L = hh < end ? pdep32(hh + 1u, S) : 0u;
-        pairs_flip<NW>(d, L, odd);
+        pairs_flip<NW>(tab, L, odd);
         unsigned long long key = ~0ull;
         uint32_t first = kFull;
         bool first_nan = false;
@@ -1406,7 +1408,7 @@ __global__ void __launch_bounds__(kBlock, 3) k_dense(const uint32_t *__restrict_
             if (is_connected(L, adj) && is_connected(S ^ L, adj)) {
                 const float4 l = __ldcg(memo + L), r = __ldcg(memo + (S ^ L));
                 JoinCost lr, rl;
-                pairs_mirror<NW>(d, pp, odd, inside, l, r, lr, rl);
+                pairs_mirror<NW>(d, pp, tab, classes, odd, l, r, lr, rl);
                 width = (int)((__float_as_uint(l.w) & kWidthMask) + (__float_as_uint(r.w) & kWidthMask));
                 found += 2u;
                 // the lane's first valid candidate is its first valid split as
@@ -1429,7 +1431,7 @@ __global__ void __launch_bounds__(kBlock, 3) k_dense(const uint32_t *__restrict_
                 }
             }
             const uint32_t next = next_subset(L, S);
-            pairs_flip<NW>(d, L ^ next, odd);
+            pairs_flip<NW>(tab, L ^ next, odd);
             L = next;
         }
         __syncwarp();
