@@ -910,13 +910,6 @@ __device__ __forceinline__ void plain_mirror(const PlainParams &c, const PlainQu
     plain_join(c, e, sel_r, r, l, dr, dl, nl_startup, nl_tuples, lb, rp, lp, rl);
 }
 
-// pext: the bits of x at the positions of mask, packed (x within mask)
-__device__ __forceinline__ uint32_t pext32(uint32_t x, uint32_t mask) {
-    uint32_t r = 0u;
-    for (; x; x &= x - 1u) r |= 1u << __popc(mask & ((x & (0u - x)) - 1u));
-    return r;
-}
-
 // One set's classes with both members in it (two members each), numbered in
 // class order without gaps: their selectivities and, per relation of the set,
 // the classes it is in.  A class has exactly one member in L when it is in an
@@ -925,48 +918,33 @@ __device__ __forceinline__ uint32_t pext32(uint32_t x, uint32_t mask) {
 // relations that change sides.
 template <int NW>
 struct PairTable {
-    float4 sel[32 * NW];
+    float4 sel[32 * NW + 2];   // two more, read ahead and not used
     uint4 row[kMaxRels][NW];
 };
 
-// by one warp; the number of classes inside S
+// by one warp, a class per lane; the number of classes inside S
 template <int NW>
 __device__ __forceinline__ int pairs_table(const DevInfoView &d, uint32_t S, uint32_t lane, PairTable<NW> &t) {
-    uint32_t odd[4 * NW], inside[4 * NW];
-#pragma unroll
-    for (int w = 0; w < 4 * NW; w++) inside[w] = odd[w] = 0u;
-    for (uint32_t x = S; x; x &= x - 1u) {
-        const uint4 *row = reinterpret_cast<const uint4 *>(d.rel_ecs + lowest_idx(x) * (4 * NW));
-#pragma unroll
-        for (int j = 0; j < NW; j++) {
-            const uint4 a = row[j];
-            const uint32_t r[4] = {a.x, a.y, a.z, a.w};
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-                inside[4 * j + q] |= odd[4 * j + q] & r[q];
-                odd[4 * j + q] ^= r[q];
-            }
-        }
-    }
     __syncwarp();   // readers of the previous set's table
-    const bool member = (S >> lane) & 1u;
-    uint32_t *row = reinterpret_cast<uint32_t *>(t.row[lane]);
-    if (member)
+    if ((S >> lane) & 1u)
 #pragma unroll
-        for (int w = 0; w < 4 * NW; w++) row[w] = 0u;
-    float *sel = reinterpret_cast<float *>(t.sel);
+        for (int j = 0; j < NW; j++) t.row[lane][j] = make_uint4(0u, 0u, 0u, 0u);
+    __syncwarp();
+    const int n_ec = d.h->n_ec;
     int base = 0;
-#pragma unroll
-    for (int w = 0; w < 4 * NW; w++) {
-        if ((inside[w] >> lane) & 1u) sel[base + popc(inside[w] & ((1u << lane) - 1u))] = d.pair_sel[64 * w + 2 * lane];
-        if (member) {
-            const uint32_t x = pext32(d.rel_ecs[lane * (4 * NW) + w] & inside[w], inside[w]);
-            const int at = base >> 5, sh = base & 31;
-            if (x) row[at] |= x << sh;
-            const uint32_t rest = sh ? x >> (32 - sh) : 0u;
-            if (rest) row[at + 1] |= rest;
+    for (int e0 = 0; e0 < n_ec; e0 += 32) {
+        const int e = e0 + (int)lane;
+        const uint32_t m = e < n_ec ? d.ec_relids[e] : 0xFFFFFFFFu;
+        const bool in = (m & ~S) == 0u;
+        const uint32_t ins = __ballot_sync(0xFFFFFFFFu, in);
+        if (in) {
+            const int at = base + popc(ins & ((1u << lane) - 1u));
+            reinterpret_cast<float *>(t.sel)[at] = d.pair_sel[2 * e];
+            const uint32_t bit = 1u << (at & 31);
+            atomicOr(reinterpret_cast<uint32_t *>(t.row[lowest_idx(m)]) + (at >> 5), bit);
+            atomicOr(reinterpret_cast<uint32_t *>(t.row[31 - __clz((int)m)]) + (at >> 5), bit);
         }
-        base += popc(inside[w]);
+        base += popc(ins);
     }
     __syncwarp();
     return base;
@@ -1000,6 +978,7 @@ __device__ __forceinline__ void pairs_mirror(const DevInfoView &d, const PlainPa
                                              const float4 r, JoinCost &lr, JoinCost &rl) {
     float sel = 1.0f;
     int quals = 0;
+    float4 a = t.sel[0], b = t.sel[1];
 #pragma unroll
     for (int w = 0; w < 4 * NW; w++) {
         if (32 * w >= classes) break;
@@ -1008,15 +987,18 @@ __device__ __forceinline__ void pairs_mirror(const DevInfoView &d, const PlainPa
 #pragma unroll
         for (int g = 0; g < 4; g++) {
             if (32 * w + 8 * g >= classes) break;
-#pragma unroll
-            for (int j = 0; j < 2; j++) {
-                const float4 s = t.sel[8 * w + 2 * g + j];
-                const uint32_t bit = 1u << (8 * g + 4 * j);
-                if (m & bit) sel *= s.x;
-                if (m & (bit << 1)) sel *= s.y;
-                if (m & (bit << 2)) sel *= s.z;
-                if (m & (bit << 3)) sel *= s.w;
-            }
+            const float4 next_a = t.sel[8 * w + 2 * g + 2], next_b = t.sel[8 * w + 2 * g + 3];
+            const uint32_t bit = 1u << (8 * g);
+            if (m & bit) sel *= a.x;
+            if (m & (bit << 1)) sel *= a.y;
+            if (m & (bit << 2)) sel *= a.z;
+            if (m & (bit << 3)) sel *= a.w;
+            if (m & (bit << 4)) sel *= b.x;
+            if (m & (bit << 5)) sel *= b.y;
+            if (m & (bit << 6)) sel *= b.z;
+            if (m & (bit << 7)) sel *= b.w;
+            a = next_a;
+            b = next_b;
         }
     }
     const PlainQuals q = reinterpret_cast<const PlainQuals *>(reinterpret_cast<const uint32_t *>(d.h) + d.h->pairs_plain)[quals];
@@ -1064,6 +1046,13 @@ struct Blocks {
     uint32_t prefix[kMaxRels + 1];
     uint32_t eprefix[kMaxRels + 1];
 };
+
+// pext: the bits of x at the positions of mask, packed (x within mask)
+__device__ __forceinline__ uint32_t pext32(uint32_t x, uint32_t mask) {
+    uint32_t r = 0u;
+    for (; x; x &= x - 1u) r |= 1u << __popc(mask & ((x & (0u - x)) - 1u));
+    return r;
+}
 
 __device__ __forceinline__ void find_blocks(uint32_t S, const uint32_t *adj, Blocks &B) {
     uint8_t disc[kMaxRels], low[kMaxRels], parent[kMaxRels];

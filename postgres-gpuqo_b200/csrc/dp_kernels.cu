@@ -1345,17 +1345,22 @@ __global__ void __launch_bounds__(kBlock) k_ovf_finalize(const uint32_t *__restr
 // ---------------------------------------------------------------------------
 // k_dense: plain DPsub over all subsets of dense graphs with plain classes
 // (DevHeader::pairs_plain; a clique of 18 relations has 193 M unordered splits,
-// every one valid).  A lane takes a contiguous slice of a set's splits
-// L = pdep(h + 1, S), h = lo .. hi - 1, and its mirror P - 1 - h, and carries the
-// matching classes from split to split (pairs_flip: two relations change sides
-// on average) instead of gathering the class rows of all relations; nearly
-// every split is valid, so none is queued.
-// Bound: issue, most of it the selectivity product in class order (about 33
-// classes a split on the clique).  share: splits per warp; a set of at most
-// that many is one warp's and written at once, otherwise the shares fold
-// their keys (as k_ovf_chunks does) and k_dense_finalize writes the winners.
+// every one valid).  The splits L = pdep(v, S), v = 1 .. 2^(k-1) - 1, and their
+// mirrors 2^k - 1 - v are a set's candidates; a lane takes an aligned slice of
+// them, so that the same relations change sides in all lanes at the same time,
+// and carries the matching classes from split to split (pairs_flip: two
+// relations change sides on average) instead of gathering the class rows of
+// all relations; nearly every split is valid, so none is queued.
+// Bound: issue (54 to 67 % of the slots), 390 to 460 instructions a split, 160 of
+// them the selectivity product in class order over the 66 classes of a set of 12
+// relations of the clique.  The 18-relation clique takes 3.7 ms; with the class
+// rows as they are and a search for each lane's matching classes it took 8.1,
+// and with 4 blocks an SM (64 registers, some spilled) 3.9.  share: values of v per warp, a power
+// of two; a set of at most that many is one warp's and written at once,
+// otherwise the shares fold their keys (as k_ovf_chunks does) and the warp of a
+// set's last share writes the winner.
 // ---------------------------------------------------------------------------
-constexpr uint32_t kDenseWhole = 1023u;   // splits of an 11-relation set
+constexpr uint32_t kDenseWhole = 1024u;   // an 11-relation set
 
 // plain DPsub keeps the all-subsets enumeration on graphs with at least half
 // of all possible edges (apply_dpsub_csg); sparse ones only come here with
@@ -1372,6 +1377,7 @@ __global__ void __launch_bounds__(kBlock, 3) k_dense(const uint32_t *__restrict_
                                                      float4 *__restrict__ memo, uint32_t *__restrict__ memo_left,
                                                      unsigned long long *__restrict__ keys,
                                                      unsigned long long *__restrict__ firsts,
+                                                     uint32_t *__restrict__ parts,
                                                      GlobalCounters *__restrict__ glob, uint32_t share) {
     extern __shared__ __align__(16) uint32_t sm[];
     __shared__ PairTable<NW> tabs[kWarpsPerBlock];
@@ -1382,31 +1388,40 @@ __global__ void __launch_bounds__(kBlock, 3) k_dense(const uint32_t *__restrict_
     const PlainParams pp = plain_params(h);
     const uint32_t lane = threadIdx.x & 31u;
     PairTable<NW> &tab = tabs[threadIdx.x >> 5];
-    const uint32_t count = lc->n_sets, W = (1u << (k - 1)) - 1u, P = 2u * W;
-    const uint32_t per_set = (W + share - 1u) / share;
+    const uint32_t count = lc->n_sets, V = 1u << (k - 1), P = 2u * V - 2u;
+    const uint32_t per_set = V / share, per = (share + 31u) / 32u;
     const unsigned long long items = (unsigned long long)count * per_set;
     uint32_t found = 0u;
     for (unsigned long long item = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5); item < items;
          item += gridDim.x * kWarpsPerBlock) {
         const uint32_t idx = (uint32_t)(item / per_set), part = (uint32_t)(item % per_set);
         const uint32_t S = sets[idx];
-        const uint32_t lo = part * share, hi = min(W, lo + share), per = (hi - lo + 31u) / 32u;
-        uint32_t hh = min(hi, lo + per * lane);
-        const uint32_t end = min(hi, hh + per);
         const int classes = pairs_table<NW>(d, S, lane, tab);
         uint32_t odd[4 * NW];
 #pragma unroll
         for (int w = 0; w < 4 * NW; w++) odd[w] = 0u;
-        uint32_t L = hh < end ? pdep32(hh + 1u, S) : 0u;
+        uint32_t v = part * share + per * lane;
+        const uint32_t end = per * lane < share ? v + per : v;
+        uint32_t L = v < end ? pdep32(v, S) : 0u;
         pairs_flip<NW>(tab, L, odd);
-        unsigned long long key = ~0ull;
+        // all relations of S joined pairwise: every split is valid
+        const bool whole_clique = __all_sync(kFull, !((S >> lane) & 1u) || (adj[lane] & S) == (S ^ (1u << lane)));
+        // The first minimum in the order of the candidates: splits come in that
+        // order, mirrors in reverse and after every split, so that a cost equal
+        // to a mirror's takes its place and one equal to a split's does not.
+        float best = INFINITY, rows = 0.0f, startup = 0.0f;
+        uint32_t best_v = 0u;
+        bool of_mirror = true;
         uint32_t first = kFull;
         bool first_nan = false;
-        float rows = 0.0f, startup = 0.0f;
         int width = 0;
-        for (; hh < end; hh++) {
-            if (is_connected(L, adj) && is_connected(S ^ L, adj)) {
-                const float4 l = __ldcg(memo + L), r = __ldcg(memo + (S ^ L));
+        float4 l = __ldcg(memo + L), r = __ldcg(memo + (S ^ L));
+        for (; v < end; v++) {
+            // the next split's entries are on their way while this one is
+            // costed (whatever they hold, if it is not valid)
+            const uint32_t next = next_subset(L, S);
+            const float4 l_next = __ldcg(memo + next), r_next = __ldcg(memo + (S ^ next));
+            if (whole_clique ? L != 0u : (is_connected(L, adj) && is_connected(S ^ L, adj))) {
                 JoinCost lr, rl;
                 pairs_mirror<NW>(d, pp, tab, classes, odd, l, r, lr, rl);
                 width = (int)((__float_as_uint(l.w) & kWidthMask) + (__float_as_uint(r.w) & kWidthMask));
@@ -1414,80 +1429,86 @@ __global__ void __launch_bounds__(kBlock, 3) k_dense(const uint32_t *__restrict_
                 // the lane's first valid candidate is its first valid split as
                 // it stands: mirrors come after every split
                 if (first == kFull) {
-                    first = hh;
+                    first = v - 1u;
                     first_nan = isnan(lr.total);
                 }
-                const unsigned long long k0 = ((unsigned long long)ord_float(lr.total) << 32) | hh;
-                if (k0 < key && !isnan(lr.total)) {
-                    key = k0;
+                if (of_mirror ? lr.total <= best : lr.total < best) {
+                    best = lr.total;
                     rows = lr.rows;
                     startup = lr.startup;
+                    best_v = v;
+                    of_mirror = false;
                 }
-                const unsigned long long k1 = ((unsigned long long)ord_float(rl.total) << 32) | (P - 1u - hh);
-                if (k1 < key && !isnan(rl.total)) {
-                    key = k1;
+                if (of_mirror ? rl.total <= best : rl.total < best) {
+                    best = rl.total;
                     rows = rl.rows;
                     startup = rl.startup;
+                    best_v = v;
+                    of_mirror = true;
                 }
             }
-            const uint32_t next = next_subset(L, S);
             pairs_flip<NW>(tab, L ^ next, odd);
             L = next;
+            l = l_next;
+            r = r_next;
         }
         __syncwarp();
-        const uint32_t kh = (uint32_t)(key >> 32), kl = (uint32_t)key;
+        const uint32_t kh = best_v ? ord_float(best) : kFull;
+        const uint32_t kl = best_v ? (of_mirror ? P - best_v : best_v - 1u) : kFull;
         const uint32_t mh = __reduce_min_sync(kFull, kh);
         const uint32_t ml = __reduce_min_sync(kFull, kh == mh ? kl : kFull);
         const uint32_t mf = __reduce_min_sync(kFull, first);
         const bool nan = __any_sync(kFull, first == mf && first_nan);
-        const unsigned long long mk = ((unsigned long long)mh << 32) | ml;
+        unsigned long long win = nan ? mf : ml;
         if (per_set > 1u) {
+            uint32_t last = 0u;
             if (lane == 0u) {
+                const unsigned long long mk = ((unsigned long long)mh << 32) | ml;
                 if (mk != ~0ull) atomicMin(keys + idx, mk);
                 atomicMin(firsts + idx, ((unsigned long long)mf << 1) | (nan ? 1ull : 0ull));
+                __threadfence();
+                if (atomicAdd(parts + idx, 1u) == per_set - 1u) {
+                    __threadfence();
+                    const unsigned long long f = __ldcg(firsts + idx);
+                    win = (f & 1ull) ? f >> 1 : __ldcg(keys + idx) & 0xFFFFFFFFull;
+                    last = 1u;
+                    keys[idx] = firsts[idx] = ~0ull;   // as the next level expects them
+                    parts[idx] = 0u;
+                }
+            }
+            if (!__shfl_sync(kFull, last, 0)) continue;
+            win = __shfl_sync(kFull, win, 0);
+        } else if (!nan) {
+            if (kh == mh && kl == ml && best_v != 0u) {
+                RelVal out;
+                out.rows = rows;
+                out.startup = startup;
+                out.total = best;
+                out.width = width;
+                memo_write(h, memo, memo_left, S, out, pdep32(ml + 1u, S));
             }
             continue;
         }
-        if (nan) {
-            if (first == mf && first_nan) {
-                const uint32_t nl = pdep32(mf + 1u, S);
-                const RelVal l = load_rel(memo, nl, h.hz_packed), r = load_rel(memo, S ^ nl, h.hz_packed);
-                memo_write(h, memo, memo_left, S, join_eval(d, nl, l, S ^ nl, r), nl);
-            }
-        } else if (key == mk && key != ~0ull) {
+        // the winning candidate of shares, or a NaN found first, once more
+        L = pdep32((uint32_t)win + 1u, S);
+#pragma unroll
+        for (int w = 0; w < 4 * NW; w++) odd[w] = 0u;
+        pairs_flip<NW>(tab, L, odd);
+        l = __ldcg(memo + L);
+        r = __ldcg(memo + (S ^ L));
+        JoinCost lr, rl;
+        pairs_mirror<NW>(d, pp, tab, classes, odd, l, r, lr, rl);
+        if (lane == 0u) {
             RelVal out;
-            out.rows = rows;
-            out.startup = startup;
-            out.total = __uint_as_float((kh & 0x80000000u) ? kh ^ 0x80000000u : ~kh);   // the inverse of ord_float
-            out.width = width;
-            memo_write(h, memo, memo_left, S, out, pdep32(kl + 1u, S));
+            out.rows = lr.rows;
+            out.startup = lr.startup;
+            out.total = lr.total;
+            out.width = (int)((__float_as_uint(l.w) & kWidthMask) + (__float_as_uint(r.w) & kWidthMask));
+            memo_write(h, memo, memo_left, S, out, L);
         }
     }
     found = __reduce_add_sync(kFull, found);
     if (lane == 0u && found) atomicAdd(&glob->evaluated_pairs, (unsigned long long)found);
-}
-
-// winners of the sets that k_dense took in shares; leaves the keys at all ones
-// for the next level
-__global__ void __launch_bounds__(kBlock) k_dense_finalize(const uint32_t *__restrict__ blob, uint32_t blob_words,
-                                                           const uint32_t *__restrict__ sets,
-                                                           const LevelCounters *__restrict__ lc, float4 *__restrict__ memo,
-                                                           uint32_t *__restrict__ memo_left,
-                                                           unsigned long long *__restrict__ keys,
-                                                           unsigned long long *__restrict__ firsts) {
-    const uint32_t count = lc->n_sets;
-    extern __shared__ __align__(16) uint32_t sm[];
-    load_blob_to_smem(blob, blob_words, sm);
-    const DevInfoView d = make_view(sm);
-    for (uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x; idx < count; idx += gridDim.x * blockDim.x) {
-        const uint32_t S = sets[idx];
-        const unsigned long long first = firsts[idx];
-        const uint32_t p = (first & 1ull) ? (uint32_t)(first >> 1) : (uint32_t)keys[idx];
-        const uint32_t L = pdep32(p + 1u, S);
-        const RelVal l = load_rel(memo, L, d.h->hz_packed), r = load_rel(memo, S ^ L, d.h->hz_packed);
-        memo_write(*d.h, memo, memo_left, S, join_eval(d, L, l, S ^ L, r), L);
-        keys[idx] = firsts[idx] = ~0ull;
-    }
 }
 
 // ---------------------------------------------------------------------------
@@ -2134,7 +2155,8 @@ public:
         const int nw = ec_stride(reinterpret_cast<const DevHeader *>(h_blob)->n_ec) / 4;
         CK(cudaMemsetAsync(d_ctl, 0, kCtlClearBytes, stream));
         CK(cudaMemsetAsync(a.seen, 0, std::max<uint64_t>((1ull << n) / 8, 4), stream));
-        if (mode == kModeDpsub && dense) {   // no winner yet (k_dense_finalize leaves them so)
+        if (mode == kModeDpsub && dense) {   // no winner and no share yet (k_dense leaves them so)
+            CK(cudaMemsetAsync(a.ovf_off, 0, max_level_sets(n) * sizeof(uint32_t), stream));
             CK(cudaMemsetAsync(a.ovf_key, 0xFF, max_level_sets(n) * sizeof(unsigned long long), stream));
             CK(cudaMemsetAsync(a.ovf_first, 0xFF, max_level_sets(n) * sizeof(unsigned long long), stream));
         }
@@ -2156,20 +2178,20 @@ public:
             n_kernels += 2;
             int eblocks = (int)std::min<uint64_t>((uint64_t)eval_max_blocks, (total + kWarpsPerBlock - 1) / kWarpsPerBlock);
             CK(cudaEventRecordWithFlags(kev[2 * k], stream, cudaEventRecordExternal));
-            const uint32_t W = (uint32_t)((1ull << (k - 1)) - 1ull);   // unordered splits of a k-set
             if (mode == kModeDpsub && dense) {
                 // whole sets per warp while a level has enough of them, shares
-                // of a set otherwise
-                const uint64_t shares = (total * W) / ((uint64_t)sm_count * 3 * kWarpsPerBlock * 4);
-                uint32_t share = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(shares, 512u), 4096u);
-                const bool whole = W <= std::max(share, kDenseWhole);
-                if (whole) share = W;
-                n_kernels += whole ? 0 : 1;
+                // of a set otherwise: four for every warp, as long as the set's
+                // table (150 instructions) is little against its splits (450 for
+                // 32), and smaller ones only where warps would have none
+                const uint32_t V = 1u << (k - 1);
+                const uint64_t warps = (uint64_t)sm_count * 3 * kWarpsPerBlock;
+                uint32_t share = 512u;
+                while (share > 128u && total * V < share * warps) share /= 2u;
+                while (share < 4096u && total * V >= 2u * share * 4u * warps) share *= 2u;
+                const bool whole = V <= std::max(share, kDenseWhole);
+                if (whole) share = V;
                 (nw == 1 ? k_dense<1> : k_dense<2>)<<<sm_count * 3, kBlock, (size_t)((blob_words + 3u) & ~3u) * 4u, stream>>>(
-                    a.blob, blob_words, k, cur_sets, lc, a.memo, a.memo_left, a.ovf_key, a.ovf_first, a.glob, share);
-                if (!whole)
-                    k_dense_finalize<<<sm_count, kBlock, (size_t)((blob_words + 3u) & ~3u) * 4u, stream>>>(
-                        a.blob, blob_words, cur_sets, lc, a.memo, a.memo_left, a.ovf_key, a.ovf_first);
+                    a.blob, blob_words, k, cur_sets, lc, a.memo, a.memo_left, a.ovf_key, a.ovf_first, a.ovf_off, a.glob, share);
             } else if (mode == kModeDpsub) {
                 k_eval<kModeDpsub><<<eblocks, kBlock, smem, stream>>>(a.blob, blob_words, k, cur_sets, lc, a.memo,
                                                                       a.memo_left, a.ovf_set, a.ovf_P, a.ovf_off,
@@ -2361,7 +2383,6 @@ public:
             CK(cudaFuncSetAttribute(k_eval<kModeMpdp>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
             CK(cudaFuncSetAttribute(k_dense<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
             CK(cudaFuncSetAttribute(k_dense<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-            CK(cudaFuncSetAttribute(k_dense_finalize, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
             CK(cudaFuncSetAttribute(k_ovf_chunks<kModeDpsub>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
             CK(cudaFuncSetAttribute(k_ovf_chunks<kModeMpdp>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
             CK(cudaFuncSetAttribute(k_ovf_finalize<kModeDpsub>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
