@@ -794,31 +794,41 @@ __device__ __forceinline__ void tree_order(const TreeRows &t, uint32_t S, uint32
 // row counts of the larger side alone, so the order of several joins does not
 // matter), hence the place is at hand and not computed on demand.
 struct TreeBest {
-    unsigned long long key;
+    float total;
+    uint32_t p;            // place, kFull: none yet
     uint32_t left;
     float rows, startup;
     uint32_t nan_p;        // lowest place of a candidate with a NaN cost, kFull: none
 
     __device__ __forceinline__ void init() {
-        key = ~0ull;
+        total = INFINITY;
+        p = kFull;
         left = 0u;
         rows = startup = 0.0f;
         nan_p = kFull;
     }
 };
 
+// a NaN compares false and leaves the best as it is
 __device__ __forceinline__ void tree_update(TreeBest &best, uint32_t p, uint32_t L, float rows, float startup,
                                             float total) {
-    if (__builtin_expect(isnan(total), 0)) {
-        best.nan_p = min(best.nan_p, p);
-        return;
-    }
-    const unsigned long long key = ((unsigned long long)ord_float(total) << 32) | p;
-    if (key < best.key) {
-        best.key = key;
+    if (total < best.total || (total == best.total && p < best.p)) {
+        best.total = total;
+        best.p = p;
         best.left = L;
         best.rows = rows;
         best.startup = startup;
+    }
+}
+
+__device__ __forceinline__ void tree_update_mirror(TreeBest &best, uint32_t S, uint32_t L0, uint32_t p0, uint32_t p1,
+                                                   float rows0, float startup0, float total0, float rows1,
+                                                   float startup1, float total1) {
+    tree_update(best, p0, L0, rows0, startup0, total0);
+    tree_update(best, p1, S ^ L0, rows1, startup1, total1);
+    if (__builtin_expect(isnan(total0) || isnan(total1), 0)) {
+        if (isnan(total0)) best.nan_p = min(best.nan_p, p0);
+        if (isnan(total1)) best.nan_p = min(best.nan_p, p1);
     }
 }
 
@@ -834,8 +844,7 @@ __device__ __forceinline__ void tree_cost(const DevInfoView &d, const PlainParam
         JoinCost lr, rl;
         plain_mirror(pp, e.quals, e.sel_lo, e.sel_hi, lv, rv, lr, rl);
         width = (int)((__float_as_uint(lv.w) & kWidthMask) + (__float_as_uint(rv.w) & kWidthMask));
-        tree_update(best, p0, L0, lr.rows, lr.startup, lr.total);
-        tree_update(best, p1, S ^ L0, rl.rows, rl.startup, rl.total);
+        tree_update_mirror(best, S, L0, p0, p1, lr.rows, lr.startup, lr.total, rl.rows, rl.startup, rl.total);
     } else {
         const RelVal l = unpack_rel(lv, h.hz_packed), r = unpack_rel(rv, h.hz_packed);
         RelVal o0, o1;
@@ -843,8 +852,7 @@ __device__ __forceinline__ void tree_cost(const DevInfoView &d, const PlainParam
             LAYOUT == kTreeMasked ? reinterpret_cast<const TreeEdge *>(t.tab + tree_edge_off(t.n))[edge].classes : 0u;
         join_eval_mirror_tree<LAYOUT == kTreeMasked>(d, L0, l, S ^ L0, r, classes, o0, o1);
         width = o0.width;
-        tree_update(best, p0, L0, o0.rows, o0.startup, o0.total);
-        tree_update(best, p1, S ^ L0, o1.rows, o1.startup, o1.total);
+        tree_update_mirror(best, S, L0, p0, p1, o0.rows, o0.startup, o0.total, o1.rows, o1.startup, o1.total);
     }
 }
 
@@ -930,7 +938,8 @@ __device__ __forceinline__ void tree_set(const DevInfoView &d, const PlainParams
         }
         if (cact) tree_cost<LAYOUT>(d, pp, t, S, cL, c0, c1, ce, clv, crv, best, width);
     }
-    uint32_t mh = (uint32_t)(best.key >> 32), ml = (uint32_t)best.key;
+    uint32_t mh = best.p == kFull ? kFull : ord_float(best.total), ml = best.p;
+    const uint32_t own = mh;
     if (G == 32) {
         const uint32_t w = __reduce_min_sync(kFull, mh);
         ml = __reduce_min_sync(kFull, mh == w ? ml : kFull);
@@ -944,7 +953,7 @@ __device__ __forceinline__ void tree_set(const DevInfoView &d, const PlainParams
             }
         }
     }
-    bool win = has && best.key == (((unsigned long long)mh << 32) | ml) && best.key != ~0ull;
+    bool win = has && best.p != kFull && own == mh && best.p == ml;
     if (__any_sync(kFull, best.nan_p != kFull)) {
         RelVal out;
         uint32_t left = 0u;
@@ -953,11 +962,9 @@ __device__ __forceinline__ void tree_set(const DevInfoView &d, const PlainParams
         if (writer) memo_write(h, memo, memo_left, S, out, left);
     }
     if (win) {
-        // the inverse of ord_float (a total is never -0: its startup cost starts from +0)
-        const float total = __uint_as_float((mh & 0x80000000u) ? mh ^ 0x80000000u : ~mh);
         const uint32_t word = LAYOUT == kTreePlain ? plain_width_word(h, best.rows, width)
                                                    : memo_width_word(h, best.rows, width);
-        memo[S] = make_float4(best.rows, best.startup, total, __uint_as_float(word));
+        memo[S] = make_float4(best.rows, best.startup, best.total, __uint_as_float(word));
         memo_left[S] = best.left;
     }
 }
