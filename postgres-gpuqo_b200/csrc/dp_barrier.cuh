@@ -36,6 +36,9 @@ __device__ __forceinline__ unsigned long long global_ns() {
 // same SM.  The verdict is the same for every thread of the block (thread 0
 // decides); blocks may disagree only after a timeout, and then every later
 // barrier sees the error flag and returns false at once, so all blocks leave.
+// A poll is one round trip to L2 (some 700 cycles); the error flag comes with
+// it, because a second trip for the flag after the count, and a third for the
+// verdict, would lengthen every level by half a microsecond.
 // epoch: the caller's count of barriers passed (thread 0); max_polls: polls
 // before the wait gives up (barrier_polls).
 template <bool ACQUIRE_POLL>
@@ -45,27 +48,30 @@ __device__ __forceinline__ bool grid_barrier(unsigned *bar, unsigned &epoch, uns
     if (threadIdx.x == 0) {
         epoch++;
         const unsigned target = base + epoch * gridDim.x;
-        volatile unsigned *verr = bar + 2;
         asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
         const unsigned long long t0 = global_ns();
-        unsigned spins = 0;
+        unsigned spins = 0, failed;
         for (;;) {
+            // error flag and count in flight together
             unsigned c;
+            asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(failed) : "l"(bar + 2) : "memory");
             if (ACQUIRE_POLL) {
                 asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(c) : "l"(bar) : "memory");
             } else {
                 asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(c) : "l"(bar) : "memory");
             }
-            if (c >= target || *verr != 0u) {
+            if (c >= target || failed != 0u) {
                 if (!ACQUIRE_POLL) __threadfence();
                 break;
             }
-            if (++spins >= max_polls || global_ns() - t0 > kBarrierTimeoutNs) {
+            ++spins;
+            if (spins >= max_polls || ((spins & 63u) == 0u && global_ns() - t0 > kBarrierTimeoutNs)) {
                 atomicExch(bar + 2, 1u);
+                failed = 1u;
                 break;
             }
         }
-        s_ok = (*verr == 0u) ? 1u : 0u;
+        s_ok = failed == 0u ? 1u : 0u;
     }
     __syncthreads();
     return s_ok != 0u;
