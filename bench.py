@@ -217,6 +217,12 @@ def cpu_model():
     return "unknown"
 
 
+def reference_built():
+    sys.path.insert(0, os.path.join(REPO, "oracle"))
+    import harness
+    return harness.ref_available()
+
+
 def cpu_reference_sample(queries, algorithm, steps=None, budget_s=20.0, min_runs=5, max_runs=40, native=False,
                          threads=None):
     """The reference's own CPU engine (oracle/_ref, or its -march=native
@@ -670,19 +676,23 @@ def main():
     # selectivities, 9 words per class member, then 16-byte aligned the
     # per-relation class masks (rows of whole 4-word groups), 2 pair
     # selectivities per class (rounded up to 4 words) and the plain-class
-    # mask, plus the 3 n^2 tree tables of a tree-shaped graph; staged in
-    # 512-word buckets); out, one copy of the engine's control block: 33 level
-    # counters (24 B), the pair counter, the barrier words, the tree size, 64
-    # plan nodes (28 B)
+    # mask, plus the tables of a tree-shaped graph: 32 words, 8 per relation
+    # and 4 n per relation that is ever the lowest of a connected set); out, the
+    # 2 n - 1 plan nodes (28 B) and their number
     q0 = qs[0]
     n_ec = len(q0.eq_classes)
     n_sels = sum(len(e.sels) for e in q0.eq_classes)
     n_fks = sum(len(e.members) for e in q0.eq_classes)
     ec_stride = (((n_ec + 31) // 32) + 3) // 4 * 4
     words = (343 + 2 * n_ec + n_sels + 9 * n_fks + 3) // 4 * 4
-    words += N_RELS * ec_stride + (2 * n_ec + 3) // 4 * 4 + ec_stride + 3 * N_RELS * N_RELS
-    h2d = 4 * ((words + 511) // 512 * 512)
-    d2h = 33 * 24 + 8 + 16 + 4 + 4 + 64 * 28
+    words += N_RELS * ec_stride + (2 * n_ec + 3) // 4 * 4 + ec_stride + 32 + 8 * N_RELS
+    degree = [0] * N_RELS
+    for e in q0.eq_classes:
+        for m in e.members:
+            degree[m] += 1
+    words += 4 * N_RELS * sum(1 for i, g in enumerate(degree) if i == 0 or g > 1)
+    h2d = 4 * words
+    d2h = (2 * N_RELS - 1) * 28 + 4
 
     if rank == 0:
         peak, peak_kind = measured_peaks()
@@ -715,13 +725,16 @@ def main():
             "gpu_launches": kernels,
             "clocks": clk.summary(),
         }
+        cpu_baseline = not args.no_cpu_baseline and reference_built()
         if world == 1 and not args.no_batched:
             line["batched"] = batched_section()
         if world == 1 and not args.no_served:
             line["served"] = served_section()
         if world == 1 and not args.no_configs:
-            line["configs"] = configs_section(cpu=not args.no_cpu_baseline)
-        if world == 1 and not args.no_cpu_baseline:
+            line["configs"] = configs_section(cpu=cpu_baseline)
+        if world == 1 and not args.no_cpu_baseline and not cpu_baseline:
+            line["cpu_baseline"] = {"skipped": "the reference's CPU engines are not built here"}
+        if world == 1 and cpu_baseline:
             med, mean, cores, ns = cpu_reference_sample(qs, capi.GPUQO_CPU_DPSUB_BICC_PARALLEL)
             line["cpu_baseline"] = {"value": med, "unit": "ms/query", "cores": cores, "kind": "reference",
                                     "mean": mean, "cpu_model": cpu_model(),

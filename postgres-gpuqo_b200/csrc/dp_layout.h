@@ -14,7 +14,6 @@
 namespace gqb {
 
 constexpr int kMaxRels = 32;      // compact masks are 32-bit
-constexpr int kWarp = 32;
 
 // ---------------------------------------------------------------------------
 // Device planner info blob (built on the host, copied into shared memory by
