@@ -1053,8 +1053,12 @@ __global__ void __launch_bounds__(kWideBlock, 2) k_wide_cactus(const unsigned ch
             for (uint32_t i = nwarps - 1u - gwarp; i < count; i += nwarps) {
                 const uint64_t S = __ldcg(sets + first + i);
                 // the arrays are outgrown: nothing more is entered (the table
-                // has twice their room and stays searchable)
-                if ((uint64_t)next + __ldcg(&ctl->level_n[k + 1u]) > total) break;
+                // has twice their room and stays searchable).  Other blocks add
+                // to the count meanwhile, and two lanes' loads may return two
+                // values: one lane reads it for the warp, which leaves together.
+                uint32_t listed = 0u;
+                if (lane == 0u) listed = __ldcg(&ctl->level_n[k + 1u]);
+                if ((uint64_t)next + __shfl_sync(kFullW, listed, 0) > total) break;
                 for (uint32_t half = 0; half < n; half += 32u) {
                     const uint32_t v = half + lane;
                     bool claimed = false;
