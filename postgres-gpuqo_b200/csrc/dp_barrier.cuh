@@ -78,7 +78,10 @@ __device__ __forceinline__ bool grid_barrier(unsigned *bar, unsigned &epoch, uns
 }
 
 // The barrier of a grid that is one thread-block cluster, in hardware (no
-// polling, nothing to time out): every thread of the cluster.
+// polling, nothing to time out): every thread of the cluster.  It follows
+// code in which single lanes write a set's winner or emit a list's entries, so
+// a warp may arrive in parts: the forms without .aligned, which every thread
+// executes for itself.
 __device__ __forceinline__ uint32_t cluster_blocks() {
     uint32_t n;
     asm volatile("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(n));
@@ -86,8 +89,8 @@ __device__ __forceinline__ uint32_t cluster_blocks() {
 }
 
 __device__ __forceinline__ void cluster_barrier() {
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
 }
 
 }  // namespace gqb
