@@ -1831,6 +1831,13 @@ uint64_t engine_bytes_needed(int n) {
 // gpuqo_b200_device_memory_mb: when > 0, a DP whose arena would need more
 // device memory than this is refused with GPUQO_B200_ERR_NOMEM before any
 // allocation (the engines keep what they hold, so later calls are unaffected)
+// A buffer's pointer is null from the moment it is freed, so that an
+// allocation that fails leaves nothing a later call could use or free again.
+template <class T> static void release(T *&p) {
+    if (p) cudaFree(p);
+    p = nullptr;
+}
+
 static int over_budget(uint64_t bytes, const char *what, std::string &err) {
     const int mb = gpuqo_b200_device_memory_mb;
     if (mb <= 0 || bytes <= ((uint64_t)mb << 20)) return 0;
@@ -1993,18 +2000,20 @@ public:
     bool barrier_timed_out = false;    // a grid barrier of k_dp_tree gave up: per-level launches until reset
     std::map<GraphKey, int> graph_kernels;
     float *flush = nullptr;            // L2 flush buffer (timing only)
+    bool ready = false;                // init has come to its end
 
     int init(std::string &err) {
-        if (stream) return 0;
+        if (ready) return 0;
         CK(cudaGetDevice(&device));
         CK(cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, device));
-        CK(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
-        CK(cudaEventCreate(&ev0));
-        CK(cudaEventCreate(&ev1));
+        if (!stream) CK(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
+        if (!ev0) CK(cudaEventCreate(&ev0));
+        if (!ev1) CK(cudaEventCreate(&ev1));
         kev.resize(2 * 34);
-        for (auto &e : kev) CK(cudaEventCreate(&e));
-        CK(cudaMalloc(&d_ctl, sizeof(EngineCtl)));
-        CK(cudaMallocHost(&h_ctl, sizeof(EngineCtl)));
+        for (auto &e : kev)
+            if (!e) CK(cudaEventCreate(&e));
+        if (!d_ctl) CK(cudaMalloc(&d_ctl, sizeof(EngineCtl)));
+        if (!h_ctl) CK(cudaMallocHost(&h_ctl, sizeof(EngineCtl)));
         a.lvl = d_ctl->lvl;
         a.glob = &d_ctl->glob;
         a.bar = d_ctl->bar;
@@ -2014,7 +2023,7 @@ public:
         h_glob = &h_ctl->glob;
         h_tree_n = &h_ctl->tree_n;
         h_tree = h_ctl->tree;
-        CK(cudaMalloc(&a.binom, 33 * 33 * sizeof(uint32_t)));
+        if (!a.binom) CK(cudaMalloc(&a.binom, 33 * 33 * sizeof(uint32_t)));
         std::vector<uint32_t> bt(33 * 33, 0);
         for (int i = 0; i <= 32; i++)
             for (int j = 0; j <= 32; j++) {
@@ -2022,6 +2031,7 @@ public:
                 bt[i * 33 + j] = v > 0xFFFFFFFFull ? 0xFFFFFFFFu : (uint32_t)v;
             }
         CK(cudaMemcpy(a.binom, bt.data(), bt.size() * 4, cudaMemcpyHostToDevice));
+        ready = true;
         return 0;
     }
 
@@ -2033,8 +2043,10 @@ public:
     int ensure(int n, uint32_t blob_words, std::string &err) {
         if (blob_words > blob_cap_words) {
             drop_graphs();
-            if (a.blob) cudaFree(a.blob);
+            blob_cap_words = 0;
+            release(a.blob);
             if (h_blob) cudaFreeHost(h_blob);
+            h_blob = nullptr;
             uint32_t cap = std::max<uint32_t>((blob_words + 511u) & ~511u, 16384u);
             CK(cudaMalloc(&a.blob, cap * 4));
             CK(cudaMallocHost(&h_blob, cap * 4));
@@ -2044,18 +2056,17 @@ public:
         if (int rc = over_budget(engine_bytes_needed(n), "the exact DP's dense memo and level lists", err)) return rc;
         if (n <= cap_n) return 0;
         drop_graphs();
-        cudaFree(a.memo);
-        cudaFree(a.memo_left);
-        cudaFree(a.sets);
-        cudaFree(a.sets2);
-        cudaFree(a.seen);
-        cudaFree(a.ovf_set);
-        cudaFree(a.ovf_P);
-        cudaFree(a.ovf_off);
-        cudaFree(a.ovf_key);
-        cudaFree(a.ovf_first);
-        a.memo = nullptr;
         cap_n = -1;
+        release(a.memo);
+        release(a.memo_left);
+        release(a.sets);
+        release(a.sets2);
+        release(a.seen);
+        release(a.ovf_set);
+        release(a.ovf_P);
+        release(a.ovf_off);
+        release(a.ovf_key);
+        release(a.ovf_first);
         uint64_t slots = 1ull << n;
         uint64_t ms = max_level_sets(n);
         CK(cudaMalloc(&a.memo, slots * sizeof(float4)));
@@ -2083,14 +2094,12 @@ public:
             return rc;
         if (n <= dpsize_cap_n) return 0;
         drop_graphs();
-        cudaFree(a.pos);
-        cudaFree(a.bmask);
-        cudaFree(a.bstart);
-        cudaFree(a.tile_sum);
-        cudaFree(a.disc);
-        a.pos = a.bmask = a.bstart = a.tile_sum = nullptr;
-        a.disc = nullptr;
         dpsize_cap_n = -1;
+        release(a.pos);
+        release(a.bmask);
+        release(a.bstart);
+        release(a.tile_sum);
+        release(a.disc);
         CK(cudaMalloc(&a.pos, (1ull << n) * sizeof(uint32_t)));
         CK(cudaMalloc(&a.bmask, ms * sizeof(uint32_t)));
         CK(cudaMalloc(&a.bstart, ms * sizeof(uint32_t)));
@@ -3782,8 +3791,9 @@ struct BatchEngine {
     int device = -1, sm_count = 148;
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-    // arena (grown on demand)
-    uint64_t cap_slots = 0, cap_items = 0, cap_seen = 0;
+    // arena (grown on demand), each buffer with its own capacity: one that
+    // could not be allocated has none, whatever the others hold
+    uint64_t cap_memo = 0, cap_left = 0, cap_seen = 0, cap_listA = 0, cap_listB = 0;
     float4 *memo = nullptr;
     uint32_t *memo_left = nullptr, *blobs = nullptr, *seen = nullptr;
     unsigned long long *listA = nullptr, *listB = nullptr;
@@ -3802,12 +3812,13 @@ struct BatchEngine {
     std::map<size_t, int> coop_one;              // dynamic shared bytes -> co-resident blocks of kb_gen<true>
     bool barrier_timed_out = false;              // a grid barrier gave up: per-level launches until reset
     BatchOvf ovf{};                              // overflow list of kb_gen
-    uint64_t cap_ovf = 0;
+    uint64_t cap_ovf[6] = {};                    // of its arrays
     void *flush = nullptr;                       // L2 flush buffer (device-resident timing only)
     // pinned staging of a wave: planner infos and descriptors in, plans and
     // counters out (grown on demand; the copies are truly asynchronous)
     unsigned char *h_in = nullptr, *h_out = nullptr;
     size_t cap_h_in = 0, cap_h_out = 0;
+    bool ready = false;                          // init has come to its end
 
     static int grow_pinned(unsigned char *&p, size_t &cap, size_t bytes, std::string &err) {
         if (bytes <= cap) return 0;
@@ -3820,12 +3831,12 @@ struct BatchEngine {
     }
 
     int init(std::string &err) {
-        if (stream) return 0;
+        if (ready) return 0;
         CK(cudaGetDevice(&device));
         CK(cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, device));
-        CK(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
-        CK(cudaEventCreate(&ev0));
-        CK(cudaEventCreate(&ev1));
+        if (!stream) CK(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
+        if (!ev0) CK(cudaEventCreate(&ev0));
+        if (!ev1) CK(cudaEventCreate(&ev1));
         int dev_coop = 0, occ = 0, occ_tree[3] = {0, 0, 0};
         cudaDeviceGetAttribute(&dev_coop, cudaDevAttrCooperativeLaunch, device);
         no_cooperative();
@@ -3838,6 +3849,7 @@ struct BatchEngine {
             for (int i = 0; i < 3; i++) coop_grid_tree[i] = occ_tree[i] * sm_count;
         }
         cudaGetLastError();
+        ready = true;
         return 0;
     }
 
@@ -3935,10 +3947,9 @@ struct BatchEngine {
     // not fit
     template <class T> int grow(T *&p, uint64_t &cap, uint64_t need, std::string &err) {
         if (need <= cap) return 0;
-        if (p) cudaFree(p);
-        p = nullptr;
         const uint64_t want = std::max(need, 2 * cap);
         cap = 0;
+        release(p);
         if (want > need && cudaMalloc(&p, want * sizeof(T)) == cudaSuccess) {
             cap = want;
             return 0;
@@ -4022,26 +4033,17 @@ struct BatchEngine {
         if (int rc = over_budget(slots * (sizeof(float4) + 4) + words * 4 + seen_words * 4 + items * 16 + ovf_need * 32,
                                  "the batch wave's arena", err))
             return rc;
-        uint64_t c1 = cap_slots, c2 = cap_slots, c4 = cap_seen, c5 = cap_items, c6 = cap_items;
-        if (int rc = grow(memo, c1, slots, err)) return rc;
-        if (int rc = grow(memo_left, c2, slots, err)) return rc;
-        cap_slots = std::min(c1, c2);
-        if (int rc = grow(seen, c4, seen_words, err)) return rc;
-        cap_seen = c4;
-        if (int rc = grow(listA, c5, items, err)) return rc;
-        if (int rc = grow(listB, c6, items, err)) return rc;
-        cap_items = std::min(c5, c6);
-        if (ovf_need > cap_ovf) {
-            uint64_t a1 = cap_ovf, a2 = cap_ovf, a3 = cap_ovf, a4 = cap_ovf, a5 = cap_ovf;
-            uint64_t a6 = cap_ovf;
-            if (int rc = grow(ovf.item, a1, ovf_need, err)) return rc;
-            if (int rc = grow(ovf.W, a2, ovf_need, err)) return rc;
-            if (int rc = grow(ovf.off, a3, ovf_need, err)) return rc;
-            if (int rc = grow(ovf.key, a4, ovf_need, err)) return rc;
-            if (int rc = grow(ovf.nan_p, a5, ovf_need, err)) return rc;
-            if (int rc = grow(ovf.done, a6, ovf_need, err)) return rc;
-            cap_ovf = ovf_need;
-        }
+        if (int rc = grow(memo, cap_memo, slots, err)) return rc;
+        if (int rc = grow(memo_left, cap_left, slots, err)) return rc;
+        if (int rc = grow(seen, cap_seen, seen_words, err)) return rc;
+        if (int rc = grow(listA, cap_listA, items, err)) return rc;
+        if (int rc = grow(listB, cap_listB, items, err)) return rc;
+        if (int rc = grow(ovf.item, cap_ovf[0], ovf_need, err)) return rc;
+        if (int rc = grow(ovf.W, cap_ovf[1], ovf_need, err)) return rc;
+        if (int rc = grow(ovf.off, cap_ovf[2], ovf_need, err)) return rc;
+        if (int rc = grow(ovf.key, cap_ovf[3], ovf_need, err)) return rc;
+        if (int rc = grow(ovf.nan_p, cap_ovf[4], ovf_need, err)) return rc;
+        if (int rc = grow(ovf.done, cap_ovf[5], ovf_need, err)) return rc;
         ovf.cap = (uint32_t)ovf_need;
         // units of the overflow shares: small enough to spread a level evenly,
         // large enough that a level's units number below 2^32 (at most 2^22
