@@ -1058,32 +1058,38 @@ __global__ void __launch_bounds__(kBlock, 3) k_eval_tree(const uint32_t *__restr
 // m2 and any other neighbour must exceed m1 (a single relation: itself).  So
 // the extensions of S are one mask, counted and placed with one atomic per
 // warp; the loop over the relations of S costs about 10 instructions each.
-__device__ __forceinline__ uint32_t above(uint32_t bit) { return ~((bit << 1) - 1u); }
+// near: the same with T's smallest leaf (m1 < m2 the two smallest, v below
+// them), for memos beyond the caches (near_order).  The sets that one S emits,
+// and those of the S next to it in the list, then share their high relations,
+// so that the memo entries a warp reads and writes lie close together; by the
+// largest leaf they share the low ones, and with them mostly the row of the
+// tables that the warp reads (the row of a set's lowest relation).
 
 // the relations v of the neighbours N of S whose addition emits S + v
 template <class Adj>
-__device__ __forceinline__ uint32_t tree_extension_mask(uint32_t S, uint32_t N, uint32_t leaves, Adj adj) {
-    const uint32_t m1 = 1u << (31 - __clz(leaves));
-    const uint32_t rest = leaves ^ m1;
-    if (rest == 0u) return N & above(m1);                      // a single relation
-    const uint32_t m2 = 1u << (31 - __clz(rest)), a1 = adj(31 - __clz(m1));
-    return N & ((above(m1) & ~a1) | (above(m2) & a1));
+__device__ __forceinline__ uint32_t tree_extension_mask(uint32_t S, uint32_t N, uint32_t leaves, bool near, Adj adj) {
+    auto end = [&](uint32_t x) { return near ? lowest(x) : 1u << (31 - __clz(x)); };
+    auto beyond = [&](uint32_t bit) { return near ? bit - 1u : ~((bit << 1) - 1u); };
+    const uint32_t m1 = end(leaves), rest = leaves ^ m1;
+    if (rest == 0u) return N & beyond(m1);                     // a single relation
+    const uint32_t a1 = adj(lowest_idx(m1));
+    return N & ((beyond(m1) & ~a1) | (beyond(end(rest)) & a1));
 }
 
 // the same from S alone (adj(v): neighbours of v)
 template <class Adj>
-__device__ __forceinline__ uint32_t tree_extensions(uint32_t S, Adj adj) {
+__device__ __forceinline__ uint32_t tree_extensions(uint32_t S, bool near, Adj adj) {
     uint32_t N = 0u, leaves = 0u;
     for (uint32_t x = S; x; x &= x - 1u) {
         const uint32_t a = adj(lowest_idx(x)), in = a & S;
         N |= a;
         if ((in & (in - 1u)) == 0u) leaves |= x & (0u - x);   // S is connected: at least one neighbour in S
     }
-    return S ? tree_extension_mask(S, N & ~S, leaves, adj) : 0u;
+    return S ? tree_extension_mask(S, N & ~S, leaves, near, adj) : 0u;
 }
 
-__device__ __forceinline__ void tree_enum_phase(const uint32_t *adj, int k, const uint32_t *prev_sets, uint32_t c_prev,
-                                                uint32_t *out_sets, LevelCounters *lc) {
+__device__ __forceinline__ void tree_enum_phase(const uint32_t *adj, int k, bool near, const uint32_t *prev_sets,
+                                                uint32_t c_prev, uint32_t *out_sets, LevelCounters *lc) {
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t nthreads = gridDim.x * blockDim.x;
     // from the far end of the grid: the first warps evaluate the first sets
@@ -1097,7 +1103,8 @@ __device__ __forceinline__ void tree_enum_phase(const uint32_t *adj, int k, cons
         const uint32_t S = (k == 2) ? (1u << i) : __ldcg(prev_sets + i);
         const uint32_t a = ((S >> lane) & 1u) ? adj[lane] : 0u, in = a & S;
         const uint32_t leaves = __ballot_sync(kFull, a != 0u && (in & (in - 1u)) == 0u);
-        const uint32_t ext = tree_extension_mask(S, __reduce_or_sync(kFull, a) & ~S, leaves, [&](int v) { return adj[v]; });
+        const uint32_t ext =
+            tree_extension_mask(S, __reduce_or_sync(kFull, a) & ~S, leaves, near, [&](int v) { return adj[v]; });
         uint32_t base = 0u;
         if (lane == 0u && ext) base = atomicAdd(&lc->n_sets, (uint32_t)__popc(ext));
         base = __shfl_sync(kFull, base, 0);
@@ -1107,7 +1114,7 @@ __device__ __forceinline__ void tree_enum_phase(const uint32_t *adj, int k, cons
     for (uint32_t first = tid & ~31u; first < c_prev; first += nthreads) {
         const uint32_t idx = first + (tid & 31u);
         const uint32_t S = idx < c_prev ? ((k == 2) ? (1u << idx) : __ldcg(prev_sets + idx)) : 0u;
-        uint32_t ext = tree_extensions(S, [&](int v) { return adj[v]; });
+        uint32_t ext = tree_extensions(S, near, [&](int v) { return adj[v]; });
         const uint32_t cnt = (uint32_t)__popc(ext);
         uint32_t incl = cnt;
 #pragma unroll
@@ -1171,6 +1178,7 @@ __device__ __forceinline__ void extract_plan(const float4 *memo, const uint32_t 
 struct TreePlan {
     uint32_t count[33];
     uint8_t group[33];
+    uint8_t near;                      // order of the lists (near_order)
 };
 
 // Bound: a warp-step (one split, both orientations) issues about 240
@@ -1230,13 +1238,13 @@ __global__ void __launch_bounds__(kBlock, MINB) k_dp_tree(const uint32_t *__rest
         memo[1u << i] = base_entry(*d.h, i);
         memo_left[1u << i] = 0u;
     }
-    if (n >= 2) tree_enum_phase(adj, 2, nullptr, (uint32_t)n, setsA, lvl + 2);
+    if (n >= 2) tree_enum_phase(adj, 2, plan.near != 0u, nullptr, (uint32_t)n, setsA, lvl + 2);
     if (!barrier()) return;
     for (int k = 2; k <= n; k++) {
         uint32_t *cur = (k & 1) ? setsB : setsA;
         uint32_t *nxt = (k & 1) ? setsA : setsB;
         const uint32_t count = plan.count[k];
-        if (k < n) tree_enum_phase(adj, k + 1, cur, count, nxt, lvl + k + 1);
+        if (k < n) tree_enum_phase(adj, k + 1, plan.near != 0u, cur, count, nxt, lvl + k + 1);
         tree_level<LAYOUT>(d, pp, gwarp, nwarps, cur, count, k, plan.group[k], memo, memo_left);
         if (!barrier()) return;
     }
@@ -1920,6 +1928,18 @@ static double tree_level_counts(const DevHeader *h, uint32_t (&count)[33]) {
     return total;
 }
 
+// The order in which the tree kernels list connected sets (tree_extension_mask)
+// for a memo of `slots` entries of which `sets` are used, a sector of 32 bytes
+// each: near once the sectors exceed the L2 cache, or, for plain trees, whose
+// cost does not cover the misses, once the memo's span exceeds 512 MB, some 256
+// pages of 2 MB (snowflake-25, 512 MB: 156 us by the largest leaf, 158 near;
+// snowflake-26: 191 and 178; -30: 732 and 453; star-22, 67 MB of sectors: 394 and
+// 391, star-24: 1438 and 1242, star-26 / 27 / 28: 11.6 / 26.4 / 57.3 ms and 5.4 /
+// 11.7 / 25.5; with statistics snowflake-28 454 and 460 us).
+static bool near_order(uint64_t slots, double sets, int layout, int l2_bytes) {
+    return 32.0 * sets > (double)l2_bytes || (layout == kTreePlain && 16ull * slots > (512ull << 20));
+}
+
 // cpu_dpsize's level-1 list (gpuqo_cpu_dpsize.cu:43-48 after
 // gpuqo_cpu_sequential.cu:73-84): the iteration order of its unordered_map
 // memo once base relation i (key 2^(i+1), whose hash is the key itself) has
@@ -1970,7 +1990,7 @@ static cudaError_t launch_cluster(const void *fn, int blocks, size_t smem, void 
 class Engine {
 public:
     int device = -1;
-    int sm_count = 148;
+    int sm_count = 148, l2_bytes = 0;
     cudaStream_t stream = nullptr;
     DevArena a;
     int cap_n = -1;                    // arena sized for this many relations
@@ -2006,6 +2026,7 @@ public:
         if (ready) return 0;
         CK(cudaGetDevice(&device));
         CK(cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, device));
+        CK(cudaDeviceGetAttribute(&l2_bytes, cudaDevAttrL2CacheSize, device));
         if (!stream) CK(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
         if (!ev0) CK(cudaEventCreate(&ev0));
         if (!ev1) CK(cudaEventCreate(&ev1));
@@ -2340,6 +2361,7 @@ public:
         for (int k = 2; k <= n; k++) plan_pairs += (uint64_t)plan.count[k] * 2u * (uint64_t)(k - 1);
         bar_after = one_cluster ? bar_base : bar_base + (unsigned)n * (unsigned)grid;   // a barrier per level and the first
         *h_tree_n = 0;
+        plan.near = near_order(1ull << n, sets, layout, l2_bytes) ? 1u : 0u;
         for (int k = 2; k <= n; k++)
             plan.group[k] = (uint8_t)tree_group(plan.count[k], k, (uint32_t)grid * kBlock, (uint32_t)std::min(grid, sm_count));
         unsigned poll_limit = (unsigned)std::max(0, gpuqo_b200_barrier_poll_limit);
@@ -3589,14 +3611,14 @@ __global__ void kb_extract(const BatchQ *__restrict__ qs, int nq, const uint32_t
 // 20 relations (77 M pairs, its wave of cycles included) 2230 -> 1000 us, of
 // 512 queries of 8 to 16 (23.7 M pairs) 1040 -> 600 us.
 __device__ __forceinline__ void batch_tree_enum(const BatchQ *qs, const uint32_t *blobs, const unsigned long long *prev,
-                                                uint32_t c_prev, unsigned long long *out, LevelCounters *lc,
-                                                uint32_t tid, uint32_t nthreads) {
+                                                uint32_t c_prev, bool near, unsigned long long *out,
+                                                LevelCounters *lc, uint32_t tid, uint32_t nthreads) {
     const uint32_t lane = threadIdx.x & 31u;
     for (uint32_t first = tid & ~31u; first < c_prev; first += nthreads) {
         const uint32_t idx = first + (tid & 31u);
         const unsigned long long it = idx < c_prev ? __ldcg(prev + idx) : 0ull;
         const uint32_t *adj = reinterpret_cast<const DevHeader *>(blobs + qs[it >> 32].blob_off)->adj;
-        uint32_t ext = tree_extensions((uint32_t)it, [&](int v) { return __ldg(adj + v); });
+        uint32_t ext = tree_extensions((uint32_t)it, near, [&](int v) { return __ldg(adj + v); });
         const uint32_t cnt = (uint32_t)__popc(ext);
         uint32_t incl = cnt;
 #pragma unroll
@@ -3638,7 +3660,8 @@ __global__ void __launch_bounds__(kBlock, 3) kb_dp(const BatchQ *__restrict__ qs
                                                    unsigned long long *__restrict__ listB,
                                                    LevelCounters *__restrict__ lvl, GlobalCounters *__restrict__ glob,
                                                    TreeNode *__restrict__ tree, int *__restrict__ tree_n,
-                                                   unsigned *__restrict__ bar, uint32_t sms, unsigned poll_limit) {
+                                                   unsigned *__restrict__ bar, uint32_t sms, uint32_t near,
+                                                   unsigned poll_limit) {
     const unsigned max_polls = barrier_polls(poll_limit);
     __shared__ unsigned long long stage[kWarpsPerBlock][64];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -3685,7 +3708,7 @@ __global__ void __launch_bounds__(kBlock, 3) kb_dp(const BatchQ *__restrict__ qs
         unsigned long long *nxt = (k & 1) ? listA : listB;
         const uint32_t count = __ldcg(&lvl[k].n_sets);
         // enumeration from the far end of the grid, evaluation from the start
-        if (k < maxn) batch_tree_enum(qs, blobs, cur, count, nxt, lvl + k + 1, nthreads - 1u - tid, nthreads);
+        if (k < maxn) batch_tree_enum(qs, blobs, cur, count, near != 0u, nxt, lvl + k + 1, nthreads - 1u - tid, nthreads);
         batch_tree_level<LAYOUT>(qs, blobs, gwarp, nwarps, cur, count, k, tree_group(count, k, nthreads, sms), memo,
                                  memo_left);
         pairs += (unsigned long long)count * 2ull * (unsigned long long)(k - 1);   // every split edge, both orientations
@@ -3788,7 +3811,7 @@ constexpr size_t kGenSmem = kWarpsPerBlock * sizeof(GenScratch);
 static_assert(kGenSmem <= 44 * 1024 && sizeof(GenScratch) % 16 == 0, "kb_gen scratch and its static shared memory");
 
 struct BatchEngine {
-    int device = -1, sm_count = 148;
+    int device = -1, sm_count = 148, l2_bytes = 0;
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     // arena (grown on demand), each buffer with its own capacity: one that
@@ -3834,6 +3857,7 @@ struct BatchEngine {
         if (ready) return 0;
         CK(cudaGetDevice(&device));
         CK(cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, device));
+        CK(cudaDeviceGetAttribute(&l2_bytes, cudaDevAttrL2CacheSize, device));
         if (!stream) CK(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
         if (!ev0) CK(cudaEventCreate(&ev0));
         if (!ev1) CK(cudaEventCreate(&ev1));
@@ -3897,7 +3921,8 @@ struct BatchEngine {
     // the wave as one cooperative launch: kb_dp<layout> when every query is
     // tree-shaped (layout: the least of the queries' tree_layout), else kb_gen
     // (layout < 0; kb_gen<true> for one query); false when it could not start
-    bool enqueue_persistent(int nq, int maxn, uint32_t words, uint64_t seen_words, int layout, uint32_t cactus_sets) {
+    bool enqueue_persistent(int nq, int maxn, uint32_t words, uint64_t slots, uint64_t seen_words, int layout,
+                            uint32_t cactus_sets) {
         const bool tree_only = layout >= 0;
         const int one = (!tree_only && nq == 1) ? one_grid(words) : 0;
         int grid = tree_only ? coop_grid_tree[layout] : (one > 0 ? one : coop_grid);
@@ -3921,9 +3946,9 @@ struct BatchEngine {
         cudaError_t e;
         if (tree_only) {
             static const void *const variants[3] = {(const void *)kb_dp<0>, (const void *)kb_dp<1>, (const void *)kb_dp<2>};
-            uint32_t sms = (uint32_t)sm_count;
+            uint32_t sms = (uint32_t)sm_count, near = near_order(slots, 0.0, layout, l2_bytes) ? 1u : 0u;
             void *args[] = {&qs, &nq, &maxn, &blobs, &memo, &memo_left, &listA, &listB,
-                            &lvl, &glob, &tree, &tree_n, &bar, &sms, &poll_limit};
+                            &lvl, &glob, &tree, &tree_n, &bar, &sms, &near, &poll_limit};
             e = cudaLaunchCooperativeKernel(variants[layout], dim3(grid), dim3(kBlock), args, 0, stream);
         } else {
             void *args[] = {&qs, &nq, &maxn, &blobs, &words, &memo, &memo_left, &seen, &listA, &listB,
@@ -4083,7 +4108,7 @@ struct BatchEngine {
         };
         uint32_t kernels = 1;
         CK(cudaEventRecord(ev0, stream));
-        bool persistent = enqueue_persistent(nq, maxn, (uint32_t)words, seen_words, layout, cactus_sets);
+        bool persistent = enqueue_persistent(nq, maxn, (uint32_t)words, slots, seen_words, layout, cactus_sets);
         CK(cudaGetLastError());
         if (!persistent) kernels = enqueue_levels(nq, maxn, seen_words);
         CK(cudaGetLastError());
