@@ -856,41 +856,57 @@ __device__ __forceinline__ void tree_cost(const DevInfoView &d, const PlainParam
     }
 }
 
-// The first candidate of a set in enumeration order has a NaN cost: the
-// reference keeps it.  Rare (overflowed row estimates): every lane finds its
-// lowest place, and when the group's lowest is a NaN one, its lane costs it
-// again and writes the entry.  Returns whether the lane's group is settled.
+// Some candidates of the warp's sets have a NaN cost (overflowed row
+// estimates); the reference keeps such a one where it is a set's first.  The
+// places of block order are 0 .. 2 (k - 1) - 1, so there it is the one at place
+// 0; plain DPsub's first is the least outer side of all splits.  The lane that
+// found it costs it again.  Returns whether the lane's group is settled.
+template <int LAYOUT>
 __device__ __noinline__ bool tree_nan_rule(const DevInfoView d, uint32_t S, bool has, int G, uint32_t nan_p,
                                            const float4 *memo, RelVal &out, uint32_t &left, bool &writer) {
     const DevHeader &h = *d.h;
     const TreeRows t = tree_rows(h, S);
-    const int gl = (int)(threadIdx.x & 31u) % G;
-    uint32_t first = kFull, nan_left = 0u;
-    uint32_t x = has ? S & (S - 1u) : 0u;
-    for (int j = 0; x; x &= x - 1u, j++) {
-        const uint32_t v = (uint32_t)lowest_idx(x);
-        if (G == 32 ? (int)v != gl : j % G != gl) continue;
-        const uint2 e = *reinterpret_cast<const uint2 *>(t.row + 2u * v);
-        const uint32_t L0 = (e.y & kTreeLower) ? S & e.x : S ^ (S & e.x);
-        uint32_t p0, p1;
-        tree_order(t, S, v, e.x, L0, h.index_order, p0, p1);
-        first = min(first, min(p0, p1));
-        if (p0 == nan_p) nan_left = L0;
-        if (p1 == nan_p) nan_left = S ^ L0;
+    const int lane = (int)(threadIdx.x & 31u), gl = lane & (G - 1);
+    uint32_t first = 0u;
+    // the lane's own child ends, as tree_set deals them out
+    uint32_t ends = has ? S & (S - 1u) : 0u;
+    if (G == 32) {
+        ends &= 1u << lane;
+    } else {
+        for (int i = 0; i < gl; i++) ends &= ends - 1u;
     }
-    uint32_t gfirst = first, gnan = nan_p;
-    for (int off = G >> 1; off >= 1; off >>= 1) {
-        gfirst = min(gfirst, __shfl_xor_sync(kFull, gfirst, off));
-        gnan = min(gnan, __shfl_xor_sync(kFull, gnan, off));
+    auto for_each_end = [&](auto body) {
+        for (uint32_t x = ends; x;) {
+            const uint32_t v = (uint32_t)lowest_idx(x);
+            const uint2 e = *reinterpret_cast<const uint2 *>(t.row + 2u * v);
+            body(v, e, (e.y & kTreeLower) ? S & e.x : S ^ (S & e.x));
+            for (int i = 0; i < G; i++) x &= x - 1u;
+        }
+    };
+    if (__any_sync(kFull, has && h.index_order != 0u)) {
+        if (h.index_order != 0u) {
+            first = kFull;
+            for_each_end([&](uint32_t, uint2, uint32_t L0) { first = min(first, min(L0, S ^ L0)); });
+        }
+        for (int off = G >> 1; off >= 1; off >>= 1) first = min(first, __shfl_xor_sync(kFull, first, off));
     }
-    const bool settled = has && gnan != kFull && gnan == gfirst;
-    writer = settled && nan_p == gnan;
+    writer = has && nan_p == first;   // kFull, no NaN, is no place
+    const uint32_t writers = __ballot_sync(kFull, writer);
     if (writer) {
-        left = nan_left;
+        uint32_t edge = 0u;
+        for_each_end([&](uint32_t v, uint2 e, uint32_t L0) {
+            uint32_t p0, p1;
+            tree_order(t, S, v, e.x, L0, h.index_order, p0, p1);
+            if (p0 != nan_p && p1 != nan_p) return;
+            left = p0 == nan_p ? L0 : S ^ L0;
+            edge = e.y & 31u;
+        });
         const RelVal l = load_rel(memo, left, h.hz_packed), r = load_rel(memo, S ^ left, h.hz_packed);
-        out = join_eval(d, left, l, S ^ left, r);
+        const uint32_t classes =
+            LAYOUT == kTreeGeneral ? 0u : reinterpret_cast<const TreeEdge *>(t.tab + tree_edge_off(t.n))[edge].classes;
+        out = join_eval_t<LAYOUT != kTreeGeneral>(d, left, l, S ^ left, r, classes);
     }
-    return settled;
+    return ((writers >> (lane - gl)) & (G == 32 ? kFull : (1u << G) - 1u)) != 0u;
 }
 
 // One set of k relations (has: the lane's group holds one) by a group of G
@@ -958,7 +974,7 @@ __device__ __forceinline__ void tree_set(const DevInfoView &d, const PlainParams
         RelVal out;
         uint32_t left = 0u;
         bool writer = false;
-        if (tree_nan_rule(d, S, has, G, best.nan_p, memo, out, left, writer)) win = false;
+        if (tree_nan_rule<LAYOUT>(d, S, has, G, best.nan_p, memo, out, left, writer)) win = false;
         if (writer) memo_write(h, memo, memo_left, S, out, left);
     }
     if (win) {
