@@ -130,17 +130,16 @@ __device__ __forceinline__ float clamp_row_est(float nrows) {
 }
 
 // :820-841 (MAXALIGN with MAXIMUM_ALIGNOF 8, RELATION_OVERHEAD 24, BLCKSZ 8192)
-// A width >= 0 stays below 2^32 after the alignment and the overhead, so it is
-// converted from 32 bits: the same integer, the same rounding.  The 64-bit
-// conversion runs at a sixteenth of the 32-bit one's rate and was executed
-// three times per costed orientation.
-static __device__ __noinline__ float row_bytes_wide(int width) {
-    unsigned long long a = ((unsigned long long)(long long)width + 7ull) & ~7ull;
-    return (float)(a + 24ull);
-}
+// The reference converts the aligned width plus overhead from 64 unsigned bits.
+// That is below 2^32 for a width >= 0, so 32 bits hold the same integer and give
+// the same rounding at 16 times the rate of the 64-bit conversion, which ran
+// three times per costed orientation.  For a width < 0 the 64-bit sum is either
+// past zero again, then 32 bits hold it too, or within 2^31 of 2^64, which as a
+// float is 2^64.  No call for the rare case: one in the cost code took 2 to 3 %
+// of the kernels that evaluate general classes (registers kept across it).
 __device__ __forceinline__ float row_bytes(int width) {
-    if (__builtin_expect(width < 0, 0)) return row_bytes_wide(width);
-    return (float)((((uint32_t)width + 7u) & ~7u) + 24u);
+    const uint32_t u = (((uint32_t)width + 7u) & ~7u) + 24u;
+    return (width & (int)u) < 0 ? 18446744073709551616.0f : (float)u;
 }
 __device__ __forceinline__ float relation_byte_size(float tuples, int width) { return tuples * row_bytes(width); }
 __device__ __forceinline__ float page_size(float tuples, int width) {

@@ -695,7 +695,7 @@ __device__ __forceinline__ void mpdp_groups(const DevInfoView &d, const uint32_t
     }
 }
 
-__global__ void __launch_bounds__(kBlock) k_eval_mpdp(const uint32_t *__restrict__ blob, uint32_t blob_words,
+__global__ void __launch_bounds__(kBlock, 2) k_eval_mpdp(const uint32_t *__restrict__ blob, uint32_t blob_words,
                                                       const uint32_t *__restrict__ sets,
                                                       LevelCounters *__restrict__ lc, float4 *__restrict__ memo,
                                                       uint32_t *__restrict__ memo_left, uint32_t *__restrict__ ovf_set,
