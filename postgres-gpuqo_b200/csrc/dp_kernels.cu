@@ -2208,7 +2208,9 @@ public:
         const int nw = ec_stride(reinterpret_cast<const DevHeader *>(h_blob)->n_ec) / 4;
         CK(cudaMemsetAsync(d_ctl, 0, kCtlClearBytes, stream));
         CK(cudaMemsetAsync(a.seen, 0, std::max<uint64_t>((1ull << n) / 8, 4), stream));
-        if (mode == kModeDpsub && dense) {   // no winner and no share yet (k_dense leaves them so)
+        // no winner and no share yet (k_dense leaves them so); sets of up to
+        // kDenseWhole splits are one warp's, so smaller queries have no shares
+        if (mode == kModeDpsub && dense && (1u << (n - 1)) > kDenseWhole) {
             CK(cudaMemsetAsync(a.ovf_off, 0, max_level_sets(n) * sizeof(uint32_t), stream));
             CK(cudaMemsetAsync(a.ovf_key, 0xFF, max_level_sets(n) * sizeof(unsigned long long), stream));
             CK(cudaMemsetAsync(a.ovf_first, 0xFF, max_level_sets(n) * sizeof(unsigned long long), stream));
