@@ -2197,6 +2197,9 @@ public:
         return (size_t)(((blob_words + 3u) & ~3u) + kWarpsPerBlock * kQueueWords) * 4u;
     }
 
+    // dynamic shared memory of k_dense: the planner info
+    static size_t dense_smem(uint32_t blob_words) { return (size_t)((blob_words + 3u) & ~3u) * 4u; }
+
     // Enqueues the whole DP for n relations on `stream`.
     int enqueue(int n, DpMode mode, bool ccc, bool profile, uint32_t blob_words, std::string &err) {
         if (mode == kModeDpsize) return enqueue_dpsize(n, blob_words, err);
@@ -2245,7 +2248,7 @@ public:
                 while (share < 4096u && total * V >= 2u * share * 4u * warps) share *= 2u;
                 const bool whole = V <= std::max(share, kDenseWhole);
                 if (whole) share = V;
-                (nw == 1 ? k_dense<1> : k_dense<2>)<<<sm_count * 3, kBlock, (size_t)((blob_words + 3u) & ~3u) * 4u, stream>>>(
+                (nw == 1 ? k_dense<1> : k_dense<2>)<<<sm_count * 3, kBlock, dense_smem(blob_words), stream>>>(
                     a.blob, blob_words, k, cur_sets, lc, a.memo, a.memo_left, a.ovf_key, a.ovf_first, a.ovf_off, a.glob, share);
             } else if (mode == kModeDpsub) {
                 k_eval<kModeDpsub><<<eblocks, kBlock, smem, stream>>>(a.blob, blob_words, k, cur_sets, lc, a.memo,
@@ -2437,20 +2440,25 @@ public:
             CK(cudaFuncSetAttribute(k_dpsize_eval, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
             CK(cudaFuncSetAttribute(k_eval<kModeDpsub>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
             CK(cudaFuncSetAttribute(k_eval<kModeMpdp>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-            CK(cudaFuncSetAttribute(k_dense<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-            CK(cudaFuncSetAttribute(k_dense<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
             CK(cudaFuncSetAttribute(k_ovf_chunks<kModeDpsub>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
             CK(cudaFuncSetAttribute(k_ovf_chunks<kModeMpdp>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
             CK(cudaFuncSetAttribute(k_ovf_finalize<kModeDpsub>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
             CK(cudaFuncSetAttribute(k_ovf_finalize<kModeMpdp>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         }
-        CK(cudaMemcpyAsync(a.blob, h_blob, words * 4, cudaMemcpyHostToDevice, stream));
-        exec = nullptr;
-        const uint32_t mb = reinterpret_cast<const DevHeader *>(h_blob)->max_block;
-        const uint32_t tm = reinterpret_cast<const DevHeader *>(h_blob)->tree_mode;
         // the dense kernels are instantiated by the words of a class row
         const DevHeader *hb = reinterpret_cast<const DevHeader *>(h_blob);
         const int dense = (mode == kModeDpsub && dense_pairs(*hb)) ? ec_stride(hb->n_ec) / 4 : 0;
+        if (dense) {
+            // their pair tables beside the planner info: 47,360 bytes for 256
+            // classes, the most there are
+            const size_t table = kWarpsPerBlock * (dense == 1 ? sizeof(PairTable<1>) : sizeof(PairTable<2>));
+            const void *fn = dense == 1 ? (const void *)k_dense<1> : (const void *)k_dense<2>;
+            if (dense_smem(words) + table > 48 * 1024)
+                CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dense_smem(words)));
+        }
+        CK(cudaMemcpyAsync(a.blob, h_blob, words * 4, cudaMemcpyHostToDevice, stream));
+        exec = nullptr;
+        const uint32_t mb = hb->max_block, tm = hb->tree_mode;
         GraphKey key{n, (((int)mode * 64 + (int)std::min<uint32_t>(mb, 63u)) * 2 + (int)(tm != 0u)) * 4 + dense,
                      ccc ? 1 : 0, (int)words};
         (void)profile;
