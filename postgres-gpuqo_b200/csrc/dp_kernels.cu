@@ -1844,11 +1844,8 @@ uint64_t engine_bytes_needed(int n) {
         cudaError_t e_ = (call);                                                          \
         if (e_ != cudaSuccess) {                                                          \
             err = std::string(#call) + ": " + cudaGetErrorString(e_);                     \
-            if (e_ == cudaErrorMemoryAllocation) {                                        \
-                cudaGetLastError();                                                       \
-                return GPUQO_B200_ERR_NOMEM;                                              \
-            }                                                                             \
-            return GPUQO_B200_ERR_CUDA;                                                   \
+            cudaGetLastError();   /* reported here: not by the next call's check too */   \
+            return e_ == cudaErrorMemoryAllocation ? GPUQO_B200_ERR_NOMEM : GPUQO_B200_ERR_CUDA; \
         }                                                                                 \
     } while (0)
 

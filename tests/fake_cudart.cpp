@@ -1,8 +1,9 @@
 // A stand-in for the CUDA runtime functions that the library calls, to be
 // loaded ahead of the real one: device memory is host memory, a launch does
-// nothing.  It fails the allocations it is told to and counts every use of a
-// pointer that no live allocation holds: freed again, cleared, copied or
-// handed to a kernel.
+// nothing.  It fails the allocations it is told to, and a request for more shared
+// memory than a block has, keeps the last error as CUDA does, and counts every
+// use of a pointer that no live allocation holds: freed again, cleared, copied
+// or handed to a kernel.
 #include <sys/mman.h>
 
 #include <cstdint>
@@ -29,6 +30,9 @@ static std::map<const void *, std::string> &names() {
 
 extern "C" {
 int fake_allocations, fake_fail_from = -1, fake_fail_count, fake_bad, fake_launches;
+static int last_error;   // of the calls that can fail here
+
+static int failed(int e) { return last_error = e; }
 
 static bool held(const void *p, size_t n) {
     auto it = live().upper_bound((uintptr_t)p);
@@ -39,9 +43,9 @@ static bool held(const void *p, size_t n) {
 
 static int allocate(void **p, size_t n) {
     const int at = fake_allocations++;
-    if (fake_fail_from >= 0 && at >= fake_fail_from && at < fake_fail_from + fake_fail_count) return 2;
+    if (fake_fail_from >= 0 && at >= fake_fail_from && at < fake_fail_from + fake_fail_count) return failed(2);
     void *m = mmap(nullptr, n ? n : 1, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS | MAP_NORESERVE, -1, 0);
-    if (m == MAP_FAILED) return 2;
+    if (m == MAP_FAILED) return failed(2);
     live()[(uintptr_t)m] = n;
     *p = m;
     return 0;
@@ -52,7 +56,7 @@ static int release(void *p) {
     auto it = live().find((uintptr_t)p);
     if (it == live().end()) {
         fake_bad++;
-        return 1;
+        return failed(1);
     }
     munmap(p, it->second ? it->second : 1);
     live().erase(it);
@@ -126,8 +130,14 @@ int cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int *n, const void *,
     *n = 2;
     return 0;
 }
-int cudaFuncSetAttribute(const void *, int, int) { return 0; }
-int cudaGetLastError() { return 0; }
+int cudaFuncSetAttribute(const void *, int attr, int value) {
+    return attr == 8 && value > 227 * 1024 ? failed(1) : 0;   // dynamic shared memory of a block
+}
+int cudaGetLastError() {
+    const int e = last_error;
+    last_error = 0;
+    return e;
+}
 const char *cudaGetErrorString(int e) { return e ? "error" : "no error"; }
 int cudaGetSymbolAddress(void **, const void *) { return 1; }
 int cudaEventCreate(void **e) {

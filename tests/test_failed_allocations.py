@@ -63,3 +63,24 @@ def test_smaller_calls_after_a_failed_allocation(fake, kind):
     for fail, (_, failed, then, bad, _) in enumerate(runs):
         assert ERR_NOMEM in failed and all(f in (b, ERR_NOMEM) for f, b in zip(failed, before)), fail
         assert then == after and bad == 0, fail
+
+
+REFUSED = """
+import sys
+from gpuqo_b200 import capi, lib, query
+big = query.star(12, 1)
+first = list(big.eq_classes)
+for i in range(6000):   # a planner info larger than a block's shared memory
+    big.eq_classes.append(query.EqClass(list(first[i % 11].members), [0.5], [[], []], [query.VarInfo()] * 2))
+for q in (query.star(12, 1), big, query.star(12, 1)):
+    print("call", lib.run(q, capi.GPUQO_DPSUB, bicc=True).error, file=sys.stderr)
+"""
+
+
+def test_a_refused_call_leaves_no_error_for_the_next(fake):
+    env = dict(os.environ, LD_PRELOAD=fake, PYTHONPATH=os.path.join(REPO, "postgres-gpuqo_b200"))
+    done = subprocess.run([sys.executable, "-c", REFUSED], env=env, capture_output=True, text=True, timeout=120)
+    _, refused, after = done.stderr.split("call 2\n")[:3]
+    assert done.returncode == 0 and "cudaFuncSetAttribute" in refused
+    # no plan comes from kernels that do nothing, but the runtime has no complaint
+    assert "nodes" in after and "cuda" not in after
