@@ -34,7 +34,7 @@ struct GenScratch {
     uint32_t half[33];            // ... unordered splits ahead of it
     // unions of the parts of a block's relations, 4 relations per group of 16
     // words (blocks of 3 and more relations that are no cycles: at most 14
-    // groups for 31 relations)
+    // groups for the 30 relations of this path, as triangles)
     uint32_t tab[16 * 16];
     uint32_t pre[64];             // cycle blocks: unions along the walk (sizes plus one, at most 48)
     uint32_t hang[32];            // relation and the parts below it outside its parent block

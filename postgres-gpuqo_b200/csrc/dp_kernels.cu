@@ -1055,15 +1055,16 @@ __global__ void __launch_bounds__(kBlock, 3) k_eval_tree(const uint32_t *__restr
 }
 
 // ---------------------------------------------------------------------------
-// k_dp_tree: the whole MPDP of a tree-shaped query in ONE cooperative,
-// persistent launch.  The planner info and the binomial table are staged in
-// shared memory once; levels are separated by a grid barrier, and each phase
-// evaluates level k while enumerating level k+1 (independent: the
-// enumeration reads only level k's sets).  Data written by other blocks is
-// read with ld.global.cg (L2), never through a possibly stale L1 line.
-// The barrier spins a bounded number of times; on timeout it raises an error
-// flag, every block leaves, and the host reruns the DP with per-level
-// launches.
+// k_dp_tree: the whole MPDP of a tree-shaped query in ONE persistent launch:
+// cooperative, or for queries of narrow levels an ordinary launch of one
+// thread-block cluster (or one block).  The planner info is staged in shared
+// memory once; levels are separated by a barrier, and each phase evaluates
+// level k while enumerating level k+1 (independent: the enumeration reads only
+// level k's sets).  Data written by other blocks is read with ld.global.cg
+// (L2), never through a possibly stale L1 line.
+// The grid barrier spins a bounded number of times; on timeout it raises an
+// error flag, every block leaves, and the host reruns the DP with per-level
+// launches.  A cluster has the hardware's barrier.
 // ---------------------------------------------------------------------------
 // One enumeration phase (level k from the connected (k-1)-sets) of a
 // tree-shaped query graph, each k-set once and without a dedup structure:
@@ -1212,7 +1213,8 @@ struct TreePlan {
 // up.  blob may be the host's too: a few blocks read it faster than a copy
 // ahead of the launch takes.
 // MINB: blocks per SM the register budget is set for (2, 3 or 4: 128, 80 or 64
-// registers, no spill but 4 bytes with 4 blocks), chosen per query from its
+// registers; spill: 16 bytes with 3 blocks and general classes, 20 with 4
+// blocks), chosen per query from its
 // connected sets per level, the total over the relation count
 // (Tuning::single_narrow_level_sets, Tuning::single_wide_level_sets); LAYOUT:
 // the evaluation (tree_layout)
@@ -1883,9 +1885,11 @@ struct Tuning {
     // tree queries with up to this many connected sets per level run
     // k_dp_tree<2>, those with more than single_wide_level_sets k_dp_tree<4>
     // (device time of the 2- / 3- / 4-blocks variant: star-18, 7 k sets per
-    // level, 98 / 104 / 111 us; star-20, 26 k, 163 / 156 / 165; star-21, 50 k,
-    // 253 / 237 / 252; star-22, 95 k, 392 / 387 / 385; star-24, 350 k,
-    // 1557 / 1441 / 1407; the third crossover is left to the autotuner)
+    // level, 95 / 103 / 120 us; star-20, 26 k, 159 / 156 / 176; star-22, 95 k,
+    // 381 / 372 / 384; star-24, 350 k, 1357 / 1210 / 1194; star-26, 1.3 M,
+    // 6182 / 5363 / 5591; star-27, 2.5 M, 13.5 / 11.8 / 12.6 ms; snowflake-28,
+    // 12 k, 217 / 227 / 268 us; snowflake-30, 39 k, 427 / 430 / 474: the third
+    // one wins by 1 % between 350 and 700 k, which is left to the autotuner)
     double single_narrow_level_sets = 16384.0;
     double single_wide_level_sets = 1e30;
     double batch_single_sets = double(1u << 20);   // a batch hands larger tree queries to k_dp_tree
@@ -3763,7 +3767,7 @@ bool batch_eligible(const std::vector<uint32_t> &blob) {
 }
 
 // true when some set of the query may have more candidates than one group
-// evaluates: those sets need the overflow phase of kb_dp
+// evaluates: those sets need the overflow phase of kb_gen
 static bool batch_needs_ovf(const std::vector<uint32_t> &blob) {
     const DevHeader *h = reinterpret_cast<const DevHeader *>(blob.data());
     return mpdp_candidate_bound(h->n, (int)h->max_block) > kOvfLimit;
@@ -3831,7 +3835,9 @@ struct alignas(16) BatchCtl {
 
 // dynamic shared memory of kb_gen besides the planner info
 constexpr size_t kGenSmem = kWarpsPerBlock * sizeof(GenScratch);
-static_assert(kGenSmem <= 44 * 1024 && sizeof(GenScratch) % 16 == 0, "kb_gen scratch and its static shared memory");
+// beside it kb_gen has the list staging (8 bytes x 64 per warp) and the
+// barrier's verdict as static shared memory: without opt-in 48 KB in all
+static_assert(kGenSmem + kWarpsPerBlock * 64 * 8 + 16 <= 48 * 1024 && sizeof(GenScratch) % 16 == 0, "kb_gen shared memory");
 
 struct BatchEngine {
     int device = -1, sm_count = 148, l2_bytes = 0;
@@ -4195,7 +4201,7 @@ int engine_run_batch(const std::vector<const std::vector<uint32_t> *> &blobs, ui
         if (int rc = eng->run(*blobs[i], n, kModeMpdp, true, false, out[i], st, err)) return rc;
         st.handoff_ms += st.device_ms - before;
     }
-    // tree-shaped queries first (waves of kb_dp<true>), then the others; the
+    // tree-shaped queries first (waves of kb_dp), then the others (kb_gen); the
     // order within each part is the caller's (largest first)
     std::stable_partition(rest.begin(), rest.end(), [&](size_t i) {
         return reinterpret_cast<const DevHeader *>(blobs[i]->data())->tree_mode != 0u;

@@ -116,7 +116,7 @@ struct DevHeader {
     // not a tree: every class plain with one selectivity for both orientations
     // and at most 256 of them, hz_packed, hash joins enabled and a row of the
     // widest set within work_mem: the word offset of PlainQuals[n_ec + 1] by
-    // the number of matching classes (pairs_match, plain_mirror); 0: no
+    // the number of matching classes (pairs_mirror, plain_mirror); 0: no
     uint32_t pairs_plain;
 };
 
@@ -144,8 +144,8 @@ struct alignas(16) PlainQuals {
 // A connected set S is a subtree; the reference's block search walks it from
 // its lowest relation r in exactly this preorder.  Every relation of S but r
 // is the child end of one split edge, so the first rows give every split with
-// one 8-byte load; the second rows serve the enumeration index, which only
-// equal costs and NaN costs ask for.
+// one 8-byte load; the second rows give its place in block order, which is
+// taken along with every split (equal costs are common).
 struct TreeEdge {
     PlainQuals quals;
     // the selectivity product over the edge's classes in class order with the
