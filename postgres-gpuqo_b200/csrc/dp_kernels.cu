@@ -2032,6 +2032,7 @@ public:
     double plan_sets = 0.0;            // connected sets and pairs of the last persistent run
     uint64_t plan_pairs = 0;
     std::map<size_t, int> coop_blocks; // (dynamic shared bytes, variant) -> co-resident blocks of k_dp_tree (0: none)
+    std::map<const void *, size_t> smem_limit;   // dynamic shared memory that its variants are allowed
     int force_minb = 0;                // autotuner: run this k_dp_tree variant (2, 3 or 4); 0 = by the tuning record
     bool coop_off = false;             // cooperative launch refused on this device
     bool barrier_timed_out = false;    // a grid barrier of k_dp_tree gave up: per-level launches until reset
@@ -2356,8 +2357,11 @@ public:
             int blocks = 0, dev_coop = 0, occ = 0;
             cudaDeviceGetAttribute(&dev_coop, cudaDevAttrCooperativeLaunch, device);
             bool ok = dev_coop != 0;
-            if (ok && smem > 48 * 1024)
+            size_t &limit = smem_limit[fn];   // only ever raised: larger sizes stay launchable
+            if (ok && smem > std::max<size_t>(limit, 48 * 1024)) {
                 ok = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess;
+                if (ok) limit = smem;
+            }
             if (ok) ok = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, kBlock, smem) == cudaSuccess;
             if (ok) blocks = occ * sm_count;
             cudaGetLastError();

@@ -17,6 +17,7 @@ struct dim3 {
 };
 struct LaunchConfig {   // the head of cudaLaunchConfig_t
     dim3 grid, block;
+    size_t smem;
 };
 
 static std::map<uintptr_t, size_t> &live() {
@@ -28,10 +29,15 @@ static std::map<const void *, std::string> &names() {
     return *m;
 }
 
+// dynamic shared memory that a kernel is allowed
+static std::map<const void *, int> &shared_limits() {
+    static auto *m = new std::map<const void *, int>;
+    return *m;
+}
+
 extern "C" {
 int fake_allocations, fake_fail_from = -1, fake_fail_count, fake_bad, fake_launches;
 static int last_error;   // of the calls that can fail here
-
 static int failed(int e) { return last_error = e; }
 
 static bool held(const void *p, size_t n) {
@@ -64,7 +70,9 @@ static int release(void *p) {
 }
 
 // the pointer arguments of the kernels, by name
-static int launch(const void *fn, void **args) {
+static int launch(const void *fn, void **args, size_t smem) {
+    auto limit = shared_limits().find(fn);
+    if (smem > 48 * 1024 && (limit == shared_limits().end() || smem > (size_t)limit->second)) return failed(1);
     fake_launches++;
     auto it = names().find(fn);
     const std::string name = it == names().end() ? "" : it->second;
@@ -108,9 +116,11 @@ int cudaMemcpyAsync(void *d, const void *s, size_t n, int kind, void *) {
     return 0;
 }
 int cudaMemcpy(void *d, const void *s, size_t n, int kind) { return cudaMemcpyAsync(d, s, n, kind, nullptr); }
-int cudaLaunchKernel(const void *fn, dim3, dim3, void **args, size_t, void *) { return launch(fn, args); }
-int cudaLaunchCooperativeKernel(const void *fn, dim3, dim3, void **args, size_t, void *) { return launch(fn, args); }
-int cudaLaunchKernelExC(const LaunchConfig *, const void *fn, void **args) { return launch(fn, args); }
+int cudaLaunchKernel(const void *fn, dim3, dim3, void **args, size_t smem, void *) { return launch(fn, args, smem); }
+int cudaLaunchCooperativeKernel(const void *fn, dim3, dim3, void **args, size_t smem, void *) {
+    return launch(fn, args, smem);
+}
+int cudaLaunchKernelExC(const LaunchConfig *c, const void *fn, void **args) { return launch(fn, args, c->smem); }
 
 int cudaGetDevice(int *d) { return *d = 0; }
 int cudaSetDevice(int) { return 0; }
@@ -130,8 +140,11 @@ int cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int *n, const void *,
     *n = 2;
     return 0;
 }
-int cudaFuncSetAttribute(const void *, int attr, int value) {
-    return attr == 8 && value > 227 * 1024 ? failed(1) : 0;   // dynamic shared memory of a block
+int cudaFuncSetAttribute(const void *fn, int attr, int value) {
+    if (attr != 8) return 0;   // dynamic shared memory of a block
+    if (value > 227 * 1024) return failed(1);
+    shared_limits()[fn] = value;
+    return 0;
 }
 int cudaGetLastError() {
     const int e = last_error;

@@ -84,3 +84,39 @@ def test_a_refused_call_leaves_no_error_for_the_next(fake):
     assert done.returncode == 0 and "cudaFuncSetAttribute" in refused
     # no plan comes from kernels that do nothing, but the runtime has no complaint
     assert "nodes" in after and "cuda" not in after
+
+
+MANY_CLASSES = """
+import ctypes, json, sys
+from gpuqo_b200 import capi, lib, query
+fake = ctypes.CDLL(sys.argv[1])
+launches = ctypes.c_int.in_dll(fake, "fake_launches")
+def call(n, classes, persistent, extra=()):   # 1,100 classes: a planner info of some 90 KB
+    L = lib.load()
+    L.gpuqo_b200_reset_persistent()   # no plan comes from the kernels here, which counts as a barrier that gave up
+    capi.set_int(L, "gpuqo_b200_persistent", persistent)
+    q = query.star(n, 1)
+    for a, b in extra:
+        q.edges[a], q.edges[b] = sorted(q.edges[a] + [b]), sorted(q.edges[b] + [a])
+    first = list(q.eq_classes)
+    for i in range(classes - len(first)):
+        q.eq_classes.append(query.EqClass(list(first[i % len(first)].members), [0.5], [[], []], [query.VarInfo()] * 2))
+    before = launches.value
+    lib.run(q, capi.GPUQO_DPSUB, bicc=True)
+    return launches.value - before
+"""
+
+
+def _many_classes(fake, calls):
+    env = dict(os.environ, LD_PRELOAD=fake, PYTHONPATH=os.path.join(REPO, "postgres-gpuqo_b200"))
+    done = subprocess.run([sys.executable, "-c", MANY_CLASSES + f"print(json.dumps({calls}))", fake], env=env,
+                          capture_output=True, text=True, timeout=120)
+    assert done.returncode == 0
+    return json.loads(done.stdout), done.stderr
+
+
+def test_a_smaller_planner_info_leaves_the_larger_one_its_shared_memory(fake):
+    """the level kernels that follow are in a captured graph by the third call: its one launch is the persistent
+    kernel's, with the shared memory that the second call's size would not allow"""
+    launched, _ = _many_classes(fake, "[call(12, 1100, 1), call(12, 850, 1), call(12, 1100, 1)]")
+    assert launched[2] == 1
