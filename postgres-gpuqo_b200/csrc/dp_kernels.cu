@@ -2445,6 +2445,8 @@ public:
             CK(cudaFuncSetAttribute(k_dpsize_eval, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
             CK(cudaFuncSetAttribute(k_eval<kModeDpsub>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
             CK(cudaFuncSetAttribute(k_eval<kModeMpdp>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            CK(cudaFuncSetAttribute(k_eval_mpdp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            CK(cudaFuncSetAttribute(k_eval_tree, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
             CK(cudaFuncSetAttribute(k_ovf_chunks<kModeDpsub>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
             CK(cudaFuncSetAttribute(k_ovf_chunks<kModeMpdp>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
             CK(cudaFuncSetAttribute(k_ovf_finalize<kModeDpsub>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));

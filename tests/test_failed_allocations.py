@@ -120,3 +120,9 @@ def test_a_smaller_planner_info_leaves_the_larger_one_its_shared_memory(fake):
     kernel's, with the shared memory that the second call's size would not allow"""
     launched, _ = _many_classes(fake, "[call(12, 1100, 1), call(12, 850, 1), call(12, 1100, 1)]")
     assert launched[2] == 1
+
+
+def test_level_kernels_are_allowed_the_planner_info(fake):
+    """a tree, and a graph with a cycle, by the launches per level"""
+    launched, said = _many_classes(fake, "[call(12, 1100, 0), call(12, 1100, 0, [(0, 1), (0, 2), (1, 2)])]")
+    assert min(launched) > 0 and "cuda" not in said
