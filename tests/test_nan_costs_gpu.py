@@ -52,4 +52,4 @@ def test_time_with_nan_costs():
     the first candidate."""
     ms = [lib.time_resident(q, capi.GPUQO_DPSUB, bicc=True, warmup=3, iters=20)[1]
           for q in (query.key_chain(31, 1, rich=True), query.chain(31, 1, rich=True))]
-    assert ms[1] < 1.45 * ms[0]
+    assert ms[1] < 1.5 * ms[0]
